@@ -94,6 +94,11 @@ def core() -> ctypes.CDLL:
                                              _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr,
                                              _c_float, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int,
                                              _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_ptr])
+        lib.tge_attention_f32_scratch_floats.argtypes = [_c_int] * 7
+        lib.tge_attention_f32_scratch_floats.restype = _c_ll
+        _declare(lib, "tge_attention_f32", [_c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr,
+                                            _c_int, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int,
+                                            _c_ptr, _c_ll, _c_ptr, _c_ptr])
         _declare(lib, "tge_attention_pooled_merge", [_c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr,
                                                      _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_int,
                                                      _c_int, _c_int, _c_int, _c_float, _c_int, _c_int, _c_ptr, _c_int, _c_ptr,
@@ -919,6 +924,19 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
                                                        status_word().data_ptr(), _stream()), core_lib)
         return out
     lib = core()
+    if (q.dtype == torch.float32 and not force_simt and value_dim == head_dim and not v_pitch and sink is None and not pool
+            and dist_bias is None and not keep_first and gate is None):
+        # plain causal or windowed float32 attention: keys in tiles that a block's rows share
+        need = lib.tge_attention_f32_scratch_floats(tokens, num_seqs, max_q_len, max_ctx_len, heads, kv_heads, head_dim)
+        if need >= 0:
+            scratch = scratch_floats(need) if need > 0 else None
+            rc = lib.tge_attention_f32(q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
+                                       max_pages, num_pages, page_size, q_start.data_ptr(), start_pos.data_ptr(),
+                                       positions.data_ptr(), num_seqs, max_q_len, max_ctx_len, out.data_ptr(), out_stride,
+                                       tokens, heads, kv_heads, head_dim, float(scale), window, _ptr(scratch), need,
+                                       status_word().data_ptr(), _stream())
+            if _check(rc, lib) != UNSUPPORTED:
+                return out
     _check(lib.tge_attention_simt(q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(),
                                   block_table.data_ptr(), max_pages, num_pages, page_size, positions.data_ptr(),
                                   seq_of_token.data_ptr(), out.data_ptr(), out_stride, tokens, heads, kv_heads,

@@ -394,6 +394,36 @@ def test_attention_simt(ops, dtype, heads, kv_heads, head_dim):
     assert err < TOL[dtype]
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim,page_size,window", [
+    (7, 1, 128, 16, 0), (12, 2, 64, 64, 0), (3, 1, 32, 16, 100), (4, 2, 16, 5, 0), (34, 2, 128, 16, 300), (4, 4, 128, 64, 1)])
+def test_attention_float32_rows_do_not_depend_on_the_step(ops, heads, kv_heads, head_dim, page_size, window):
+    """The tiled float32 kernel: lengths at the edges of its tiles (64 keys) and runs (256), and one request whole, in
+    portions and token by token (16 and 64 rows to a block, runs inside a block and merged) to the same bits."""
+    case = lambda q_lens, starts, **kw: _attention_case(ops, torch.float32, heads, kv_heads, head_dim, q_lens, starts,
+                                                        page_size=page_size, window=window, **kw)
+    err, out, ref = case([1, 1, 9, 65, 1, 257], [0, 63, 64, 190, 256, 511])
+    simt, _, _ = case([1, 1, 9, 65, 1, 257], [0, 63, 64, 190, 256, 511], force_simt=True)
+    # 64 keys are summed before they join the rest and a score in four parts, so no more error than key by key;
+    # a quarter more for rounding's luck
+    assert err < TOL[torch.float32] and err <= 1.25 * simt + 1e-8
+    if page_size != 16:
+        return
+    # the same keys and queries in other cuts
+    lengths = 600
+    k_pages, v_pages, table, _k, _v = paged_cache([lengths], kv_heads, head_dim, page_size, torch.float32, DEV, seed=3)
+    q = torch.randn(lengths, heads * head_dim, generator=torch.Generator().manual_seed(4)).to(DEV)
+
+    def rows(start, count, bound=lengths):
+        positions, seq_of_token, q_start, start_pos = batch_index([count], [start], DEV)
+        return ops.attention(q[start:start + count], k_pages, v_pages, table, q_start, start_pos, positions, seq_of_token, 1,
+                             count, bound, heads, kv_heads, head_dim, head_dim ** -0.5, window=window)
+    whole = rows(0, lengths)
+    for start, count in ((0, 1), (63, 1), (64, 2), (255, 3), (256, 1), (300, 30), (599, 1), (410, 190)):
+        assert torch.equal(rows(start, count), whole[start:start + count]), (start, count)
+    assert torch.equal(rows(520, 1, bound=4096), whole[520:521])
+    ops.check_status()
+
+
 def test_leading_single_tokens_deep_in_long_contexts_get_splits_of_their_own(ops):
     """A mixed step: nine single tokens at contexts of about 4,000 beside a prompt of 300 tokens.  The prompt's
     keys are not cut; the single tokens, a decode batch of their own, have theirs cut (the choice is automatic
