@@ -94,6 +94,10 @@ def core() -> ctypes.CDLL:
                                              _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr,
                                              _c_float, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int,
                                              _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_ptr])
+        lib.tge_gemm_f32_tcgen05_scratch_floats.argtypes = [_c_ptr, _c_ll, _c_int, _c_int, _c_int]
+        lib.tge_gemm_f32_tcgen05_scratch_floats.restype = _c_ll
+        _declare(lib, "tge_gemm_f32_tcgen05", [_c_ptr, _c_ll, _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ll, _c_int, _c_int, _c_int, _c_int,
+                                               _c_ptr, _c_ll, _c_float, _c_int, _c_ptr, _c_ptr])
         lib.tge_attention_f32_scratch_floats.argtypes = [_c_int] * 7
         lib.tge_attention_f32_scratch_floats.restype = _c_ll
         _declare(lib, "tge_attention_f32", [_c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr,
@@ -606,8 +610,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], epilo
     GEMM_GELU / GEMM_GELU_TANH: out [M, N] run dtype = gelu(product + bias) in the erf / the tanh form for the
     columns from ``act_from`` on, the plain product below (for row-concatenated weights).
     ``alpha`` multiplies product + bias in the store and add epilogues (a residual multiplier, a logit scale).
-    bfloat16 goes to the tcgen05 kernel when the shape allows TMA, else (and all of
-    float32) to the CUDA-core kernel.
+    Both types go to their tcgen05 kernel when the shape allows TMA (float32, split into three bfloat16 numbers, from
+    512 x 512 weights on), else to the CUDA-core kernel.
     """
     deferred = x if isinstance(x, DeferredRows) else None
     if deferred is not None:
@@ -654,6 +658,15 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], epilo
     if deferred is not None:
         x = deferred.complete()
         ldx = _rows_2d(x, "linear input")
+    if x.dtype == torch.float32 and USE_TCGEN05 and not force_simt:
+        need = lib.tge_gemm_f32_tcgen05_scratch_floats(w.data_ptr(), ldw, M, N, K)
+        if need >= 0:
+            scratch = scratch_floats(need)
+            rc = lib.tge_gemm_f32_tcgen05(x.data_ptr(), ldx, w.data_ptr(), ldw, _ptr(bias), out.data_ptr(), ldo, M, N, K, epilogue,
+                                          scratch.data_ptr(), scratch.numel(), float(alpha), int(act_from),
+                                          status_word().data_ptr(), _stream())
+            if _check(rc, lib) != UNSUPPORTED:
+                return out
     _check(lib.tge_gemm_simt(x.data_ptr(), ldx, w.data_ptr(), ldw, _ptr(bias), out.data_ptr(), ldo, M, N, K,
                              int(x.dtype == torch.bfloat16), epilogue, float(alpha), int(act_from), _stream()), lib)
     return out

@@ -112,6 +112,52 @@ def test_gemm_simt_value_does_not_depend_on_the_batch(ops):
         assert torch.equal(alone[0], whole[row])
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 512, 512), (8, 1000, 516), (16, 512, 3584), (17, 4608, 1536), (33, 640, 700), (65, 520, 640),
+                                   (129, 3584, 512), (300, 514, 4100), (513, 2048, 516)])
+def test_gemm_float32_on_the_tensor_cores(ops, M, N, K):
+    """Every token tile and ragged edge, products cut along k and whole, panels of tokens; epilogues; a row alone to the same
+    bits; an error against float64 no larger than that of one FMA chain along k."""
+    gen = torch.Generator().manual_seed(M + N + K)
+    x, w, b = (torch.randn(M, K, generator=gen).to(DEV), (torch.randn(N, K, generator=gen) * 0.1).to(DEV),
+               torch.randn(N, generator=gen).to(DEV))
+    assert ops.core().tge_gemm_f32_tcgen05_scratch_floats(w.data_ptr(), K, M, N, K) > 0
+    ref = x.double() @ w.double().T
+    out = ops.linear(x, w, None, ops.GEMM_STORE_F32)
+    chain = ops.linear(x, w, None, ops.GEMM_STORE_F32, force_simt=True)
+    rms = lambda t: float((t.double() - ref).norm() / ref.norm())
+    assert rms(out) <= rms(chain)
+    for row in (0, M // 2, M - 1):
+        assert torch.equal(ops.linear(x[row:row + 1], w, None, ops.GEMM_STORE_F32)[0], out[row])
+    # bounds: a sum's error here is below 4e-7 of its root mean square, the largest of a million five times that
+    stream = torch.randn(M, N, generator=gen).to(DEV)
+    added = stream.clone()
+    ops.linear(x, w, b, ops.GEMM_ADD_F32, out=added, alpha=0.5)
+    assert rel_error(added, stream.double() + 0.5 * (ref + b.double())) < 2e-6
+    wide = torch.zeros(M, N + 3, device=DEV)
+    ops.linear(x, w, b, ops.GEMM_GELU, out=wide[:, :N], act_from=100)
+    full = ref + b.double()
+    act = torch.cat([full[:, :100], torch.nn.functional.gelu(full[:, 100:])], dim=1)
+    assert rel_error(wide[:, :N], act) < 2e-6 and float(wide[:, N:].abs().max()) == 0
+    g, u = full[:, 0::2], full[:, 1::2]
+    assert rel_error(ops.linear(x, w, b, ops.GEMM_SWIGLU), torch.nn.functional.silu(g) * u) < 5e-6    # two sums' errors
+    ops.check_status()
+
+
+def test_gemm_float32_on_the_tensor_cores_keeps_what_is_not_finite(ops):
+    gen = torch.Generator().manual_seed(1)
+    x, w = torch.randn(20, 600, generator=gen).to(DEV), torch.randn(700, 600, generator=gen).to(DEV)
+    x[3, 5], x[4, 599], w[8, 6], w[9, 0] = math.inf, -math.inf, math.nan, 3.4e38
+    x[5] = 2e38                                    # parts and sums beyond the range
+    for epilogue in (ops.GEMM_STORE_F32, ops.GEMM_SWIGLU):
+        out, chain = (ops.linear(x, w, None, epilogue, force_simt=simt) for simt in (False, True))
+        odd = ~torch.isfinite(chain)
+        assert odd.any() and torch.equal(torch.isfinite(out), ~odd)
+        assert torch.equal(torch.nan_to_num(out[odd], nan=7.0), torch.nan_to_num(chain[odd], nan=7.0))
+    # tiny numbers keep what a sum of three parts holds of them
+    out = ops.linear(x[6:9] * 1e-30, w[10:], None, ops.GEMM_STORE_F32)
+    assert rel_error(out * 1e30, x[6:9].double() @ w[10:].double().T) < 1e-6
+
+
 TC_SHAPES = [(1, 128, 64), (8, 384, 176), (16, 200, 256), (33, 130, 72), (64, 512, 1024), (100, 300, 512),
              (200, 640, 320), (300, 1024, 512), (520, 256, 192)]
 
