@@ -145,6 +145,118 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const T* __restrict__ x,
   }
 }
 
+// Few tokens, float32, aligned rows: the same chain of FMAs per element, organised for latency.
+//
+// The tile above waits for its loads in each of K / 16 rounds and has 64 x 64 elements whatever M is: a tiny model's product
+// of 3 rows took 8.4 us at K = 64 and 20 us at K = 384, nearly all of it round trips to L2.  Here a block owns 16 x 32 elements
+// (a lane per weight row, a warp per four tokens), so a product spreads over four times the SMs and more, and
+// four blocks of 64 k are on their way at once by cp.async, the weights' (nobody's result) before the wait for
+// the kernel in front.  Measured (B200), the tile above and this kernel, us, at 4 tokens:
+// 128 x 64 6.3 -> 2.3, 512 x 96 8.5 -> 2.8, 64 x 176 12.9 -> 3.8, 96 x 256 17.8 -> 4.9, 500 x 3,000 181 -> 47; 300 tokens
+// of 384 x 96 8.5 -> 4.3 and of 500 x 3,000 180 -> 101.
+constexpr int SKINNY_M = 16, SKINNY_N = 32, SKINNY_K = 64, SKINNY_PITCH = SKINNY_K + 4, SKINNY_STAGES = 4;
+constexpr int SKINNY_STAGE = (SKINNY_M + SKINNY_N) * SKINNY_PITCH;
+
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool live) {
+  const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+  const int bytes = live ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to), "l"(src), "r"(bytes) : "memory");
+}
+
+__global__ void __launch_bounds__(128) gemm_skinny_kernel(const float* __restrict__ x, size_t ldx, const float* __restrict__ w, size_t ldw,
+                                                          const float* __restrict__ bias, float* __restrict__ out, size_t ldo, int M,
+                                                          int N, int K, int epilogue, float alpha, int act_from) {
+  extern __shared__ __align__(16) float ring[];
+  pdl_trigger();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m0 = blockIdx.y * SKINNY_M, n0 = blockIdx.x * SKINNY_N;
+  const int blocks = (K + SKINNY_K - 1) / SKINNY_K;
+  auto fetch_w = [&](int kb) {
+    float* stage = ring + (kb % SKINNY_STAGES) * SKINNY_STAGE + SKINNY_M * SKINNY_PITCH;
+#pragma unroll
+    for (int i = 0; i < SKINNY_N * SKINNY_K / 4 / 128; ++i) {
+      const int c = tid + i * 128, row = c >> 4, k = kb * SKINNY_K + (c & 15) * 4;
+      const bool live = n0 + row < N && k < K;
+      copy16(stage + row * SKINNY_PITCH + (c & 15) * 4, live ? w + (size_t)(n0 + row) * ldw + k : w, live);
+    }
+  };
+  auto fetch_x = [&](int kb) {
+    float* stage = ring + (kb % SKINNY_STAGES) * SKINNY_STAGE;
+#pragma unroll
+    for (int i = 0; i < SKINNY_M * SKINNY_K / 4 / 128; ++i) {
+      const int c = tid + i * 128, row = c >> 4, k = kb * SKINNY_K + (c & 15) * 4;
+      const bool live = m0 + row < M && k < K;
+      copy16(stage + row * SKINNY_PITCH + (c & 15) * 4, live ? x + (size_t)(m0 + row) * ldx + k : x, live);
+    }
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
+  const int n = n0 + lane;
+  const float add = bias != nullptr && n < N ? bias[n] : 0.0f;
+#pragma unroll
+  for (int kb = 0; kb < SKINNY_STAGES - 1; ++kb)
+    if (kb < blocks) fetch_w(kb);
+  pdl_wait();
+#pragma unroll
+  for (int kb = 0; kb < SKINNY_STAGES - 1; ++kb) {      // the weights above land with the first group
+    if (kb < blocks) fetch_x(kb);
+    commit();
+  }
+  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  for (int kb = 0; kb < blocks; ++kb) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(SKINNY_STAGES - 2) : "memory");
+    __syncthreads();                                    // everyone's part of block kb is there, and block kb - 1 is read
+    if (kb + SKINNY_STAGES - 1 < blocks) {
+      fetch_w(kb + SKINNY_STAGES - 1);
+      fetch_x(kb + SKINNY_STAGES - 1);
+    }
+    commit();
+    if (m0 + warp * 4 >= M) continue;                   // uniform over the warp
+    const float* xs = ring + (kb % SKINNY_STAGES) * SKINNY_STAGE + warp * 4 * SKINNY_PITCH;
+    const float* ws = ring + (kb % SKINNY_STAGES) * SKINNY_STAGE + (SKINNY_M + lane) * SKINNY_PITCH;
+    const int held = min(K - kb * SKINNY_K, SKINNY_K);  // a multiple of four
+#pragma unroll 4
+    for (int k = 0; k < held; k += 4) {
+      const float4 b = *reinterpret_cast<const float4*>(ws + k);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 a = *reinterpret_cast<const float4*>(xs + i * SKINNY_PITCH + k);
+        acc[i] = fmaf(a.x, b.x, acc[i]);
+        acc[i] = fmaf(a.y, b.y, acc[i]);
+        acc[i] = fmaf(a.z, b.z, acc[i]);
+        acc[i] = fmaf(a.w, b.w, acc[i]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int m = m0 + warp * 4 + i;
+    if (m >= M) break;
+    float v = acc[i];
+    if (bias) v += add;
+    if (epilogue == GEMM_SWIGLU || epilogue == GEMM_GLU_CLAMPED) {
+      float u = __shfl_down_sync(0xffffffffu, v, 1);    // an even lane's neighbour holds the row above
+      if (epilogue == GEMM_GLU_CLAMPED) {
+        v = fminf(v, alpha);
+        u = fminf(fmaxf(u, -alpha), alpha) + 1.0f;
+        v *= 1.702f;
+        u *= 1.0f / 1.702f;
+      }
+      if (!(lane & 1) && n + 1 < N) out[(size_t)m * ldo + (n >> 1)] = v / (1.0f + expf(-v)) * u;
+      continue;
+    }
+    if (n >= N) continue;
+    float* dst = out + (size_t)m * ldo + n;
+    if (epilogue >= GEMM_GELU) {
+      if (n >= act_from) v = epilogue == GEMM_GELU ? gelu_erf(v) : gelu_tanh(v);
+      *dst = v;
+    } else if (epilogue == GEMM_ADD_F32) {
+      *dst += v * alpha;
+    } else {
+      *dst = v * alpha;
+    }
+  }
+}
+
 }  // namespace
 
 // x [M, K] (row stride ldx), w [N, K] (row stride ldw), both in the run dtype;
@@ -161,6 +273,24 @@ TGE_API int tge_gemm_simt(const void* x, long long ldx, const void* w, long long
   const size_t align = is_bf16 ? 8 : 16;
   const int vec = (K % 4 == 0) && ((ldx * elem) % align == 0) && ((ldw * elem) % align == 0) &&
                   ((uintptr_t)x % align == 0) && ((uintptr_t)w % align == 0);
+  // Float32 rows that 16-byte copies can read: up to 64 tokens always, more while the small tiles of all of them fit the
+  // chip at once (then latency counts, not the number of shared-memory reads per FMA: 1,000 tokens of 512 x 96, beyond
+  // the line, take 8.5 us either way).
+  const long long small_tiles = (long long)((N + SKINNY_N - 1) / SKINNY_N) * ((M + SKINNY_M - 1) / SKINNY_M);
+  if (!is_bf16 && vec && (M <= 64 || small_tiles <= 4 * tge_sm_count())) {
+    constexpr int smem = SKINNY_STAGES * SKINNY_STAGE * (int)sizeof(float);
+    cudaError_t err = cudaFuncSetAttribute(gemm_skinny_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (err == cudaSuccess)
+      err = tge_launch(gemm_skinny_kernel, dim3((N + SKINNY_N - 1) / SKINNY_N, (M + SKINNY_M - 1) / SKINNY_M), dim3(128), smem, stream,
+                       (const float*)x, (size_t)ldx, (const float*)w, (size_t)ldw, bias, (float*)out, (size_t)ldo, M, N, K, epilogue,
+                       alpha, act_from);
+    if (err != cudaSuccess) {
+      tge_set_error("gemm_simt: launch failed: %s", cudaGetErrorString(err));
+      cudaGetLastError();
+      return -2;
+    }
+    return tge_launched("gemm_simt", 1);
+  }
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (is_bf16)
     gemm_simt_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, (size_t)ldx,

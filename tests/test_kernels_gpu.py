@@ -112,6 +112,23 @@ def test_gemm_simt_value_does_not_depend_on_the_batch(ops):
         assert torch.equal(alone[0], whole[row])
 
 
+@pytest.mark.parametrize("N,K", [(33, 4), (31, 64), (130, 68), (96, 256), (64, 700)])
+def test_gemm_float32_few_tokens_have_the_bits_of_many(ops, N, K):
+    """The kernel for few float32 tokens against the one for many, whose small tiles no longer fit the chip: the same
+    chain of FMAs per element, at the edges of its 16 x 32 tiles and k-blocks of 64, in every epilogue."""
+    gen = torch.Generator().manual_seed(N + K)
+    many = 600 * 16 + 1
+    x, w, b = torch.randn(many, K, generator=gen).to(DEV), torch.randn(N, K, generator=gen).to(DEV), torch.randn(N, generator=gen).to(DEV)
+    for epilogue in (ops.GEMM_STORE, ops.GEMM_STORE_F32, ops.GEMM_ADD_F32, ops.GEMM_GELU, ops.GEMM_GELU_TANH) + (
+            (ops.GEMM_SWIGLU, ops.GEMM_GLU_CLAMPED) if N % 2 == 0 else ()):
+        def run(rows):
+            out = torch.ones(rows.shape[0], N, device=DEV) if epilogue == ops.GEMM_ADD_F32 else None
+            return ops.linear(rows, w, b, epilogue, out=out, force_simt=True, alpha=0.75, act_from=7)
+        whole = run(x)
+        for first, count in ((0, 1), (17, 16), (100, 19), (many - 64, 64)):
+            assert torch.equal(run(x[first:first + count]), whole[first:first + count]), (epilogue, first, count)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 512, 512), (8, 1000, 516), (16, 512, 3584), (17, 4608, 1536), (33, 640, 700), (65, 520, 640),
                                    (129, 3584, 512), (300, 514, 4100), (513, 2048, 516)])
 def test_gemm_float32_on_the_tensor_cores(ops, M, N, K):
