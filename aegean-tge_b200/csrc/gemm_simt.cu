@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(128) gemm_skinny_kernel(const float* __restric
       if (n >= act_from) v = epilogue == GEMM_GELU ? gelu_erf(v) : gelu_tanh(v);
       *dst = v;
     } else if (epilogue == GEMM_ADD_F32) {
-      *dst += v * alpha;
+      *dst = __fadd_rn(*dst, __fmul_rn(v, alpha));      // rounded twice, as above
     } else {
       *dst = v * alpha;
     }
