@@ -21,6 +21,12 @@
 
 #include "common.cuh"
 
+// decay_scan_tc.cu
+int decay_tc_chunk(int dim, int vdim);
+int launch_decay_tc(const void* rows, long long ld, const float* prepared, int v_off, int heads, int dim, int vdim, int activation,
+                    const float* decay, const int* q_start, float* carry, float* out, int num_seqs, int pieces, bool readout, int* status,
+                    cudaStream_t stream);
+
 namespace {
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
@@ -910,6 +916,17 @@ __global__ void __launch_bounds__(128) pool_kv_kernel(
   }
 }
 
+// Tokens per segment where a step's portions are shared out over blocks of their own (0: they are not): chunks of 128
+// on the tensor cores for bfloat16 and the sizes decay_scan_tc.cu is built for from one whole chunk on; else segments of 256
+// on the FMA pipes from two on.
+int segment_tokens(bool is_bf16, int dim, int vdim, int max_q_len) {
+  static const bool chunks_ok = getenv("TGE_NO_CHUNKED_SCAN") == nullptr || getenv("TGE_NO_CHUNKED_SCAN")[0] == '\0';
+  if (!chunks_ok) return 0;
+  const int chunk = is_bf16 ? decay_tc_chunk(dim, vdim) : 0;
+  if (chunk > 0 && max_q_len >= chunk) return chunk;
+  return max_q_len >= 2 * SEGMENT && dim <= 128 && dim % 4 == 0 ? SEGMENT : 0;
+}
+
 template <typename T>
 int launch_decay_scan(const void* rows, long long ld, int q_off, int k_off, int v_off, int heads, int dim, int vdim,
                       int activation, const float* cos_table, const float* sin_table, int table_positions, int rotary,
@@ -940,9 +957,22 @@ int launch_decay_scan(const void* rows, long long ld, int q_off, int k_off, int 
     decay_prepare_kernel<T><<<dim3(tokens, heads), 128, 0, stream>>>((const T*)rows, ld, q_off, k_off, heads, dim, activation,
                                                                      cos_table, sin_table, table_positions, rotary, k_scale,
                                                                      positions, prepared, status);
+    const int segment = carry != nullptr ? segment_tokens(sizeof(T) == 2, dim, vdim, max_q_len) : 0;
+    if (segment > 0 && segment != SEGMENT && tokens / segment + num_seqs <= 65535) {
+      const int pieces = tokens / segment + num_seqs;
+      int rc = launch_decay_tc(rows, ld, prepared, v_off, heads, dim, vdim, activation, decay, q_start, carry, out, num_seqs, pieces, false,
+                               status, stream);
+      if (rc < 0) return rc;
+      decay_segment_carry_kernel<<<dim3((dim * vdim + 255) / 256, heads, num_seqs), 256, 0, stream>>>(
+          carry, state, decay, slots, q_start, heads, dim, vdim, segment);
+      rc = launch_decay_tc(rows, ld, prepared, v_off, heads, dim, vdim, activation, decay, q_start, carry, out, num_seqs, pieces, true,
+                           status, stream);
+      if (rc < 0) return rc;
+      return tge_launched("decay_scan_tc", 4);
+    }
     // few blocks and long portions: segments, so that the whole device works on one prompt
     const long long blocks = (long long)wide_grid.x * heads * num_seqs;
-    if (carry != nullptr && max_q_len >= 2 * SEGMENT && blocks < 2LL * tge_sm_count() && tokens / SEGMENT + num_seqs <= 65535) {
+    if (segment == SEGMENT && blocks < 2LL * tge_sm_count() && tokens / SEGMENT + num_seqs <= 65535) {
       dim3 pieces(wide_grid.x, heads, tokens / SEGMENT + num_seqs);      // an upper bound; blocks beyond the last segment leave at once
       decay_scan_wide_kernel<T, 1><<<pieces, 256, wide, stream>>>((const T*)rows, ld, prepared, v_off, heads, dim, vdim, activation,
                                                                   decay, state, slots, q_start, out, carry, num_seqs, SEGMENT);
@@ -1031,6 +1061,10 @@ TGE_API int tge_scale_add_norm(float* x, const float* y, long long ldy, const fl
     scale_add_norm_kernel<float><<<rows, 256, 0, stream>>>(x, y, ldy, weight, (float*)copy, hidden, alpha, eps);
   return tge_launched("scale_add_norm", 1);
 }
+
+// Tokens of a segment in steps whose longest portion is max_q_len, 0: no segments.  With them `carry` holds a state for each of
+// tokens / segment + num_seqs.
+TGE_API int tge_decay_scan_segment(int is_bf16, int dim, int vdim, int max_q_len) { return segment_tokens(is_bf16 != 0, dim, vdim, max_q_len); }
 
 TGE_API int tge_decay_scan(const void* rows, int is_bf16, long long ld, int q_off, int k_off, int v_off, int heads,
                            int dim, int vdim, int activation, const float* cos_table, const float* sin_table,

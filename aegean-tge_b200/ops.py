@@ -155,6 +155,7 @@ def core() -> ctypes.CDLL:
         _declare(lib, "tge_to_run_dtype", [_c_ptr, _c_ptr, _c_int, _c_ll, _c_ptr])
         _declare(lib, "tge_scale_add_norm", [_c_ptr, _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_float,
                                              _c_float, _c_ptr])
+        _declare(lib, "tge_decay_scan_segment", [_c_int] * 4)
         _declare(lib, "tge_decay_scan", [_c_ptr, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                          _c_ptr, _c_ptr, _c_int, _c_int, _c_float, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr,
                                          _c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_ptr])
@@ -1027,10 +1028,11 @@ def decay_scan(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, heads: in
     # the chunked kernels read q and k as the recurrence takes them from a buffer that one kernel fills per step
     prepared = (torch.empty((tokens, heads, 2, dim), dtype=torch.float32, device=rows.device)
                 if longest >= 16 and dim <= 256 else None)
-    # one long portion is shared out over many blocks in segments of 256 tokens: a state per segment in between
-    carry = (torch.empty((tokens // 256 + num_seqs, heads, dim, vdim), dtype=torch.float32, device=rows.device)
-             if prepared is not None and longest >= 512 and dim <= 128 and dim % 4 == 0 else None)
     lib = core()
+    # long portions are shared out over many blocks in segments of 128 or 256 tokens: a state per segment in between
+    segment = lib.tge_decay_scan_segment(int(rows.dtype == torch.bfloat16), dim, vdim, longest) if prepared is not None else 0
+    carry = (torch.empty((tokens // segment + num_seqs, heads, dim, vdim), dtype=torch.float32, device=rows.device)
+             if segment > 0 else None)
     _check(lib.tge_decay_scan(rows.data_ptr(), int(rows.dtype == torch.bfloat16), ld, q_off, k_off, v_off, heads, dim,
                               vdim, int(activation), _ptr(cos) if rotary else None, _ptr(sin) if rotary else None,
                               table_positions, rotary, float(k_scale), decay.data_ptr(), state.data_ptr(),
