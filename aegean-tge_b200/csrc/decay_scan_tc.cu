@@ -120,6 +120,12 @@ __device__ __forceinline__ float value_at(const ScanTcParams& p, int token, int 
   return p.activation ? silu_of(v) : v;
 }
 
+// 32 bytes, one sector, in one store: lanes write rows of their own, and 16-byte stores would fill each sector in two
+__device__ __forceinline__ void store8(float* dst, const float v[8]) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]),
+               "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+
 // 32 numbers of this thread's lane as columns [col, col + 16) of each part of a first operand (parts `part_cols` columns apart).
 __device__ __forceinline__ void store_lane32(uint32_t taddr, int part_cols, const float v[32]) {
   uint32_t h[16], m[16], l[16];
@@ -199,6 +205,8 @@ __device__ __forceinline__ BlockSetup set_up(unsigned char* smem_raw, uint32_t* 
   __syncthreads();
   tc_fence_after();
   s.tmem = *tmem_slot;
+  pdl_trigger();                           // tensor memory is held: a block of the next kernel can at worst wait for it
+  pdl_wait();
   return s;
 }
 __device__ __forceinline__ void tear_down(uint32_t tmem, int warp) {
@@ -276,7 +284,7 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_state_kernel(const Sca
     }
   } else if (ok && row < DIM) {
 #pragma unroll
-    for (int c = 0; c < VDIM / 2; c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(sums[c], sums[c + 1], sums[c + 2], sums[c + 3]);
+    for (int c = 0; c < VDIM / 2; c += 8) store8(dst + c, sums + c);
   }
   tear_down(s.tmem, warp);
 }
@@ -414,9 +422,9 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
     read_sums<16, 2>(s.tmem + lane_base + half * (VDIM / 2) + c, 128, more);
     if (ok && row < count && !by_formula) {
 #pragma unroll
-      for (int j = 0; j < 16; j += 4)
-        *reinterpret_cast<float4*>(dst + c + j) =
-            make_float4(o[c + j] + more[j], o[c + j + 1] + more[j + 1], o[c + j + 2] + more[j + 2], o[c + j + 3] + more[j + 3]);
+      for (int j = 0; j < 16; ++j) more[j] += o[c + j];
+      store8(dst + c, more);
+      store8(dst + c + 8, more + 8);
     }
   }
   tear_down(s.tmem, warp);
@@ -429,11 +437,11 @@ int run(const ScanTcParams& p, int pieces, bool readout, cudaStream_t stream) {
   auto kernel = readout ? decay_chunk_readout_kernel<DIM, VDIM> : decay_chunk_state_kernel<DIM, VDIM>;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 + 6 * OPERAND_BYTES);
   if (err == cudaSuccess) {
-    kernel<<<dim3(p.heads, pieces), THREADS, smem, stream>>>(p);
-    err = cudaGetLastError();
+    err = tge_launch(kernel, dim3(p.heads, pieces), dim3(THREADS), smem, stream, p);
   }
   if (err != cudaSuccess) {
     tge_set_error("decay_scan_tc: launch failed: %s", cudaGetErrorString(err));
+    cudaGetLastError();
     return -2;
   }
   return 1;

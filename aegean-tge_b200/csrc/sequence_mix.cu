@@ -264,6 +264,64 @@ __global__ void __launch_bounds__(128) decay_prepare_kernel(
   }
 }
 
+// The same two numbers at a time, a warp per head and eight heads to a block (bfloat16; offsets, strides, the key size and half the
+// rotated numbers even).  Bound by its bytes: a block of 128 threads per (token, head) with two-byte loads took 40 us
+// for 2,048 tokens of 28 heads of 128, this 33.
+__global__ void __launch_bounds__(256) decay_prepare_vec_kernel(
+    const __nv_bfloat16* __restrict__ rows, long long ld, int q_off, int k_off, int heads, int dim, int activation,
+    const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary,
+    float k_scale, const int* __restrict__ positions, float* __restrict__ prepared, int* status) {
+  pdl_trigger();
+  const int t = blockIdx.x, head = blockIdx.y * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int half = rotary >> 1;
+  int position = positions[t];
+  if (rotary > 0 && (position < 0 || position >= table_positions)) {
+    if (lane == 0 && head == 0) atomicOr(status, TGE_STATUS_BAD_ROW);
+    position = 0;
+  }
+  pdl_wait();
+  if (head >= heads) return;
+  const __nv_bfloat16* q_row = rows + (size_t)t * ld + q_off + head * dim;
+  const __nv_bfloat16* k_row = rows + (size_t)t * ld + k_off + head * dim;
+  float* dst = prepared + ((size_t)t * heads + head) * 2 * dim;
+  auto two = [&](const __nv_bfloat16* at) {
+    const uint32_t raw = *reinterpret_cast<const uint32_t*>(at);
+    float2 v = make_float2(__uint_as_float(raw << 16), __uint_as_float(raw & 0xffff0000u));
+    if (activation) v = make_float2(silu_f(v.x), silu_f(v.y));
+    return v;
+  };
+#pragma unroll 2
+  for (int i = 2 * lane; i < dim; i += 64) {
+    float2 q = two(q_row + i), k = two(k_row + i);
+    if (i < rotary) {
+      const bool low = i < half;
+      const int other = low ? i + half : i - half, angle = low ? i : i - half;
+      const float2 q2 = two(q_row + other), k2 = two(k_row + other);
+      const float2 cs = *reinterpret_cast<const float2*>(cos_table + (size_t)position * half + angle);
+      const float2 sn = *reinterpret_cast<const float2*>(sin_table + (size_t)position * half + angle);
+      // the pair (u, v) = (element i, element i + half) becomes (u cos - v sin, v cos + u sin)
+      q = low ? make_float2(q.x * cs.x - q2.x * sn.x, q.y * cs.y - q2.y * sn.y) : make_float2(q.x * cs.x + q2.x * sn.x, q.y * cs.y + q2.y * sn.y);
+      k = low ? make_float2(k.x * cs.x - k2.x * sn.x, k.y * cs.y - k2.y * sn.y) : make_float2(k.x * cs.x + k2.x * sn.x, k.y * cs.y + k2.y * sn.y);
+    }
+    *reinterpret_cast<float2*>(dst + i) = q;
+    *reinterpret_cast<float2*>(dst + dim + i) = make_float2(k.x * k_scale, k.y * k_scale);
+  }
+}
+
+template <typename T>
+void launch_decay_prepare(const T* rows, long long ld, int q_off, int k_off, int heads, int dim, int activation, const float* cos_table,
+                          const float* sin_table, int table_positions, int rotary, float k_scale, const int* positions, float* prepared,
+                          int tokens, int* status, cudaStream_t stream) {
+  const bool pairs = sizeof(T) == 2 && ld % 2 == 0 && q_off % 2 == 0 && k_off % 2 == 0 && dim % 2 == 0 && rotary % 4 == 0 &&
+                     (uintptr_t)rows % 4 == 0 && (uintptr_t)cos_table % 8 == 0 && (uintptr_t)sin_table % 8 == 0 && (uintptr_t)prepared % 8 == 0;
+  if (pairs)
+    tge_launch(decay_prepare_vec_kernel, dim3(tokens, (heads + 7) / 8), dim3(256), 0, stream, (const __nv_bfloat16*)rows, ld, q_off, k_off, heads,
+               dim, activation, cos_table, sin_table, table_positions, rotary, k_scale, positions, prepared, status);
+  else
+    decay_prepare_kernel<T><<<dim3(tokens, heads), 128, 0, stream>>>(rows, ld, q_off, k_off, heads, dim, activation, cos_table, sin_table,
+                                                                     table_positions, rotary, k_scale, positions, prepared, status);
+}
+
 // The same recurrence for portions of many tokens, CHUNK tokens at a time.  With S the state before a chunk of n
 // tokens, c the head's decay and t, j places in the chunk:
 //   o_t   = c^(t+1) S^T q_t + sum_(j <= t) c^(t-j) (q_t . k_j) v_j
@@ -654,16 +712,20 @@ __global__ void decay_segment_carry_kernel(float* __restrict__ carry, float* __r
   const int seq = blockIdx.z, head = blockIdx.y;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int cells = dim * vdim;
-  if (e >= cells) return;
+  __shared__ float power_of[2];            // c^segment and c^(length of the last segment): float64, so by two threads of a block only
+  pdl_trigger();
   int before = 0;
   for (int s = 0; s < seq; ++s) before += (q_start[s + 1] - q_start[s] + segment - 1) / segment;
   const int count = q_start[seq + 1] - q_start[seq];
   if (count <= 0) return;
   const int pieces = (count + segment - 1) / segment;
-  const double c = (double)decay[head];
+  if (threadIdx.x < 2)
+    power_of[threadIdx.x] = (float)pow((double)decay[head], (double)(threadIdx.x == 0 ? segment : count - (pieces - 1) * segment));
+  __syncthreads();
+  pdl_wait();
+  if (e >= cells) return;
   float* slot = state + ((size_t)slots[seq] * heads + head) * cells + e;
   float running = *slot;
-  const float whole = (float)pow(c, (double)segment);                 // every segment but a request's last is whole
   for (int k0 = 0; k0 < pieces; k0 += 16) {
     // sixteen segments' contributions are asked for at once; the stores that follow would otherwise keep each
     // load behind the one before
@@ -675,8 +737,7 @@ __global__ void decay_segment_carry_kernel(float* __restrict__ carry, float* __r
     for (int k = 0; k < 16; ++k) {
       if (k0 + k < pieces) {
         carry[((size_t)(before + k0 + k) * heads + head) * cells + e] = running;
-        const int length = min(segment, count - (k0 + k) * segment);
-        running = fmaf(length == segment ? whole : (float)pow(c, (double)length), running, own[k]);
+        running = fmaf(power_of[k0 + k + 1 < pieces ? 0 : 1], running, own[k]);
       }
     }
   }
@@ -720,6 +781,57 @@ __global__ void __launch_bounds__(128) gated_norm_kernel(const float* __restrict
     const float z = to_float<T>(gt[e]);
     const float w = weight != nullptr ? weight[(size_t)g * size + e] : 1.0f;
     dst[e] = from_float<TO>(src[e] * scale * w * (act == 0 ? silu_f(z) : sigmoid_f(z)));
+  }
+}
+
+// The same for a bfloat16 gate and rows that four-number accesses can read: UNIT threads to a group (a warp, or a block for wide
+// groups), every number loaded once and kept in registers.  Bound by its bytes; the kernel above read a group twice, four
+// bytes to a lane: 2,048 tokens of 28 groups of 128 took 27 us and take 24,
+// one group of 1,792 (a warp per token before) 33 us and 12.
+constexpr int GATED_QUADS = 4;            // per thread at most
+template <int UNIT>
+__global__ void __launch_bounds__(256) gated_norm_vec_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ gate, long long ld_gate,
+                                                             const float* __restrict__ weight, __nv_bfloat16* __restrict__ out, long long ld_out,
+                                                             int tokens, int groups, int size, float eps, int act) {
+  __shared__ float scratch[32];
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x % UNIT;
+  const long long unit = (long long)blockIdx.x * (256 / UNIT) + threadIdx.x / UNIT;
+  if (unit >= (long long)tokens * groups) return;                 // a whole warp, or the whole block
+  const int t = (int)(unit / groups), g = (int)(unit - (long long)t * groups);
+  const float4* src = reinterpret_cast<const float4*>(o + ((size_t)t * groups + g) * size);
+  const uint2* gt = reinterpret_cast<const uint2*>(gate + (size_t)t * ld_gate + (size_t)g * size);
+  const int quads = size >> 2;
+  float4 y[GATED_QUADS];
+  float sum = 0.0f;
+#pragma unroll
+  for (int k = 0; k < GATED_QUADS; ++k) {
+    const int i = lane + k * UNIT;
+    y[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < quads) {
+      float4 v = src[i];
+      const uint2 raw = gt[i];
+      const float z[4] = {__uint_as_float(raw.x << 16), __uint_as_float(raw.x & 0xffff0000u), __uint_as_float(raw.y << 16), __uint_as_float(raw.y & 0xffff0000u)};
+      float a[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[e] = act == 1 ? sigmoid_f(z[e]) : silu_f(z[e]);
+      const float4 gated = make_float4(v.x * a[0], v.y * a[1], v.z * a[2], v.w * a[3]);
+      if (act == 2) v = gated;
+      sum = fmaf(v.x, v.x, sum); sum = fmaf(v.y, v.y, sum); sum = fmaf(v.z, v.z, sum); sum = fmaf(v.w, v.w, sum);
+      y[k] = gated;
+    }
+  }
+  sum = UNIT == 32 ? warp_sum(sum) : block_sum(sum, scratch);
+  const float scale = 1.0f / sqrtf(sum / (float)size + eps);
+  __nv_bfloat16* dst = out + (size_t)t * ld_out + (size_t)g * size;
+#pragma unroll
+  for (int k = 0; k < GATED_QUADS; ++k) {
+    const int i = lane + k * UNIT;
+    if (i < quads) {
+      const float4 w = weight != nullptr ? reinterpret_cast<const float4*>(weight + (size_t)g * size)[i] : make_float4(1.f, 1.f, 1.f, 1.f);
+      store_quad(dst + 4 * (size_t)i, make_float4(y[k].x * scale * w.x, y[k].y * scale * w.y, y[k].z * scale * w.z, y[k].w * scale * w.w));
+    }
   }
 }
 
@@ -954,17 +1066,16 @@ int launch_decay_scan(const void* rows, long long ld, int q_off, int k_off, int 
       configured[which] = wide;
     }
     dim3 wide_grid((vdim + WIDE - 1) / WIDE, heads, num_seqs);
-    decay_prepare_kernel<T><<<dim3(tokens, heads), 128, 0, stream>>>((const T*)rows, ld, q_off, k_off, heads, dim, activation,
-                                                                     cos_table, sin_table, table_positions, rotary, k_scale,
-                                                                     positions, prepared, status);
+    launch_decay_prepare((const T*)rows, ld, q_off, k_off, heads, dim, activation, cos_table, sin_table, table_positions, rotary, k_scale,
+                         positions, prepared, tokens, status, stream);
     const int segment = carry != nullptr ? segment_tokens(sizeof(T) == 2, dim, vdim, max_q_len) : 0;
     if (segment > 0 && segment != SEGMENT && tokens / segment + num_seqs <= 65535) {
       const int pieces = tokens / segment + num_seqs;
       int rc = launch_decay_tc(rows, ld, prepared, v_off, heads, dim, vdim, activation, decay, q_start, carry, out, num_seqs, pieces, false,
                                status, stream);
       if (rc < 0) return rc;
-      decay_segment_carry_kernel<<<dim3((dim * vdim + 255) / 256, heads, num_seqs), 256, 0, stream>>>(
-          carry, state, decay, slots, q_start, heads, dim, vdim, segment);
+      tge_launch(decay_segment_carry_kernel, dim3((dim * vdim + 255) / 256, heads, num_seqs), dim3(256), 0, stream, carry, state, decay, slots,
+                 q_start, heads, dim, vdim, segment);
       rc = launch_decay_tc(rows, ld, prepared, v_off, heads, dim, vdim, activation, decay, q_start, carry, out, num_seqs, pieces, true,
                            status, stream);
       if (rc < 0) return rc;
@@ -976,8 +1087,8 @@ int launch_decay_scan(const void* rows, long long ld, int q_off, int k_off, int 
       dim3 pieces(wide_grid.x, heads, tokens / SEGMENT + num_seqs);      // an upper bound; blocks beyond the last segment leave at once
       decay_scan_wide_kernel<T, 1><<<pieces, 256, wide, stream>>>((const T*)rows, ld, prepared, v_off, heads, dim, vdim, activation,
                                                                   decay, state, slots, q_start, out, carry, num_seqs, SEGMENT);
-      decay_segment_carry_kernel<<<dim3((dim * vdim + 255) / 256, heads, num_seqs), 256, 0, stream>>>(
-          carry, state, decay, slots, q_start, heads, dim, vdim, SEGMENT);
+      tge_launch(decay_segment_carry_kernel, dim3((dim * vdim + 255) / 256, heads, num_seqs), dim3(256), 0, stream, carry, state, decay, slots,
+                 q_start, heads, dim, vdim, (int)SEGMENT);
       decay_scan_wide_kernel<T, 2><<<pieces, 256, wide, stream>>>((const T*)rows, ld, prepared, v_off, heads, dim, vdim, activation,
                                                                   decay, state, slots, q_start, out, carry, num_seqs, SEGMENT);
       return tge_launched("decay_scan_segments", 4);
@@ -997,9 +1108,8 @@ int launch_decay_scan(const void* rows, long long ld, int q_off, int k_off, int 
       }
       configured[which] = chunked;
     }
-    decay_prepare_kernel<T><<<dim3(tokens, heads), 128, 0, stream>>>((const T*)rows, ld, q_off, k_off, heads, dim, activation,
-                                                                     cos_table, sin_table, table_positions, rotary, k_scale,
-                                                                     positions, prepared, status);
+    launch_decay_prepare((const T*)rows, ld, q_off, k_off, heads, dim, activation, cos_table, sin_table, table_positions, rotary, k_scale,
+                         positions, prepared, tokens, status, stream);
     decay_scan_chunked_kernel<T><<<grid, CHUNK_THREADS, chunked, stream>>>((const T*)rows, ld, prepared, v_off, heads, dim, vdim,
                                                                           activation, decay, state, slots, q_start, out);
     return tge_launched("decay_scan_chunked", 2);
@@ -1097,7 +1207,16 @@ TGE_API int tge_gated_norm(const float* o, const void* gate, int is_bf16, long l
   if (tokens == 0) return 0;
   const long long units = (long long)tokens * groups;
   const unsigned blocks = (unsigned)((units + 3) / 4);
-  if (!is_bf16 && out_is_bf16)
+  // four numbers at a time where the rows allow it: a warp to a group of up to 512 numbers, a block up to 4,096
+  const bool quads = is_bf16 && size % 4 == 0 && ld_gate % 4 == 0 && ld_out % 4 == 0 && size <= 256 * 4 * GATED_QUADS && units <= 0x7fffffffll &&
+                     (uintptr_t)o % 16 == 0 && (uintptr_t)gate % 8 == 0 && (uintptr_t)out % 8 == 0 && (uintptr_t)weight % 16 == 0;
+  if (quads && size <= 32 * 4 * GATED_QUADS)
+    tge_launch(gated_norm_vec_kernel<32>, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, stream, o, (const __nv_bfloat16*)gate, ld_gate, weight,
+               (__nv_bfloat16*)out, ld_out, tokens, groups, size, eps, act);
+  else if (quads)
+    tge_launch(gated_norm_vec_kernel<256>, dim3((unsigned)units), dim3(256), 0, stream, o, (const __nv_bfloat16*)gate, ld_gate, weight,
+               (__nv_bfloat16*)out, ld_out, tokens, groups, size, eps, act);
+  else if (!is_bf16 && out_is_bf16)
     tge_launch(gated_norm_kernel<float, __nv_bfloat16>, dim3(blocks), dim3(128), 0, stream, o, (const float*)gate, ld_gate, weight,
                (__nv_bfloat16*)out, ld_out, tokens, groups, size, eps, act);
   else if (is_bf16)
