@@ -1279,8 +1279,15 @@ const CUtensorMap* pool_map(const void* pages, int num_pages, int kv_heads, int 
 #endif  // TGE_TMA_KERNELS
 
 // Merges the split states of one (token, head): out = sum_s 2^(m_s - M) acc_s / sum_s 2^(m_s - M) l_s,
-// over the splits that hold keys visible to the row, in split order.
-template <int HELD>                                                  // splits whose state is held in registers
+// over the splits that hold keys visible to the row, in split order.  A thread per number of a head; every warp holds the
+// splits' maxima and denominators, lane by lane, and hands them round by shuffles.
+//
+// Bound by latency: one round trip for maxima and the first sixteen states together, then the arithmetic.  The code is
+// kept short on purpose: with every state of sixteen or 48 splits in registers of its own the unrolled instances were several
+// times as long, and a step that runs nine other kernels in between fetched them anew each time: one
+// request of 2,048 tokens in 17 splits 8.5 us a layer and now 5.9, eight in 8 splits 4.9 and 4.8 (7B shape, in place).
+constexpr int MERGE_LANES = 4;                                          // splits per lane at most: 128 in all
+constexpr int MERGE_BATCH = 16;                                         // states on their way together
 __global__ void attention_merge_kernel(const float* __restrict__ partial_o, const float* __restrict__ partial_ml,
                                        const int* __restrict__ positions, __nv_bfloat16* __restrict__ out,
                                        int out_stride, int total_tokens, int heads, int window, int split_tokens,
@@ -1288,98 +1295,88 @@ __global__ void attention_merge_kernel(const float* __restrict__ partial_o, cons
                                        const __nv_bfloat16* __restrict__ gate, int gate_stride, int gate_elements,
                                        int window_runs) {
   pdl_trigger();
-  const int t = blockIdx.x + first_token, h = blockIdx.y;
+  const int t = blockIdx.x + first_token, h = blockIdx.y, lane = threadIdx.x & 31;
   const int pos = positions[t];                                     // given to the step: not the previous kernel's work
   const float sink_log2 = sink != nullptr ? sink[h] * LOG2E : -INFINITY;   // the sink joins the merged denominator once
-  pdl_wait();
-  const __nv_bfloat16* gates = gate != nullptr && gate_elements ? gate + (size_t)t * gate_stride + (size_t)h * DV : nullptr;
-  const float factor = gate != nullptr && !gate_elements ? gate_of(__bfloat162float(gate[(size_t)t * gate_stride + h])) : 1.0f;
-  const size_t stride = (size_t)total_tokens * heads;               // slots per split
-  const size_t slot0 = (size_t)t * heads + h;
-  if (num_splits <= HELD) {
-    // Every load is asked for before the first result is needed, the row's position among them: one round
-    // trip instead of four.  Splits without a key visible to the row are read too (the scratch holds all
-    // splits; what lies there is old) and dropped by selection, never by a weight of zero.
-    float2 ml[HELD];
-#pragma unroll
-    for (int i = 0; i < HELD; ++i)
-      ml[i] = i < num_splits ? *reinterpret_cast<const float2*>(partial_ml + ((size_t)i * stride + slot0) * 2)
-                             : make_float2(-INFINITY, 0.0f);
-    const int base = run_base(window_runs ? window : 0, pos);
-    const int first_key = window > 0 ? max(pos - window + 1, 0) : 0;
-    const int s_lo = (first_key - base) / split_tokens;
-    const int s_hi = min((pos - base) / split_tokens, num_splits - 1);
-    for (int d = threadIdx.x; d < DV; d += blockDim.x) {
-      float o[HELD];
-#pragma unroll
-      for (int i = 0; i < HELD; ++i) o[i] = i < num_splits ? partial_o[((size_t)i * stride + slot0) * DV + d] : 0.0f;
-#pragma unroll
-      for (int i = 0; i < HELD; ++i) {
-        const bool live = i <= s_hi && (i >= s_lo || i * split_tokens < keep_first);
-        ml[i] = live ? ml[i] : make_float2(-INFINITY, 0.0f);
-        o[i] = live ? o[i] : 0.0f;
-      }
-      float m = -INFINITY;
-#pragma unroll
-      for (int i = 0; i < HELD; ++i) m = fmaxf(m, ml[i].x);
-      const float m_use = m == -INFINITY ? 0.0f : m;
-      float l = 0.0f, acc = 0.0f;
-#pragma unroll
-      for (int i = 0; i < HELD; ++i) {          // in split order; a split beyond s_hi has m = -inf: weight 0
-        const float scale = exp2f(ml[i].x - m_use);
-        l += scale * ml[i].y;
-        acc += scale * o[i];
-      }
-      if (sink != nullptr) l += exp2f(sink_log2 - m_use);
-      out[(size_t)t * out_stride + (size_t)h * DV + d] = __float2bfloat16_rn(acc * (l > 0.0f ? 1.0f / l : 0.0f) * (gates != nullptr ? gate_of(__bfloat162float(gates[d])) : factor));
-    }
-    return;
-  }
   const int base = run_base(window_runs ? window : 0, pos);
   const int first_key = window > 0 ? max(pos - window + 1, 0) : 0;
   const int s_lo = (first_key - base) / split_tokens;
   const int s_hi = min((pos - base) / split_tokens, num_splits - 1);
   // the runs of the kept first tokens, then those of the window
   const int kept_runs = min(s_lo, (keep_first + split_tokens - 1) / split_tokens);
-  const int skipped = s_lo - kept_runs;
+  const int skipped = s_lo - kept_runs, count = s_hi - skipped + 1;
+  const size_t stride = (size_t)total_tokens * heads;               // slots per split
+  const size_t slot0 = (size_t)t * heads + h;
+  auto slot_of = [&](int i) { return (size_t)(i < kept_runs ? i : i + skipped) * stride + slot0; };
+  pdl_wait();
+  const __nv_bfloat16* gates = gate != nullptr && gate_elements ? gate + (size_t)t * gate_stride + (size_t)h * DV : nullptr;
+  const float factor = gate != nullptr && !gate_elements ? gate_of(__bfloat162float(gate[(size_t)t * gate_stride + h])) : 1.0f;
+  const bool held = count <= 32 * MERGE_LANES;
+  float2 ml[MERGE_LANES];
   float m = -INFINITY;
-  for (int i = 0; i <= s_hi - skipped; ++i) {
-    const int s = i < kept_runs ? i : i + skipped;
-    m = fmaxf(m, partial_ml[((size_t)s * stride + slot0) * 2]);
-  }
-  const float m_use = m == -INFINITY ? 0.0f : m;
-  float l = 0.0f;
-  for (int i = 0; i <= s_hi - skipped; ++i) {
-    const int s = i < kept_runs ? i : i + skipped;
-    const size_t slot = (size_t)s * stride + slot0;
-    l += exp2f(partial_ml[slot * 2] - m_use) * partial_ml[slot * 2 + 1];
-  }
-  if (sink != nullptr) l += exp2f(sink_log2 - m_use);
-  const float inv = (l > 0.0f ? 1.0f / l : 0.0f) * factor;
-  for (int d = threadIdx.x; d < DV; d += blockDim.x) {
-    float acc = 0.0f;
-    for (int i = 0; i <= s_hi - skipped; ++i) {
-      const int s = i < kept_runs ? i : i + skipped;
-      const size_t slot = (size_t)s * stride + slot0;
-      acc += exp2f(partial_ml[slot * 2] - m_use) * partial_o[slot * DV + d];
+  if (held) {
+#pragma unroll
+    for (int k = 0; k < MERGE_LANES; ++k) {
+      const int i = lane + 32 * k;
+      ml[k] = i < count ? *reinterpret_cast<const float2*>(partial_ml + slot_of(i) * 2) : make_float2(-INFINITY, 0.0f);
     }
-    out[(size_t)t * out_stride + (size_t)h * DV + d] =
-        __float2bfloat16_rn(acc * inv * (gates != nullptr ? gate_of(__bfloat162float(gates[d])) : 1.0f));
+  } else {
+    for (int i = 0; i < count; ++i) m = fmaxf(m, partial_ml[slot_of(i) * 2]);
+  }
+  for (int d0 = 0; d0 < DV; d0 += blockDim.x) {                       // every lane takes part in the shuffles
+    const int d = d0 + (int)threadIdx.x, d_read = min(d, DV - 1);
+    float l = 0.0f, acc = 0.0f, m_use = 0.0f;
+    for (int i0 = 0; i0 < count; i0 += MERGE_BATCH) {
+      float o[MERGE_BATCH];
+#pragma unroll
+      for (int i = 0; i < MERGE_BATCH; ++i) o[i] = i0 + i < count ? partial_o[slot_of(i0 + i) * DV + d_read] : 0.0f;
+      if (i0 == 0) {
+        if (held && d0 == 0) {
+#pragma unroll
+          for (int k = 0; k < MERGE_LANES; ++k) m = fmaxf(m, ml[k].x);
+#pragma unroll
+          for (int offset = 16; offset > 0; offset >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, offset));
+        }
+        m_use = m == -INFINITY ? 0.0f : m;
+        if (held && d0 == 0) {
+#pragma unroll
+          for (int k = 0; k < MERGE_LANES; ++k) ml[k].x = exp2f(ml[k].x - m_use);       // from here on the split's weight
+        }
+      }
+      float2 part = make_float2(0.0f, 0.0f);                          // this lane's split of the thirty-two around i0
+      if (held) {
+#pragma unroll
+        for (int k = 0; k < MERGE_LANES; ++k)
+          if (i0 >> 5 == k) part = ml[k];
+      }
+#pragma unroll
+      for (int i = 0; i < MERGE_BATCH; ++i) {                         // in split order
+        float scale, denominator;
+        if (held) {
+          scale = __shfl_sync(0xffffffffu, part.x, (i0 & 16) + i);
+          denominator = __shfl_sync(0xffffffffu, part.y, (i0 & 16) + i);
+        } else {
+          const bool live = i0 + i < count;
+          scale = live ? exp2f(partial_ml[slot_of(i0 + i) * 2] - m_use) : 0.0f;
+          denominator = live ? partial_ml[slot_of(i0 + i) * 2 + 1] : 0.0f;
+        }
+        l += scale * denominator;
+        acc += scale * o[i];
+      }
+    }
+    if (sink != nullptr) l += exp2f(sink_log2 - m_use);
+    if (d < DV)
+      out[(size_t)t * out_stride + (size_t)h * DV + d] =
+          __float2bfloat16_rn(acc * (l > 0.0f ? 1.0f / l : 0.0f) * (gates != nullptr ? gate_of(__bfloat162float(gates[d])) : factor));
   }
 }
 
-// Sixteen states in registers serve most steps; a single long request cut into up to 48 splits takes the wider
-// instance, and beyond that the kernel walks the splits in a loop.
 void launch_merge(const AttnParams& p, const int* positions, int first_token, cudaStream_t stream) {
   const dim3 grid(p.total_tokens - first_token, p.heads);
   const int threads = DV >= 128 ? 128 : (DV >= 64 ? 64 : 32);
-  auto run = [&](auto kernel) {
-    tge_launch(kernel, grid, threads, 0, stream, (const float*)p.partial_o, (const float*)p.partial_ml, positions, p.out, p.out_stride,
-               p.total_tokens, p.heads, p.window, p.split_tokens, p.num_splits, first_token, p.sink, p.keep_first, p.gate,
-               p.gate_stride, p.gate_elements, p.window_runs);
-  };
-  if (p.num_splits <= 16) run(attention_merge_kernel<16>);
-  else run(attention_merge_kernel<48>);
+  tge_launch(attention_merge_kernel, grid, threads, 0, stream, (const float*)p.partial_o, (const float*)p.partial_ml, positions, p.out, p.out_stride,
+             p.total_tokens, p.heads, p.window, p.split_tokens, p.num_splits, first_token, p.sink, p.keep_first, p.gate,
+             p.gate_stride, p.gate_elements, p.window_runs);
 }
 
 template <int NWARPS>
