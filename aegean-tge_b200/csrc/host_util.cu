@@ -47,6 +47,25 @@ int tge_sm_count() {
 
 TGE_API int tge_device_sm_count() { return tge_sm_count(); }
 
+// What a step does around its kernels, on the raw stream: torch's own calls look up a stream object and build event and
+// copy objects each time (5 to 9 us apiece, against 1 to 2 here, three copies and two events to a step of a small model).
+static int checked(const char* what, cudaError_t err) {
+  if (err == cudaSuccess) return 0;
+  cudaGetLastError();
+  tge_set_error("%s: %s", what, cudaGetErrorString(err));
+  return -2;
+}
+TGE_API int tge_event_create(void** event) {
+  return checked("event", cudaEventCreateWithFlags(reinterpret_cast<cudaEvent_t*>(event), cudaEventDisableTiming));
+}
+TGE_API int tge_event_record(void* event, cudaStream_t stream) { return checked("event record", cudaEventRecord((cudaEvent_t)event, stream)); }
+TGE_API int tge_event_synchronize(void* event) { return checked("event wait", cudaEventSynchronize((cudaEvent_t)event)); }
+TGE_API int tge_event_destroy(void* event) { return checked("event", cudaEventDestroy((cudaEvent_t)event)); }
+// The caller keeps both ends alive until the copy is done.
+TGE_API int tge_copy(void* dst, const void* src, long long bytes, cudaStream_t stream) {
+  return checked("copy", cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyDefault, stream));
+}
+
 TGE_API const char* tge_last_error() { return g_error; }
 
 TGE_API int tge_abi_version() { return 1; }

@@ -18,6 +18,7 @@ from typing import Callable, Dict, Hashable, List, Optional, Sequence
 import numpy as np
 import torch
 
+from .. import ops as _ops
 from .. import runtime as _rt
 from ..cache.manager import CacheManager
 from ..cache.pages import PoolExhausted
@@ -36,26 +37,28 @@ class Staging:
         self.ring = ring
         self.hosts = [torch.zeros(ints, dtype=torch.int32).pin_memory() for _ in range(ring)]
         self.views = [host.numpy() for host in self.hosts]
-        self.copied: List[Optional[torch.cuda.Event]] = [None] * ring
+        self.copied = [_ops.StepEvent() for _ in range(ring)]
         self.turn = 0
 
     def take(self, ints: int = 0) -> int:
         """The next buffer's index, free to be written, at least ``ints`` long."""
         turn = self.turn
         self.turn = (turn + 1) % self.ring
-        if self.copied[turn] is not None:
-            self.copied[turn].synchronize()
-            self.copied[turn] = None
+        self.copied[turn].synchronize()
         if self.hosts[turn].numel() < ints:
             self.hosts[turn] = torch.zeros(max(ints, 2 * self.hosts[turn].numel()), dtype=torch.int32).pin_memory()
             self.views[turn] = self.hosts[turn].numpy()
         return turn
 
-    def queued(self, turn: int) -> None:
-        """Call after the copy out of buffer ``turn`` was queued on the current stream."""
-        event = torch.cuda.Event()
-        event.record()
-        self.copied[turn] = event
+    def send(self, turn: int, ints: int, to: torch.Tensor) -> None:
+        """Queues the copy of buffer ``turn``'s first ``ints`` into ``to`` (int32 on the device) on the current stream."""
+        _ops.copy_bytes(to, self.hosts[turn], 4 * ints)
+        self.copied[turn].record()
+
+    def __del__(self):
+        # the pinned buffers go back to their allocator, which knows nothing of the copies out of them
+        for event in getattr(self, "copied", ()):
+            event.synchronize()
 
 
 def graph_batch(batch: int) -> int:
@@ -221,8 +224,8 @@ class ModelRunner:
             total = pack(0, 0, staging.views[turn], layout)
             if packed is not None:
                 packed()
-            dev = staging.hosts[turn][:total].to(self.device, non_blocking=True)
-            staging.queued(turn)
+            dev = torch.empty(total, dtype=torch.int32, device=self.device)
+            staging.send(turn, total, dev)
             self.h2d_bytes_last = total * 4
             ctx, rows = context_from_packed(dev, staging.views[turn], layout, groups)
             logits = self.model.forward(ctx, rows)
@@ -322,8 +325,7 @@ class DecodeGraph:
             raise RuntimeError("decode graph: the packed step does not have the captured layout")
         if packed is not None:
             packed()
-        self.dev.copy_(staging.hosts[turn], non_blocking=True)
-        staging.queued(turn)
+        staging.send(turn, total, self.dev)
         if device_tokens is not None:      # the token ids are still on the device: they overwrite the packed placeholders
             first = self.layout.token_ids
             self.dev[first:first + device_tokens.numel()].copy_(device_tokens, non_blocking=True)

@@ -56,6 +56,11 @@ def core() -> ctypes.CDLL:
         path = _build.build_core()
         lib = ctypes.CDLL(path)
         lib.tge_last_error.restype = ctypes.c_char_p
+        _declare(lib, "tge_event_create", [_c_ptr])
+        _declare(lib, "tge_event_record", [_c_ptr, _c_ptr])
+        _declare(lib, "tge_event_synchronize", [_c_ptr])
+        _declare(lib, "tge_event_destroy", [_c_ptr])
+        _declare(lib, "tge_copy", [_c_ptr, _c_ptr, _c_ll, _c_ptr])
         _declare(lib, "tge_embedding", [_c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_ptr])
         _declare(lib, "tge_rmsnorm", [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_float,
                                       _c_ptr, _c_ptr])
@@ -247,13 +252,50 @@ def _check(rc: int, lib: ctypes.CDLL) -> int:
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+# torch.cuda.current_device looks whether CUDA is initialised first; here there are tensors on the device already
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
 
 
 def _stream() -> int:
     """The current stream's handle (asked on every launch: a graph capture switches streams)."""
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_current_device())
     return torch.cuda.current_stream().cuda_stream
+
+
+class StepEvent:
+    """An event without timing, recorded on the current stream, again and again."""
+
+    __slots__ = ("_handle", "_recorded")
+
+    def __init__(self):
+        self._handle, self._recorded = ctypes.c_void_p(), False
+        lib = core()
+        if lib.tge_event_create(ctypes.addressof(self._handle)) < 0:
+            self._handle = None
+            raise KernelError(lib.tge_last_error().decode("utf-8", "replace"))
+
+    def record(self) -> None:
+        _check(_core_lib.tge_event_record(self._handle, _stream()), _core_lib)
+        self._recorded = True
+
+    def synchronize(self) -> None:
+        """Waits for what was queued before the last record (nothing if there was none)."""
+        if self._recorded and _core_lib is not None:         # None: the interpreter is on its way out
+            _check(_core_lib.tge_event_synchronize(self._handle), _core_lib)
+
+    def __del__(self):
+        if getattr(self, "_handle", None) and _core_lib is not None:
+            _core_lib.tge_event_destroy(self._handle)
+
+
+def copy_bytes(dst: torch.Tensor, src: torch.Tensor, count: int) -> None:
+    """Queues a copy of the first ``count`` bytes of ``src`` to ``dst`` on the current stream (host memory pinned).  Nothing keeps
+    the two tensors alive for it: the caller does, until an event recorded behind the copy has passed."""
+    if not (dst.is_contiguous() and src.is_contiguous() and count <= dst.nbytes and count <= src.nbytes):
+        raise KernelError(f"copy: {count} bytes between tensors of {src.nbytes} and {dst.nbytes}")
+    lib = core()
+    _check(lib.tge_copy(dst.data_ptr(), src.data_ptr(), count, _stream()), lib)
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -263,7 +305,7 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 def _want(t: torch.Tensor, name: str, dtype=None, contiguous: bool = True) -> None:
     if not t.is_cuda:
         raise KernelError(f"{name} must be a CUDA tensor (this engine has no CPU path)")
-    if dtype is not None and t.dtype not in (dtype if isinstance(dtype, tuple) else (dtype,)):
+    if dtype is not None and t.dtype != dtype and not (isinstance(dtype, tuple) and t.dtype in dtype):
         raise KernelError(f"{name} must be {dtype}, got {t.dtype}")
     if contiguous and not t.is_contiguous():
         raise KernelError(f"{name} must be contiguous")
@@ -271,9 +313,10 @@ def _want(t: torch.Tensor, name: str, dtype=None, contiguous: bool = True) -> No
 
 def _rows_2d(t: torch.Tensor, name: str) -> int:
     """Row stride (elements) of a 2-D tensor whose rows are dense."""
-    if t.dim() != 2 or (t.shape[1] > 1 and t.stride(1) != 1):
-        raise KernelError(f"{name} must be 2-D with dense rows, got shape {tuple(t.shape)} strides {t.stride()}")
-    return t.stride(0) if t.shape[0] > 1 else max(t.stride(0), t.shape[1])
+    shape, strides = t.shape, t.stride()
+    if len(shape) != 2 or (shape[1] > 1 and strides[1] != 1):
+        raise KernelError(f"{name} must be 2-D with dense rows, got shape {tuple(shape)} strides {strides}")
+    return strides[0] if shape[0] > 1 else max(strides[0], shape[1])
 
 
 _FLOAT = (torch.float32, torch.bfloat16)
@@ -287,10 +330,11 @@ _outgrown: Dict[int, list] = {}       # earlier scratch buffers, kept alive for 
 
 
 def status_word(device: Optional[torch.device] = None) -> torch.Tensor:
-    index = torch.cuda.current_device() if device is None or device.index is None else device.index
-    if index not in _status:
-        _status[index] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{index}")
-    return _status[index]
+    index = _current_device() if device is None or device.index is None else device.index
+    word = _status.get(index)
+    if word is None:
+        word = _status[index] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{index}")
+    return word
 
 
 def check_status() -> None:
@@ -322,7 +366,7 @@ def scratch_floats(count: int) -> torch.Tensor:
     writing partial sums there whenever it is replayed.  Buffers at least double, so what is kept is less
     than what is in use.
     """
-    index = torch.cuda.current_device()
+    index = _current_device()
     have = _scratch.get(index)
     if have is None or have.numel() < count:
         if torch.cuda.is_current_stream_capturing():
@@ -1198,7 +1242,7 @@ def choose_attention_split(tokens: int, num_seqs: int, max_q_len: int, max_ctx_l
         want_splits = min(2 * sms // blocks, most)
         return keys_per_split(want_splits) if want_splits > 1 else 0
     # Single tokens.  About one block per SM is best: every split more is a state more to write and to merge, and
-    # the merging kernel holds sixteen states in registers (A/B in one process, ms per step of the 7B shape, 296
+    # the merging kernel asks for sixteen states at a time (A/B in one process, ms per step of the 7B shape, 296
     # blocks against 148: batch 16 at context 2,048 3.33 / 3.22; batch 8 at 4,096 3.30 / 3.13; batch 4 at 4,096
     # 3.23 / 3.04; batch 4 at 30,000 4.05 / 3.89; batch 1 at 32,000 3.71 / 3.38).  Two exceptions, both measured:
     # splits of no more than 256 keys, sixteen at most over the whole bound, are better taken twice as many

@@ -24,7 +24,7 @@ class Sampler:
         self.ops = ops
         self.device = device
         self._zeros = {}            # rows -> float32 zeros [2, rows] on the device (greedy: temperature 0, no draw)
-        self._pinned = {}           # rows -> ring of pinned int32 buffers for ids on their way to the host
+        self._pinned = {}           # rows -> ring of (pinned int32 buffer for ids on their way to the host, event)
 
     def _to_device(self, values, dtype) -> torch.Tensor:
         host = torch.tensor(values, dtype=dtype)
@@ -67,12 +67,17 @@ class Sampler:
         ids = self._draw(logits, params, rngs)
         turn = self._turn = (getattr(self, "_turn", -1) + 1) % 4
         if rows not in self._pinned:
-            self._pinned[rows] = [torch.empty(rows, dtype=torch.int32).pin_memory() for _ in range(4)]
-        host = self._pinned[rows][turn]
-        host.copy_(ids, non_blocking=True)
-        event = torch.cuda.Event()
+            self._pinned[rows] = [(torch.empty(rows, dtype=torch.int32).pin_memory(), self.ops.StepEvent()) for _ in range(4)]
+        host, event = self._pinned[rows][turn]
+        self.ops.copy_bytes(host, ids, 4 * rows)
         event.record()
         return ids, host, event
+
+    def __del__(self):
+        # the pinned buffers go back to their allocator, which knows nothing of the copies into them
+        for ring in getattr(self, "_pinned", {}).values():
+            for _host, event in ring:
+                event.synchronize()
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], rngs: Sequence[XorShift32],
                histories: Optional[Sequence[Sequence[int]]] = None) -> List[int]:
