@@ -175,6 +175,21 @@ def test_gemm_float32_on_the_tensor_cores_keeps_what_is_not_finite(ops):
     assert rel_error(out * 1e30, x[6:9].double() @ w[10:].double().T) < 1e-6
 
 
+def test_gemm_float32_without_room_for_scratch_is_one_chain(ops, monkeypatch):
+    """Where the scratch buffer cannot grow (while a graph is captured) the product runs as the FMA chain, as it always did."""
+    gen = torch.Generator().manual_seed(2)
+    x, w = torch.randn(5, 600, generator=gen).to(DEV), torch.randn(640, 600, generator=gen).to(DEV)
+    chain = ops.linear(x, w, None, ops.GEMM_STORE_F32, force_simt=True)
+    out = torch.zeros(5, 640, device=DEV)
+    torch.cuda.synchronize()
+    monkeypatch.setattr(ops, "_scratch", {})
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.linear(x, w, None, ops.GEMM_STORE_F32, out=out)
+    graph.replay()
+    assert torch.equal(out, chain)
+
+
 TC_SHAPES = [(1, 128, 64), (8, 384, 176), (16, 200, 256), (33, 130, 72), (64, 512, 1024), (100, 300, 512),
              (200, 640, 320), (300, 1024, 512), (520, 256, 192)]
 
@@ -506,6 +521,15 @@ def test_attention_float32_rows_do_not_depend_on_the_step(ops, heads, kv_heads, 
         assert torch.equal(rows(start, count), whole[start:start + count]), (start, count)
     assert torch.equal(rows(520, 1, bound=4096), whole[520:521])
     ops.check_status()
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,page_size,window,q_lens,starts", [
+    (28, 4, 128, 16, 0, [1500, 37, 1], [0, 300, 70]), (40, 8, 64, 64, 200, [1030, 260], [15, 0]), (16, 8, 32, 16, 0, [900, 333, 300], [1, 64, 0]),
+    (28, 4, 128, 16, 0, [1024], [0]), (28, 4, 128, 64, 0, [250], [5]), (28, 4, 128, 16, 0, [300], [4100]), (12, 2, 128, 64, 0, [130] * 9, [0] * 9)])
+def test_attention_prefill_on_both_sides_of_the_two_tile_rule(ops, heads, kv_heads, head_dim, page_size, window, q_lens, starts):
+    """Portions that take two query tiles to a block (many blocks or long keys) and portions that take one."""
+    err, _, _ = _attention_case(ops, torch.bfloat16, heads, kv_heads, head_dim, q_lens, starts, page_size=page_size, window=window)
+    assert err < TOL[torch.bfloat16]
 
 
 def test_leading_single_tokens_deep_in_long_contexts_get_splits_of_their_own(ops):
