@@ -1558,7 +1558,16 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
         out_stride % 8 == 0 && (uintptr_t)out % 16 == 0) {
       // the tcgen05 kernels: 128 rows per query tile as well
       static const bool one_tile = getenv("TGE_ATTENTION_ONE_TILE") != nullptr && getenv("TGE_ATTENTION_ONE_TILE")[0] != '\0';
-      if (tc2::FITS && !one_tile && tc2::smem_bytes(range >> p.page_shift) <= 227 * 1024) {
+      // Two query tiles to a block share K and V and one SM; where blocks are few or short, one tile to a block has the SMs'
+      // tensor cores to itself and less to set up.  The line, measured at 28 heads over 4 of 128 (two tiles / one, us): keys of
+      // up to 256 in any number (16 prompts of 120: 31.2 / 26.5); blocks for no more than the SMs and up to 1,024 keys (1,024
+      // tokens: 30.5 / 28.5; 1,500: 39.5 / 40.9); for half of them and up to 4,096 (512 after 1,024: 37.4 / 34.8; 512 after
+      // 6,144: 117 / 120); for a quarter (200 after 6,144: 73.3 / 68.9).  40 heads over 8 and 12 over 2 lie the same way.
+      const long long pair_blocks = (long long)(((tokens - first_token + p.bq - 1) / p.bq + 1) / 2 + num_seqs) * kv_heads * num_splits;
+      const int sms = tge_sm_count();
+      const bool few = max_ctx_len <= 256 || (pair_blocks <= sms && max_ctx_len <= 1024) || (2 * pair_blocks <= sms && max_ctx_len <= 4096) ||
+                       4 * pair_blocks <= sms;
+      if (tc2::FITS && !one_tile && !few && tc2::smem_bytes(range >> p.page_shift) <= 227 * 1024) {
         // two query tiles per block, one block per SM
         const size_t smem2 = tc2::smem_bytes(range >> p.page_shift);
         static size_t configured_tc2 = 0;
