@@ -739,21 +739,25 @@ Plan make_plan(int M, int N, int K, long long scratch_floats, int force_bn, int 
   else if (M <= 128) bn = 128;
   else {
     // More than 128 tokens: every width of the token tile (a multiple of 16 in 128..256, the tokens shared out
-    // evenly) with every cut along k that the scratch holds, by the cost above; ties go to the wider tile and
+    // evenly, or 128 with the rest in the last: q/k/v of the 7B shape at 320 / 400 tokens 18.1 / 18.4 us at widths 160 / 208 and
+    // 16.2 / 16.7 at 128, o 18.5 / 18.9 and 16.7 / 16.5) with every cut along k that the scratch holds, by the cost above; ties go to the wider tile and
     // the fewer splits.
     const int k_blocks_here = (K + BK - 1) / BK;
     long long best = -1;
     bn = 256;
     for (int count = (M + 255) / 256;; ++count) {
-      const int width = ((M + count - 1) / count + 15) / 16 * 16;
-      if (width < 128) break;
+      // The last choice is 128 wide with a part of the last tile empty: few weight tiles then share the SMs without a cut, if
+      // that occupies half of them (193 tokens of q/k/v on 72 SMs: 15.6 against 17.1 us alone, but the step was slower for it).
+      const int even = ((M + count - 1) / count + 15) / 16 * 16, width = even < 128 ? 128 : even;
       const long long items = (long long)tiles_w * ((M + width - 1) / width);
+      if (even < 128 && 2 * items < sms) break;
       const int most = force_splits > 0 ? force_splits : (items >= sms || k_blocks_here < 8 ? 1 : (k_blocks_here / 4 < 32 ? k_blocks_here / 4 : 32));
       for (int s = force_splits > 0 ? force_splits : 1; s <= most; ++s) {
         if (s > 1 && (long long)s * M * N > scratch_floats) break;
         const long long cost = plan_cost(items, sms, k_blocks_here, s, one_sm_kblock_cycles(width), (long long)M * N);
         if (best < 0 || cost < best) { best = cost; bn = width; wide_splits = s; }
       }
+      if (even < 128) break;
     }
   }
   plan.bn = bn;
@@ -869,7 +873,9 @@ bool choose_pair(int M, int N, int K, long long scratch_floats, const Plan& sing
   // From about a thousand tokens on the pair does better than these figures say (every SM fetches half as many
   // token rows, which counts once the operands no longer sit in L2: o at 4,096 tokens 78 us against 92, down 375
   // against 420, where the figures put the SM alone ahead by a few per cent), so it is given 15 % there.
+  // From 256 on the same counts for 5 % (320 tokens, gate and up 76 against 71 us, down 48.7 against 45.6; 512, down 66 against 63).
   if (M >= 1024) single_cost += single_cost * 15 / 100;
+  else if (M >= 256) single_cost += single_cost * 5 / 100;
   return g_pair_mode == 2 || pair_cost <= single_cost;
 }
 
