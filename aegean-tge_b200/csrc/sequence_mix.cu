@@ -985,6 +985,8 @@ __global__ void conv_state_update_kernel(const T* __restrict__ raw, long long ld
   }
 }
 
+constexpr int POOL_AHEAD = 8;
+
 // The mean key and mean value of every block of `pool` positions whose last token this step brings: one block of
 // threads per (token, kv head); only tokens at a block's last position do anything.  The means are taken over the
 // keys and values as their pages hold them, and entry b of a request lies where position b would in the pooled pages.
@@ -1013,11 +1015,25 @@ __global__ void __launch_bounds__(128) pool_kv_kernel(
     const T* pages = is_key ? k_pages : v_pages;
     float sum = 0.0f;
     bool ok = true;
-    for (int p = position - pool + 1; p <= position; ++p) {
-      const int page_index = p / page_size;
-      const int page = page_index < max_pages ? block_table[(size_t)seq * max_pages + page_index] : -1;
-      if (page < 0 || page >= num_pages) { ok = false; break; }
-      sum += to_float<T>(pages[(((size_t)page * kv_heads + head) * page_size + p % page_size) * size + d]);
+    // eight positions' pages, then their numbers, on their way together; added in order.  (One after the other, each behind the
+    // look at its page, the 64 of a block were a chain of loads:
+    // 2,048 tokens, 4 kv heads of 128, blocks of 64: 69 us, now 37.)
+    for (int p0 = position - pool + 1; p0 <= position && ok; p0 += POOL_AHEAD) {
+      const T* at[POOL_AHEAD];
+      T value[POOL_AHEAD];
+#pragma unroll
+      for (int j = 0; j < POOL_AHEAD; ++j) {
+        const int p = min(p0 + j, position), page_index = p / page_size;
+        const int page = page_index < max_pages ? block_table[(size_t)seq * max_pages + page_index] : -1;
+        const bool good = page >= 0 && page < num_pages;
+        ok = ok && good;
+        at[j] = pages + (((size_t)(good ? page : 0) * kv_heads + head) * page_size + (p - page_index * page_size)) * size + d;
+      }
+#pragma unroll
+      for (int j = 0; j < POOL_AHEAD; ++j) value[j] = *at[j];
+#pragma unroll
+      for (int j = 0; j < POOL_AHEAD; ++j)
+        if (p0 + j <= position) sum += to_float<T>(value[j]);
     }
     if (!ok) {
       atomicOr(status, TGE_STATUS_BAD_PAGE);
