@@ -1,7 +1,7 @@
 // Paged causal attention of the float32 path, float32 arithmetic, keys in tiles shared by a block's rows.
 //
 // attention_simt.cu gives a warp one (token, head) and walks the keys one at a time: a key costs a chain of loads, a
-// butterfly over the warp and two exponentials, about 1.4 us of it per 1,000 keys and nothing to hide it behind, and
+// butterfly over the warp and two exponentials, about 1.4 us a key and nothing to hide it behind, and
 // every head of a group fetches the keys for itself.  Bound by that chain, not by bytes: a step of 8 requests of 1,000
 // tokens at 28 heads over 4 of 128 took 1,403 us a layer, against 5 us for its 33 MB of keys and values.  Here
 //   * a block owns up to 16 or 64 rows, (query, head of the group) pairs of one request and kv head, and 64 keys at a time
