@@ -970,14 +970,13 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
                                                   heads, kv_heads, bound=span)
             # the single tokens at the head of a mixed step are a decode batch of their own: a few of them deep in
             # long contexts want their keys cut although the portions beside them do not
-            prefix_split = choose_prefix_split(prefix, span, kv_heads) if prefix else 0
+            prefix_split = choose_attention_split(prefix, prefix, 1, span, heads, kv_heads, bound=span) if prefix else 0
         # single tokens over a window cut the window's span (from its first tile on), everything else the whole context
         narrow = heads // kv_heads <= 16 and window > 0 and keep_first == 0 and not pool
         one_window = min(max_ctx_len, window + 63) if narrow else max_ctx_len
         count = lambda split, reach: 1 if split == 0 or reach <= split else -(-reach // split)
-        splits = count(split_tokens, one_window if max_q_len <= 1 else max_ctx_len)
-        need = max(lib.tge_attention_mma_scratch_floats(tokens, heads, splits),
-                   lib.tge_attention_mma_scratch_floats(prefix, heads, count(prefix_split, one_window)) if prefix else 0)
+        splits = max(count(split_tokens, one_window if max_q_len <= 1 else max_ctx_len), count(prefix_split, one_window) if prefix else 1)
+        need = lib.tge_attention_mma_scratch_floats(tokens, heads, splits)
         scratch = scratch_floats(need) if need > 0 else None
         _check(lib.tge_attention_mma(q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(),
                                      block_table.data_ptr(), max_pages, num_pages, page_size, q_start.data_ptr(),
@@ -1272,19 +1271,6 @@ def choose_attention_split(tokens: int, num_seqs: int, max_q_len: int, max_ctx_l
     if want_splits <= 1 and 2 * blocks <= 2 * sms and max_ctx_len >= 4096:
         want_splits = 2
     return keys_per_split(want_splits) if want_splits > 1 else 0
-
-
-def choose_prefix_split(prefix: int, span: int, kv_heads: int) -> int:
-    """Keys per split for the single tokens at the head of a mixed step (0: not cut).
-
-    Such a step's requests hold contexts of all lengths up to ``span``, half of it on average: cut so that there are about
-    three blocks to two SMs, into runs of 256 to 1,536 keys.  Not cut, the longest request's block runs on alone (us a layer, lengths
-    even between 128 and the span, the rule for equal lengths above / this one: 31 requests up to 4,096 at 8 kv heads 79.3 / 74.7, 24
-    up to 2,500 47.1 / 31.9; at 4 kv heads 40 up to 4,096 75.0 / 43.0, 31 up to 1,500 31.1 / 21.9; at 2 kv heads 31 up to
-    1,500 21.8 / 14.5)."""
-    even = -(-prefix * kv_heads * span // (3 * core().tge_device_sm_count()))
-    split = min(max(-(-even // 64) * 64, 256), 1536)
-    return split if span > split else 0
 
 
 def sample(logits: torch.Tensor, temperature: torch.Tensor, uniform: torch.Tensor,

@@ -546,6 +546,25 @@ def test_leading_single_tokens_deep_in_long_contexts_get_splits_of_their_own(ops
     assert ops.choose_attention_split(1509, 10, 1500, 4400, 14, 2, bound=4400) == 0  # whose keys are not cut
 
 
+def test_leading_single_tokens_that_fill_the_chip_are_not_cut(ops, monkeypatch):
+    """A mixed step whose single tokens occupy the SMs as they are: cut, they would cost more states to write and to merge than
+    the parallel runs give back, and with kept first tokens scratch memory for runs of the whole context.  They have the
+    bits of the uncut walk, and the step asks for no scratch memory."""
+    for heads, kv_heads, starts, options in ((28, 4, [900] * 40, {}), (28, 4, [1500 + 3 * i for i in range(38)], dict(window=300, keep_first=64))):
+        q_lens = [1] * len(starts) + [70]
+        k_pages, v_pages, table, _k, _v = paged_cache([s + n for s, n in zip(starts + [0], q_lens)], kv_heads, 128, 64, torch.bfloat16, DEV, seed=5)
+        positions, seq_of_token, q_start, start_pos = batch_index(q_lens, starts + [0], DEV)
+        q = torch.randn(sum(q_lens), heads * 128, generator=torch.Generator().manual_seed(6)).to(torch.bfloat16).to(DEV)
+        run = lambda **kw: ops.attention(q, k_pages, v_pages, table, q_start, start_pos, positions, seq_of_token, len(q_lens), 70,
+                                         max(starts) + 1, heads, kv_heads, 128, 128 ** -0.5, decode_prefix=len(starts), **options, **kw)
+        with monkeypatch.context() as patch:
+            patch.setattr(ops, "_scratch", {})
+            chosen = run()
+            assert not ops._scratch
+        assert torch.equal(chosen, run(split_tokens=1 << 20))
+    ops.check_status()
+
+
 @pytest.mark.parametrize("split,window", [(256, 0), (128, 0), (64, 0), (64, 700)])
 def test_attention_merges_many_splits(ops, split, window):
     """Single tokens deep in a context, their keys cut into 14, 28 and 55 splits: the merging kernel holds up to 16
