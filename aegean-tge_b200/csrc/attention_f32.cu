@@ -450,7 +450,7 @@ TGE_API int tge_attention_f32(const float* q, int q_stride, const float* k_pages
   TGE_REQUIRE(page_size > 0 && max_pages > 0 && num_pages > 0 && window >= 0, "attention: bad page geometry or window");
   const long long need = tge_attention_f32_scratch_floats(tokens, num_seqs, max_q_len, max_ctx_len, heads, kv_heads, head_dim);
   if (need < 0 || (uintptr_t)k_pages % 16 != 0 || (uintptr_t)v_pages % 16 != 0) return TGE_UNSUPPORTED;
-  TGE_REQUIRE(need == 0 || (scratch != nullptr && scratch_floats >= need), "attention: the runs need %lld floats of scratch memory", need);
+  TGE_REQUIRE(scratch == nullptr || scratch_floats >= need, "attention: the runs need %lld floats of scratch memory", need);
   F32AttnParams p;
   p.q = q; p.k_pages = k_pages; p.v_pages = v_pages; p.block_table = block_table; p.q_start = q_start; p.start_pos = start_pos;
   p.positions = positions; p.out = out; p.partial = scratch; p.status = status;
@@ -458,7 +458,8 @@ TGE_API int tge_attention_f32(const float* q, int q_stride, const float* k_pages
   p.page_shift = (page_size & (page_size - 1)) == 0 ? __builtin_ctz((unsigned)page_size) : -1;
   p.num_seqs = num_seqs; p.tokens = tokens; p.heads = heads; p.kv_heads = kv_heads; p.group = heads / kv_heads; p.window = window;
   p.scale = scale;
-  p.runs = runs_of(tokens, num_seqs, max_q_len, max_ctx_len, kv_heads, p.group, head_dim);
+  // without scratch memory every block walks its runs itself, to the same bits
+  p.runs = scratch != nullptr ? runs_of(tokens, num_seqs, max_q_len, max_ctx_len, kv_heads, p.group, head_dim) : 1;
   const bool few = rows_per_thread(p.group, max_q_len) == 1;
   switch (head_dim) {
     case 16: return few ? launch<16, 1>(p, max_q_len, stream) : launch<16, 4>(p, max_q_len, stream);

@@ -379,17 +379,15 @@ def scratch_floats(count: int) -> torch.Tensor:
     return _scratch[index]
 
 
-def scratch_if_any(count: int) -> Optional[torch.Tensor]:
-    """:func:`scratch_floats` for a kernel that another one can stand in for: None where the buffer would have to grow while a graph
-    is captured, or where the device has no room for it."""
-    have = _scratch.get(_current_device())
-    if have is not None and have.numel() >= count:
-        return have
-    if torch.cuda.is_current_stream_capturing():
-        return None
+def call_floats(count: int) -> Optional[torch.Tensor]:
+    """Float32 memory of one call's own, for a kernel that another one (or another way through the same one) can stand in for: None
+    where the device has no room for it.  Calls on several streams or from several threads share nothing.  A capture
+    that meets no room raises instead, as its other buffers do: who captures can give back what the allocator only caches."""
     try:
-        return scratch_floats(count)
+        return torch.empty(count, dtype=torch.float32, device=f"cuda:{_current_device()}")
     except torch.OutOfMemoryError:
+        if torch.cuda.is_current_stream_capturing():
+            raise
         return None
 
 
@@ -720,7 +718,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], epilo
     if x.dtype == torch.float32 and USE_TCGEN05 and not force_simt:
         need = lib.tge_gemm_f32_tcgen05_scratch_floats(w.data_ptr(), ldw, M, N, K)
         if need >= 0:
-            scratch = scratch_if_any(need)
+            scratch = call_floats(need)
             if scratch is not None:
                 rc = lib.tge_gemm_f32_tcgen05(x.data_ptr(), ldx, w.data_ptr(), ldw, _ptr(bias), out.data_ptr(), ldo, M, N, K, epilogue,
                                               scratch.data_ptr(), scratch.numel(), float(alpha), int(act_from),
@@ -1002,15 +1000,14 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
         # plain causal or windowed float32 attention: keys in tiles that a block's rows share
         need = lib.tge_attention_f32_scratch_floats(tokens, num_seqs, max_q_len, max_ctx_len, heads, kv_heads, head_dim)
         if need >= 0:
-            scratch = scratch_if_any(need) if need > 0 else None
-            if need == 0 or scratch is not None:
-                rc = lib.tge_attention_f32(q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
-                                           max_pages, num_pages, page_size, q_start.data_ptr(), start_pos.data_ptr(),
-                                           positions.data_ptr(), num_seqs, max_q_len, max_ctx_len, out.data_ptr(), out_stride,
-                                           tokens, heads, kv_heads, head_dim, float(scale), window, _ptr(scratch), need,
-                                           status_word().data_ptr(), _stream())
-                if _check(rc, lib) != UNSUPPORTED:
-                    return out
+            scratch = call_floats(need) if need > 0 else None
+            rc = lib.tge_attention_f32(q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
+                                       max_pages, num_pages, page_size, q_start.data_ptr(), start_pos.data_ptr(),
+                                       positions.data_ptr(), num_seqs, max_q_len, max_ctx_len, out.data_ptr(), out_stride,
+                                       tokens, heads, kv_heads, head_dim, float(scale), window, _ptr(scratch),
+                                       0 if scratch is None else need, status_word().data_ptr(), _stream())
+            if _check(rc, lib) != UNSUPPORTED:
+                return out
     _check(lib.tge_attention_simt(q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(),
                                   block_table.data_ptr(), max_pages, num_pages, page_size, positions.data_ptr(),
                                   seq_of_token.data_ptr(), out.data_ptr(), out_stride, tokens, heads, kv_heads,

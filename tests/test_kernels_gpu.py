@@ -175,19 +175,60 @@ def test_gemm_float32_on_the_tensor_cores_keeps_what_is_not_finite(ops):
     assert rel_error(out * 1e30, x[6:9].double() @ w[10:].double().T) < 1e-6
 
 
+def test_float32_calls_on_two_streams_share_no_memory(ops, monkeypatch):
+    """Products and attention in float32 keep what passes between their launches in memory of the call: nothing comes out of the
+    device's scratch buffer, and calls on two streams at once have the results they have alone."""
+    gen = torch.Generator().manual_seed(2)
+    w = torch.randn(640, 2048, generator=gen).to(DEV)
+    lengths, heads, kv_heads = [700, 900], 7, 1
+    k_pages, v_pages, table, _k, _v = paged_cache(lengths, kv_heads, 128, 16, torch.float32, DEV, seed=8)
+    positions, seq_of_token, q_start, start_pos = batch_index([1, 1], [n - 1 for n in lengths], DEV)
+    assert ops.core().tge_attention_f32_scratch_floats(2, 2, 1, 900, heads, kv_heads, 128) > 0
+
+    def calls(x, q):
+        return (ops.linear(x, w, None, ops.GEMM_STORE_F32), ops.attention(q, k_pages, v_pages, table, q_start, start_pos, positions, seq_of_token,
+                                                                          2, 1, 900, heads, kv_heads, 128, 0.1))
+    inputs = [(torch.randn(300, 2048, generator=gen).to(DEV), torch.randn(2, heads * 128, generator=gen).to(DEV)) for _ in range(2)]
+    monkeypatch.setattr(ops, "_scratch", {})
+    alone = [calls(*pair) for pair in inputs]
+    assert not ops._scratch
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in inputs]
+    together = [[], []]
+    for _ in range(20):
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                together[i].append(calls(*inputs[i]))
+    torch.cuda.synchronize()
+    for i in range(2):
+        for product, attended in together[i]:
+            assert torch.equal(product, alone[i][0]) and torch.equal(attended, alone[i][1])
+    ops.check_status()
+
+
 def test_gemm_float32_without_room_for_scratch_is_one_chain(ops, monkeypatch):
-    """Where the scratch buffer cannot grow (while a graph is captured) the product runs as the FMA chain, as it always did."""
+    """Where the device has no room for the call's memory the product runs as the FMA chain, as it always did.  A captured
+    product finds it in the graph's pool."""
     gen = torch.Generator().manual_seed(2)
     x, w = torch.randn(5, 600, generator=gen).to(DEV), torch.randn(640, 600, generator=gen).to(DEV)
     chain = ops.linear(x, w, None, ops.GEMM_STORE_F32, force_simt=True)
+    roomy = ops.linear(x, w, None, ops.GEMM_STORE_F32)
     out = torch.zeros(5, 640, device=DEV)
     torch.cuda.synchronize()
-    monkeypatch.setattr(ops, "_scratch", {})
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         ops.linear(x, w, None, ops.GEMM_STORE_F32, out=out)
     graph.replay()
-    assert torch.equal(out, chain)
+    assert torch.equal(out, roomy) and not torch.equal(out, chain)
+    monkeypatch.setattr(ops, "call_floats", lambda count: None)
+    assert torch.equal(ops.linear(x, w, None, ops.GEMM_STORE_F32), chain)
+
+
+def test_attention_float32_without_room_for_scratch_has_the_same_bits(ops, monkeypatch):
+    case = lambda: _attention_case(ops, torch.float32, 7, 1, 128, [1, 1, 3], [1000, 63, 254])[1]
+    roomy = case()
+    monkeypatch.setattr(ops, "call_floats", lambda count: None)
+    assert torch.equal(case(), roomy)
 
 
 TC_SHAPES = [(1, 128, 64), (8, 384, 176), (16, 200, 256), (33, 130, 72), (64, 512, 1024), (100, 300, 512),
