@@ -7,8 +7,8 @@
 // about 1e-33), and of the nine products of two such sums the three of 2^-24 and below are left out; the other six are
 // tensor-core products of 16 times the FMA pipes' rate.  Measured alone (B200), FMA kernel and this one, us:
 //   weights           8 tokens           40 tokens        128 tokens        512 tokens
-//   3,584 x  3,584      218 ->  16        215 ->  20        221 ->  26        524 ->  75
-//   37,888 x 3,584      523 ->  89        528 -> 114      1,048 -> 210      3,912 -> 734  (189 TFLOP/s of float32 work)
+//   3,584 x  3,584      218 ->  17        215 ->  20        221 ->  26        524 ->  75
+//   37,888 x 3,584      523 ->  90        528 -> 114      1,048 -> 210      3,912 -> 734  (189 TFLOP/s of float32 work)
 //   3,584 x 18,944    1,601 ->  52      1,571 ->  59      1,475 ->  89      2,686 -> 334
 //   152,064 x 3,584   2,063 -> 342 (6.4 TB/s of weights)  1 token: 2,065 -> 331
 // With few tokens the weights' bytes bound it; with many, the shared memory that feeds the products.
@@ -115,8 +115,10 @@ __device__ __forceinline__ void finish(const F32GemmParams& p, float v, int m, i
 // ---- the token rows in three parts: planes [3][M][Kp] of bfloat16, zeros behind column K ----
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long long ldx, __nv_bfloat16* __restrict__ planes,
                                                          int M, int K, int Kp, int vec) {
-  pdl_trigger();
+  // Trigger behind the wait: the product then starts once whatever came before this call is done, so its loader may ask for the
+  // weights, and the kernel that adds the cuts for the bias, ahead of their own waits, whoever wrote those.
   pdl_wait();
+  pdl_trigger();
   const int m = blockIdx.y, k = ((int)blockIdx.x * 256 + (int)threadIdx.x) * 8;
   if (k >= Kp) return;
   const float* src = x + (size_t)m * ldx + k;
@@ -175,7 +177,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const __gr
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
   pdl_trigger();                               // tensor memory is held: the next kernel's blocks can at worst wait for it
-  if (warp != 0) pdl_wait();                   // weights are nobody's result: their loader goes ahead
+  if (warp != 0) pdl_wait();                   // the weights are there (see split_rows_kernel): their loader goes ahead
 
   const int units = p.tiles_w * p.tiles_t * p.splits;
   // unit -> cut along k, token tile, weight tile (the cuts of a tile and the token tiles of a weight tile side by side)
@@ -393,6 +395,7 @@ __global__ void __launch_bounds__(256) gemm_f32_combine_kernel(const F32GemmPara
   const int m = blockIdx.y, n = 2 * ((int)blockIdx.x * 256 + (int)threadIdx.x);
   if (n >= p.N) return;
   const bool second = n + 1 < p.N;
+  // the bias is there already (see split_rows_kernel)
   const float bias0 = p.bias ? p.bias[n] : 0.0f, bias1 = p.bias && second ? p.bias[n + 1] : 0.0f;
   pdl_wait();
   const float* src = p.partial + (size_t)m * p.N + n;

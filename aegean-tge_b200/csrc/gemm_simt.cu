@@ -150,10 +150,10 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const T* __restrict__ x,
 // The tile above waits for its loads in each of K / 16 rounds and has 64 x 64 elements whatever M is: a tiny model's product
 // of 3 rows took 8.4 us at K = 64 and 20 us at K = 384, nearly all of it round trips to L2.  Here a block owns 16 x 32 elements
 // (a lane per weight row, a warp per four tokens), so a product spreads over four times the SMs and more, and
-// four blocks of 64 k are on their way at once by cp.async, the weights' (nobody's result) before the wait for
-// the kernel in front.  Measured (B200), the tile above and this kernel, us, at 4 tokens:
-// 128 x 64 6.3 -> 2.3, 512 x 96 8.5 -> 2.8, 64 x 176 12.9 -> 3.8, 96 x 256 17.8 -> 4.9, 500 x 3,000 181 -> 47; 300 tokens
-// of 384 x 96 8.5 -> 4.3 and of 500 x 3,000 180 -> 101.
+// four blocks of 64 k are on their way at once by cp.async.  Measured (B200), the tile above and this kernel, us, at 4 tokens:
+// 128 x 64 6.3 -> 2.3, 512 x 96 8.5 -> 2.8, 64 x 176 12.9 -> 3.8, 96 x 256 17.8 -> 5.0, 500 x 3,000 181 -> 48; 512 tokens
+// of 384 x 96 4.9 and of 500 x 3,000 104.  (Weights asked for ahead of the wait for the kernel in front were 0.2 to 0.4 us faster, and
+// wrong where that kernel had written them.)
 constexpr int SKINNY_M = 16, SKINNY_N = 32, SKINNY_K = 64, SKINNY_PITCH = SKINNY_K + 4, SKINNY_STAGES = 4;
 constexpr int SKINNY_STAGE = (SKINNY_M + SKINNY_N) * SKINNY_PITCH;
 
@@ -191,14 +191,14 @@ __global__ void __launch_bounds__(128) gemm_skinny_kernel(const float* __restric
   };
   auto commit = [] { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
   const int n = n0 + lane;
+  pdl_wait();                                           // weights and bias may be the kernel in front's result as well
   const float add = bias != nullptr && n < N ? bias[n] : 0.0f;
 #pragma unroll
-  for (int kb = 0; kb < SKINNY_STAGES - 1; ++kb)
-    if (kb < blocks) fetch_w(kb);
-  pdl_wait();
-#pragma unroll
-  for (int kb = 0; kb < SKINNY_STAGES - 1; ++kb) {      // the weights above land with the first group
-    if (kb < blocks) fetch_x(kb);
+  for (int kb = 0; kb < SKINNY_STAGES - 1; ++kb) {
+    if (kb < blocks) {
+      fetch_w(kb);
+      fetch_x(kb);
+    }
     commit();
   }
   float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};

@@ -175,6 +175,33 @@ def test_gemm_float32_on_the_tensor_cores_keeps_what_is_not_finite(ops):
     assert rel_error(out * 1e30, x[6:9].double() @ w[10:].double().T) < 1e-6
 
 
+@pytest.mark.parametrize("N,K,M", [(640, 1024, 8), (2304, 512, 600), (96, 256, 4)])
+def test_gemm_float32_weights_and_bias_may_be_the_last_kernels_result(ops, N, K, M):
+    """Weights and bias that the kernels just before have written (here by products themselves, long ones, into memory that held
+    others) are read after they are there, on the tensor cores (cut along k and whole) and by the kernel for few tokens."""
+    gen = torch.Generator().manual_seed(N)
+    x = torch.randn(M, K, generator=gen).to(DEV)
+    a, b = torch.randn(12, N, 900, generator=gen).to(DEV), torch.randn(K, 900, generator=gen).to(DEV)
+    ones = torch.randn(12, N, 3000, generator=gen).to(DEV)
+    w, bias = torch.zeros(N, K, device=DEV), torch.zeros(N, device=DEV)
+    got, want = [], []
+    for i in range(12):
+        ops.linear(a[i], b, None, ops.GEMM_STORE_F32, out=w)
+        ops.linear(ones[i, :1], ones[i], None, ops.GEMM_STORE_F32, out=bias.view(1, N))
+        got.append(ops.linear(x, w, bias, ops.GEMM_STORE_F32))
+    for i in range(12):
+        ops.linear(a[i], b, None, ops.GEMM_STORE_F32, out=w)
+        torch.cuda.synchronize()
+        got.append(ops.linear(x, w, None, ops.GEMM_STORE_F32))          # ... the weights alone
+        ops.linear(a[i], b, None, ops.GEMM_STORE_F32, out=w)
+        want.append(ops.linear(x, w, None, ops.GEMM_STORE_F32))
+        ops.linear(ones[i, :1], ones[i], None, ops.GEMM_STORE_F32, out=bias.view(1, N))
+        torch.cuda.synchronize()
+        assert torch.equal(got[i], ops.linear(x, w, bias, ops.GEMM_STORE_F32))
+    assert all(torch.equal(g, h) for g, h in zip(got[12:], want))
+    ops.check_status()
+
+
 def test_float32_calls_on_two_streams_share_no_memory(ops, monkeypatch):
     """Products and attention in float32 keep what passes between their launches in memory of the call: nothing comes out of the
     device's scratch buffer, and calls on two streams at once have the results they have alone."""
