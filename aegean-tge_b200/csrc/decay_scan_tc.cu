@@ -35,7 +35,7 @@ struct ScanTcParams {
   float* carry;              // [chunks][heads][dim][vdim]
   float* out;                // [tokens][heads * vdim]
   int* status;
-  int v_off, heads, num_seqs, activation, aligned;
+  int v_off, heads, num_seqs, shortest, activation, aligned;
 };
 
 __device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t block_stride) {
@@ -46,17 +46,28 @@ __device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t block_stride
 __device__ __forceinline__ bool odd_number(float v) { return !(fabsf(v) <= 3.38e38f); }
 __device__ __forceinline__ float silu_of(float z) { return z / (1.0f + expf(-z)); }
 
-// Which tokens block `piece` works on: chunks are counted over all requests of the step.
+// Which tokens block `piece` works on: chunks are counted over the step's portions of p.shortest tokens and more, 32 requests
+// at a time, one to a lane (one after the other, every block of a step of many requests waited for that many loads).
 __device__ __forceinline__ bool find_chunk(const ScanTcParams& p, int piece, int& first, int& count) {
-  for (int s = 0; s < p.num_seqs; ++s) {
-    const int begin = p.q_start[s], length = p.q_start[s + 1] - begin;
-    const int pieces = (length + CHUNK - 1) / CHUNK;
-    if (piece < pieces) {
-      first = begin + piece * CHUNK;
-      count = min(CHUNK, length - piece * CHUNK);
+  const int lane = threadIdx.x & 31;
+  for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
+    const int s = s0 + lane;
+    const int begin = s < p.num_seqs ? p.q_start[s] : 0, length = s < p.num_seqs ? p.q_start[s + 1] - begin : 0;
+    const int mine = length >= p.shortest ? (length + CHUNK - 1) / CHUNK : 0;
+    int upto = mine;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+      const int other = __shfl_up_sync(0xffffffffu, upto, offset);
+      if (lane >= offset) upto += other;
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, piece < upto);
+    if (hit != 0) {
+      const int at = __ffs(hit) - 1, place = (piece - __shfl_sync(0xffffffffu, upto - mine, at)) * CHUNK;
+      first = __shfl_sync(0xffffffffu, begin, at) + place;
+      count = min(CHUNK, __shfl_sync(0xffffffffu, length, at) - place);
       return true;
     }
-    piece -= pieces;
+    piece -= __shfl_sync(0xffffffffu, upto, 31);
   }
   return false;
 }
@@ -452,13 +463,14 @@ int run(const ScanTcParams& p, int pieces, bool readout, cudaStream_t stream) {
 // Tokens per chunk, or 0: key and value sizes the kernels are not built for.
 int decay_tc_chunk(int dim, int vdim) { return (dim == 64 || dim == 128) && (vdim == 64 || vdim == 128) ? CHUNK : 0; }
 
-// One of the two launches around decay_segment_carry_kernel; `pieces` is an upper bound of the chunks.  Returns 1 or an error.
+// One of the two launches around decay_segment_carry_kernel, for portions of `shortest` tokens and more; `pieces` is an upper bound of
+// their chunks.  Returns 1 or an error.
 int launch_decay_tc(const void* rows, long long ld, const float* prepared, int v_off, int heads, int dim, int vdim, int activation,
-                    const float* decay, const int* q_start, float* carry, float* out, int num_seqs, int pieces, bool readout, int* status,
-                    cudaStream_t stream) {
+                    const float* decay, const int* q_start, float* carry, float* out, int num_seqs, int shortest, int pieces, bool readout,
+                    int* status, cudaStream_t stream) {
   ScanTcParams p;
   p.rows = (const __nv_bfloat16*)rows; p.ld = ld; p.prepared = prepared; p.decay = decay; p.q_start = q_start; p.carry = carry; p.out = out;
-  p.status = status; p.v_off = v_off; p.heads = heads; p.num_seqs = num_seqs; p.activation = activation;
+  p.status = status; p.v_off = v_off; p.heads = heads; p.num_seqs = num_seqs; p.shortest = shortest; p.activation = activation;
   p.aligned = ((uintptr_t)(p.rows + v_off) % 16 == 0) && (ld * 2) % 16 == 0;
   if (dim == 64) return vdim == 64 ? run<64, 64>(p, pieces, readout, stream) : run<64, 128>(p, pieces, readout, stream);
   return vdim == 64 ? run<128, 64>(p, pieces, readout, stream) : run<128, 128>(p, pieces, readout, stream);

@@ -24,8 +24,8 @@
 // decay_scan_tc.cu
 int decay_tc_chunk(int dim, int vdim);
 int launch_decay_tc(const void* rows, long long ld, const float* prepared, int v_off, int heads, int dim, int vdim, int activation,
-                    const float* decay, const int* q_start, float* carry, float* out, int num_seqs, int pieces, bool readout, int* status,
-                    cudaStream_t stream);
+                    const float* decay, const int* q_start, float* carry, float* out, int num_seqs, int shortest, int pieces, bool readout,
+                    int* status, cudaStream_t stream);
 
 namespace {
 
@@ -491,6 +491,7 @@ __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_grou
 // state, from zero, into `carry[segment]`), `decay_segment_carry_kernel` (per request, in order: carry[k] <- the
 // state the segment starts from, state <- c^len state + contribution; the last one goes to the slot), MODE 2 (a
 // block per segment: the readout, from carry[segment]).  blockIdx.z counts segments over all requests of the step.
+// In MODE 0 `segment` > 0 leaves portions of that many tokens and more to the kernels of decay_scan_tc.cu.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(256) decay_scan_wide_kernel(
     const T* __restrict__ rows, long long ld, const float* __restrict__ prepared, int v_off, int heads, int dim, int vdim,
@@ -513,6 +514,7 @@ __global__ void __launch_bounds__(256) decay_scan_wide_kernel(
     seq = blockIdx.z;
     first = q_start[seq];
     last = q_start[seq + 1];
+    if (segment > 0 && last - first >= segment) return;
   } else {
     int z = blockIdx.z;
     for (int s = 0; s < num_seqs; ++s) {
@@ -706,18 +708,41 @@ __global__ void __launch_bounds__(256) decay_scan_wide_kernel(
 
 // Between the two segment launches: every request's segments in order.  carry[k] holds segment k's own contribution
 // on the way in and the state it starts from on the way out; the request's slot gets the state after its last one.
+// Portions below `shortest` tokens have no segments; blockIdx.z counts the others (with a grid over all requests, blocks that only
+// left took 85 us of a step of 64 single tokens beside a prompt).  They are counted 32 requests at a time, one to a lane.
 __global__ void decay_segment_carry_kernel(float* __restrict__ carry, float* __restrict__ state, const float* __restrict__ decay,
-                                           const int* __restrict__ slots, const int* __restrict__ q_start, int heads,
-                                           int dim, int vdim, int segment) {
-  const int seq = blockIdx.z, head = blockIdx.y;
+                                           const int* __restrict__ slots, const int* __restrict__ q_start, int num_seqs, int heads,
+                                           int dim, int vdim, int segment, int shortest) {
+  const int head = blockIdx.y;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   const int cells = dim * vdim;
   __shared__ float power_of[2];            // c^segment and c^(length of the last segment): float64, so by two threads of a block only
   pdl_trigger();
-  int before = 0;
-  for (int s = 0; s < seq; ++s) before += (q_start[s + 1] - q_start[s] + segment - 1) / segment;
-  const int count = q_start[seq + 1] - q_start[seq];
-  if (count <= 0) return;
+  int seq = -1, before = 0, count = 0;
+  for (int s0 = 0, z = blockIdx.z; s0 < num_seqs; s0 += 32) {
+    const int lane = threadIdx.x & 31, s = s0 + lane;
+    const int length = s < num_seqs ? q_start[s + 1] - q_start[s] : 0;
+    const bool cut = s < num_seqs && length >= shortest;
+    int upto = cut ? (length + segment - 1) / segment : 0;
+    const int mine = upto;
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+      const int other = __shfl_up_sync(0xffffffffu, upto, offset);
+      if (lane >= offset) upto += other;
+    }
+    const unsigned cuts = __ballot_sync(0xffffffffu, cut);
+    const unsigned hit = __ballot_sync(0xffffffffu, cut && __popc(cuts & ((1u << lane) - 1)) == z);
+    if (hit != 0) {
+      const int at = __ffs(hit) - 1;
+      seq = s0 + at;
+      before += __shfl_sync(0xffffffffu, upto - mine, at);
+      count = __shfl_sync(0xffffffffu, length, at);
+      break;
+    }
+    z -= __popc(cuts);
+    before += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  if (seq < 0) return;
   const int pieces = (count + segment - 1) / segment;
   if (threadIdx.x < 2)
     power_of[threadIdx.x] = (float)pow((double)decay[head], (double)(threadIdx.x == 0 ? segment : count - (pieces - 1) * segment));
@@ -1044,15 +1069,27 @@ __global__ void __launch_bounds__(128) pool_kv_kernel(
   }
 }
 
-// Tokens per segment where a step's portions are shared out over blocks of their own (0: they are not): chunks of 128
-// on the tensor cores for bfloat16 and the sizes decay_scan_tc.cu is built for from one whole chunk on; else segments of 256
-// on the FMA pipes from two on.
-int segment_tokens(bool is_bf16, int dim, int vdim, int max_q_len) {
+// How a step's portions are shared out over blocks of their own: segments of `tokens` (0: they are not), for portions of
+// `shortest` tokens and more, of which there are at most `portions` with `states` segments in all.
+struct Segments {
+  int tokens, shortest, portions;
+  long long states;
+};
+// Portions below this many tokens stay on the FMA pipes, one block each from end to end: chunks of 128 on the tensor cores gain from
+// their second on, and the states between them cost a trip to memory (us a layer, 28 heads of 128, FMA pipes / tensor cores: one
+// portion of 256 102 / 46, ten of 200 421 / 296, sixteen of 128 428 / 510, 128 beside 16 single tokens 164 / 195).
+constexpr int TC_PORTION = 160;
+Segments segments_of(bool is_bf16, int dim, int vdim, int max_q_len, int tokens, int num_seqs) {
   static const bool chunks_ok = getenv("TGE_NO_CHUNKED_SCAN") == nullptr || getenv("TGE_NO_CHUNKED_SCAN")[0] == '\0';
-  if (!chunks_ok) return 0;
-  const int chunk = is_bf16 ? decay_tc_chunk(dim, vdim) : 0;
-  if (chunk > 0 && max_q_len >= chunk) return chunk;
-  return max_q_len >= 2 * SEGMENT && dim <= 128 && dim % 4 == 0 ? SEGMENT : 0;
+  const int chunk = chunks_ok && is_bf16 ? decay_tc_chunk(dim, vdim) : 0;
+  if (chunk > 0 && max_q_len >= TC_PORTION) {
+    // a request alone goes there whatever its length is (max_q_len may be a bound)
+    if (num_seqs == 1) return {chunk, 1, 1, (tokens + chunk - 1) / chunk};
+    const int most = tokens / TC_PORTION < num_seqs ? tokens / TC_PORTION : num_seqs;      // portions that long
+    return {chunk, TC_PORTION, most, tokens / chunk + most};
+  }
+  if (chunks_ok && max_q_len >= 2 * SEGMENT && dim <= 128 && dim % 4 == 0) return {SEGMENT, 1, num_seqs, (long long)tokens / SEGMENT + num_seqs};
+  return {0, 0, 0, 0};
 }
 
 template <typename T>
@@ -1084,29 +1121,34 @@ int launch_decay_scan(const void* rows, long long ld, int q_off, int k_off, int 
     dim3 wide_grid((vdim + WIDE - 1) / WIDE, heads, num_seqs);
     launch_decay_prepare((const T*)rows, ld, q_off, k_off, heads, dim, activation, cos_table, sin_table, table_positions, rotary, k_scale,
                          positions, prepared, tokens, status, stream);
-    const int segment = carry != nullptr ? segment_tokens(sizeof(T) == 2, dim, vdim, max_q_len) : 0;
-    if (segment > 0 && segment != SEGMENT && tokens / segment + num_seqs <= 65535) {
-      const int pieces = tokens / segment + num_seqs;
-      int rc = launch_decay_tc(rows, ld, prepared, v_off, heads, dim, vdim, activation, decay, q_start, carry, out, num_seqs, pieces, false,
-                               status, stream);
+    const Segments cut = carry != nullptr ? segments_of(sizeof(T) == 2, dim, vdim, max_q_len, tokens, num_seqs) : Segments{0, 0, 0, 0};
+    const int pieces = cut.states <= 65535 ? (int)cut.states : 0;        // an upper bound; blocks beyond the last segment leave at once
+    const dim3 carry_grid((dim * vdim + 255) / 256, heads, cut.portions);
+    if (pieces > 0 && cut.tokens != SEGMENT) {
+      // long portions in chunks on the tensor cores, the single tokens and short portions beside them as in any other step
+      if (num_seqs > 1)
+        decay_scan_wide_kernel<T, 0><<<wide_grid, 256, wide, stream>>>((const T*)rows, ld, prepared, v_off, heads, dim, vdim, activation,
+                                                                       decay, state, slots, q_start, out, nullptr, num_seqs, cut.shortest);
+      int rc = launch_decay_tc(rows, ld, prepared, v_off, heads, dim, vdim, activation, decay, q_start, carry, out, num_seqs, cut.shortest,
+                               pieces, false, status, stream);
       if (rc < 0) return rc;
-      tge_launch(decay_segment_carry_kernel, dim3((dim * vdim + 255) / 256, heads, num_seqs), dim3(256), 0, stream, carry, state, decay, slots,
-                 q_start, heads, dim, vdim, segment);
-      rc = launch_decay_tc(rows, ld, prepared, v_off, heads, dim, vdim, activation, decay, q_start, carry, out, num_seqs, pieces, true,
-                           status, stream);
+      tge_launch(decay_segment_carry_kernel, carry_grid, dim3(256), 0, stream, carry, state, decay, slots, q_start, num_seqs, heads, dim,
+                 vdim, cut.tokens, cut.shortest);
+      rc = launch_decay_tc(rows, ld, prepared, v_off, heads, dim, vdim, activation, decay, q_start, carry, out, num_seqs, cut.shortest, pieces,
+                           true, status, stream);
       if (rc < 0) return rc;
-      return tge_launched("decay_scan_tc", 4);
+      return tge_launched("decay_scan_tc", num_seqs > 1 ? 5 : 4);
     }
     // few blocks and long portions: segments, so that the whole device works on one prompt
     const long long blocks = (long long)wide_grid.x * heads * num_seqs;
-    if (segment == SEGMENT && blocks < 2LL * tge_sm_count() && tokens / SEGMENT + num_seqs <= 65535) {
-      dim3 pieces(wide_grid.x, heads, tokens / SEGMENT + num_seqs);      // an upper bound; blocks beyond the last segment leave at once
-      decay_scan_wide_kernel<T, 1><<<pieces, 256, wide, stream>>>((const T*)rows, ld, prepared, v_off, heads, dim, vdim, activation,
-                                                                  decay, state, slots, q_start, out, carry, num_seqs, SEGMENT);
-      tge_launch(decay_segment_carry_kernel, dim3((dim * vdim + 255) / 256, heads, num_seqs), dim3(256), 0, stream, carry, state, decay, slots,
-                 q_start, heads, dim, vdim, (int)SEGMENT);
-      decay_scan_wide_kernel<T, 2><<<pieces, 256, wide, stream>>>((const T*)rows, ld, prepared, v_off, heads, dim, vdim, activation,
-                                                                  decay, state, slots, q_start, out, carry, num_seqs, SEGMENT);
+    if (pieces > 0 && blocks < 2LL * tge_sm_count()) {
+      const dim3 segment_grid(wide_grid.x, heads, pieces);
+      decay_scan_wide_kernel<T, 1><<<segment_grid, 256, wide, stream>>>((const T*)rows, ld, prepared, v_off, heads, dim, vdim, activation,
+                                                                        decay, state, slots, q_start, out, carry, num_seqs, SEGMENT);
+      tge_launch(decay_segment_carry_kernel, carry_grid, dim3(256), 0, stream, carry, state, decay, slots, q_start, num_seqs, heads, dim,
+                 vdim, (int)SEGMENT, 1);
+      decay_scan_wide_kernel<T, 2><<<segment_grid, 256, wide, stream>>>((const T*)rows, ld, prepared, v_off, heads, dim, vdim, activation,
+                                                                        decay, state, slots, q_start, out, carry, num_seqs, SEGMENT);
       return tge_launched("decay_scan_segments", 4);
     }
     decay_scan_wide_kernel<T, 0><<<wide_grid, 256, wide, stream>>>((const T*)rows, ld, prepared, v_off, heads, dim, vdim,
@@ -1188,9 +1230,10 @@ TGE_API int tge_scale_add_norm(float* x, const float* y, long long ldy, const fl
   return tge_launched("scale_add_norm", 1);
 }
 
-// Tokens of a segment in steps whose longest portion is max_q_len, 0: no segments.  With them `carry` holds a state for each of
-// tokens / segment + num_seqs.
-TGE_API int tge_decay_scan_segment(int is_bf16, int dim, int vdim, int max_q_len) { return segment_tokens(is_bf16 != 0, dim, vdim, max_q_len); }
+// States that `carry` holds in a step of `tokens` tokens of num_seqs requests whose longest portion is max_q_len, 0: it has no use for any.
+TGE_API long long tge_decay_scan_carry_states(int is_bf16, int dim, int vdim, int max_q_len, int tokens, int num_seqs) {
+  return segments_of(is_bf16 != 0, dim, vdim, max_q_len, tokens, num_seqs).states;
+}
 
 TGE_API int tge_decay_scan(const void* rows, int is_bf16, long long ld, int q_off, int k_off, int v_off, int heads,
                            int dim, int vdim, int activation, const float* cos_table, const float* sin_table,

@@ -160,7 +160,8 @@ def core() -> ctypes.CDLL:
         _declare(lib, "tge_to_run_dtype", [_c_ptr, _c_ptr, _c_int, _c_ll, _c_ptr])
         _declare(lib, "tge_scale_add_norm", [_c_ptr, _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_float,
                                              _c_float, _c_ptr])
-        _declare(lib, "tge_decay_scan_segment", [_c_int] * 4)
+        lib.tge_decay_scan_carry_states.argtypes = [_c_int] * 6
+        lib.tge_decay_scan_carry_states.restype = _c_ll
         _declare(lib, "tge_decay_scan", [_c_ptr, _c_int, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                          _c_ptr, _c_ptr, _c_int, _c_int, _c_float, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr,
                                          _c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_ptr])
@@ -1087,9 +1088,9 @@ def decay_scan(rows: torch.Tensor, q_off: int, k_off: int, v_off: int, heads: in
                 if longest >= 16 and dim <= 256 else None)
     lib = core()
     # long portions are shared out over many blocks in segments of 128 or 256 tokens: a state per segment in between
-    segment = lib.tge_decay_scan_segment(int(rows.dtype == torch.bfloat16), dim, vdim, longest) if prepared is not None else 0
-    carry = (torch.empty((tokens // segment + num_seqs, heads, dim, vdim), dtype=torch.float32, device=rows.device)
-             if segment > 0 else None)
+    states = (lib.tge_decay_scan_carry_states(int(rows.dtype == torch.bfloat16), dim, vdim, longest, tokens, num_seqs)
+              if prepared is not None else 0)
+    carry = call_floats(states * heads * dim * vdim) if states > 0 else None
     _check(lib.tge_decay_scan(rows.data_ptr(), int(rows.dtype == torch.bfloat16), ld, q_off, k_off, v_off, heads, dim,
                               vdim, int(activation), _ptr(cos) if rotary else None, _ptr(sin) if rotary else None,
                               table_positions, rotary, float(k_scale), decay.data_ptr(), state.data_ptr(),

@@ -272,6 +272,42 @@ def test_decayed_state_in_portions_and_batches(ops, dtype, heads, dim, vdim, rot
         assert rel_error(torch.cat(got[s]), torch.from_numpy(ref)) < 3e-5        # float32 arithmetic in both formats
 
 
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (64, 64)])
+@pytest.mark.parametrize("step", [[1] * 37 + [300], [160], [1, 159, 160, 161, 3, 512, 2], [1] * 70 + [700, 130], [200] * 5])
+def test_short_portions_beside_a_long_one_go_as_they_go_without_it(ops, dim, vdim, step):
+    """A portion's route is by its own length: single tokens and short portions keep their bits whether or not a prompt is in the
+    step, long ones theirs whatever is beside them, and the states between chunks take memory for the long ones only."""
+    heads = 3
+    gen = torch.Generator().manual_seed(dim + len(step))
+    rows = (torch.randn(sum(step), 3 * heads * 128, generator=gen) * 0.7).to(torch.bfloat16).to(DEV)
+    decay = torch.tensor([0.9, 0.99, 1.0], device=DEV)
+    start = torch.randn(len(step), heads, dim, vdim, generator=gen).to(DEV)
+
+    def run(chosen, bound):
+        cuts = [step[s] for s in chosen]
+        positions, _seq, q_start = _steps(cuts)
+        state = start.clone()
+        begin = [sum(step[:s]) for s in chosen]
+        part = torch.cat([rows[b:b + n] for b, n in zip(begin, cuts)])
+        out = ops.decay_scan(part, 0, heads * 128, 2 * heads * 128, heads, dim, vdim, decay, state, _i32(chosen), q_start, positions,
+                             len(cuts), max_q_len=bound)
+        return [out[sum(cuts[:i]):sum(cuts[:i + 1])] for i in range(len(cuts))], state
+    every = list(range(len(step)))
+    whole, state = run(every, max(step))
+    for s in every:
+        if step[s] >= 160:
+            alone, after = run([s], step[s])
+            assert torch.equal(alone[0], whole[s]) and torch.equal(after[s], state[s])
+    short = [s for s in every if step[s] < 160]
+    if short:
+        alone, after = run(short, 159)
+        for s, out in zip(short, alone):
+            assert torch.equal(out, whole[s]) and torch.equal(after[s], state[s])
+    states = ops.core().tge_decay_scan_carry_states(1, dim, vdim, max(step), sum(step), len(step))
+    assert sum(-(-n // 128) for n in step if n >= 160) <= states <= 2 * (sum(step) // 128) + 1
+    ops.check_status()
+
+
 def test_a_lost_state_would_show(ops):
     """With a decay of 1 the first token's key and value stay in every later readout: zeroing the state between two
     portions changes the second portion's rows by far more than the tolerance."""
