@@ -11,8 +11,9 @@
 //   1. decay_chunk_state_kernel: a chunk's own contribution to the state, sum_j c^(n-1-j) k_j v_j^T, into carry[chunk];
 //   2. decay_segment_carry_kernel of sequence_mix.cu: carry[chunk] <- the state the chunk starts from, the last state to its slot;
 //   3. decay_chunk_readout_kernel: o = c^(t+1) q S0 + (c^(t-j) q k^T below the diagonal) v.
-// A chunk that meets a number which is not finite (or too large for its high part) is computed by the formulas themselves instead: the
-// split would make infinity - infinity of it, and zeros above the diagonal times infinity would reach earlier tokens.
+// A number that is not finite, or too large for its high part, makes NaN of every product it meets: as an input its split is
+// infinity - infinity, zeros above the diagonal times infinity reach earlier tokens, and so does a score that overflows.  A chunk one of
+// whose results is not finite is therefore computed by the formulas themselves.
 // First operands lie in tensor memory (a lane per token or state row), second operands in shared memory, split on their way in.
 // Measured (B200, 2,048 tokens, 28 heads of 128): states 150 -> 57 us, readout 337 -> 91 us; 14 heads of 64 with activated values of
 // 128: 108 -> 33 us and 137 -> 45 us.  Error against float64 2.85e-7 -> 1.7e-7, activated 1.97e-7 -> 1.44e-7.
@@ -42,8 +43,14 @@ __device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t block_stride
   return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(block_stride >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// neither splits into parts nor multiplies with zero as a number should
-__device__ __forceinline__ bool odd_number(float v) { return !(fabsf(v) <= 3.38e38f); }
+// NaN from the first infinity or NaN on, else zero
+template <int N>
+__device__ __forceinline__ float not_finite(const float v[N]) {
+  float poison = 0.0f;
+#pragma unroll
+  for (int i = 0; i < N; ++i) poison = fmaf(v[i], 0.0f, poison);
+  return poison;
+}
 __device__ __forceinline__ float silu_of(float z) { return z / (1.0f + expf(-z)); }
 
 // Which tokens block `piece` works on: chunks are counted over the step's portions of p.shortest tokens and more, 32 requests
@@ -91,8 +98,7 @@ __device__ __forceinline__ void store_parts(unsigned char* base, int block, int 
 // The chunk's values [token][column] as a second operand whose contiguous direction is the column: blocks of 64 columns, a row of
 // 128 bytes per token.  Plain values are bfloat16 (one part), activated ones float32 (three).
 template <int VDIM>
-__device__ __forceinline__ bool load_values(const ScanTcParams& p, unsigned char* base, int first, int count, int head, int tid) {
-  bool odd = false;
+__device__ __forceinline__ void load_values(const ScanTcParams& p, unsigned char* base, int first, int count, int head, int tid) {
 #pragma unroll 4
   for (int e = tid; e < CHUNK * VDIM / 8; e += THREADS) {
     const int t = e / (VDIM / 8), c = (e % (VDIM / 8)) * 8;
@@ -117,11 +123,8 @@ __device__ __forceinline__ bool load_values(const ScanTcParams& p, unsigned char
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = silu_of(v[i]);
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) odd = odd || odd_number(v[i]);
     store_parts(base, c >> 6, CHUNK, t, (c & 63) >> 3, v, p.activation ? 3 : 1);
   }
-  return odd;
 }
 
 // One value as the products take it.
@@ -254,7 +257,6 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_state_kernel(const Sca
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t a = s.tmem + ACC_COLS;
   const int half = warp >> 2, row = (warp & 3) * 32 + lane;
-  bool odd = false;
   // first operand: k_j[row] c^(n-1-j), this warp's 64 of the 128 tokens
 #pragma unroll
   for (int t0 = half * 64; t0 < half * 64 + 64; t0 += 32) {
@@ -265,13 +267,10 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_state_kernel(const Sca
       v[i] = row < DIM && t < count ? p.prepared[((size_t)(first + t) * p.heads + head) * 2 * DIM + DIM + row] : 0.0f;
     }
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      odd = odd || odd_number(v[i]);
-      v[i] *= powers[max(count - 1 - (t0 + i), 0)];
-    }
+    for (int i = 0; i < 32; ++i) v[i] *= powers[max(count - 1 - (t0 + i), 0)];
     store_lane32(a + lane_base + t0 / 2, CHUNK / 2, v);
   }
-  odd = load_values<VDIM>(p, s.generic, first, count, head, tid) || odd;
+  load_values<VDIM>(p, s.generic, first, count, head, tid);
   operands_ready();
   if (warp == 0) {
     if (elect_one()) {
@@ -285,7 +284,7 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_state_kernel(const Sca
   float* dst = p.carry + (((size_t)piece * p.heads + head) * DIM + row) * VDIM + half * (VDIM / 2);
   float sums[VDIM / 2];
   read_sums<VDIM / 2, 2>(s.tmem + lane_base + half * (VDIM / 2), 128, sums);
-  if (__syncthreads_or(odd)) {
+  if (__syncthreads_or(!(not_finite<VDIM / 2>(sums) == 0.0f))) {
     for (int c = 0; c < VDIM / 2 && row < DIM; ++c) {
       float sum = 0.0f;
       for (int j = 0; j < count; ++j)
@@ -320,7 +319,6 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
   unsigned char* second = s.generic;                          // the state, then the keys
   unsigned char* values = s.generic + 3 * OPERAND_BYTES;
   const float* own = p.prepared + ((size_t)(first + min(row, count - 1)) * p.heads + head) * 2 * DIM + half * (DIM / 2);
-  bool odd = false;
   // the token's query, this warp's half of it
 #pragma unroll
   for (int i0 = 0; i0 < DIM / 2; i0 += 32) {
@@ -330,8 +328,6 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
       const float4 q = row < count ? *reinterpret_cast<const float4*>(own + i0 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
       v[i] = q.x; v[i + 1] = q.y; v[i + 2] = q.z; v[i + 3] = q.w;
     }
-#pragma unroll
-    for (int i = 0; i < 32; ++i) odd = odd || odd_number(v[i]);
     store_lane32(a + lane_base + (half * (DIM / 2) + i0) / 2, DIM / 2, v);
   }
   // the state the chunk starts from, [dim][vdim]: contiguous along vdim
@@ -341,8 +337,6 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
     const int i = e / (VDIM / 8), c = (e % (VDIM / 8)) * 8;
     const float4 x = *reinterpret_cast<const float4*>(state + (size_t)i * VDIM + c), y = *reinterpret_cast<const float4*>(state + (size_t)i * VDIM + c + 4);
     const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-#pragma unroll
-    for (int k = 0; k < 8; ++k) odd = odd || odd_number(v[k]);
     store_parts(second, c >> 6, DIM, i, (c & 63) >> 3, v, 3);
   }
   operands_ready();
@@ -353,7 +347,7 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
     }
     __syncwarp();
   }
-  odd = load_values<VDIM>(p, values, first, count, head, tid) || odd;      // while the products run
+  load_values<VDIM>(p, values, first, count, head, tid);      // while the products run
   bool ok = mbar_wait(bar, 0, p.status, &abort_word);
   tc_fence_after();
   float o[VDIM / 2];
@@ -373,8 +367,6 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
       const float4 x = *reinterpret_cast<const float4*>(src), y = *reinterpret_cast<const float4*>(src + 4);
       v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
     }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) odd = odd || odd_number(v[k]);
     store_parts(second, i >> 6, CHUNK, t, (i & 63) >> 3, v, 3);
   }
   operands_ready();
@@ -410,11 +402,17 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
   }
   ok = mbar_wait(bar, 0, p.status, &abort_word) && ok;
   tc_fence_after();
+#pragma unroll
+  for (int c = 0; c < VDIM / 2; c += 16) {
+    float more[16];
+    read_sums<16, 2>(s.tmem + lane_base + half * (VDIM / 2) + c, 128, more);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) o[c + j] += more[j];
+  }
   float* dst = p.out + (size_t)(first + row) * p.heads * VDIM + (size_t)head * VDIM + half * (VDIM / 2);
-  const bool by_formula = __syncthreads_or(odd);
-  if (by_formula && row < count) {
+  if (__syncthreads_or(!(not_finite<VDIM / 2>(o) == 0.0f))) {
     const float* q = p.prepared + ((size_t)(first + row) * p.heads + head) * 2 * DIM;
-    for (int c = 0; c < VDIM / 2; ++c) {
+    for (int c = 0; c < VDIM / 2 && row < count; ++c) {
       float sum = 0.0f;
       for (int i = 0; i < DIM; ++i) sum = fmaf(q[i], state[(size_t)i * VDIM + half * (VDIM / 2) + c], sum);
       sum *= powers[row + 1];
@@ -426,17 +424,9 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
       }
       dst[c] = sum;
     }
-  }
+  } else if (ok && row < count) {
 #pragma unroll
-  for (int c = 0; c < VDIM / 2; c += 16) {
-    float more[16];
-    read_sums<16, 2>(s.tmem + lane_base + half * (VDIM / 2) + c, 128, more);
-    if (ok && row < count && !by_formula) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) more[j] += o[c + j];
-      store8(dst + c, more);
-      store8(dst + c + 8, more + 8);
-    }
+    for (int c = 0; c < VDIM / 2; c += 8) store8(dst + c, o + c);
   }
   tear_down(s.tmem, warp);
 }

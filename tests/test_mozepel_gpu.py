@@ -8,6 +8,7 @@ option, cut and batched in every way, both number formats.
 """
 import copy
 import json
+import math
 import os
 import random
 
@@ -305,6 +306,86 @@ def test_short_portions_beside_a_long_one_go_as_they_go_without_it(ops, dim, vdi
             assert torch.equal(out, whole[s]) and torch.equal(after[s], state[s])
     states = ops.core().tge_decay_scan_carry_states(1, dim, vdim, max(step), sum(step), len(step))
     assert sum(-(-n // 128) for n in step if n >= 160) <= states <= 2 * (sum(step) // 128) + 1
+    ops.check_status()
+
+
+@pytest.mark.parametrize("dim,vdim,activation", [(128, 128, False), (64, 64, False), (64, 128, True)])
+def test_chunks_that_meet_numbers_which_are_not_finite(ops, dim, vdim, activation):
+    """Infinities, NaN and numbers near the type's largest, given or arising inside a chunk: they reach what the formulas let them
+    reach and nothing else, and an overflow is an infinity of the right sign.  300 tokens in three chunks, the odd number in the second."""
+    heads, tokens, at, head, i0 = 2, 300, 170, 1, 5
+    gen = torch.Generator().manual_seed(dim + vdim)
+    q0, k0, v0 = 0, heads * dim, 2 * heads * dim
+    clean = (torch.randn(tokens, 2 * heads * dim + heads * vdim, generator=gen) * 0.5).to(torch.bfloat16)
+    decay = [1.0, 0.97]
+    begin = torch.randn(1, heads, dim, vdim, generator=gen)
+
+    def run(rows, state):
+        state = state.clone().to(DEV)
+        positions, _seq, q_start = _steps([tokens])
+        out = ops.decay_scan(rows.to(DEV), q0, k0, v0, heads, dim, vdim, torch.tensor(decay, device=DEV), state, _i32([0]), q_start,
+                             positions, 1, activation=activation, max_q_len=tokens)
+        return out.double().cpu().view(tokens, heads, vdim), state.double().cpu()
+
+    def reference(rows, state):
+        x = rows.double().numpy()
+        take = lambda first, size: x[:, first:first + heads * size].reshape(tokens, heads, size)
+        q, k, v = take(q0, dim), take(k0, dim), take(v0, vdim)
+        if activation:
+            q, k, v = plain.silu(q), plain.silu(k), plain.silu(v)
+        s, out = state[0].double().numpy().copy(), []
+        for t in range(tokens):
+            s = s * np.array(decay)[:, None, None] + k[t][:, :, None] * v[t][:, None, :]
+            out.append(np.einsum("hdv,hd->hv", s, q[t]))
+        return torch.from_numpy(np.stack(out))
+    close = lambda got, ref: bool(torch.isfinite(got).all()) and float((got - ref).norm() / ref.norm()) < 3e-5
+    want = reference(clean, begin)
+    got, _ = run(clean, begin)
+    assert close(got, want)
+    other = 1 - head
+
+    # a value: its column of its head from its token on
+    for number in (math.inf, math.nan):
+        rows = clean.clone()
+        rows[at, v0 + head * vdim + 3] = number
+        got, state = run(rows, begin)
+        hit = torch.zeros(vdim, dtype=torch.bool)
+        hit[3] = True
+        assert close(got[:at], want[:at]) and close(got[:, other], want[:, other]) and close(got[at:, head][:, ~hit], want[at:, head][:, ~hit])
+        assert not torch.isfinite(got[at:, head, 3]).any() and not torch.isfinite(state[0, head, :, 3]).any()
+    # a query: its token's row; a key: its head's rows from its token on
+    rows = clean.clone()
+    rows[at, q0 + head * dim + i0] = math.inf
+    got, state = run(rows, begin)
+    keep = torch.arange(tokens) != at
+    assert close(got[keep], want[keep]) and close(got[:, other], want[:, other])
+    assert not torch.isfinite(got[at, head]).any() and bool(torch.isfinite(state).all())
+    rows = clean.clone()
+    rows[at, k0 + head * dim + i0] = math.nan
+    got, _ = run(rows, begin)
+    assert close(got[:at], want[:at]) and close(got[:, other], want[:, other]) and not torch.isfinite(got[at:, head]).any()
+    # the state the portion starts from
+    odd = begin.clone()
+    odd[0, head, i0, 3] = math.inf
+    got, _ = run(clean, odd)
+    assert close(got[:, head, 4:], want[:, head, 4:]) and close(got[:, other], want[:, other]) and not torch.isfinite(got[:, head, 3]).any()
+    # a score beyond float32's range, of finite numbers: infinite with its value's sign, in its row alone
+    rows = clean.clone()
+    rows[at, k0 + head * dim + i0] = 2e19
+    rows[at + 30, q0 + head * dim + i0] = 2e20
+    ref = reference(rows, begin)
+    got, _ = run(rows, begin)
+    v = rows[at, v0 + head * vdim:v0 + (head + 1) * vdim].double()
+    assert torch.isinf(got[at + 30, head]).all() and torch.equal(torch.sign(got[at + 30, head]), torch.sign(v))
+    keep = torch.arange(tokens) != at + 30
+    assert close(got[keep], ref[keep]) and close(got[at + 30, other], ref[at + 30, other])
+    # a value near the largest number, behind small keys: everything stays finite
+    rows = clean.clone()
+    rows[at, v0 + head * vdim + 3] = 3.3e38
+    rows[at, k0 + head * dim:k0 + (head + 1) * dim] *= 1e-3
+    ref = reference(rows, begin)
+    got, _ = run(rows, begin)
+    assert float(ref.abs().max()) < 1e38 and close(got[:, head, 3], ref[:, head, 3]) and close(got[:, head, 4:], ref[:, head, 4:])
     ops.check_status()
 
 
