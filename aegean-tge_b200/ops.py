@@ -374,9 +374,10 @@ def scratch_floats(count: int) -> torch.Tensor:
             raise KernelError("scratch memory must be sized before a CUDA graph is captured "
                               f"(need {count} floats, have {0 if have is None else have.numel()})")
         size = max(count, 1 << 22, 0 if have is None else 2 * have.numel())
-        if have is not None:
+        grown = torch.empty(size, dtype=torch.float32, device=f"cuda:{index}")
+        if have is not None:       # only now: an allocation that fails leaves everything as it was
             _outgrown.setdefault(index, []).append(have)
-        _scratch[index] = torch.empty(size, dtype=torch.float32, device=f"cuda:{index}")
+        _scratch[index] = grown
     return _scratch[index]
 
 

@@ -258,6 +258,23 @@ def test_attention_float32_without_room_for_scratch_has_the_same_bits(ops, monke
     assert torch.equal(case(), roomy)
 
 
+def test_scratch_memory_that_cannot_grow_stays_as_it_was(ops, monkeypatch):
+    """A buffer too large for the device raises, time and again, without filing the one in use among the outgrown."""
+    def no_room(*_args, **_kw):
+        raise torch.OutOfMemoryError("no room")
+    monkeypatch.setattr(ops, "_scratch", {})
+    monkeypatch.setattr(ops, "_outgrown", {})
+    held = ops.scratch_floats(10)
+    with monkeypatch.context() as patch:
+        patch.setattr(torch, "empty", no_room)
+        for _ in range(3):
+            with pytest.raises(torch.OutOfMemoryError):
+                ops.scratch_floats(held.numel() + 1)
+        assert ops.scratch_floats(held.numel()) is held and not ops._outgrown
+    grown = ops.scratch_floats(held.numel() + 1)
+    assert grown.numel() >= 2 * held.numel() and [t is held for kept in ops._outgrown.values() for t in kept] == [True]
+
+
 TC_SHAPES = [(1, 128, 64), (8, 384, 176), (16, 200, 256), (33, 130, 72), (64, 512, 1024), (100, 300, 512),
              (200, 640, 320), (300, 1024, 512), (520, 256, 192)]
 
