@@ -1559,14 +1559,21 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
       // the tcgen05 kernels: 128 rows per query tile as well
       static const bool one_tile = getenv("TGE_ATTENTION_ONE_TILE") != nullptr && getenv("TGE_ATTENTION_ONE_TILE")[0] != '\0';
       // Two query tiles to a block share K and V and one SM; where blocks are few or short, one tile to a block has the SMs'
-      // tensor cores to itself and less to set up.  The line, measured at 28 heads over 4 of 128 (two tiles / one, us): keys of
-      // up to 256 in any number (16 prompts of 120: 31.2 / 26.5); blocks for no more than the SMs and up to 1,024 keys (1,024
-      // tokens: 30.5 / 28.5; 1,500: 39.5 / 40.9); for half of them and up to 4,096 (512 after 1,024: 37.4 / 34.8; 512 after
-      // 6,144: 117 / 120); for a quarter (200 after 6,144: 73.3 / 68.9).  40 heads over 8 and 12 over 2 lie the same way.
-      const long long pair_blocks = (long long)(((tokens - first_token + p.bq - 1) / p.bq + 1) / 2 + num_seqs) * kv_heads * num_splits;
+      // tensor cores to itself and less to set up.  The lines, measured at 28 heads over 4, 40 over 8, 12 over 2, 32 over 8, 16 over 16
+      // of 128 and 14 over 2 of 64 (two tiles / one, us).  Up to 320 keys, any number of blocks: unless the single tiles take twice
+      // the waves (28/4: 16 x 64 13.4 / 14.0, 20 x 64 24.5 / 20.8; 12/2: 64 x 32 16.9 / 20.3, 12 x 100 13.6 / 10.3, 8 x 300 17.4 / 19.7;
+      // 40/8: 6 x 128 14.8 / 16.9, 32 x 64 51.4 / 41.7), or tiles are whole ones of a head's queries (16/16: 8 x 200 19.1 / 17.0);
+      // what still loses: 40/8 64 x 32, seven waves for four, 61.8 / 64.6.  More
+      // keys: blocks for no more than the SMs and up to 1,024 (28/4: 1,024 tokens 30.5 / 27.8; 1,500 38.8 / 40.2; 12/2: 3 x 512 20.9 / 17.0), for half of
+      // them and up to 4,096 (512 after 1,024: 36.8 / 34.3; 40/8: 512 after 3,000 70.4 / 75.4), for a quarter (12/2: 200 after 6,144 40.1 / 40.1).
       const int sms = tge_sm_count();
-      const bool few = max_ctx_len <= 256 || (pair_blocks <= sms && max_ctx_len <= 1024) || (2 * pair_blocks <= sms && max_ctx_len <= 4096) ||
-                       4 * pair_blocks <= sms;
+      const long long portions = num_seqs > first_token ? num_seqs - first_token : 1;          // the single tokens at the head: one each
+      const long long own_tiles = ((tokens - first_token + portions - 1) / portions + p.bq - 1) / p.bq;      // of a portion, were all alike
+      auto waves = [&](long long blocks) { return (blocks * portions * kv_heads * num_splits + sms - 1) / sms; };
+      const long long pair_blocks = (long long)(((tokens - first_token + p.bq - 1) / p.bq + 1) / 2 + num_seqs) * kv_heads * num_splits;
+      const bool few = max_ctx_len <= 320 ? group == 1 || waves(own_tiles) < 2 * waves((own_tiles + 1) / 2)
+                                          : (pair_blocks <= sms && max_ctx_len <= 1024) || (2 * pair_blocks <= sms && max_ctx_len <= 4096) ||
+                                                4 * pair_blocks <= sms;
       if (tc2::FITS && !one_tile && !few && tc2::smem_bytes(range >> p.page_shift) <= 227 * 1024) {
         // two query tiles per block, one block per SM
         const size_t smem2 = tc2::smem_bytes(range >> p.page_shift);

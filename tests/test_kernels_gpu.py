@@ -617,6 +617,14 @@ def test_attention_prefill_on_both_sides_of_the_two_tile_rule(ops, heads, kv_hea
     assert err < TOL[torch.bfloat16]
 
 
+@pytest.mark.parametrize("heads,kv_heads,head_dim,count,length", [
+    (12, 2, 128, 32, 64), (12, 2, 128, 8, 300), (28, 4, 128, 20, 64), (40, 8, 128, 6, 128), (4, 4, 128, 40, 200), (14, 2, 64, 40, 17)])
+def test_attention_of_short_prompts_on_both_sides_of_the_rule_for_waves(ops, heads, kv_heads, head_dim, count, length):
+    """Many short prompts: one query tile to a block unless that takes twice the waves of two, the last prompt longer than the rest."""
+    err, _, _ = _attention_case(ops, torch.bfloat16, heads, kv_heads, head_dim, [length] * (count - 1) + [length + 9], [0] * count, page_size=64)
+    assert err < TOL[torch.bfloat16]
+
+
 def test_leading_single_tokens_deep_in_long_contexts_get_splits_of_their_own(ops):
     """A mixed step: nine single tokens at contexts of about 4,000 beside a prompt of 300 tokens.  The prompt's
     keys are not cut; the single tokens, a decode batch of their own, have theirs cut (the choice is automatic
