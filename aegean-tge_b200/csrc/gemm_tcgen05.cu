@@ -873,9 +873,12 @@ bool choose_pair(int M, int N, int K, long long scratch_floats, const Plan& sing
   // From about a thousand tokens on the pair does better than these figures say (every SM fetches half as many
   // token rows, which counts once the operands no longer sit in L2: o at 4,096 tokens 78 us against 92, down 375
   // against 420, where the figures put the SM alone ahead by a few per cent), so it is given 15 % there.
-  // From 256 on the same counts for 5 % (320 tokens, gate and up 76 against 71 us, down 48.7 against 45.6; 512, down 66 against 63).
+  // From 256 on the same counts for 5 % where the weights are 13 M numbers and more (one SM / pair, us: 37,888 x 3,584 at 320 tokens 76 / 71;
+  // 3,584 x 18,944 at 320 48.7 / 45.6; 7,168 x 5,120 at 448 32.3 / 31.6; 1,536 x 8,960 at 448 17.9 / 17.0, at 960 28.2 / 26.8).  Below, setting up a
+  // pair costs more than its loads save (1,536 x 1,536 at 320 11.3 / 12.3; 2,048 x 2,048 at 448 13.1 / 13.8; 8,192 x 1,536 at 448 15.2 / 15.8).
+  constexpr long long PAIR_WEIGHTS = 13000000;
   if (M >= 1024) single_cost += single_cost * 15 / 100;
-  else if (M >= 256) single_cost += single_cost * 5 / 100;
+  else if (M >= 256 && (long long)N * K >= PAIR_WEIGHTS) single_cost += single_cost * 5 / 100;
   return g_pair_mode == 2 || pair_cost <= single_cost;
 }
 
