@@ -17,8 +17,10 @@
 // lives longer than one k-block of 64, is filled from the smallest products to the largest (l h, h l, m m, m h, h m, h h), and is
 // added into registers with rounding to nearest: the error against float64 is a tenth of one FMA chain's along k
 // (relative, random numbers: 1.1e-7 against 1.07e-6 at K = 3,584, 1.7e-7 against 2.5e-6 at 18,944).
-// Numbers that are not finite, or products beyond float32's range, do not survive the split (infinity - infinity): an
-// output that is not finite is computed again as one FMA chain along k, so it is what that chain makes of it.
+// Numbers that are not finite, or products beyond float32's range, do not survive the split (infinity - infinity), and below about
+// 1e-33 the low parts run out of exponents: an output that is not finite, or below 2^-100 without being zero, is computed
+// again as one FMA chain along k, so it is what that chain makes of it.  (A part lost below 2^-133 is worth 2^-134 of the other side's
+// number: against an output of 2^-100 nothing.  What remains is an output that the chain makes of numbers below 2^-134 alone: zero here.)
 //
 // An output element depends on its own row of x and of w only: the k-blocks' order, the cut along k (a rule on N and K) and
 // the order in which the cuts are added do not depend on how many tokens there are or on the tile a token falls in.
@@ -61,7 +63,7 @@ struct Shape {
 };
 
 struct F32GemmParams {
-  const float* x;       // for outputs that are not finite
+  const float* x;       // for outputs outside the usual range
   const float* w;
   long long ldx, ldw;
   int M, N, K;
@@ -86,8 +88,9 @@ __device__ __noinline__ float fma_chain(const float* x, const float* w, int K) {
   for (int k = 0; k < K; ++k) acc = fmaf(x[k], w[k], acc);
   return acc;
 }
-__device__ __forceinline__ float finite_or_chain(const F32GemmParams& p, float v, int m, int n) {
-  return fabsf(v) <= 3.402823466e38f ? v : fma_chain(p.x + (size_t)m * p.ldx, p.w + (size_t)n * p.ldw, p.K);
+__device__ __forceinline__ float usual_or_chain(const F32GemmParams& p, float v, int m, int n) {
+  const float size = fabsf(v);
+  return (size <= 3.402823466e38f && size >= 7.8886090522e-31f) || size == 0.0f ? v : fma_chain(p.x + (size_t)m * p.ldx, p.w + (size_t)n * p.ldw, p.K);
 }
 
 __device__ __forceinline__ float gated(const F32GemmParams& p, float g, float u) {
@@ -370,7 +373,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const __gr
       for (int c = 0; c < COLS; ++c) {
         const int m = m0 + c;
         if (m >= p.M) continue;                // uniform over the warp
-        const float v = (n_ok ? finite_or_chain(p, sum[c], m, n) : 0.0f) + bias;
+        const float v = (n_ok ? usual_or_chain(p, sum[c], m, n) : 0.0f) + bias;
         if (is_gated) {
           const float up = __shfl_down_sync(0xffffffffu, v, 1);      // N is even: an even row's partner exists
           if (n_ok && !(lane & 1)) p.out[(size_t)m * p.ldo + (n >> 1)] = gated(p, v, up);
@@ -418,8 +421,8 @@ __global__ void __launch_bounds__(256) gemm_f32_combine_kernel(const F32GemmPara
       b += v[i].y;
     }
   }
-  a = finite_or_chain(p, a, m, n) + bias0;
-  if (second) b = finite_or_chain(p, b, m, n + 1) + bias1;
+  a = usual_or_chain(p, a, m, n) + bias0;
+  if (second) b = usual_or_chain(p, b, m, n + 1) + bias1;
   if (p.epilogue == F32_SWIGLU || p.epilogue == F32_GLU_CLAMPED) {
     p.out[(size_t)m * p.ldo + (n >> 1)] = gated(p, a, b);
     return;

@@ -202,6 +202,24 @@ def test_gemm_float32_weights_and_bias_may_be_the_last_kernels_result(ops, N, K,
     ops.check_status()
 
 
+@pytest.mark.parametrize("N,K", [(700, 600), (4736, 2048)])
+def test_gemm_float32_on_the_tensor_cores_keeps_tiny_numbers(ops, N, K):
+    """Rows around and below 1e-33, where three bfloat16 parts no longer hold a float32 number: no more error than one FMA chain's
+    (cut along k and whole), and the rows beside them as they are without them.  Zeros stay zeros."""
+    gen = torch.Generator().manual_seed(N)
+    x, w = torch.randn(12, K, generator=gen).to(DEV), torch.randn(N, K, generator=gen).to(DEV)
+    plain = ops.linear(x, w, None, ops.GEMM_STORE_F32)
+    for row, scale in ((1, 1e-28), (3, 1e-31), (5, 1e-33), (7, 1e-35), (9, 3e-38), (11, 0.0)):
+        x[row] *= scale
+    out, chain = (ops.linear(x, w, None, ops.GEMM_STORE_F32, force_simt=simt) for simt in (False, True))
+    ref = x.double() @ w.double().T
+    assert torch.equal(out[0::2], plain[0::2]) and not out[11].any()
+    for row in (1, 3, 5, 7, 9):
+        error = lambda got: float((got[row].double() - ref[row]).norm() / ref[row].norm())
+        assert error(out) <= 1.05 * error(chain), row
+    ops.check_status()
+
+
 def test_float32_calls_on_two_streams_share_no_memory(ops, monkeypatch):
     """Products and attention in float32 keep what passes between their launches in memory of the call: nothing comes out of the
     device's scratch buffer, and calls on two streams at once have the results they have alone."""
