@@ -4,17 +4,17 @@
 // butterfly over the warp and two exponentials, about 1.4 us a key and nothing to hide it behind, and
 // every head of a group fetches the keys for itself.  Bound by that chain, not by bytes: a step of 8 requests of 1,000
 // tokens at 28 heads over 4 of 128 took 1,403 us a layer, against 5 us for its 33 MB of keys and values.  Here
-//   * a block owns up to 16 or 64 rows, (query, head of the group) pairs of one request and kv head, and 64 keys at a time
+//   * a block owns up to 16, 32 or 64 rows, (query, head of the group) pairs of one request and kv head, and 64 keys at a time
 //     lie in shared memory for all of them, the next 64 under way (cp.async, two buffers);
 //   * 16 x 16 threads hold the scores as a matrix product does (rows by 4 keys each, paired float32 FMAs over the head),
 //     so a tile costs one round of maxima, exponentials and sums, not 64;
 //   * where the rows are few the keys are cut into runs, each a block of its own, merged by a second kernel.
 // Measured in place (B200, float32): that step 1,403 -> 25 us a layer, 512 prompt tokens 639 -> 122 us; 100 prompt tokens at 12
-// heads over 2 of 128 56 -> 25 us alone, three single tokens at 4 heads of 16 18 -> 3 us; 7 prompt tokens at 28 heads, one short tile,
-// went from 6 to 9 us (a block's copies and barriers cost more there than they save).
+// heads over 2 of 128 56 -> 15 us alone, three single tokens at 4 heads of 16 18 -> 3 us, 7 prompt tokens at 28 heads 5.8 -> 4.9; one to three
+// tokens at a request's very beginning lose (28 heads: one 2.3 -> 3.3, three 3.7 -> 4.6: a block's copies and barriers cost more there than they save).
 //
 // A row's result depends only on its own keys, not on the batch, on how its request was cut into portions or on which of
-// the two row counts serves it: keys go in tiles of 64 and runs of RUN_KEYS that start at multiples of these positions, a
+// the three row counts serves it: keys go in tiles of 64 and runs of RUN_KEYS that start at multiples of these positions, a
 // tile that a row does not see changes nothing of its state, every sum over keys or numbers of a head has one order, and
 // the runs are merged in order by the same code inside a block and in the merging kernel.
 #include "common.cuh"
@@ -390,15 +390,22 @@ int row_blocks(int tokens, int num_seqs, int max_q_len, int bq) {
   return (int)(((long long)tokens + (long long)num_seqs * (bq - 1)) / bq);
 }
 
-// Sixteen rows where a request brings no more (and the group fits), 64 otherwise: a block of 64 rows with 14 in use
-// computes the other 50 all the same (single tokens bring group rows each).
-int rows_per_thread(int group, int max_q_len) { return group * (long long)max_q_len <= 16 ? 1 : MAX_ROWS_PER_THREAD; }
+// Sixteen rows to a block where a request brings no more (single tokens bring group rows each), thirty-two where it brings no more or where
+// blocks of that many still find an SM each, 64 otherwise: a block computes all its rows, in use or not, and while SMs are idle
+// smaller blocks finish sooner (us, 64 / 32 rows, 28 heads over 4 of 128: three prompt tokens 6.6 / 4.6,
+// seven 7.5 / 4.9, forty 11.5 / 8.1, a hundred 20.7 / 15.0; sixteen at 3,000 find no room: 47 / 66).
+int rows_per_thread(int tokens, int num_seqs, int max_q_len, int max_ctx_len, int kv_heads, int group) {
+  const long long rows = group * (long long)max_q_len, runs = (max_ctx_len + RUN_KEYS - 1) / RUN_KEYS;
+  if (rows <= 16) return 1;
+  if (rows <= 32 || (group <= 32 && row_blocks(tokens, num_seqs, max_q_len, 32 / group) * kv_heads * runs <= tge_sm_count())) return 2;
+  return MAX_ROWS_PER_THREAD;
+}
 
 // Runs that are blocks of their own, 1: none.  Only where the row blocks alone leave the chip half empty, and where the
 // states stay within 64 MB: a long portion deep in a long context has keys enough for every block.
 constexpr long long MAX_STATE_FLOATS = 16 << 20;
 int runs_of(int tokens, int num_seqs, int max_q_len, int max_ctx_len, int kv_heads, int group, int head_dim) {
-  const int bq = 16 * rows_per_thread(group, max_q_len) / group;
+  const int bq = 16 * rows_per_thread(tokens, num_seqs, max_q_len, max_ctx_len, kv_heads, group) / group;
   const long long blocks = (long long)row_blocks(tokens, num_seqs, max_q_len, bq) * kv_heads;
   const int runs = (max_ctx_len + RUN_KEYS - 1) / RUN_KEYS;
   const bool fits = (long long)runs * tokens * kv_heads * group * (head_dim + 2) <= MAX_STATE_FLOATS;
@@ -421,6 +428,12 @@ int launch(const F32AttnParams& p, int max_q_len, cudaStream_t stream) {
     return -2;
   }
   return tge_launched("attention_f32", p.runs > 1 ? 2 : 1);
+}
+
+template <int HD>
+int launch_rows(const F32AttnParams& p, int max_q_len, int max_ctx_len, cudaStream_t stream) {
+  const int rows = rows_per_thread(p.tokens, p.num_seqs, max_q_len, max_ctx_len, p.kv_heads, p.group);
+  return rows == 1 ? launch<HD, 1>(p, max_q_len, stream) : rows == 2 ? launch<HD, 2>(p, max_q_len, stream) : launch<HD, MAX_ROWS_PER_THREAD>(p, max_q_len, stream);
 }
 
 bool f32_attention_takes(int heads, int kv_heads, int head_dim) {
@@ -460,11 +473,10 @@ TGE_API int tge_attention_f32(const float* q, int q_stride, const float* k_pages
   p.scale = scale;
   // without scratch memory every block walks its runs itself, to the same bits
   p.runs = scratch != nullptr ? runs_of(tokens, num_seqs, max_q_len, max_ctx_len, kv_heads, p.group, head_dim) : 1;
-  const bool few = rows_per_thread(p.group, max_q_len) == 1;
   switch (head_dim) {
-    case 16: return few ? launch<16, 1>(p, max_q_len, stream) : launch<16, 4>(p, max_q_len, stream);
-    case 32: return few ? launch<32, 1>(p, max_q_len, stream) : launch<32, 4>(p, max_q_len, stream);
-    case 64: return few ? launch<64, 1>(p, max_q_len, stream) : launch<64, 4>(p, max_q_len, stream);
-    default: return few ? launch<128, 1>(p, max_q_len, stream) : launch<128, 4>(p, max_q_len, stream);
+    case 16: return launch_rows<16>(p, max_q_len, max_ctx_len, stream);
+    case 32: return launch_rows<32>(p, max_q_len, max_ctx_len, stream);
+    case 64: return launch_rows<64>(p, max_q_len, max_ctx_len, stream);
+    default: return launch_rows<128>(p, max_q_len, max_ctx_len, stream);
   }
 }

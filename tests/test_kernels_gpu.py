@@ -626,6 +626,29 @@ def test_attention_float32_rows_do_not_depend_on_the_step(ops, heads, kv_heads, 
     ops.check_status()
 
 
+@pytest.mark.parametrize("group,counts", [(1, (16, 17, 32, 33, 64, 65)), (7, (2, 3, 4, 5, 9)), (16, (1, 2, 3)), (17, (1, 2)), (32, (1, 2)), (33, (1, 2)), (64, (1, 2))])
+def test_attention_float32_rows_have_the_bits_of_any_block(ops, group, counts):
+    """Portions around the lines between 16, 32 and 64 rows to a block, alone (blocks find an SM each) and repeated in a step of many
+    requests (they do not), against the whole prompt in one step."""
+    length, head_dim = 330, 64
+    k_pages, v_pages, table, _k, _v = paged_cache([length], 2, head_dim, 16, torch.float32, DEV, seed=3)
+    q = torch.randn(length, 2 * group * head_dim, generator=torch.Generator().manual_seed(4)).to(DEV)
+
+    def rows(starts, count):
+        positions, seq_of_token, q_start, start_pos = batch_index([count] * len(starts), starts, DEV)
+        return ops.attention(torch.cat([q[s:s + count] for s in starts]), k_pages, v_pages, table.expand(len(starts), -1).contiguous(), q_start,
+                             start_pos, positions, seq_of_token, len(starts), count, length, 2 * group, 2, head_dim, 0.1)
+    whole = rows([0], length)
+    for count in counts:
+        starts = [0, 63, 255, length - count] * 50
+        alone, many = rows(starts[:1], count), rows(starts, count)
+        assert torch.equal(alone, whole[:count])
+        for i, s in enumerate(starts[:4]):
+            assert torch.equal(many[i * count:(i + 1) * count], whole[s:s + count]), (count, s)
+        assert torch.equal(many.view(50, -1), many.view(50, -1)[:1].expand(50, -1))
+    ops.check_status()
+
+
 @pytest.mark.parametrize("heads,kv_heads,head_dim,page_size,window,q_lens,starts", [
     (28, 4, 128, 16, 0, [1500, 37, 1], [0, 300, 70]), (40, 8, 64, 64, 200, [1030, 260], [15, 0]), (16, 8, 32, 16, 0, [900, 333, 300], [1, 64, 0]),
     (28, 4, 128, 16, 0, [1024], [0]), (28, 4, 128, 64, 0, [250], [5]), (28, 4, 128, 16, 0, [300], [4100]), (12, 2, 128, 64, 0, [130] * 9, [0] * 9)])
