@@ -701,12 +701,22 @@ def test_leading_single_tokens_that_fill_the_chip_are_not_cut(ops, monkeypatch):
 
 @pytest.mark.parametrize("split,window", [(256, 0), (128, 0), (64, 0), (64, 700)])
 def test_attention_merges_many_splits(ops, split, window):
-    """Single tokens deep in a context, their keys cut into 14, 28 and 55 splits: the merging kernel holds up to 16
-    or 48 split states in registers and walks more than that in a loop; with a window most splits hold no
+    """Single tokens deep in a context, their keys cut into 14, 28 and 55 splits: the merging kernel hands round the splits'
+    weights lane by lane, up to four to a lane, and asks for sixteen states at a time; with a window most splits hold no
     visible key.  One far key is made to dominate, so a split dropped or counted twice would show."""
     err, _, _ = _attention_case(ops, torch.bfloat16, 14, 2, 128, [1, 1, 1], [3499, 1200, 65], window=window, split=split,
                                 spike=(0, 3000 if window else 17))
     assert err < TOL[torch.bfloat16]
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,start,window", [
+    (7, 1, 128, 8191, 0), (7, 1, 128, 8192, 0), (4, 1, 64, 9100, 0), (2, 1, 32, 12000, 0), (7, 1, 128, 9000, 8300)])
+def test_attention_merges_more_splits_than_a_warp_holds(ops, heads, kv_heads, head_dim, start, window):
+    """Keys in splits of 64: 128 of them, the most whose weights a warp holds, and more, which are walked one by one; far keys
+    at both ends of the walk dominate in turn."""
+    for spike in ((0, 5 if not window else start - window + 3), (0, start - 1)):
+        err, _, _ = _attention_case(ops, torch.bfloat16, heads, kv_heads, head_dim, [1, 1], [start, 70], window=window, split=64, spike=spike)
+        assert err < TOL[torch.bfloat16]
 
 
 @pytest.mark.parametrize("heads,kv_heads,head_dim", [(7, 1, 128), (28, 4, 64), (6, 2, 48), (40, 2, 16)])

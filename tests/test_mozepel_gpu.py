@@ -389,6 +389,45 @@ def test_chunks_that_meet_numbers_which_are_not_finite(ops, dim, vdim, activatio
     ops.check_status()
 
 
+@pytest.mark.parametrize("heads,dim,vdim,rotary,activation,k_scale", [
+    (9, 128, 128, 128, False, 128 ** -0.5), (3, 64, 64, 32, True, 1.0), (2, 128, 64, 64, True, 0.5), (5, 64, 128, 0, False, 0.125),
+    (5, 20, 24, 12, False, 0.25), (1, 200, 72, 100, True, 0.5)])
+@pytest.mark.parametrize("cuts", [[17], [300, 1, 40, 161], [128], [129], [640, 255]])
+def test_decayed_state_of_rows_that_wide_accesses_can_read(ops, heads, dim, vdim, rotary, activation, k_scale, cuts):
+    """Even offsets and strides: q and k two numbers at a time, values eight at a time; chunks whole, of one token and ragged,
+    on the tensor cores and beside them, from states that are not zero."""
+    from aegean_tge_b200.parts.rope import rotary_tables
+    gen = torch.Generator().manual_seed(heads * 1000 + dim + len(cuts))
+    decay = [1.0 - 0.5 ** (2 + h) for h in range(heads)]
+    tokens, positions_from = sum(cuts), [11 * s for s in range(len(cuts))]
+    rows = (torch.randn(tokens, 2 * heads * dim + heads * vdim, generator=gen) * 0.7).to(torch.bfloat16)
+    cos, sin = rotary_tables(300.0, max(rotary, 2), 2048, None, precise=True)
+    begin = torch.randn(len(cuts), heads, dim, vdim, generator=gen)
+    state = begin.clone().to(DEV)
+    positions, _seq, q_start = _steps(cuts, positions_from)
+    out = ops.decay_scan(rows.to(DEV), 0, heads * dim, 2 * heads * dim, heads, dim, vdim, torch.tensor(decay, dtype=torch.float32, device=DEV),
+                         state, _i32(list(range(len(cuts)))), q_start, positions, len(cuts), activation=activation, cos=cos.to(DEV),
+                         sin=sin.to(DEV), rotary=rotary, k_scale=k_scale, max_q_len=max(cuts)).double().cpu()
+    ops.check_status()
+    freq, first = plain.frequencies(max(rotary, 2), 300.0), 0
+    for s, n in enumerate(cuts):
+        x = rows[first:first + n].double().numpy()
+        q, k = x[:, :heads * dim].reshape(n, heads, dim), x[:, heads * dim:2 * heads * dim].reshape(n, heads, dim)
+        v = x[:, 2 * heads * dim:].reshape(n, heads, vdim)
+        if activation:
+            q, k, v = plain.silu(q), plain.silu(k), plain.silu(v)
+        if rotary:
+            at = positions_from[s] + np.arange(n)
+            q, k = plain.rotate(q, at, rotary, freq), plain.rotate(k, at, rotary, freq)
+        held, ref = begin[s].double().numpy().copy(), []
+        for t in range(n):
+            held = held * np.array(decay)[:, None, None] + k_scale * k[t][:, :, None] * v[t][:, None, :]
+            ref.append(np.einsum("hdv,hd->hv", held, q[t]).reshape(-1))
+        assert rel_error(out[first:first + n], torch.from_numpy(np.stack(ref))) < 3e-5        # float32 arithmetic
+        assert rel_error(state[s], torch.from_numpy(held)) < 3e-5
+        first += n
+
+
 def test_a_lost_state_would_show(ops):
     """With a decay of 1 the first token's key and value stay in every later readout: zeroing the state between two
     portions changes the second portion's rows by far more than the tolerance."""
@@ -427,6 +466,38 @@ def test_gated_norm(ops, dtype, groups, size, weighted, sigmoid):
     gate = wide[:, 9:].double().numpy()
     ref = normed * (plain.sigmoid(gate) if sigmoid else plain.silu(gate))
     assert got.dtype == dtype and rel_error(got, torch.from_numpy(ref)) < KERNEL_TOL[dtype]
+
+
+@pytest.mark.parametrize("groups,size,weighted,gate_first,sigmoid", [
+    (1, 4, True, False, False), (28, 128, True, False, False), (3, 508, True, True, False), (5, 512, False, False, True),
+    (2, 516, True, False, False), (1, 1792, True, False, True), (1, 4096, True, True, False), (1, 4100, True, False, False)])
+def test_gated_norm_of_rows_that_four_number_accesses_can_read(ops, groups, size, weighted, gate_first, sigmoid):
+    """A warp to a group up to 512 numbers, a block up to 4,096 (the kernel for any rows beyond), at the edges of both, the last group's
+    block not full; and each against the kernel for any rows, which odd strides go to, on the same numbers."""
+    gen = torch.Generator().manual_seed(groups + size)
+    tokens, eps, n = 37, 1e-5, groups * size
+    o = torch.randn(tokens, n, generator=gen) * 3.0
+    gate = torch.randn(tokens, n + 8, generator=gen).to(torch.bfloat16)[:, 8:]
+    weight = (1.0 + 0.1 * torch.randn(n, generator=gen)) if weighted else None
+    on_dev = lambda t: None if t is None else t.to(DEV)
+    wide = torch.zeros(tokens, n + 8, dtype=torch.bfloat16, device=DEV)
+    wide[:, 8:] = gate.to(DEV)
+    got = ops.gated_norm(o.to(DEV), wide[:, 8:], on_dev(weight), groups, eps, sigmoid, gate_first=gate_first)
+    odd = torch.zeros(tokens, n + 9, dtype=torch.bfloat16, device=DEV)
+    odd[:, 9:] = gate.to(DEV)
+    other = ops.gated_norm(o.to(DEV), odd[:, 9:], on_dev(weight), groups, eps, sigmoid, gate_first=gate_first)
+    x, z = o.double().numpy(), gate.double().numpy()
+    act = plain.sigmoid(z) if sigmoid else plain.silu(z)
+    if gate_first:
+        x = x * act
+    ref = plain.unit_rms(x.reshape(tokens, groups, size), eps).reshape(tokens, n)
+    if weighted:
+        ref = ref * weight.double().numpy()
+    if not gate_first:
+        ref = ref * act
+    assert rel_error(got, torch.from_numpy(ref)) < KERNEL_TOL[torch.bfloat16]
+    # sums in another order: a rounding of bfloat16 apart at most
+    assert bool(((got.float() - other.float()).abs() <= 2.0 ** -7 * other.float().abs()).all())
 
 
 @pytest.mark.parametrize("hidden", [48, 100, 1024])
