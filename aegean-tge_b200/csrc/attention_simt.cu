@@ -3,8 +3,9 @@
 // One warp per (token, query head).  Keys are visited in position order with a
 // running maximum, so a row's result depends only on its own keys, never on
 // the batch it arrives in or on how its request was cut into portions.  It is
-// the attention of the whole float32 path and of head sizes the tensor-core
-// kernel was not compiled for.
+// the attention of head sizes the tensor-core kernel was not compiled for and of
+// the float32 path where attention_f32.cu does not go: other head sizes, values of
+// a size of their own, sinks, biases, gates, pooled blocks, kept first tokens.
 //
 // Per query head h at position p (reference: src/cpu/scalar/attention_scalar.cpp:48-115,
 // src/models/qwen2.cpp:1243-1304): kv head = h / group; for t in [first, p]:

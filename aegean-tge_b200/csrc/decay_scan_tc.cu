@@ -14,6 +14,7 @@
 // A number that is not finite, or too large for its high part, makes NaN of every product it meets: as an input its split is
 // infinity - infinity, zeros above the diagonal times infinity reach earlier tokens, and so does a score that overflows.  A chunk one of
 // whose results is not finite is therefore computed by the formulas themselves.
+// Numbers below about 1e-33 keep fewer than 24 bits in their parts; beside anything larger in the same sum that is nothing.
 // First operands lie in tensor memory (a lane per token or state row), second operands in shared memory, split on their way in.
 // Measured (B200, 2,048 tokens, 28 heads of 128): states 150 -> 57 us, readout 337 -> 91 us; 14 heads of 64 with activated values of
 // 128: 108 -> 33 us and 137 -> 45 us.  Error against float64 2.85e-7 -> 1.7e-7, activated 1.97e-7 -> 1.44e-7.

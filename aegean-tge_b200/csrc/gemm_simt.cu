@@ -1,8 +1,9 @@
 // Matrix product on the CUDA cores with float32 accumulation: out = x . w^T (+ epilogue).
 //
-// This is the whole float32 path's product (plain FFMA, no reduced-precision
-// matrix mode) and the fallback of the bfloat16 path for shapes the tensor-core
-// kernel refuses.  Every output element is accumulated over k in ascending
+// This is the float32 path's product (plain FFMA, no reduced-precision matrix
+// mode) for weights smaller than 512 x 512 or not aligned for TMA (the others go
+// to gemm_f32_tcgen05.cu) and the fallback of the bfloat16 path for shapes the
+// tensor-core kernel refuses.  Every output element is accumulated over k in ascending
 // order by one thread, so its value depends on neither the tile it falls in
 // nor on what else is in the batch.  The formula is the reference's
 // row-times-vector product (src/tensor/reference.cpp:29-45) followed by the
