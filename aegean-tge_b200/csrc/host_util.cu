@@ -60,6 +60,16 @@ TGE_API int tge_event_create(void** event) {
 }
 TGE_API int tge_event_record(void* event, cudaStream_t stream) { return checked("event record", cudaEventRecord((cudaEvent_t)event, stream)); }
 TGE_API int tge_event_synchronize(void* event) { return checked("event wait", cudaEventSynchronize((cudaEvent_t)event)); }
+// 1: what was queued before the last record is done, 0: not yet
+TGE_API int tge_event_query(void* event) {
+  const cudaError_t err = cudaEventQuery((cudaEvent_t)event);
+  if (err == cudaErrorNotReady) {
+    cudaGetLastError();
+    return 0;
+  }
+  return err == cudaSuccess ? 1 : checked("event query", err);
+}
+TGE_API int tge_event_wait(void* event, cudaStream_t stream) { return checked("wait of a stream", cudaStreamWaitEvent(stream, (cudaEvent_t)event, 0)); }
 TGE_API int tge_event_destroy(void* event) { return checked("event", cudaEventDestroy((cudaEvent_t)event)); }
 // The caller keeps both ends alive until the copy is done.
 TGE_API int tge_copy(void* dst, const void* src, long long bytes, cudaStream_t stream) {

@@ -59,6 +59,8 @@ def core() -> ctypes.CDLL:
         _declare(lib, "tge_event_create", [_c_ptr])
         _declare(lib, "tge_event_record", [_c_ptr, _c_ptr])
         _declare(lib, "tge_event_synchronize", [_c_ptr])
+        _declare(lib, "tge_event_query", [_c_ptr])
+        _declare(lib, "tge_event_wait", [_c_ptr, _c_ptr])
         _declare(lib, "tge_event_destroy", [_c_ptr])
         _declare(lib, "tge_copy", [_c_ptr, _c_ptr, _c_ll, _c_ptr])
         _declare(lib, "tge_embedding", [_c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_ptr])
@@ -284,6 +286,18 @@ class StepEvent:
         """Waits for what was queued before the last record (nothing if there was none)."""
         if self._recorded and _core_lib is not None:         # None: the interpreter is on its way out
             _check(_core_lib.tge_event_synchronize(self._handle), _core_lib)
+
+    def query(self) -> bool:
+        """Whether what was queued before the last record is done (True if there was none)."""
+        if not self._recorded:
+            return True
+        done = _core_lib.tge_event_query(self._handle)
+        return done > 0 or bool(_check(min(done, 0), _core_lib))
+
+    def wait(self, stream: Optional["torch.cuda.Stream"] = None) -> None:
+        """Lets ``stream`` (the current one if None) wait for what was queued before the last record; the host goes on."""
+        if self._recorded:
+            _check(_core_lib.tge_event_wait(self._handle, _stream() if stream is None else stream.cuda_stream), _core_lib)
 
     def __del__(self):
         if getattr(self, "_handle", None) and _core_lib is not None:

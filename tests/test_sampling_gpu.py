@@ -162,3 +162,27 @@ def test_engine_samples_with_cuts_and_penalty(model_dirs):
     assert penalised[0] == plain_greedy[0] or plain_greedy[0] in prompt
     mixed = engine.generate([prompt, prompt], n=6, sampling=[cut, SamplingParams()])
     assert mixed[0] == a[:6] and mixed[1] == plain_greedy[:6]
+
+
+def test_the_event_of_a_draw_on_its_way_can_be_asked_and_waited_for(ops):
+    """What ``sample_async`` returns beside the ids: an event that tells whether the host's copy is complete, that another stream
+    may wait for and that the host may, without counting as a kernel."""
+    from aegean_tge_b200.sampling import Sampler, SamplingParams
+    sampler = Sampler(ops, torch.device(DEV))
+    logits = torch.randn(5, 3000, generator=torch.Generator().manual_seed(3)).to(DEV)
+    best = logits.argmax(dim=1).tolist()
+    greedy = [SamplingParams(temperature=0.0)] * 5
+    assert ops.StepEvent().query()                       # nothing was queued before it
+    side = torch.cuda.Stream()
+    for _ in range(6):                                   # past the ring of four
+        ids, host, event = sampler.sample_async(logits, greedy, [None] * 5)
+        before = ops.launches
+        event.wait(side)
+        with torch.cuda.stream(side):
+            seen = ids.clone()
+        event.wait()
+        event.query()
+        event.synchronize()
+        assert event.query() and host.tolist() == best and ops.launches == before
+        side.synchronize()
+        assert seen.tolist() == best
