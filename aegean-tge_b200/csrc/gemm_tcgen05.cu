@@ -94,97 +94,170 @@ __device__ __forceinline__ float row_factor_of(const float* __restrict__ ss, int
   return 1.0f / sqrtf(sum / (float)width + eps);
 }
 
+// What a finished tile's epilogue needs besides the accumulator, asked for while the tensor cores still work on the tile:
+// the lane's bias and, where the product is added to the float32 stream, the old values under its first sixteen columns.
+struct TileAhead {
+  float bias;
+  float old[16];
+};
+
+__device__ __forceinline__ bool adds_to_stream(const GemmParams& p) { return !p.to_partial && p.epilogue == GEMM_ADD_F32; }
+
+// the stream's values at weight row n and token columns m0 .. m0 + 15
+__device__ __forceinline__ void load_old(const GemmParams& p, int n, int m0, float old[16]) {
+  const int inside = n < p.n_w ? p.m_tok - m0 : 0;
+  const float* src = reinterpret_cast<const float*>(p.out) + (size_t)m0 * p.ldo + n;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) old[j] = j < inside ? src[(size_t)j * p.ldo] : 0.0f;
+}
+
+__device__ __forceinline__ void epilogue_ahead(const GemmParams& p, int n, int m0, TileAhead& ahead) {
+  ahead.bias = (p.bias && n < p.n_w && !p.to_partial) ? p.bias[n] : 0.0f;
+  if (adds_to_stream(p)) load_old(p, n, m0, ahead.old);
+}
+
+// sixteen float32 results of one weight row, a row of `dst` each: 32 lanes write 128 neighbouring bytes per store
+__device__ __forceinline__ void store_columns(float* dst, long long ld, int inside, const float v[16]) {
+  if (inside >= 16) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) dst[(size_t)j * ld] = v[j];
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (j < inside) dst[(size_t)j * ld] = v[j];
+  }
+}
+
+// bfloat16 results v of rows n (a lane each) and token columns m0 .. m0 + 15.  Neighbouring lanes exchange every other column, so
+// that a lane holds two rows of eight columns, and then lanes two apart exchange every other one of those: four rows of
+// four columns, an 8-byte store each (`quads`: rows of the output that allow it; `pairs`: 4-byte stores after the
+// first exchange).
+__device__ __forceinline__ void store_bf16(const GemmParams& p, int lane, int n, int m0, const float v[16], bool quads, bool pairs) {
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out);
+  if (!pairs) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (n < p.n_w && m0 + j < p.m_tok) out[(size_t)(m0 + j) * p.ldo + n] = __float2bfloat16_rn(v[j]);
+    return;
+  }
+  const int odd = lane & 1, upper = (lane >> 1) & 1;
+  uint32_t w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
+    const __nv_bfloat162 both = __floats2bfloat162_rn(odd ? got : v[2 * j], odd ? v[2 * j + 1] : got);
+    w[j] = *reinterpret_cast<const uint32_t*>(&both);
+  }
+  if (quads) {
+    const int row = n & ~3;
+    __nv_bfloat16* dst = out + (size_t)(m0 + 2 * upper + odd) * p.ldo + row;
+    const int inside = row < p.n_w ? p.m_tok - m0 - 2 * upper - odd : 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? w[2 * i] : w[2 * i + 1], 2);
+      const uint2 four = make_uint2(upper ? got : w[2 * i], upper ? w[2 * i + 1] : got);
+      if (4 * i < inside) *reinterpret_cast<uint2*>(dst + (size_t)(4 * i) * p.ldo) = four;
+    }
+    return;
+  }
+  const int row = n & ~1;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int m = m0 + 2 * j + odd;
+    if (m >= p.m_tok || row >= p.n_w) continue;
+    __nv_bfloat16* dst = out + (size_t)m * p.ldo + row;
+    if (row + 1 < p.n_w) *reinterpret_cast<uint32_t*>(dst) = w[j];
+    else *dst = __ushort_as_bfloat16((unsigned short)w[j]);
+  }
+}
+
+// Gated results: even lanes hold gate rows, odd lanes the matching up rows.  Per pair of token columns one exchange gives the even
+// lane (gate, up) of the first column and the odd lane those of the second; where the output's rows allow it (`pairs`), lanes
+// two apart then exchange halves, so that a lane stores two neighbouring results of four columns, 4 bytes each.
+template <bool CLAMPED>
+__device__ __forceinline__ void store_gated(const GemmParams& p, int lane, int n, int m0, const float v[16], bool pairs) {
+  const int odd = lane & 1, upper = (lane >> 1) & 1;
+  float x[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
+    const float g = odd ? got : v[2 * j], u = odd ? v[2 * j + 1] : got;
+    x[j] = CLAMPED ? clamped_gate_mul(g, u, p.alpha) : __fdividef(g, 1.0f + __expf(-g)) * u;
+  }
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out);
+  if (!pairs) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (n < p.n_w && m0 + 2 * j + odd < p.m_tok) out[(size_t)(m0 + 2 * j + odd) * p.ldo + (n >> 1)] = __float2bfloat16_rn(x[j]);
+    return;
+  }
+  __nv_bfloat16* dst = out + (size_t)(m0 + 2 * upper + odd) * p.ldo + ((n & ~3) >> 1);
+  const int inside = (n & ~3) < p.n_w ? p.m_tok - m0 - 2 * upper - odd : 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 two = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+    const uint32_t mine = *reinterpret_cast<const uint32_t*>(&two), got = __shfl_xor_sync(0xffffffffu, mine, 2);
+    const uint32_t both = upper ? __byte_perm(got, mine, 0x7632) : __byte_perm(mine, got, 0x5410);
+    if (4 * i < inside) *reinterpret_cast<uint32_t*>(dst + (size_t)(4 * i) * p.ldo) = both;
+  }
+}
+
 // The epilogue of one finished tile: this warp's 32 lanes (weight rows n) by its columns [c_begin, c_end)
-// of the accumulator buffer `acc`.
+// of the accumulator buffer `acc`.  A block's last epilogue has no products beside it, so it is bound by its own latency and
+// instructions: what to do is decided per sixteen columns and not per element, the stream's old values are asked for a group ahead,
+// and stores are wide.  (Time stamps, 193 tokens of the 7B shape, decided and stored element by element / so: gate and up 6.1 / 3.8 us
+// of a launch's 56 / 54, q/k/v's partial sums 4.9 / 2.1 of 17.3 / 14.7.)
 __device__ __forceinline__ void epilogue_tile(const GemmParams& p, uint32_t tmem_base, int acc, int quarter, int lane,
-                                              int c_begin, int c_end, int n, int tile_t, int split,
+                                              int c_begin, int c_end, int n, int tile_t, int split, TileAhead& ahead,
                                               const float* row_factor = nullptr) {
-  const bool n_ok = n < p.n_w;
-  const float bias = (p.bias && n_ok && !p.to_partial) ? p.bias[n] : 0.0f;
+  const bool to_f32 = p.to_partial || p.epilogue == GEMM_STORE_F32, adds = adds_to_stream(p);
+  const bool gated = gated_epilogue(p.epilogue), n_ok = n < p.n_w;
+  const uintptr_t at = (uintptr_t)p.out;
+  const bool pairs = (p.ldo & 1) == 0 && (at & 3) == 0 && (!gated || (p.n_w & 3) == 0);
+  const bool quads = (p.ldo & 3) == 0 && (at & 7) == 0 && (p.n_w & 3) == 0;
   for (int c0 = c_begin; c0 < c_end; c0 += 16) {
-    uint32_t r[16];
-    const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * p.bn + c0);
-    tc_load16(taddr, r);
     const int m0 = tile_t * p.bn + c0;
-    if (m0 >= p.m_tok) continue;                              // uniform over the warp
+    if (m0 >= p.m_tok) break;                                 // uniform over the warp
+    float next[16];
+    if (adds && c0 + 16 < c_end) load_old(p, n, m0 + 16, next);
+    uint32_t r[16];
+    tc_load16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * p.bn + c0), r);
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
     if (row_factor != nullptr && !p.to_partial) {             // partial sums stay as they are: who adds them scales
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        r[j] = __float_as_uint(__uint_as_float(r[j]) * row_factor[min(m0 + j, DEFER_MAX_TOKENS - 1)]);
+      for (int j = 0; j < 16; ++j) v[j] *= row_factor[min(m0 + j, DEFER_MAX_TOKENS - 1)];
     }
-    if (!p.to_partial && p.epilogue == GEMM_ADD_F32) {
-      // read all sixteen old values before the first store, so the loads overlap
-      float* dst = reinterpret_cast<float*>(p.out) + (size_t)m0 * p.ldo + n;
-      float old[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) old[j] = (n_ok && m0 + j < p.m_tok) ? dst[(size_t)j * p.ldo] : 0.0f;
-#pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (n_ok && m0 + j < p.m_tok) dst[(size_t)j * p.ldo] = old[j] + p.alpha * (__uint_as_float(r[j]) + bias);
+    for (int j = 0; j < 16; ++j) v[j] += ahead.bias;
+    if (gated && !p.to_partial) {
+      if (p.epilogue == GEMM_SWIGLU) store_gated<false>(p, lane, n, m0, v, pairs);
+      else store_gated<true>(p, lane, n, m0, v, pairs);
       continue;
     }
-    if (!p.to_partial && gated_epilogue(p.epilogue)) {
-      // Even lanes hold gate rows, odd lanes the matching up rows.  Per pair of token columns one
-      // exchange gives the even lane (gate, up) of the first column and the odd lane those of the second.
-      const bool odd = lane & 1;
+    if (!p.to_partial) {
+      if (p.epilogue == GEMM_GELU || p.epilogue == GEMM_GELU_TANH) {
+        if (n >= p.act_from) {
 #pragma unroll
-      for (int j = 0; j < 16; j += 2) {
-        const float a = __uint_as_float(r[j]) + bias, b = __uint_as_float(r[j + 1]) + bias;
-        const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
-        const float g = odd ? got : a, u = odd ? b : got;
-        const int m = m0 + j + (odd ? 1 : 0);
-        if (n_ok && m < p.m_tok)
-          reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)m * p.ldo + (n >> 1)] =
-              __float2bfloat16_rn(p.epilogue == GEMM_SWIGLU ? __fdividef(g, 1.0f + __expf(-g)) * u : clamped_gate_mul(g, u, p.alpha));
+          for (int j = 0; j < 16; ++j) v[j] = p.epilogue == GEMM_GELU ? gelu_erf_fast(v[j]) : gelu_tanh(v[j]);
+        }
+      } else if (adds) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = fmaf(p.alpha, v[j], ahead.old[j]);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) ahead.old[j] = next[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] *= p.alpha;
       }
-      continue;
     }
-    if (!p.to_partial && p.epilogue != GEMM_STORE_F32 && (p.ldo & 1) == 0 && ((uintptr_t)p.out & 3) == 0) {
-      // bfloat16 results, two weight rows to a store: neighbouring lanes exchange every other token column, the
-      // even lane then holds (row n, row n + 1) of the even columns and the odd lane those of the odd columns,
-      // so a lane issues eight 4-byte stores where it would issue sixteen of 2 bytes (the gated epilogue's way).
-      const bool odd = lane & 1;
-      const bool activate = p.epilogue >= GEMM_GELU && n >= p.act_from;
-      const int nn = odd ? n - 1 : n;
-#pragma unroll
-      for (int j = 0; j < 16; j += 2) {
-        float a = __uint_as_float(r[j]) + bias, b = __uint_as_float(r[j + 1]) + bias;
-        if (p.epilogue >= GEMM_GELU) {
-          if (activate) {
-            a = p.epilogue == GEMM_GELU ? gelu_erf_fast(a) : gelu_tanh(a);
-            b = p.epilogue == GEMM_GELU ? gelu_erf_fast(b) : gelu_tanh(b);
-          }
-        } else {
-          a *= p.alpha;
-          b *= p.alpha;
-        }
-        const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
-        const float lo = odd ? got : a, hi = odd ? b : got;
-        const int m = m0 + j + (odd ? 1 : 0);
-        if (m < p.m_tok && nn < p.n_w) {
-          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + (size_t)m * p.ldo + nn;
-          if (nn + 1 < p.n_w) *reinterpret_cast<__nv_bfloat162*>(dst) = __floats2bfloat162_rn(lo, hi);
-          else *dst = __float2bfloat16_rn(lo);
-        }
-      }
-      continue;
-    }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const int m = m0 + j;
-      float v = __uint_as_float(r[j]) + bias;
-      if (p.to_partial) {
-        if (n_ok && m < p.m_tok) p.partial[((size_t)split * p.m_tok + m) * p.n_w + n] = v;
-      } else if (n_ok && m < p.m_tok) {
-        if (p.epilogue >= GEMM_GELU) {
-          if (n >= p.act_from) v = p.epilogue == GEMM_GELU ? gelu_erf_fast(v) : gelu_tanh(v);
-          reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)m * p.ldo + n] = __float2bfloat16_rn(v);
-        } else if (p.epilogue == GEMM_STORE) {
-          reinterpret_cast<__nv_bfloat16*>(p.out)[(size_t)m * p.ldo + n] = __float2bfloat16_rn(p.alpha * v);
-        } else {
-          reinterpret_cast<float*>(p.out)[(size_t)m * p.ldo + n] = p.alpha * v;
-        }
-      }
+    if (to_f32 || adds) {
+      float* dst = p.to_partial ? p.partial + ((size_t)split * p.m_tok + m0) * p.n_w + n
+                                : reinterpret_cast<float*>(p.out) + (size_t)m0 * p.ldo + n;
+      store_columns(dst, p.to_partial ? p.n_w : p.ldo, n_ok ? p.m_tok - m0 : 0, v);
+    } else {
+      store_bf16(p, lane, n, m0, v, quads, pairs);
     }
   }
 }
@@ -354,10 +427,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       const int split = work % p.splits;
       const int rest = work / p.splits;
       const int tile_t = rest % p.tiles_t, tile_w = rest / p.tiles_t;
+      const int n = tile_w * BM + quarter * 32 + lane;
+      TileAhead ahead;
+      if (c_begin < c_end) epilogue_ahead(p, n, tile_t * p.bn + c_begin, ahead);
       if (!mbar_wait(tfull_bar(acc), acc_phase, p.status, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      epilogue_tile(p, tmem_base, acc, quarter, lane, c_begin, c_end, tile_w * BM + quarter * 32 + lane, tile_t, split,
-                    row_factor);
+      epilogue_tile(p, tmem_base, acc, quarter, lane, c_begin, c_end, n, tile_t, split, ahead, row_factor);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty_bar(acc));
@@ -552,10 +627,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
       const int split = work % p.splits;
       const int rest = work / p.splits;
       const int tile_t = rest % p.tiles_t, tile_w = rest / p.tiles_t;
+      const int n = tile_w * PAIR_BM + (int)rank * BM + quarter * 32 + lane;
+      TileAhead ahead;
+      if (c_begin < c_end) epilogue_ahead(p, n, tile_t * p.bn + c_begin, ahead);
       if (!mbar_wait(tfull_bar(acc), acc_phase, p.status, abort_flag)) { ok = false; break; }
       tc_fence_after();
-      epilogue_tile(p, tmem_base, acc, quarter, lane, c_begin, c_end,
-                    tile_w * PAIR_BM + (int)rank * BM + quarter * 32 + lane, tile_t, split);
+      epilogue_tile(p, tmem_base, acc, quarter, lane, c_begin, c_end, n, tile_t, split, ahead);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(map_to_rank(tempty_bar(acc), 0));

@@ -408,6 +408,39 @@ def test_gemm_pair_epilogues(ops, pair_everywhere, M, N, K):
     ops.check_status()
 
 
+@pytest.mark.parametrize("pair", [0, 2])
+@pytest.mark.parametrize("M,N,K", [(1, 128, 64), (15, 260, 128), (17, 132, 64), (145, 130, 192), (193, 388, 320), (257, 131, 64), (500, 640, 128)])
+def test_gemm_tcgen05_stores_of_any_width_hold_the_same(ops, pair, M, N, K):
+    """Outputs whose rows allow 8-byte stores, 4-byte stores or single ones only, over tokens and weight rows that end inside a tile: the
+    same bits in every epilogue, and nothing beside them touched."""
+    gen = torch.Generator().manual_seed(N + M)
+    x, w = torch.randn(M, K, generator=gen).to(torch.bfloat16).to(DEV), (torch.randn(N, K, generator=gen) * 0.1).to(torch.bfloat16).to(DEV)
+    b = torch.randn(N, generator=gen).to(DEV)
+    plain_rows = ops_plain.linear(x.cpu(), w.cpu(), b.cpu())
+    ops.set_pair_gemm(pair)
+    try:
+        for epilogue in (ops.GEMM_STORE, ops.GEMM_STORE_F32, ops.GEMM_ADD_F32, ops.GEMM_SWIGLU, ops.GEMM_GELU, ops.GEMM_GELU_TANH, ops.GEMM_GLU_CLAMPED):
+            gated = epilogue in (ops.GEMM_SWIGLU, ops.GEMM_GLU_CLAMPED)
+            if gated and N % 2:
+                continue
+            dtype = torch.float32 if epilogue in (ops.GEMM_STORE_F32, ops.GEMM_ADD_F32) else torch.bfloat16
+            columns, results = N // 2 if gated else N, []
+            for before, width in ((0, -(-columns // 8) * 8), (4, -(-columns // 8) * 8 + 8), (2, -(-columns // 2) * 2 + 4), (3, columns + 5)):
+                out = torch.ones(M, width, dtype=dtype, device=DEV)
+                view = out[:, before:before + columns]
+                ops.linear(x, w, b, epilogue, out=view, alpha=0.75, act_from=5)
+                results.append(view.clone())
+                assert bool((out[:, :before] == 1).all()) and bool((out[:, before + columns:] == 1).all())
+            ops.check_status()
+            assert all(torch.equal(results[0], other) for other in results[1:]), epilogue
+            if epilogue == ops.GEMM_STORE:
+                assert rel_error(results[0], 0.75 * plain_rows) < TOL[torch.bfloat16]
+            if epilogue == ops.GEMM_ADD_F32:
+                assert rel_error(results[0], 1.0 + 0.75 * plain_rows) < 2e-5
+    finally:
+        ops.set_pair_gemm(1)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 256, 128), (8, 3584, 512), (33, 520, 264), (128, 1024, 320), (140, 384, 192), (150, 384, 192)])
 @pytest.mark.parametrize("defer", [False, True])
 def test_linear_add_norm_and_rows_without_their_factor(ops, M, N, K, defer):
