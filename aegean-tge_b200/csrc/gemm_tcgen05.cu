@@ -31,6 +31,8 @@
 
 enum GemmEpilogue : int { GEMM_STORE = 0, GEMM_STORE_F32 = 1, GEMM_ADD_F32 = 2, GEMM_SWIGLU = 3, GEMM_GELU = 4,
                           GEMM_GELU_TANH = 5, GEMM_GLU_CLAMPED = 6 };
+// Added to the epilogue by a caller whose weights no kernel still in flight can have written (a model's, once it is loaded).
+constexpr int GEMM_WEIGHTS_SETTLED = 256;
 // GEMM_GLU_CLAMPED: the gated epilogue with both halves clamped at L = `alpha`: g <- min(g, L), u <- clamp(u, -L, L),
 // out = g sigmoid(1.702 g) (u + 1).
 // GEMM_GELU / GEMM_GELU_TANH: bfloat16 out = gelu(acc + bias) in the erf or the tanh form for weight rows n >= act_from,
@@ -67,6 +69,7 @@ struct GemmParams {
   float ss_eps;
   float alpha;         // multiplies acc + bias in the plain epilogues (1: none)
   int act_from;        // first weight row the GELU epilogues activate
+  int settled;         // the weights were there before any kernel that may still run: the pair kernel asks for them early
 };
 constexpr int DEFER_MAX_TOKENS = 128;
 
@@ -545,7 +548,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
   pdl_trigger();
-  pdl_wait();
+  // Settled weights (the caller says so): their loader asks for a ring-full of them while the kernel in front still runs.
+  // (193 tokens in three prompts, 12 layers of the 7B shape, with the shorter epilogue: 2,087 -> 1,955 us.)
+  if (warp != 0 || !p.settled) pdl_wait();
 
   const int total_work = p.tiles_w * p.tiles_t * p.splits;
   const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
@@ -556,6 +561,21 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
+      int ahead = 0;      // stages of the first item whose weight tile is already on its way
+      if (p.settled) {
+        if (pair < total_work) {
+          const int split = pair % p.splits, tile_w = pair / p.splits / p.tiles_t;
+          const int kb_begin = (int)((long long)split * p.k_blocks / p.splits);
+          const int kb_end = (int)((long long)(split + 1) * p.k_blocks / p.splits);
+          ahead = kb_end - kb_begin < p.stages ? kb_end - kb_begin : p.stages;
+          for (int s = 0; s < ahead; ++s) {
+            if (rank == 0) mbar_expect_tx(full_bar(s), 2u * stage_bytes);
+            tma_load_2d_pair(base + (uint32_t)s * stage_bytes, &map_w, map_to_rank(full_bar(s), 0), (kb_begin + s) * BK,
+                             tile_w * PAIR_BM + (int)rank * BM);
+          }
+        }
+        pdl_wait();
+      }
       for (int work = pair; work < total_work && ok; work += pairs) {
         const int split = work % p.splits;
         const int rest = work / p.splits;
@@ -563,11 +583,15 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
         const int kb_begin = (int)((long long)split * p.k_blocks / p.splits);
         const int kb_end = (int)((long long)(split + 1) * p.k_blocks / p.splits);
         for (int kb = kb_begin; kb < kb_end; ++kb) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1u, p.status, abort_flag)) { ok = false; break; }
-          if (rank == 0) mbar_expect_tx(full_bar(stage), 2u * stage_bytes);
           const uint32_t leader_full = map_to_rank(full_bar(stage), 0);
           const uint32_t a_dst = base + (uint32_t)stage * stage_bytes;
-          tma_load_2d_pair(a_dst, &map_w, leader_full, kb * BK, tile_w * PAIR_BM + (int)rank * BM);
+          if (ahead > 0) {
+            --ahead;      // first pass over the ring: the stage is free and its weight tile was requested above
+          } else {
+            if (!mbar_wait(empty_bar(stage), phase ^ 1u, p.status, abort_flag)) { ok = false; break; }
+            if (rank == 0) mbar_expect_tx(full_bar(stage), 2u * stage_bytes);
+            tma_load_2d_pair(a_dst, &map_w, leader_full, kb * BK, tile_w * PAIR_BM + (int)rank * BM);
+          }
           tma_load_2d_pair(a_dst + A_STAGE_BYTES, &map_x, leader_full, kb * BK, tile_t * p.bn + (int)rank * (p.bn / 2));
           if (++stage == p.stages) { stage = 0; phase ^= 1u; }
         }
@@ -1016,7 +1040,7 @@ namespace {
 int launch_product(const void* x, long long ldx, const void* w, long long ldw, const float* bias, void* out,
                    long long ldo, int M, int N, int K, int epilogue, float* scratch, long long scratch_floats,
                    int force_bn, int force_splits, bool partial_always, int* status, cudaStream_t stream,
-                   int* splits_out, const RowSums& sums = RowSums(), float alpha = 1.0f, int act_from = 0) {
+                   int* splits_out, const RowSums& sums = RowSums(), float alpha = 1.0f, int act_from = 0, bool settled = false) {
   if (K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || (uintptr_t)x % 16 != 0 || (uintptr_t)w % 16 != 0) return TGE_UNSUPPORTED;
   if (scratch == nullptr) scratch_floats = 0;
   const Plan plan = make_plan(M, N, K, scratch_floats, force_bn, force_splits);
@@ -1052,7 +1076,7 @@ int launch_product(const void* x, long long ldx, const void* w, long long ldw, c
     p.to_partial = pair_partial ? 1 : 0;
     p.bias = bias; p.out = out; p.ldo = ldo; p.partial = scratch; p.status = status;
     p.ss = nullptr; p.ss_slices = 0; p.ss_width = 0; p.ss_eps = 0.0f;
-    p.alpha = alpha; p.act_from = act_from;
+    p.alpha = alpha; p.act_from = act_from; p.settled = settled ? 1 : 0;
     const size_t smem = 1024 + (size_t)pair_plan.stages * (A_STAGE_BYTES + (pair_plan.bn / 2) * BK * 2) +
                         8 * (2 * pair_plan.stages + 4) + 16;
     const long long total = (long long)p.tiles_w * p.tiles_t * p.splits;
@@ -1081,7 +1105,7 @@ int launch_product(const void* x, long long ldx, const void* w, long long ldw, c
   p.to_partial = to_partial ? 1 : 0;
   p.bias = bias; p.out = out; p.ldo = ldo; p.partial = scratch; p.status = status;
   p.ss = sums.ss; p.ss_slices = sums.slices; p.ss_width = sums.width; p.ss_eps = sums.eps;
-  p.alpha = alpha; p.act_from = act_from;
+  p.alpha = alpha; p.act_from = act_from; p.settled = 0;
 
   const size_t smem = 1024 + (size_t)plan.stages * (A_STAGE_BYTES + plan.bn * BK * 2) + 8 * (2 * plan.stages + 4) + 16 +
                       DEFER_MAX_TOKENS * sizeof(float);
@@ -1435,6 +1459,8 @@ TGE_API int tge_gemm_tcgen05(const void* x, long long ldx, const void* w, long l
                              long long scratch_floats, int force_bn, int force_splits, int* status,
                              const float* x_ss, int x_ss_slices, int x_ss_width, float x_ss_eps, float alpha,
                              int act_from, cudaStream_t stream) {
+  const bool settled = epilogue > 0 && (epilogue & GEMM_WEIGHTS_SETTLED) != 0;
+  if (settled) epilogue -= GEMM_WEIGHTS_SETTLED;
   TGE_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm: bad sizes M=%d N=%d K=%d", M, N, K);
   TGE_REQUIRE(epilogue >= GEMM_STORE && epilogue <= GEMM_GLU_CLAMPED, "gemm: unknown epilogue %d", epilogue);
   TGE_REQUIRE((epilogue != GEMM_SWIGLU && epilogue != GEMM_GLU_CLAMPED) || N % 2 == 0, "gemm: the gated epilogue needs an even number of weight rows, got %d", N);
@@ -1445,7 +1471,7 @@ TGE_API int tge_gemm_tcgen05(const void* x, long long ldx, const void* w, long l
   RowSums sums;
   sums.ss = x_ss; sums.slices = x_ss_slices; sums.width = x_ss_width; sums.eps = x_ss_eps;
   int rc = launch_product(x, ldx, w, ldw, bias, out, ldo, M, N, K, epilogue, scratch, scratch_floats, force_bn,
-                          force_splits, false, status, stream, &splits, sums, alpha, act_from);
+                          force_splits, false, status, stream, &splits, sums, alpha, act_from, settled);
   if (rc != 1) return rc;
   if (splits > 0) {
     // bytes of four columns of the result: two bfloat16 where they are gated, four bfloat16, or four float32

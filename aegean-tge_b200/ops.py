@@ -667,11 +667,12 @@ class DeferredRows:
 
 
 _NO_FACTOR = (None, 0, 0, 0.0)
+_SETTLED = 256          # added to the epilogue: GEMM_WEIGHTS_SETTLED of csrc/gemm_tcgen05.cu
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], epilogue: int,
            out: Optional[torch.Tensor] = None, force_simt: bool = False, force_bn: int = 0,
-           force_splits: int = 0, alpha: float = 1.0, act_from: int = 0) -> torch.Tensor:
+           force_splits: int = 0, alpha: float = 1.0, act_from: int = 0, settled: bool = False) -> torch.Tensor:
     """out = x . w^T with an epilogue.
 
     x [M, K] and w [N, K] in the run dtype; bias float32 [N] or None.
@@ -685,6 +686,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], epilo
     ``alpha`` multiplies product + bias in the store and add epilogues (a residual multiplier, a logit scale).
     Both types go to their tcgen05 kernel when the shape allows TMA (float32, split into three bfloat16 numbers, from
     512 x 512 weights on), else to the CUDA-core kernel.
+    ``settled``: no kernel that may still run has written ``w`` (a loaded model's weights): they may be read before the kernel
+    in front is done.
     """
     deferred = x if isinstance(x, DeferredRows) else None
     if deferred is not None:
@@ -724,7 +727,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], epilo
         scratch = scratch_floats(need) if need > 0 else None
         factor = _NO_FACTOR if deferred is None else deferred.factor_args()
         rc = lib.tge_gemm_tcgen05(x.data_ptr(), ldx, w.data_ptr(), ldw, _ptr(bias), out.data_ptr(), ldo, M, N, K,
-                                  epilogue, _ptr(scratch), 0 if scratch is None else scratch.numel(), force_bn,
+                                  epilogue + (_SETTLED if settled else 0), _ptr(scratch), 0 if scratch is None else scratch.numel(), force_bn,
                                   force_splits, status_word().data_ptr(), *factor, float(alpha), int(act_from), _stream())
         if _check(rc, lib) != UNSUPPORTED:
             return out
@@ -761,7 +764,7 @@ FUSED_MAX_TOKENS = 144
 
 def linear_add_norm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], stream: torch.Tensor,
                     norm_weight: torch.Tensor, eps: float, out_dtype: torch.dtype, defer: bool = False,
-                    alpha: float = 1.0):
+                    alpha: float = 1.0, settled: bool = False):
     """stream (float32 [M, N]) += alpha * (x . w^T (+ bias)); returns RMSNorm(stream) * norm_weight in ``out_dtype``.
 
     For a small bfloat16 batch the partial sums of the product are added into the stream and the new
@@ -801,14 +804,14 @@ def linear_add_norm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tenso
                                            status_word().data_ptr(), float(alpha), _stream())
         if _check(rc, lib) != UNSUPPORTED:
             return out
-    linear(x, w, bias, GEMM_ADD_F32, out=stream, alpha=alpha)
+    linear(x, w, bias, GEMM_ADD_F32, out=stream, alpha=alpha, settled=settled)
     return rmsnorm(stream, norm_weight, eps, out_dtype)
 
 
 def linear_qkv_rope_store(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], cos: Optional[torch.Tensor],
                           sin: Optional[torch.Tensor], rotary: int, positions: torch.Tensor,
                           seq_of_token: torch.Tensor, block_table: torch.Tensor, k_pages: torch.Tensor,
-                          v_pages: torch.Tensor, heads: int, kv_heads: int, head_dim: int) -> torch.Tensor:
+                          v_pages: torch.Tensor, heads: int, kv_heads: int, head_dim: int, settled: bool = False) -> torch.Tensor:
     """The fused q/k/v product of an attention layer followed by rotation and the cache store.
 
     Returns the qkv buffer [T, (heads + 2 kv_heads) * head_dim] whose first heads*head_dim columns hold the
@@ -850,7 +853,7 @@ def linear_qkv_rope_store(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch
                                            *(_NO_FACTOR if deferred is None else deferred.factor_args()), _stream())
         if _check(rc, lib) != UNSUPPORTED:
             return qkv
-    qkv = linear(x if deferred is None else deferred, w, bias, GEMM_STORE)
+    qkv = linear(x if deferred is None else deferred, w, bias, GEMM_STORE, settled=settled)
     rope_kv_store(qkv, cos, sin, rotary, positions, seq_of_token, block_table, k_pages, v_pages, heads, kv_heads,
                   head_dim)
     return qkv

@@ -326,7 +326,7 @@ class GQAttention(Mixer):
             h = complete()
         k_pages, v_pages = cache.paged["k"], cache.paged["v"]
         table = ctx.block_tables[cache.group]
-        qk = ops.linear(h, self.w_qkv, self.b_qkv, ops.GEMM_STORE)
+        qk = ops.linear(h, self.w_qkv, self.b_qkv, ops.GEMM_STORE, settled=True)
         coef, every = self.q_temp if self.q_temp is not None else (0.0, 0)
         ops.qk_temp_store(qk, self.q_norm_w, self.k_norm_w, self.qk_norm[1] if self.qk_norm else 1.0, coef, every,
                           ctx.positions, ctx.seq_of_token, table if cache.owner else None, k_pages if cache.owner else None,
@@ -345,7 +345,7 @@ class GQAttention(Mixer):
             h = complete()
         k_pages, v_pages = cache.paged["k"], cache.paged["v"]
         table = ctx.block_tables[cache.group]
-        rows = ops.linear(h, self.w_qkv, None, ops.GEMM_STORE)
+        rows = ops.linear(h, self.w_qkv, None, ops.GEMM_STORE, settled=True)
         if self.own_kv and not cache.owner:
             raise RuntimeError("attention: a layer with keys of its own was given another layer's cache")
         if self.own_kv or self.qk_norm is not None:
@@ -387,7 +387,7 @@ class GQAttention(Mixer):
         k_pages, v_pages = cache.paged["k"], cache.paged["v"]
         table = ctx.block_tables[cache.group]
         cos, sin, rotary = self.position.rotary_tables()
-        raw = ops.linear(h, self.w_qkv, None, ops.GEMM_STORE)
+        raw = ops.linear(h, self.w_qkv, None, ops.GEMM_STORE, settled=True)
         q = ops.conv_norm_rope_store(raw, self.conv_w, self.taps, cache.state.get("conv"), ctx.slots, ctx.q_start,
                                      ctx.num_seqs, self.q_norm_w, self.k_norm_w, self.qk_norm[1] if self.qk_norm else 1.0,
                                      cos, sin, rotary, ctx.positions, ctx.seq_of_token, table,
@@ -460,7 +460,7 @@ class GQAttention(Mixer):
                     act_out=beside[0] if shared else None, activation=beside[1] if shared else ops.GEMM_GELU)
                 did_beside = shared and qkv is not None
             if qkv is None:
-                qkv = ops.linear(h, self.w_qkv, self.b_qkv, ops.GEMM_STORE)
+                qkv = ops.linear(h, self.w_qkv, self.b_qkv, ops.GEMM_STORE, settled=True)
                 ops.qk_norm_kv_store(qkv, q_w, k_w, eps, per_head, ctx.positions, ctx.seq_of_token,
                                      table if store_here else None, k_pages if store_here else None,
                                      v_pages if store_here else None, self.heads, self.kv_heads, self.head_dim,
@@ -484,9 +484,9 @@ class GQAttention(Mixer):
             cos, sin, rotary = tables
             qkv = ops.linear_qkv_rope_store(h, self.w_qkv, self.b_qkv, cos, sin, rotary, ctx.positions,
                                             ctx.seq_of_token, table, k_pages, v_pages, self.heads, self.kv_heads,
-                                            self.head_dim)
+                                            self.head_dim, settled=True)
         else:
-            qkv = ops.linear(h, self.w_qkv, self.b_qkv, ops.GEMM_STORE)
+            qkv = ops.linear(h, self.w_qkv, self.b_qkv, ops.GEMM_STORE, settled=True)
             if tables is None:
                 q = qkv[:, :self.q_dim].view(-1, self.heads, self.head_dim)
                 k = qkv[:, self.q_dim:self.q_dim + self.kv_dim].view(-1, self.kv_heads, self.head_dim)
@@ -512,18 +512,19 @@ class GQAttention(Mixer):
         return self.w_o, self.b_o
 
     def forward(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
-        return self.ops.linear(self.attend(h, ctx, cache), self.w_o, self.b_o, self.ops.GEMM_STORE)
+        return self.ops.linear(self.attend(h, ctx, cache), self.w_o, self.b_o, self.ops.GEMM_STORE, settled=True)
 
     def forward_f32(self, h, ctx: StepContext, cache: LayerCache, out=None, alpha: float = 1.0, accumulate: bool = False):
         a = self.attend(h, ctx, cache)
         epilogue = self.ops.GEMM_ADD_F32 if accumulate else self.ops.GEMM_STORE_F32
-        return self.ops.linear(a, self.w_o, self.b_o, epilogue, out=out, alpha=alpha)
+        return self.ops.linear(a, self.w_o, self.b_o, epilogue, out=out, alpha=alpha, settled=True)
 
     def forward_add(self, h: torch.Tensor, x: torch.Tensor, ctx: StepContext, cache: LayerCache, next_norm=None,
                     defer: bool = False):
         a = self.attend(h, ctx, cache)
         fused = next_norm.fusable() if next_norm is not None else None
         if fused is not None:
-            return self.ops.linear_add_norm(a, self.w_o, self.b_o, x, fused[0], fused[1], self.env.dtype, defer=defer)
-        self.ops.linear(a, self.w_o, self.b_o, self.ops.GEMM_ADD_F32, out=x)
+            return self.ops.linear_add_norm(a, self.w_o, self.b_o, x, fused[0], fused[1], self.env.dtype, defer=defer,
+                                            settled=True)
+        self.ops.linear(a, self.w_o, self.b_o, self.ops.GEMM_ADD_F32, out=x, settled=True)
         return None

@@ -138,8 +138,8 @@ class ParallelBlock(Block):
         fused = next_norm.fusable() if next_norm is not None else None
         if fused is not None:
             return ops.linear_add_norm(inner, self.w_out, self.b_out, x, fused[0], fused[1], self.env.dtype,
-                                       defer=bool(next_takes_deferred), alpha=self.mult)
-        ops.linear(inner, self.w_out, self.b_out, ops.GEMM_ADD_F32, out=x, alpha=self.mult)
+                                       defer=bool(next_takes_deferred), alpha=self.mult, settled=True)
+        ops.linear(inner, self.w_out, self.b_out, ops.GEMM_ADD_F32, out=x, alpha=self.mult, settled=True)
         return None
 
 

@@ -83,5 +83,5 @@ class LinearHead(Part):
         return 2.0 * tokens * self.vocab * self.hidden
 
     def forward(self, h: torch.Tensor) -> torch.Tensor:
-        logits = self.ops.linear(h, self.weight, None, self.ops.GEMM_STORE_F32, alpha=self.logit_scale)
+        logits = self.ops.linear(h, self.weight, None, self.ops.GEMM_STORE_F32, alpha=self.logit_scale, settled=True)
         return logits if self.cap is None else self.ops.soft_cap(logits, self.cap)

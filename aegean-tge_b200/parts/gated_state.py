@@ -70,18 +70,18 @@ class _MatrixStateMixer(Mixer):
         return self.w_o, None
 
     def forward(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
-        return self.ops.linear(self.inner(h, ctx, cache), self.w_o, None, self.ops.GEMM_STORE)
+        return self.ops.linear(self.inner(h, ctx, cache), self.w_o, None, self.ops.GEMM_STORE, settled=True)
 
     def forward_f32(self, h, ctx: StepContext, cache: LayerCache, out=None, alpha: float = 1.0, accumulate: bool = False):
         epilogue = self.ops.GEMM_ADD_F32 if accumulate else self.ops.GEMM_STORE_F32
-        return self.ops.linear(self.inner(h, ctx, cache), self.w_o, None, epilogue, out=out, alpha=alpha)
+        return self.ops.linear(self.inner(h, ctx, cache), self.w_o, None, epilogue, out=out, alpha=alpha, settled=True)
 
     def forward_add(self, h: torch.Tensor, x: torch.Tensor, ctx: StepContext, cache: LayerCache, next_norm=None):
         a = self.inner(h, ctx, cache)
         fused = next_norm.fusable() if next_norm is not None else None
         if fused is not None:
-            return self.ops.linear_add_norm(a, self.w_o, None, x, fused[0], fused[1], self.env.dtype)
-        self.ops.linear(a, self.w_o, None, self.ops.GEMM_ADD_F32, out=x)
+            return self.ops.linear_add_norm(a, self.w_o, None, x, fused[0], fused[1], self.env.dtype, settled=True)
+        self.ops.linear(a, self.w_o, None, self.ops.GEMM_ADD_F32, out=x, settled=True)
         return None
 
 
@@ -138,7 +138,7 @@ class GatedDeltaRule(_MatrixStateMixer):
 
     def inner(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache, out: Optional[torch.Tensor] = None):
         ops = self.ops
-        raw = ops.linear(h, self.w_in, None, ops.GEMM_STORE_F32)
+        raw = ops.linear(h, self.w_in, None, ops.GEMM_STORE_F32, settled=True)
         qk, v, gates = ops.gated_prepare(raw, ops.GATED_DELTA, self.groups, self.heads, self.key_dim, self.value_dim,
                                          self.taps, self.conv_w, None, cache.state.get("conv"), ctx.slots, ctx.q_start,
                                          ctx.seq_of_token, ctx.num_seqs, self.a_log, self.dt_bias, unit_eps=self.unit_eps,
@@ -198,7 +198,7 @@ class StateSpace(_MatrixStateMixer):
 
     def inner(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache, out: Optional[torch.Tensor] = None):
         ops = self.ops
-        raw = ops.linear(h, self.w_in, None, ops.GEMM_STORE_F32)
+        raw = ops.linear(h, self.w_in, None, ops.GEMM_STORE_F32, settled=True)
         qk, v, gates = ops.gated_prepare(raw, ops.GATED_STATE_SPACE, self.groups, self.heads, self.key_dim, self.value_dim,
                                          self.taps, self.conv_w, self.conv_b, cache.state.get("conv"), ctx.slots, ctx.q_start,
                                          ctx.seq_of_token, ctx.num_seqs, self.a_log, self.dt_bias)
@@ -264,8 +264,8 @@ class MatrixLSTM(Mixer):
         complete = getattr(h, "complete", None)
         if complete is not None:
             h = complete()
-        rows = ops.linear(h, self.w_in, None, ops.GEMM_STORE)
-        gates = ops.linear(h, self.w_gates, self.b_gates, ops.GEMM_STORE_F32)
+        rows = ops.linear(h, self.w_in, None, ops.GEMM_STORE, settled=True)
+        gates = ops.linear(h, self.w_gates, self.b_gates, ops.GEMM_STORE_F32, settled=True)
         state = cache.state
         return ops.mlstm(rows, gates, self.heads, self.key_dim, self.value_dim, self.norm_w, state["state"],
                          state["normaliser"], state["maximum"], ctx.slots, ctx.q_start, ctx.host_q_lens, self.cap,
@@ -275,16 +275,16 @@ class MatrixLSTM(Mixer):
         return self.w_o, None
 
     def forward(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
-        return self.ops.linear(self.inner(h, ctx, cache), self.w_o, None, self.ops.GEMM_STORE)
+        return self.ops.linear(self.inner(h, ctx, cache), self.w_o, None, self.ops.GEMM_STORE, settled=True)
 
     def forward_f32(self, h, ctx: StepContext, cache: LayerCache, out=None, alpha: float = 1.0, accumulate: bool = False):
         epilogue = self.ops.GEMM_ADD_F32 if accumulate else self.ops.GEMM_STORE_F32
-        return self.ops.linear(self.inner(h, ctx, cache), self.w_o, None, epilogue, out=out, alpha=alpha)
+        return self.ops.linear(self.inner(h, ctx, cache), self.w_o, None, epilogue, out=out, alpha=alpha, settled=True)
 
     def forward_add(self, h: torch.Tensor, x: torch.Tensor, ctx: StepContext, cache: LayerCache, next_norm=None):
         a = self.inner(h, ctx, cache)
         fused = next_norm.fusable() if next_norm is not None else None
         if fused is not None:
-            return self.ops.linear_add_norm(a, self.w_o, None, x, fused[0], fused[1], self.env.dtype)
-        self.ops.linear(a, self.w_o, None, self.ops.GEMM_ADD_F32, out=x)
+            return self.ops.linear_add_norm(a, self.w_o, None, x, fused[0], fused[1], self.env.dtype, settled=True)
+        self.ops.linear(a, self.w_o, None, self.ops.GEMM_ADD_F32, out=x, settled=True)
         return None

@@ -167,12 +167,12 @@ class LatentAttention(Mixer):
         table = ctx.block_tables[cache.group]
         dtype = self.env.dtype
         own = not self.shared_kv
-        raw = ops.linear(h, self.w_in, None, ops.GEMM_STORE_F32)
+        raw = ops.linear(h, self.w_in, None, ops.GEMM_STORE_F32, settled=True)
         q_latent, gate = ops.latent_prepare(raw, self.q_rank, self.kv_rank, self.rot, self.gate_n, own, self.q_norm_w,
                                             self.kv_norm_w, self.eps, self.cos, self.sin, self.rot_dims, ctx.positions,
                                             ctx.seq_of_token, table, pages if (own and cache.owner) else None, dtype,
                                             halves=self.halves)
-        q = ops.linear(q_latent, self.w_uq, None, ops.GEMM_STORE)
+        q = ops.linear(q_latent, self.w_uq, None, ops.GEMM_STORE, settled=True)
         per_head = self.dim + self.rot
         if self.expands(ctx, pages):
             return self.attend_expanded(q, gate, ctx, pages, table, out)
@@ -264,7 +264,7 @@ class LatentAttention(Mixer):
         keys, values = held
         latents = torch.empty((count * page_size, self.kv_rank), dtype=dtype, device=device)
         ops.latent_gather(pages, table, owners, indices, ctx.ctx_len, self.kv_rank, self.heads, latents, keys)
-        expanded = ops.linear(latents, self.w_ukv, None, ops.GEMM_STORE)
+        expanded = ops.linear(latents, self.w_ukv, None, ops.GEMM_STORE, settled=True)
         ops.latent_scatter(expanded, count, self.dim, keys, values)
         queries = torch.empty_like(q)
         ops.rotate_runs(q, per, queries, per, self.heads, per, self.cos, self.sin, self.rot_dims, ctx.positions,
@@ -283,14 +283,14 @@ class LatentAttention(Mixer):
         return self.w_o, None
 
     def forward(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
-        return self.ops.linear(self.attend(h, ctx, cache), self.w_o, None, self.ops.GEMM_STORE)
+        return self.ops.linear(self.attend(h, ctx, cache), self.w_o, None, self.ops.GEMM_STORE, settled=True)
 
     def forward_f32(self, h, ctx: StepContext, cache: LayerCache, out=None, alpha: float = 1.0, accumulate: bool = False):
         epilogue = self.ops.GEMM_ADD_F32 if accumulate else self.ops.GEMM_STORE_F32
-        return self.ops.linear(self.attend(h, ctx, cache), self.w_o, None, epilogue, out=out, alpha=alpha)
+        return self.ops.linear(self.attend(h, ctx, cache), self.w_o, None, epilogue, out=out, alpha=alpha, settled=True)
 
     def forward_add(self, h: torch.Tensor, x: torch.Tensor, ctx: StepContext, cache: LayerCache, next_norm=None):
-        self.ops.linear(self.attend(h, ctx, cache), self.w_o, None, self.ops.GEMM_ADD_F32, out=x)
+        self.ops.linear(self.attend(h, ctx, cache), self.w_o, None, self.ops.GEMM_ADD_F32, out=x, settled=True)
         return None
 
 

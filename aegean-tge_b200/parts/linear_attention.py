@@ -92,7 +92,7 @@ class DecayLinearAttention(Mixer):
 
     def inner(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache, out: Optional[torch.Tensor] = None):
         ops = self.ops
-        rows = ops.linear(h, self.w_in, None, ops.GEMM_STORE)
+        rows = ops.linear(h, self.w_in, None, ops.GEMM_STORE, settled=True)
         o = ops.decay_scan(rows, 0, self.q_dim, 2 * self.q_dim, self.heads, self.head_dim, self.value_dim, self.decay,
                            cache.state["state"], ctx.slots, ctx.q_start, ctx.positions, ctx.num_seqs,
                            activation=self.activation == "silu", cos=self.cos, sin=self.sin, rotary=self.rotary,
@@ -105,14 +105,14 @@ class DecayLinearAttention(Mixer):
         return self.w_o, None
 
     def forward(self, h: torch.Tensor, ctx: StepContext, cache: LayerCache) -> torch.Tensor:
-        return self.ops.linear(self.inner(h, ctx, cache), self.w_o, None, self.ops.GEMM_STORE)
+        return self.ops.linear(self.inner(h, ctx, cache), self.w_o, None, self.ops.GEMM_STORE, settled=True)
 
     def forward_f32(self, h, ctx: StepContext, cache: LayerCache, out=None, alpha: float = 1.0, accumulate: bool = False):
         ops = self.ops
         a = self.inner(h, ctx, cache)
         if accumulate:
-            return ops.linear(a, self.w_o, None, ops.GEMM_ADD_F32, out=out, alpha=alpha)
-        return ops.linear(a, self.w_o, None, ops.GEMM_STORE_F32, out=out, alpha=alpha)
+            return ops.linear(a, self.w_o, None, ops.GEMM_ADD_F32, out=out, alpha=alpha, settled=True)
+        return ops.linear(a, self.w_o, None, ops.GEMM_STORE_F32, out=out, alpha=alpha, settled=True)
 
 
 @MIXERS.register("mixer_sum")

@@ -55,19 +55,19 @@ class SwiGLU(FeedForward):
         self.w_gate_up, self.w_down = gate_up, down
 
     def forward(self, h: torch.Tensor, ctx: StepContext) -> torch.Tensor:
-        a = self.ops.linear(h, self.w_gate_up, None, self.ops.GEMM_SWIGLU)
-        return self.ops.linear(a, self.w_down, None, self.ops.GEMM_STORE)
+        a = self.ops.linear(h, self.w_gate_up, None, self.ops.GEMM_SWIGLU, settled=True)
+        return self.ops.linear(a, self.w_down, None, self.ops.GEMM_STORE, settled=True)
 
     def forward_f32(self, h: torch.Tensor, ctx: StepContext) -> torch.Tensor:
-        a = self.ops.linear(h, self.w_gate_up, None, self.ops.GEMM_SWIGLU)
-        return self.ops.linear(a, self.w_down, None, self.ops.GEMM_STORE_F32)
+        a = self.ops.linear(h, self.w_gate_up, None, self.ops.GEMM_SWIGLU, settled=True)
+        return self.ops.linear(a, self.w_down, None, self.ops.GEMM_STORE_F32, settled=True)
 
     def forward_add(self, h: torch.Tensor, x: torch.Tensor, ctx: StepContext, next_norm=None, defer: bool = False):
-        a = self.ops.linear(h, self.w_gate_up, None, self.ops.GEMM_SWIGLU)
+        a = self.ops.linear(h, self.w_gate_up, None, self.ops.GEMM_SWIGLU, settled=True)
         fused = next_norm.fusable() if next_norm is not None else None
         if fused is not None:
-            return self.ops.linear_add_norm(a, self.w_down, None, x, fused[0], fused[1], self.env.dtype, defer=defer)
-        self.ops.linear(a, self.w_down, None, self.ops.GEMM_ADD_F32, out=x)
+            return self.ops.linear_add_norm(a, self.w_down, None, x, fused[0], fused[1], self.env.dtype, defer=defer, settled=True)
+        self.ops.linear(a, self.w_down, None, self.ops.GEMM_ADD_F32, out=x, settled=True)
         return None
 
 
@@ -137,7 +137,7 @@ class DenseMLP(FeedForward):
         self.w_up = view
 
     def inner(self, h, ctx: StepContext, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        rows = self.ops.linear(h, self.w_up, self.b_up, self.epilogue(), out=out)
+        rows = self.ops.linear(h, self.w_up, self.b_up, self.epilogue(), out=out, settled=True)
         if self.activation == "xielu":
             self.ops.activation(rows, self.ops.ACT_XIELU, self.act)
         elif self.activation == "relu_squared":
@@ -148,14 +148,14 @@ class DenseMLP(FeedForward):
         return self.w_down, self.b_down
 
     def forward(self, h: torch.Tensor, ctx: StepContext) -> torch.Tensor:
-        return self.ops.linear(self.inner(h, ctx), self.w_down, self.b_down, self.ops.GEMM_STORE)
+        return self.ops.linear(self.inner(h, ctx), self.w_down, self.b_down, self.ops.GEMM_STORE, settled=True)
 
     def forward_add(self, h: torch.Tensor, x: torch.Tensor, ctx: StepContext, next_norm=None, defer: bool = False):
         a = self.inner(h, ctx)
         fused = next_norm.fusable() if next_norm is not None else None
         if fused is not None:
-            return self.ops.linear_add_norm(a, self.w_down, self.b_down, x, fused[0], fused[1], self.env.dtype, defer=defer)
-        self.ops.linear(a, self.w_down, self.b_down, self.ops.GEMM_ADD_F32, out=x)
+            return self.ops.linear_add_norm(a, self.w_down, self.b_down, x, fused[0], fused[1], self.env.dtype, defer=defer, settled=True)
+        self.ops.linear(a, self.w_down, self.b_down, self.ops.GEMM_ADD_F32, out=x, settled=True)
         return None
 
 
@@ -200,24 +200,24 @@ class ClampedGLU(FeedForward):
     def inner(self, h, ctx: StepContext, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         if self.alpha == 1.702 and self.offset == 1.0:
             # the product's own epilogue clamps and gates (its constants are these two)
-            return self.ops.linear(h, self.w_gate_up, None, self.ops.GEMM_GLU_CLAMPED, out=out, alpha=self.limit)
+            return self.ops.linear(h, self.w_gate_up, None, self.ops.GEMM_GLU_CLAMPED, out=out, alpha=self.limit, settled=True)
         complete = getattr(h, "complete", None)
-        rows = self.ops.linear(h if complete is None else complete(), self.w_gate_up, None, self.ops.GEMM_STORE_F32)
+        rows = self.ops.linear(h if complete is None else complete(), self.w_gate_up, None, self.ops.GEMM_STORE_F32, settled=True)
         return self.ops.gated_clamp_act(rows, self.limit, self.alpha, self.offset, self.env.dtype, out=out)
 
     def output_projection(self):
         return self.w_down, None
 
     def forward(self, h: torch.Tensor, ctx: StepContext) -> torch.Tensor:
-        return self.ops.linear(self.inner(h, ctx), self.w_down, None, self.ops.GEMM_STORE)
+        return self.ops.linear(self.inner(h, ctx), self.w_down, None, self.ops.GEMM_STORE, settled=True)
 
     def forward_f32(self, h: torch.Tensor, ctx: StepContext) -> torch.Tensor:
-        return self.ops.linear(self.inner(h, ctx), self.w_down, None, self.ops.GEMM_STORE_F32)
+        return self.ops.linear(self.inner(h, ctx), self.w_down, None, self.ops.GEMM_STORE_F32, settled=True)
 
     def forward_add(self, h: torch.Tensor, x: torch.Tensor, ctx: StepContext, next_norm=None, defer: bool = False):
         a = self.inner(h, ctx)
         fused = next_norm.fusable() if next_norm is not None else None
         if fused is not None:
-            return self.ops.linear_add_norm(a, self.w_down, None, x, fused[0], fused[1], self.env.dtype, defer=defer)
-        self.ops.linear(a, self.w_down, None, self.ops.GEMM_ADD_F32, out=x)
+            return self.ops.linear_add_norm(a, self.w_down, None, x, fused[0], fused[1], self.env.dtype, defer=defer, settled=True)
+        self.ops.linear(a, self.w_down, None, self.ops.GEMM_ADD_F32, out=x, settled=True)
         return None

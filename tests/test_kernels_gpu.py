@@ -441,6 +441,23 @@ def test_gemm_tcgen05_stores_of_any_width_hold_the_same(ops, pair, M, N, K):
         ops.set_pair_gemm(1)
 
 
+@pytest.mark.parametrize("M,N,K", [(150, 256, 64), (193, 3584, 704), (300, 4608, 512), (2048, 768, 1024)])
+def test_gemm_pair_settled_weights_change_no_bit(ops, pair_everywhere, M, N, K):
+    """Weights asked for ahead of the kernel in front (fewer k-blocks than stages, cuts along k, several tiles to a pair), each product
+    reading what the one before it has written."""
+    gen = torch.Generator().manual_seed(N)
+    x, w = torch.randn(M, K, generator=gen).to(torch.bfloat16).to(DEV), (torch.randn(N, K, generator=gen) * 0.1).to(torch.bfloat16).to(DEV)
+    back = (torch.randn(K, N, generator=gen) * 0.05).to(torch.bfloat16).to(DEV)
+    results = []
+    for settled in (False, True):
+        rows = x
+        for _ in range(6):
+            rows = ops.linear(ops.linear(rows, w, None, ops.GEMM_STORE, settled=settled), back, None, ops.GEMM_STORE, settled=settled)
+        results.append(rows)
+    ops.check_status()
+    assert torch.equal(results[0], results[1]) and bool(torch.isfinite(results[0]).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 256, 128), (8, 3584, 512), (33, 520, 264), (128, 1024, 320), (140, 384, 192), (150, 384, 192)])
 @pytest.mark.parametrize("defer", [False, True])
 def test_linear_add_norm_and_rows_without_their_factor(ops, M, N, K, defer):
