@@ -18,12 +18,15 @@
 // First operands lie in tensor memory (a lane per token or state row), second operands in shared memory, split on their way in.
 // Measured (B200, 2,048 tokens, 28 heads of 128): states 150 -> 57 us, readout 337 -> 91 us; 14 heads of 64 with activated values of
 // 128: 108 -> 33 us and 137 -> 45 us.  Error against float64 2.85e-7 -> 1.7e-7, activated 1.97e-7 -> 1.44e-7.
+// One block holds an SM (all of its tensor memory), and its phases follow one another, so it is bound by their latencies: with sixteen
+// warps in place of eight (in a prompt of 2,048, us a layer) states 52 -> 45, readout 84 -> 75, activated 31 -> 23 and 37 -> 33.
 #include "tcgen05_ptx.cuh"
 
 namespace {
 
 constexpr int CHUNK = 128;               // tokens per chunk = lanes of tensor memory
-constexpr int THREADS = 256;             // two warps per 32-lane quarter, half of the columns each
+constexpr int THREADS = 512;             // four warps per 32-lane quarter, a quarter of the columns each
+constexpr int PARTS = THREADS / 128;
 constexpr int ACC_COLS = 256;            // two accumulators of up to 128 columns
 constexpr int OPERAND_BYTES = 128 * 128 * 2;   // one part of a second operand of up to 128 x 128
 constexpr int TMEM_COLS = 512;
@@ -100,7 +103,7 @@ __device__ __forceinline__ void store_parts(unsigned char* base, int block, int 
 // 128 bytes per token.  Plain values are bfloat16 (one part), activated ones float32 (three).
 template <int VDIM>
 __device__ __forceinline__ void load_values(const ScanTcParams& p, unsigned char* base, int first, int count, int head, int tid) {
-#pragma unroll 4
+#pragma unroll 2
   for (int e = tid; e < CHUNK * VDIM / 8; e += THREADS) {
     const int t = e / (VDIM / 8), c = (e % (VDIM / 8)) * 8;
     float v[8];
@@ -244,6 +247,7 @@ __device__ __forceinline__ void operands_ready() {
 // ---- a chunk's own contribution to the state: lanes are the state's rows, the contraction runs over the tokens ----
 template <int DIM, int VDIM>
 __global__ void __launch_bounds__(THREADS, 1) decay_chunk_state_kernel(const ScanTcParams p) {
+  constexpr int COLS = VDIM / PARTS;       // result columns of a warp
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
@@ -257,10 +261,10 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_state_kernel(const Sca
   const BlockSetup s = set_up(smem_raw, &tmem_slot, &abort_word, bar, powers, p.decay[head], tid, warp);
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t a = s.tmem + ACC_COLS;
-  const int half = warp >> 2, row = (warp & 3) * 32 + lane;
-  // first operand: k_j[row] c^(n-1-j), this warp's 64 of the 128 tokens
-#pragma unroll
-  for (int t0 = half * 64; t0 < half * 64 + 64; t0 += 32) {
+  const int part = warp >> 2, row = (warp & 3) * 32 + lane;
+  // first operand: k_j[row] c^(n-1-j), this warp's 32 of the 128 tokens
+  {
+    const int t0 = part * (CHUNK / PARTS);
     float v[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
@@ -282,20 +286,20 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_state_kernel(const Sca
   }
   const bool ok = mbar_wait(bar, 0, p.status, &abort_word);
   tc_fence_after();
-  float* dst = p.carry + (((size_t)piece * p.heads + head) * DIM + row) * VDIM + half * (VDIM / 2);
-  float sums[VDIM / 2];
-  read_sums<VDIM / 2, 2>(s.tmem + lane_base + half * (VDIM / 2), 128, sums);
-  if (__syncthreads_or(!(not_finite<VDIM / 2>(sums) == 0.0f))) {
-    for (int c = 0; c < VDIM / 2 && row < DIM; ++c) {
+  float* dst = p.carry + (((size_t)piece * p.heads + head) * DIM + row) * VDIM + part * COLS;
+  float sums[COLS];
+  read_sums<COLS, 2>(s.tmem + lane_base + part * COLS, 128, sums);
+  if (__syncthreads_or(!(not_finite<COLS>(sums) == 0.0f))) {
+    for (int c = 0; c < COLS && row < DIM; ++c) {
       float sum = 0.0f;
       for (int j = 0; j < count; ++j)
         sum = fmaf(p.prepared[((size_t)(first + j) * p.heads + head) * 2 * DIM + DIM + row] * powers[count - 1 - j],
-                   value_at<VDIM>(p, first + j, head, half * (VDIM / 2) + c), sum);
+                   value_at<VDIM>(p, first + j, head, part * COLS + c), sum);
       dst[c] = sum;
     }
   } else if (ok && row < DIM) {
 #pragma unroll
-    for (int c = 0; c < VDIM / 2; c += 8) store8(dst + c, sums + c);
+    for (int c = 0; c < COLS; c += 8) store8(dst + c, sums + c);
   }
   tear_down(s.tmem, warp);
 }
@@ -303,6 +307,7 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_state_kernel(const Sca
 // ---- the readout of a chunk: lanes are its tokens ----
 template <int DIM, int VDIM>
 __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const ScanTcParams p) {
+  constexpr int COLS = VDIM / PARTS;       // result columns of a warp
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
@@ -316,24 +321,23 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
   const BlockSetup s = set_up(smem_raw, &tmem_slot, &abort_word, bar, powers, p.decay[head], tid, warp);
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t a = s.tmem + ACC_COLS;
-  const int half = warp >> 2, row = (warp & 3) * 32 + lane;
+  const int part = warp >> 2, row = (warp & 3) * 32 + lane;
   unsigned char* second = s.generic;                          // the state, then the keys
   unsigned char* values = s.generic + 3 * OPERAND_BYTES;
-  const float* own = p.prepared + ((size_t)(first + min(row, count - 1)) * p.heads + head) * 2 * DIM + half * (DIM / 2);
-  // the token's query, this warp's half of it
-#pragma unroll
-  for (int i0 = 0; i0 < DIM / 2; i0 += 32) {
+  const float* own = p.prepared + ((size_t)(first + min(row, count - 1)) * p.heads + head) * 2 * DIM + part * 32;
+  // the token's query, 32 numbers to a warp
+  if (part * 32 < DIM) {
     float v[32];
 #pragma unroll
     for (int i = 0; i < 32; i += 4) {
-      const float4 q = row < count ? *reinterpret_cast<const float4*>(own + i0 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 q = row < count ? *reinterpret_cast<const float4*>(own + i) : make_float4(0.f, 0.f, 0.f, 0.f);
       v[i] = q.x; v[i + 1] = q.y; v[i + 2] = q.z; v[i + 3] = q.w;
     }
-    store_lane32(a + lane_base + (half * (DIM / 2) + i0) / 2, DIM / 2, v);
+    store_lane32(a + lane_base + part * 16, DIM / 2, v);
   }
   // the state the chunk starts from, [dim][vdim]: contiguous along vdim
   const float* state = p.carry + ((size_t)piece * p.heads + head) * DIM * VDIM;
-#pragma unroll 4
+#pragma unroll 2
   for (int e = tid; e < DIM * VDIM / 8; e += THREADS) {
     const int i = e / (VDIM / 8), c = (e % (VDIM / 8)) * 8;
     const float4 x = *reinterpret_cast<const float4*>(state + (size_t)i * VDIM + c), y = *reinterpret_cast<const float4*>(state + (size_t)i * VDIM + c + 4);
@@ -351,15 +355,15 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
   load_values<VDIM>(p, values, first, count, head, tid);      // while the products run
   bool ok = mbar_wait(bar, 0, p.status, &abort_word);
   tc_fence_after();
-  float o[VDIM / 2];
-  read_sums<VDIM / 2, DIM / 64>(s.tmem + lane_base + half * (VDIM / 2), 128, o);
+  float o[COLS];
+  read_sums<COLS, DIM / 64>(s.tmem + lane_base + part * COLS, 128, o);
   {
     const float carried = powers[row + 1];
 #pragma unroll
-    for (int c = 0; c < VDIM / 2; ++c) o[c] *= carried;
+    for (int c = 0; c < COLS; ++c) o[c] *= carried;
   }
   // the keys [token][dim] over the state, contiguous along the contraction
-#pragma unroll 4
+#pragma unroll 2
   for (int e = tid; e < CHUNK * DIM / 8; e += THREADS) {
     const int t = e / (DIM / 8), i = (e % (DIM / 8)) * 8;
     float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -380,17 +384,16 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
   }
   ok = mbar_wait(bar, 1, p.status, &abort_word) && ok;
   tc_fence_after();
-  // decayed scores of this token with keys 64 half ... 64 half + 63, as first operand of the next product (over the query)
-#pragma unroll
-  for (int j0 = 0; j0 < 64; j0 += 32) {
+  // decayed scores of this token with keys 32 part ... 32 part + 31, as first operand of the next product (over the query)
+  {
     float v[32];
-    read_sums<32, DIM / 64>(s.tmem + lane_base + half * 64 + j0, 128, v);
+    read_sums<32, DIM / 64>(s.tmem + lane_base + part * 32, 128, v);
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
-      const int gap = row - (half * 64 + j0 + j);
+      const int gap = row - (part * 32 + j);
       v[j] = gap >= 0 ? v[j] * powers[max(gap, 0)] : 0.0f;
     }
-    store_lane32(a + lane_base + (half * 64 + j0) / 2, CHUNK / 2, v);
+    store_lane32(a + lane_base + part * 16, CHUNK / 2, v);
   }
   operands_ready();
   if (warp == 0) {
@@ -404,30 +407,30 @@ __global__ void __launch_bounds__(THREADS, 1) decay_chunk_readout_kernel(const S
   ok = mbar_wait(bar, 0, p.status, &abort_word) && ok;
   tc_fence_after();
 #pragma unroll
-  for (int c = 0; c < VDIM / 2; c += 16) {
+  for (int c = 0; c < COLS; c += 16) {
     float more[16];
-    read_sums<16, 2>(s.tmem + lane_base + half * (VDIM / 2) + c, 128, more);
+    read_sums<16, 2>(s.tmem + lane_base + part * COLS + c, 128, more);
 #pragma unroll
     for (int j = 0; j < 16; ++j) o[c + j] += more[j];
   }
-  float* dst = p.out + (size_t)(first + row) * p.heads * VDIM + (size_t)head * VDIM + half * (VDIM / 2);
-  if (__syncthreads_or(!(not_finite<VDIM / 2>(o) == 0.0f))) {
+  float* dst = p.out + (size_t)(first + row) * p.heads * VDIM + (size_t)head * VDIM + part * COLS;
+  if (__syncthreads_or(!(not_finite<COLS>(o) == 0.0f))) {
     const float* q = p.prepared + ((size_t)(first + row) * p.heads + head) * 2 * DIM;
-    for (int c = 0; c < VDIM / 2 && row < count; ++c) {
+    for (int c = 0; c < COLS && row < count; ++c) {
       float sum = 0.0f;
-      for (int i = 0; i < DIM; ++i) sum = fmaf(q[i], state[(size_t)i * VDIM + half * (VDIM / 2) + c], sum);
+      for (int i = 0; i < DIM; ++i) sum = fmaf(q[i], state[(size_t)i * VDIM + part * COLS + c], sum);
       sum *= powers[row + 1];
       for (int j = 0; j <= row; ++j) {
         const float* k = p.prepared + ((size_t)(first + j) * p.heads + head) * 2 * DIM + DIM;
         float score = 0.0f;
         for (int i = 0; i < DIM; ++i) score = fmaf(q[i], k[i], score);
-        sum = fmaf(score * powers[row - j], value_at<VDIM>(p, first + j, head, half * (VDIM / 2) + c), sum);
+        sum = fmaf(score * powers[row - j], value_at<VDIM>(p, first + j, head, part * COLS + c), sum);
       }
       dst[c] = sum;
     }
   } else if (ok && row < count) {
 #pragma unroll
-    for (int c = 0; c < VDIM / 2; c += 8) store8(dst + c, o + c);
+    for (int c = 0; c < COLS; c += 8) store8(dst + c, o + c);
   }
   tear_down(s.tmem, warp);
 }
