@@ -598,6 +598,40 @@ def test_convolution_norm_rotation_and_store(ops, dtype, heads, kv_heads, dim, v
             assert rel_error(state[slots[s]].cpu(), torch.from_numpy(tail)) < 1e-6
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps,rotary", [(5, 1, 128, 128, 4, 64), (4, 2, 64, 32, 3, 64), (3, 1, 24, 40, 2, 16), (28, 4, 128, 128, 4, 0)])
+@pytest.mark.parametrize("norm_last", [0, 1])
+@pytest.mark.parametrize("q_lens", [[16], [1, 2, 3, 9, 2], [33, 1, 30]])
+def test_convolution_by_eights_against_single_channels(ops, heads, kv_heads, dim, vdim, taps, rotary, norm_last, q_lens):
+    """The kernel for eight channels and four tokens at a time against the one for single channels (whose rows start on odd elements),
+    requests of fewer tokens than taps beside longer ones, each with a state: the sums of squares alone are added in another order."""
+    from aegean_tge_b200.parts.rope import rotary_tables
+    gen = torch.Generator().manual_seed(dim + taps)
+    channels, tokens = (heads + kv_heads) * dim + kv_heads * vdim, sum(q_lens)
+    raw = torch.randn(tokens, channels + 16, generator=gen).to(torch.bfloat16).to(DEV)
+    odd = torch.zeros(tokens, channels + 17, dtype=torch.bfloat16, device=DEV)
+    odd[:, 1:] = raw
+    conv_w = torch.randn(channels, taps, generator=gen).to(DEV)
+    q_norm, k_norm = (1.0 + 0.2 * torch.randn(dim, generator=gen).to(DEV) for _ in range(2))
+    cos, sin = (t.to(DEV) for t in rotary_tables(5000.0, max(rotary, 2), 256))
+    starts = [7 * s for s in range(len(q_lens))]
+    positions, seq, q_start = _steps(q_lens, starts)
+    slots = _i32([(3 * s + 2) % 7 for s in range(len(q_lens))])
+    first_state = torch.randn(7, taps - 1, channels, generator=gen).to(DEV)
+    results = []
+    for rows in (raw[:, :channels], odd[:, 1:1 + channels]):
+        k_pages, table = _paged([a + n for a, n in zip(starts, q_lens)], kv_heads, dim, 16, torch.bfloat16, 7)
+        v_pages, _ = _paged([a + n for a, n in zip(starts, q_lens)], kv_heads, vdim, 16, torch.bfloat16, 7)
+        state = first_state.clone()
+        q = ops.conv_norm_rope_store(rows, conv_w, taps, state, slots, q_start, len(q_lens), q_norm, k_norm, 1e-5, cos, sin, rotary,
+                                     positions, seq, table, k_pages, v_pages, heads, kv_heads, dim, vdim, norm_last=bool(norm_last))
+        results.append((q, k_pages, v_pages, state))
+    ops.check_status()
+    # a bfloat16 step apart at most where the norm's factor differs in its last bits (and those, where a rotation cancels)
+    for got, want in zip(*results):
+        assert torch.allclose(got.float(), want.float(), rtol=2.0 ** -7, atol=2e-6)
+    assert torch.equal(results[0][2], results[1][2]) and torch.equal(results[0][3], results[1][3])
+
+
 def _window_pool_case(ops, dtype, heads, kv_heads, dim, vdim, size, pool, lengths, tails, page_size, spike=None):
     """Requests of ``lengths`` whose last ``tails[s]`` tokens come in a second step (0: all at once).  Keys and
     values are stored and pooled by the kernels; the queries of both steps are checked.  ``spike`` = (request, key
