@@ -308,13 +308,90 @@ __global__ void __launch_bounds__(256) decay_prepare_vec_kernel(
   }
 }
 
+// The same eight numbers at a time, sixteen where a unit is turned (eight of the lower half and the eight they are paired with), a block per
+// token (everything a multiple of eight).  Bound by its bytes, two thirds of them the float32 results (88 MB for 2,048 tokens of 28 heads
+// of 128, where the kernel above takes 32 us).
+__global__ void __launch_bounds__(256) decay_prepare_eights_kernel(
+    const __nv_bfloat16* __restrict__ rows, long long ld, int q_off, int k_off, int heads, int dim, int activation,
+    const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary,
+    float k_scale, const int* __restrict__ positions, float* __restrict__ prepared, int* status) {
+  pdl_trigger();
+  const int t = blockIdx.x, half = rotary >> 1;
+  int position = positions[t];
+  if (rotary > 0 && (position < 0 || position >= table_positions)) {
+    if (threadIdx.x == 0) atomicOr(status, TGE_STATUS_BAD_ROW);
+    position = 0;
+  }
+  const int turned = half >> 3, units = turned + ((dim - rotary) >> 3);
+  pdl_wait();
+  auto eight = [&](const __nv_bfloat16* at, float v[8]) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(at);
+    const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      v[2 * i] = __uint_as_float(w[i] << 16);
+      v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+    if (activation) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = silu_f(v[i]);
+    }
+  };
+  auto store = [&](float* at, const float v[8]) {
+    reinterpret_cast<float4*>(at)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(at)[1] = make_float4(v[4], v[5], v[6], v[7]);
+  };
+  for (int u = threadIdx.x; u < heads * units; u += 256) {
+    const int head = u / units, unit = u - head * units;
+    const __nv_bfloat16* q_row = rows + (size_t)t * ld + q_off + head * dim;
+    const __nv_bfloat16* k_row = rows + (size_t)t * ld + k_off + head * dim;
+    float* dst = prepared + ((size_t)t * heads + head) * 2 * dim;
+    const bool turns = unit < turned;
+    const int i = turns ? unit * 8 : rotary + (unit - turned) * 8;
+    float q[8], k[8];
+    eight(q_row + i, q);
+    eight(k_row + i, k);
+    if (turns) {
+      float q2[8], k2[8], cs[8], sn[8];
+      eight(q_row + i + half, q2);
+      eight(k_row + i + half, k2);
+#pragma unroll
+      for (int e = 0; e < 8; e += 4) {
+        const float4 c = *reinterpret_cast<const float4*>(cos_table + (size_t)position * half + i + e);
+        const float4 n = *reinterpret_cast<const float4*>(sin_table + (size_t)position * half + i + e);
+        cs[e] = c.x; cs[e + 1] = c.y; cs[e + 2] = c.z; cs[e + 3] = c.w;
+        sn[e] = n.x; sn[e + 1] = n.y; sn[e + 2] = n.z; sn[e + 3] = n.w;
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {     // the pair (u, v) = (element i, element i + half) becomes (u cos - v sin, v cos + u sin)
+        const float u0 = q[e], v0 = q2[e], u1 = k[e], v1 = k2[e];
+        q[e] = u0 * cs[e] - v0 * sn[e];
+        q2[e] = v0 * cs[e] + u0 * sn[e];
+        k[e] = u1 * cs[e] - v1 * sn[e];
+        k2[e] = (v1 * cs[e] + u1 * sn[e]) * k_scale;
+      }
+      store(dst + i + half, q2);
+      store(dst + dim + i + half, k2);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) k[e] *= k_scale;
+    store(dst + i, q);
+    store(dst + dim + i, k);
+  }
+}
+
 template <typename T>
 void launch_decay_prepare(const T* rows, long long ld, int q_off, int k_off, int heads, int dim, int activation, const float* cos_table,
                           const float* sin_table, int table_positions, int rotary, float k_scale, const int* positions, float* prepared,
                           int tokens, int* status, cudaStream_t stream) {
   const bool pairs = sizeof(T) == 2 && ld % 2 == 0 && q_off % 2 == 0 && k_off % 2 == 0 && dim % 2 == 0 && rotary % 4 == 0 &&
                      (uintptr_t)rows % 4 == 0 && (uintptr_t)cos_table % 8 == 0 && (uintptr_t)sin_table % 8 == 0 && (uintptr_t)prepared % 8 == 0;
-  if (pairs)
+  const bool eights = pairs && dim % 8 == 0 && rotary % 16 == 0 && ld % 8 == 0 && q_off % 8 == 0 && k_off % 8 == 0 &&
+                      (((uintptr_t)rows | (uintptr_t)cos_table | (uintptr_t)sin_table | (uintptr_t)prepared) & 15) == 0;
+  if (eights)
+    tge_launch(decay_prepare_eights_kernel, dim3(tokens), dim3(256), 0, stream, (const __nv_bfloat16*)rows, ld, q_off, k_off, heads,
+               dim, activation, cos_table, sin_table, table_positions, rotary, k_scale, positions, prepared, status);
+  else if (pairs)
     tge_launch(decay_prepare_vec_kernel, dim3(tokens, (heads + 7) / 8), dim3(256), 0, stream, (const __nv_bfloat16*)rows, ld, q_off, k_off, heads,
                dim, activation, cos_table, sin_table, table_positions, rotary, k_scale, positions, prepared, status);
   else
@@ -860,6 +937,49 @@ __global__ void __launch_bounds__(256) gated_norm_vec_kernel(const float* __rest
   }
 }
 
+// Groups of up to 128 numbers, four to a warp, so that four rows' loads are on their way together (with a group to a warp each waited
+// for one: 2,048 tokens, 28 groups of 128, 22 us); a group's sum is the kernel's above.
+constexpr int GATED_EACH = 4;
+__global__ void __launch_bounds__(256) gated_norm_small_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ gate, long long ld_gate,
+                                                               const float* __restrict__ weight, __nv_bfloat16* __restrict__ out, long long ld_out,
+                                                               int tokens, int groups, int size, float eps, int act) {
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, quads = size >> 2;
+  const unsigned unit0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * GATED_EACH, units = (unsigned)tokens * groups;      // below 2^31
+  pdl_wait();
+  float4 y[GATED_EACH];
+  uint2 raw[GATED_EACH];
+#pragma unroll
+  for (int k = 0; k < GATED_EACH; ++k) {
+    y[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    raw[k] = make_uint2(0u, 0u);
+    if (unit0 + k < units && lane < quads) {
+      const unsigned t = (unit0 + k) / groups, g = unit0 + k - t * groups;
+      y[k] = reinterpret_cast<const float4*>(o + (size_t)(unit0 + k) * size)[lane];
+      raw[k] = reinterpret_cast<const uint2*>(gate + (size_t)t * ld_gate + (size_t)g * size)[lane];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < GATED_EACH; ++k) {
+    const float z[4] = {__uint_as_float(raw[k].x << 16), __uint_as_float(raw[k].x & 0xffff0000u), __uint_as_float(raw[k].y << 16),
+                        __uint_as_float(raw[k].y & 0xffff0000u)};
+    float a[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) a[e] = act == 1 ? sigmoid_f(z[e]) : silu_f(z[e]);
+    const float4 gated = make_float4(y[k].x * a[0], y[k].y * a[1], y[k].z * a[2], y[k].w * a[3]);
+    const float4 v = act == 2 ? gated : y[k];
+    float sum = fmaf(v.x, v.x, 0.0f);
+    sum = fmaf(v.y, v.y, sum); sum = fmaf(v.z, v.z, sum); sum = fmaf(v.w, v.w, sum);
+    const float scale = 1.0f / sqrtf(warp_sum(sum) / (float)size + eps);
+    if (unit0 + k < units && lane < quads) {
+      const unsigned t = (unit0 + k) / groups, g = unit0 + k - t * groups;
+      const float4 w = weight != nullptr ? reinterpret_cast<const float4*>(weight + (size_t)g * size)[lane] : make_float4(1.f, 1.f, 1.f, 1.f);
+      store_quad(out + (size_t)t * ld_out + (size_t)g * size + 4 * lane,
+                 make_float4(gated.x * scale * w.x, gated.y * scale * w.y, gated.z * scale * w.z, gated.w * scale * w.w));
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // After the q/k/v product: the short convolution over time, the per-head norm of q and k, their rotation, and the
 // store.  One warp per (token, head of q, k or v).  `raw` holds the projections of this step's tokens [T, q | k | v];
@@ -1010,62 +1130,65 @@ __global__ void conv_state_update_kernel(const T* __restrict__ raw, long long ld
   }
 }
 
-constexpr int POOL_AHEAD = 8;
+constexpr int POOL_AHEAD = 16, POOL_THREADS = 256;
 
 // The mean key and mean value of every block of `pool` positions whose last token this step brings: one block of
-// threads per (token, kv head); only tokens at a block's last position do anything.  The means are taken over the
+// threads per (32 tokens, kv head), which looks for the tokens at a block's last position among them.  The means are taken over the
 // keys and values as their pages hold them, and entry b of a request lies where position b would in the pooled pages.
+// Bound by round trips: POOL_AHEAD positions' pages, then their numbers, are on their way together, added in order.  2,048 tokens, 4 kv heads
+// of 128, blocks of 64: 69 us one position after the other; 34 eight at a time, a block of threads per token (63 of 64 only left).
 template <typename T>
-__global__ void __launch_bounds__(128) pool_kv_kernel(
+__global__ void __launch_bounds__(POOL_THREADS) pool_kv_kernel(
     const T* __restrict__ k_pages, const T* __restrict__ v_pages, const int* __restrict__ block_table, int max_pages,
     int num_pages, T* __restrict__ kp_pages, T* __restrict__ vp_pages, const int* __restrict__ pool_table,
     int pool_max_pages, int pool_num_pages, int page_size, const int* __restrict__ positions,
-    const int* __restrict__ seq_of_token, int kv_heads, int dim, int vdim, int pool, int* status) {
+    const int* __restrict__ seq_of_token, int tokens, int kv_heads, int dim, int vdim, int pool, int* status) {
   pdl_trigger();
+  const int first = blockIdx.x * 32, head = blockIdx.y, lane = threadIdx.x & 31;
+  const int mine = first + lane < tokens ? positions[first + lane] : -1;
+  unsigned ends = __ballot_sync(0xffffffffu, mine >= 0 && (mine + 1) % pool == 0);      // the same in every warp
   pdl_wait();
-  const int t = blockIdx.x, head = blockIdx.y;
-  const int position = positions[t];
-  if (position < 0 || (position + 1) % pool != 0) return;
-  const int seq = seq_of_token[t];
-  const int entry = (position + 1) / pool - 1;
-  const int entry_page = entry / page_size;
-  const int out_page = entry_page < pool_max_pages ? pool_table[(size_t)seq * pool_max_pages + entry_page] : -1;
-  if (out_page < 0 || out_page >= pool_num_pages) {
-    if (threadIdx.x == 0) atomicOr(status, TGE_STATUS_BAD_PAGE);
-    return;
-  }
-  for (int e = threadIdx.x; e < dim + vdim; e += blockDim.x) {
-    const bool is_key = e < dim;
-    const int size = is_key ? dim : vdim, d = is_key ? e : e - dim;
-    const T* pages = is_key ? k_pages : v_pages;
-    float sum = 0.0f;
-    bool ok = true;
-    // eight positions' pages, then their numbers, on their way together; added in order.  (One after the other, each behind the
-    // look at its page, the 64 of a block were a chain of loads:
-    // 2,048 tokens, 4 kv heads of 128, blocks of 64: 69 us, now 37.)
-    for (int p0 = position - pool + 1; p0 <= position && ok; p0 += POOL_AHEAD) {
-      const T* at[POOL_AHEAD];
-      T value[POOL_AHEAD];
-#pragma unroll
-      for (int j = 0; j < POOL_AHEAD; ++j) {
-        const int p = min(p0 + j, position), page_index = p / page_size;
-        const int page = page_index < max_pages ? block_table[(size_t)seq * max_pages + page_index] : -1;
-        const bool good = page >= 0 && page < num_pages;
-        ok = ok && good;
-        at[j] = pages + (((size_t)(good ? page : 0) * kv_heads + head) * page_size + (p - page_index * page_size)) * size + d;
-      }
-#pragma unroll
-      for (int j = 0; j < POOL_AHEAD; ++j) value[j] = *at[j];
-#pragma unroll
-      for (int j = 0; j < POOL_AHEAD; ++j)
-        if (p0 + j <= position) sum += to_float<T>(value[j]);
-    }
-    if (!ok) {
-      atomicOr(status, TGE_STATUS_BAD_PAGE);
+  for (; ends != 0; ends &= ends - 1) {
+    const int t = first + __ffs(ends) - 1;
+    const int position = __shfl_sync(0xffffffffu, mine, t - first);
+    const int seq = seq_of_token[t];
+    const int entry = (position + 1) / pool - 1;
+    const int entry_page = entry / page_size;
+    const int out_page = entry_page < pool_max_pages ? pool_table[(size_t)seq * pool_max_pages + entry_page] : -1;
+    if (out_page < 0 || out_page >= pool_num_pages) {
+      if (threadIdx.x == 0) atomicOr(status, TGE_STATUS_BAD_PAGE);
       continue;
     }
-    T* dst = (is_key ? kp_pages : vp_pages) + (((size_t)out_page * kv_heads + head) * page_size + entry % page_size) * size + d;
-    *dst = from_float<T>(sum / (float)pool);
+    for (int e = threadIdx.x; e < dim + vdim; e += POOL_THREADS) {
+      const bool is_key = e < dim;
+      const int size = is_key ? dim : vdim, d = is_key ? e : e - dim;
+      const T* pages = is_key ? k_pages : v_pages;
+      float sum = 0.0f;
+      bool ok = true;
+      for (int p0 = position - pool + 1; p0 <= position && ok; p0 += POOL_AHEAD) {
+        const T* at[POOL_AHEAD];
+        T value[POOL_AHEAD];
+#pragma unroll
+        for (int j = 0; j < POOL_AHEAD; ++j) {
+          const int p = min(p0 + j, position), page_index = p / page_size;
+          const int page = page_index < max_pages ? block_table[(size_t)seq * max_pages + page_index] : -1;
+          const bool good = page >= 0 && page < num_pages;
+          ok = ok && good;
+          at[j] = pages + (((size_t)(good ? page : 0) * kv_heads + head) * page_size + (p - page_index * page_size)) * size + d;
+        }
+#pragma unroll
+        for (int j = 0; j < POOL_AHEAD; ++j) value[j] = *at[j];
+#pragma unroll
+        for (int j = 0; j < POOL_AHEAD; ++j)
+          if (p0 + j <= position) sum += to_float<T>(value[j]);
+      }
+      if (!ok) {
+        atomicOr(status, TGE_STATUS_BAD_PAGE);
+        continue;
+      }
+      T* dst = (is_key ? kp_pages : vp_pages) + (((size_t)out_page * kv_heads + head) * page_size + entry % page_size) * size + d;
+      *dst = from_float<T>(sum / (float)pool);
+    }
   }
 }
 
@@ -1269,7 +1392,11 @@ TGE_API int tge_gated_norm(const float* o, const void* gate, int is_bf16, long l
   // four numbers at a time where the rows allow it: a warp to a group of up to 512 numbers, a block up to 4,096
   const bool quads = is_bf16 && size % 4 == 0 && ld_gate % 4 == 0 && ld_out % 4 == 0 && size <= 256 * 4 * GATED_QUADS && units <= 0x7fffffffll &&
                      (uintptr_t)o % 16 == 0 && (uintptr_t)gate % 8 == 0 && (uintptr_t)out % 8 == 0 && (uintptr_t)weight % 16 == 0;
-  if (quads && size <= 32 * 4 * GATED_QUADS)
+  // four groups to a warp where they fill the chip that way
+  if (quads && size <= 128 && units >= (long long)GATED_EACH * 32 * tge_sm_count())
+    tge_launch(gated_norm_small_kernel, dim3((unsigned)((units + 8 * GATED_EACH - 1) / (8 * GATED_EACH))), dim3(256), 0, stream, o,
+               (const __nv_bfloat16*)gate, ld_gate, weight, (__nv_bfloat16*)out, ld_out, tokens, groups, size, eps, act);
+  else if (quads && size <= 32 * 4 * GATED_QUADS)
     tge_launch(gated_norm_vec_kernel<32>, dim3((unsigned)((units + 7) / 8)), dim3(256), 0, stream, o, (const __nv_bfloat16*)gate, ld_gate, weight,
                (__nv_bfloat16*)out, ld_out, tokens, groups, size, eps, act);
   else if (quads)
@@ -1609,16 +1736,16 @@ TGE_API int tge_pool_kv(const void* k_pages, const void* v_pages, int is_bf16, c
                         int kv_heads, int dim, int vdim, int pool, int* status, cudaStream_t stream) {
   TGE_REQUIRE(pool > 0 && kv_heads > 0 && dim > 0 && vdim > 0 && page_size > 0, "pool_kv: bad shape");
   if (tokens == 0) return 0;
-  dim3 grid(tokens, kv_heads);
+  dim3 grid((tokens + 31) / 32, kv_heads);
   if (is_bf16)
-    tge_launch(pool_kv_kernel<__nv_bfloat16>, grid, dim3(128), 0, stream,
+    tge_launch(pool_kv_kernel<__nv_bfloat16>, grid, dim3(POOL_THREADS), 0, stream,
         (const __nv_bfloat16*)k_pages, (const __nv_bfloat16*)v_pages, block_table, max_pages, num_pages,
         (__nv_bfloat16*)kp_pages, (__nv_bfloat16*)vp_pages, pool_table, pool_max_pages, pool_num_pages, page_size, positions,
-        seq_of_token, kv_heads, dim, vdim, pool, status);
+        seq_of_token, tokens, kv_heads, dim, vdim, pool, status);
   else
-    tge_launch(pool_kv_kernel<float>, grid, dim3(128), 0, stream, (const float*)k_pages, (const float*)v_pages, block_table, max_pages,
+    tge_launch(pool_kv_kernel<float>, grid, dim3(POOL_THREADS), 0, stream, (const float*)k_pages, (const float*)v_pages, block_table, max_pages,
                                                      num_pages, (float*)kp_pages, (float*)vp_pages, pool_table,
-                                                     pool_max_pages, pool_num_pages, page_size, positions, seq_of_token,
+                                                     pool_max_pages, pool_num_pages, page_size, positions, seq_of_token, tokens,
                                                      kv_heads, dim, vdim, pool, status);
   return tge_launched("pool_kv", 1);
 }

@@ -632,6 +632,43 @@ def test_convolution_by_eights_against_single_channels(ops, heads, kv_heads, dim
     assert torch.equal(results[0][2], results[1][2]) and torch.equal(results[0][3], results[1][3])
 
 
+@pytest.mark.parametrize("heads,dim,rotary,activation", [(3, 128, 128, False), (5, 64, 16, True), (2, 24, 0, False), (1, 40, 32, True)])
+def test_decay_scan_prepares_by_eights_as_by_single_numbers(ops, heads, dim, rotary, activation):
+    """q and k prepared eight numbers at a time against rows that start on odd elements (prepared singly), through the scan: whole heads turned,
+    their first numbers, none; a last unit behind the turned ones."""
+    from aegean_tge_b200.parts.rope import rotary_tables
+    gen = torch.Generator().manual_seed(dim)
+    tokens, vdim = 96, 32
+    width = heads * (2 * dim + vdim)
+    even = torch.randn(tokens, width + 8, generator=gen).to(torch.bfloat16).to(DEV)
+    odd = torch.zeros(tokens, width + 9, dtype=torch.bfloat16, device=DEV)
+    odd[:, 1:] = even
+    cos, sin = (t.to(DEV) for t in rotary_tables(5000.0, max(rotary, 2), 256))
+    decay = torch.linspace(0.9, 0.99, heads, device=DEV)
+    positions = torch.arange(3, 3 + tokens, dtype=torch.int32, device=DEV)
+    results = []
+    for rows in (even, odd[:, 1:]):
+        state = torch.zeros(1, heads, dim, vdim, device=DEV)
+        out = ops.decay_scan(rows, 0, heads * dim, 2 * heads * dim, heads, dim, vdim, decay, state, _i32([0]), _i32([0, tokens]), positions, 1,
+                             activation=activation, cos=cos, sin=sin, rotary=rotary, k_scale=0.125, max_q_len=tokens)
+        results.append((out, state))
+    ops.check_status()
+    for got, want in zip(*results):         # a multiply-add contracted the other way round: the last bit of a prepared number
+        assert rel_error(got, want.cpu().double()) < 1e-6
+
+
+@pytest.mark.parametrize("tokens,groups,size", [(1200, 16, 128), (700, 28, 100), (19000, 1, 4)])
+@pytest.mark.parametrize("sigmoid,gate_first", [(False, False), (True, False), (False, True)])
+def test_gated_norm_four_groups_to_a_warp_has_the_bits_of_one(ops, tokens, groups, size, sigmoid, gate_first):
+    gen = torch.Generator().manual_seed(size)
+    o, gate = torch.randn(tokens, groups * size, generator=gen).to(DEV), torch.randn(tokens, groups * size, generator=gen).to(torch.bfloat16).to(DEV)
+    weight = 1.0 + 0.1 * torch.randn(groups * size, generator=gen).to(DEV)
+    many = ops.gated_norm(o, gate, weight, groups, 1e-5, sigmoid, gate_first=gate_first)
+    few = torch.cat([ops.gated_norm(o[a:a + 100].contiguous(), gate[a:a + 100], weight, groups, 1e-5, sigmoid, gate_first=gate_first)
+                     for a in range(0, tokens, 100)])
+    assert torch.equal(many, few)
+
+
 def _window_pool_case(ops, dtype, heads, kv_heads, dim, vdim, size, pool, lengths, tails, page_size, spike=None):
     """Requests of ``lengths`` whose last ``tails[s]`` tokens come in a second step (0: all at once).  Keys and
     values are stored and pooled by the kernels; the queries of both steps are checked.  ``spike`` = (request, key
