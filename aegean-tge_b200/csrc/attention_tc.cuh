@@ -175,19 +175,6 @@ __global__ void __launch_bounds__(THREADS, 2) attention_prefill_tc_kernel(
   const int row_token = q_begin + q_first + (row_valid ? qi : 0);
   const int row_pos = pos0 + qi;
   const int row_head = kvh * p.group + gg;
-  // Everything above read what the step was given (lengths, positions, the block table) and cleared this block's own
-  // shared memory, while the kernel before this one was still running; the queries and the newest keys are its work.
-  pdl_wait();
-  if (tid < ROWS) {
-    // Q row into the K-major swizzled tile: 64-column blocks of [128 rows][128 bytes]
-    const uint4* src = reinterpret_cast<const uint4*>(p.q + (size_t)row_token * p.q_stride + (size_t)row_head * HD);
-#pragma unroll
-    for (int c = 0; c < HD / 8; ++c) {
-      const uint4 v = row_valid ? src[c] : make_uint4(0, 0, 0, 0);
-      const int block = c >> 3, chunk = c & 7;
-      *reinterpret_cast<uint4*>(generic + block * (ROWS * 128) + r * 128 + ((chunk ^ (r & 7)) << 4)) = v;
-    }
-  }
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar + 8 * s, 1);
@@ -204,12 +191,15 @@ __global__ void __launch_bounds__(THREADS, 2) attention_prefill_tc_kernel(
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");     // Q tile and cleared stages, before the async proxy reads or writes them
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");     // the cleared stages, before the async proxy writes them
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem_base = tmem_slot;
   pdl_trigger();                                                      // tensor memory is held: the next kernel may be scheduled
+  // Everything above read what the step was given (lengths, positions, the block table) and set up this block's own
+  // memory, while the kernel before this one was still running; the queries and the newest keys are its work.
+  pdl_wait();
   const uint32_t s_tmem = tmem_base, o_tmem = tmem_base + 2 * BKV;
 
   if (warp == 5) {
@@ -248,6 +238,7 @@ __global__ void __launch_bounds__(THREADS, 2) attention_prefill_tc_kernel(
     }
   } else if (warp == 4) {
     // ------------------------------- products -------------------------------
+    asm volatile("bar.sync 1, %0;\n" ::"n"(ROWS + 32) : "memory");          // the queries are there
     if (elect_one()) {
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BKV >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
       const uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
@@ -286,6 +277,16 @@ __global__ void __launch_bounds__(THREADS, 2) attention_prefill_tc_kernel(
     }
   } else {
     // ------------------------------- softmax, one row per thread -------------------------------
+    // Q row into the K-major swizzled tile: 64-column blocks of [128 rows][128 bytes]
+    const uint4* src = reinterpret_cast<const uint4*>(p.q + (size_t)row_token * p.q_stride + (size_t)row_head * HD);
+#pragma unroll
+    for (int c = 0; c < HD / 8; ++c) {
+      const uint4 v = row_valid ? src[c] : make_uint4(0, 0, 0, 0);
+      const int block = c >> 3, chunk = c & 7;
+      *reinterpret_cast<uint4*>(generic + block * (ROWS * 128) + r * 128 + ((chunk ^ (r & 7)) << 4)) = v;
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");     // the queries, before the tensor core reads them
+    asm volatile("bar.sync 1, %0;\n" ::"n"(ROWS + 32) : "memory");
     // The output accumulates in tensor memory across tiles.  A row's running maximum is in raw score
     // units; when it rises, the row's accumulator is rescaled in tensor memory before the next product
     // is added (a whole warp does it together, rows whose maximum stood still use a factor of one).

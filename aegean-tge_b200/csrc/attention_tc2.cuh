@@ -113,20 +113,6 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc2_kernel(
   const int row_token = q_begin + q_first + (row_valid ? q_in_pair : 0);
   const int row_pos = pos0 + q_in_pair;
   const int row_head = kvh * p.group + gg;
-  // Everything above read what the step was given (lengths, positions, the block table) and cleared this block's own
-  // shared memory, while the kernel before this one was still running; the queries and the newest keys are its work.
-  pdl_wait();
-  if (warp < SOFTMAX_WARPS) {
-    // Q row into the K-major swizzled tile of its query tile: 64-column blocks of [128 rows][128 bytes]
-    const uint4* src = reinterpret_cast<const uint4*>(p.q + (size_t)row_token * p.q_stride + (size_t)row_head * HD);
-    unsigned char* q_tile = generic + qt * Q_BYTES;
-#pragma unroll
-    for (int c = 0; c < HD / 8; ++c) {
-      const uint4 v = row_valid ? src[c] : make_uint4(0, 0, 0, 0);
-      const int block = c >> 3, chunk = c & 7;
-      *reinterpret_cast<uint4*>(q_tile + block * (ROWS * 128) + r * 128 + ((chunk ^ (r & 7)) << 4)) = v;
-    }
-  }
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(k_bar + 8 * s, 1);
@@ -147,12 +133,15 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc2_kernel(
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_slot)), "r"((uint32_t)TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");     // Q tiles and cleared stages, before the async proxy touches them
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");     // the cleared stages, before the async proxy touches them
   fence_before();
   __syncthreads();
   fence_after();
   const uint32_t tmem_base = tmem_slot;
   pdl_trigger();                                                      // tensor memory is held: the next kernel may be scheduled
+  // Everything above read what the step was given (lengths, positions, the block table) and set up this block's own
+  // memory, while the kernel before this one was still running; the queries and the newest keys are its work.
+  pdl_wait();
   auto s_tmem = [&](int tile, int buffer) { return tmem_base + (uint32_t)((tile * 2 + buffer) * BKV); };
   auto o_tmem = [&](int tile) { return tmem_base + (uint32_t)(2 * QTILES * BKV + tile * HD); };
 
@@ -191,6 +180,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc2_kernel(
     // S = Q K^T of key tile j for both query tiles, into their score buffers (j & 1).  A buffer is free
     // once the softmax warps have read tile j - 2 out of it (a barrier of its own: a waiter that could fall
     // two phases behind cannot tell them apart by parity).
+    asm volatile("bar.sync 1, %0;\n" ::"n"((SOFTMAX_WARPS + 1) * 32) : "memory");          // the queries are there
     if (elect_one()) {
       const uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BKV >> 3) << 17) | ((uint32_t)(ROWS >> 4) << 24);
       for (int tile = 0; tile < num_tiles; ++tile) {
@@ -238,6 +228,17 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc2_kernel(
     }
   } else {
     // ------------------------------- softmax, one row per thread -------------------------------
+    // Q row into the K-major swizzled tile of its query tile: 64-column blocks of [128 rows][128 bytes]
+    const uint4* src = reinterpret_cast<const uint4*>(p.q + (size_t)row_token * p.q_stride + (size_t)row_head * HD);
+    unsigned char* q_tile = generic + qt * Q_BYTES;
+#pragma unroll
+    for (int c = 0; c < HD / 8; ++c) {
+      const uint4 v = row_valid ? src[c] : make_uint4(0, 0, 0, 0);
+      const int block = c >> 3, chunk = c & 7;
+      *reinterpret_cast<uint4*>(q_tile + block * (ROWS * 128) + r * 128 + ((chunk ^ (r & 7)) << 4)) = v;
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");     // the queries, before the tensor core reads them
+    asm volatile("bar.sync 1, %0;\n" ::"n"((SOFTMAX_WARPS + 1) * 32) : "memory");
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     const int first_key = p.window > 0 ? row_pos - p.window + 1 : 0;
     const uint32_t my_s_bar = s_bar + 8 * (qt * 2), my_p_bar = p_bar + 8 * qt, my_o_bar = o_bar + 8 * qt;
