@@ -78,6 +78,10 @@ struct AttnParams {
   const __nv_bfloat16* gate; // null, or [tokens, heads] logits: a head's output is multiplied by their logistic function
   int gate_stride;
   int gate_elements;         // the logits are [tokens, heads * DV] instead: one gate per number of a head's output
+  // The single tokens at the head of a step and the longer portions behind them share nothing, so their two kernels may run side by
+  // side: the first one lets its dependents start only behind its own wait (trigger_late), the second one then needs
+  // nothing of the kernel in front and waits for it at its very end alone (beside), so that whoever follows finds both done.
+  int trigger_late, beside;
   float scale_log2;
 };
 
@@ -709,7 +713,7 @@ __global__ void __launch_bounds__((4 * GROUPS + 1) * 32) attention_decode_tma_ke
   constexpr int WARPS = 4 * GROUPS, STAGES = GROUPS == 1 ? DEC_STAGES : 4, THREADS = (WARPS + 1) * 32;
   static_assert(STAGES % GROUPS == 0, "a stage must always serve the same group");
   extern __shared__ unsigned char smem_dyn[];
-  pdl_trigger();
+  if (!p.trigger_late) pdl_trigger();
   const uint32_t raw = smem_u32(smem_dyn);
   const uint32_t base = (raw + 1023u) & ~1023u;                       // swizzle atoms are 1024 bytes
   unsigned char* generic = smem_dyn + (base - raw);
@@ -793,6 +797,7 @@ __global__ void __launch_bounds__((4 * GROUPS + 1) * 32) attention_decode_tma_ke
     }
   }
   pdl_wait();
+  if (p.trigger_late) pdl_trigger();
 
   uint32_t qf[HD / 16][4];
 #pragma unroll
@@ -1406,12 +1411,21 @@ TGE_API long long tge_attention_mma_scratch_floats(int tokens, int heads, int nu
   return num_splits > 1 ? (long long)num_splits * tokens * heads * (DV + 2) : 0;
 }
 
+// What a call for the single tokens at a step's head leaves for its caller to do.
+struct LeadingTokens {
+  bool late = false;         // the decode kernel ran and triggers behind its wait
+  bool unmerged = false;     // the key runs' states wait for launch_merge(p, ...)
+  AttnParams p;
+};
+
 // q: [tokens, heads*HD] with row stride q_stride (elements); pages: [num_pages, kv_heads, page_size, HD].
 // q_start [num_seqs+1], start_pos [num_seqs], positions [tokens] are int32 on the device.
 // max_q_len / max_ctx_len are host-side bounds used only for launch geometry.
 // split_tokens: 0 = one split; else a multiple of 64 (keys per split).  scratch: see above.
 // `first_token`: the sequences given here start at this token of the step (earlier tokens belong to sequences
 // that another launch serves); q, out, positions and the scratch layout stay those of the whole step.
+// `lead`: the call is for such earlier tokens (not null: their kernel triggers late where it can); `beside`: the call follows one whose
+// kernel did.
 static int attention_dispatch(const void* q, int q_stride, const void* k_pages, const void* v_pages,
                               const int* block_table, int max_pages, int num_pages, int page_size,
                               const int* q_start, const int* start_pos, const int* positions, int num_seqs,
@@ -1419,7 +1433,7 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
                               int kv_heads, float scale, int window, int split_tokens, float* scratch, int* status,
                               int first_token, const float* sink, int leave_states, int v_pitch, const float* dist_bias,
                               int dist_span, int keep_first, const void* gate, int gate_stride, int gate_elements,
-                              int shared_keys, cudaStream_t stream) {
+                              int shared_keys, cudaStream_t stream, LeadingTokens* lead = nullptr, bool beside = false) {
   TGE_REQUIRE(tokens >= 0 && num_seqs >= 0, "attention_mma: negative sizes");
   TGE_REQUIRE(dist_bias == nullptr || (dist_span > 0 && scale != 0.0f), "attention_mma: a bias by distance needs its span");
   TGE_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0,
@@ -1455,6 +1469,8 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
   const bool single = max_q_len <= 1 && tokens == num_seqs && group <= 16;
   TGE_REQUIRE(!shared_keys || (single && p.v_in_keys), "attention_mma: runs of heads over the same keys are for single tokens and values inside the keys");
   p.kv_pool = shared_keys ? 1 : kv_heads;
+  p.trigger_late = 0;
+  p.beside = beside ? 1 : 0;
   p.q_stride = q_stride; p.out_stride = out_stride;
   p.max_pages = max_pages; p.num_pages = num_pages; p.page_size = page_size;
   p.page_shift = 0;
@@ -1508,11 +1524,18 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
     }
     p.bq = 1;
     p.early_tiles = p.early_tiles ? stages : 0;
+    p.trigger_late = lead != nullptr ? 1 : 0;
     dim3 grid(num_seqs, kv_heads, num_splits);
     if (two_groups) tge_launch(attention_decode_tma_kernel<2>, grid, 9 * 32, smem, stream, *map_k, *map_v, p);
     else tge_launch(attention_decode_tma_kernel<1>, grid, DEC_TMA_THREADS, smem, stream, *map_k, *map_v, p);
     int rc = tge_check_launch("attention_decode_tma");
     if (rc != 0) return rc;
+    if (lead != nullptr) {
+      lead->late = true;
+      lead->unmerged = num_splits > 1;
+      lead->p = p;
+      return 1;
+    }
     if (num_splits > 1 && !p.leave_states) {
       launch_merge(p, positions, first_token, stream);
       return tge_launched("attention_merge", 2);
@@ -1691,15 +1714,27 @@ TGE_API int tge_attention_mma(const void* q, int q_stride, const void* k_pages, 
     return attention_dispatch(q, q_stride, k_pages, v_pages, block_table, max_pages, num_pages, page_size, q_start, start_pos,
                               positions, num_seqs, tokens, max_q_len, max_ctx_len, out, out_stride, heads, kv_heads, scale,
                               window, split_tokens, scratch, status, 0, sink, leave_states, v_pitch, dist_bias, dist_span, keep_first, gate, gate_stride, gate_elements, shared_keys, stream);
+  // Side by side where nothing but keys, queries and constants is read (gates may be the kernel in front's work) and where the
+  // scratch memory holds the states of one of the two calls only.
+  const bool rest_cut = split_tokens > 0 && max_ctx_len > split_tokens, lead_cut = prefix_split_tokens > 0 && max_ctx_len > prefix_split_tokens;
+  LeadingTokens lead;
+  LeadingTokens* const ask = gate == nullptr && !leave_states && !(rest_cut && lead_cut) ? &lead : nullptr;
   const int first = attention_dispatch(q, q_stride, k_pages, v_pages, block_table, max_pages, num_pages, page_size, q_start,
                                        start_pos, positions, decode_prefix, decode_prefix, 1, max_ctx_len, out, out_stride,
                                        heads, kv_heads, scale, window, prefix_split_tokens, scratch, status, 0, sink, leave_states, v_pitch, dist_bias,
-                                       dist_span, keep_first, gate, gate_stride, gate_elements, shared_keys, stream);
+                                       dist_span, keep_first, gate, gate_stride, gate_elements, shared_keys, stream, ask);
   if (first < 0) return first;
-  const int rest = attention_dispatch(q, q_stride, k_pages, v_pages, block_table + (size_t)decode_prefix * max_pages, max_pages,
-                                      num_pages, page_size, q_start + decode_prefix, start_pos + decode_prefix, positions,
-                                      num_seqs - decode_prefix, tokens, max_q_len, max_ctx_len, out, out_stride, heads,
-                                      kv_heads, scale, window, split_tokens, scratch, status, decode_prefix, sink, leave_states, v_pitch, dist_bias,
-                                      dist_span, keep_first, gate, gate_stride, gate_elements, shared_keys, stream);
-  return rest < 0 ? rest : first + rest;
+  int rest = attention_dispatch(q, q_stride, k_pages, v_pages, block_table + (size_t)decode_prefix * max_pages, max_pages,
+                                num_pages, page_size, q_start + decode_prefix, start_pos + decode_prefix, positions,
+                                num_seqs - decode_prefix, tokens, max_q_len, max_ctx_len, out, out_stride, heads,
+                                kv_heads, scale, window, split_tokens, scratch, status, decode_prefix, sink, leave_states, v_pitch, dist_bias,
+                                dist_span, keep_first, gate, gate_stride, gate_elements, shared_keys, stream, nullptr, lead.late);
+  if (rest < 0) return rest;
+  if (lead.unmerged) {
+    launch_merge(lead.p, positions, 0, stream);
+    const int rc = tge_check_launch("attention_merge");
+    if (rc != 0) return rc;
+    ++rest;
+  }
+  return first + rest;
 }

@@ -198,8 +198,10 @@ __global__ void __launch_bounds__(THREADS, 2) attention_prefill_tc_kernel(
   const uint32_t tmem_base = tmem_slot;
   pdl_trigger();                                                      // tensor memory is held: the next kernel may be scheduled
   // Everything above read what the step was given (lengths, positions, the block table) and set up this block's own
-  // memory, while the kernel before this one was still running; the queries and the newest keys are its work.
-  pdl_wait();
+  // memory, while the kernel before this one was still running; the queries and the newest keys are its work (or
+  // that of the kernel before it: p.beside).
+  if (!p.beside) pdl_wait();
+  else __threadfence();                                               // what that one wrote, and not what an L1 still holds
   const uint32_t s_tmem = tmem_base, o_tmem = tmem_base + 2 * BKV;
 
   if (warp == 5) {
@@ -446,6 +448,7 @@ __global__ void __launch_bounds__(THREADS, 2) attention_prefill_tc_kernel(
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS) : "memory");
   }
+  if (p.beside) pdl_wait();                                           // who follows this kernel finds the one in front done as well
 }
 
 constexpr size_t smem_bytes(int table_entries) {

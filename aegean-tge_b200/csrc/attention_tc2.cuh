@@ -140,8 +140,10 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc2_kernel(
   const uint32_t tmem_base = tmem_slot;
   pdl_trigger();                                                      // tensor memory is held: the next kernel may be scheduled
   // Everything above read what the step was given (lengths, positions, the block table) and set up this block's own
-  // memory, while the kernel before this one was still running; the queries and the newest keys are its work.
-  pdl_wait();
+  // memory, while the kernel before this one was still running; the queries and the newest keys are its work (or
+  // that of the kernel before it: p.beside).
+  if (!p.beside) pdl_wait();
+  else __threadfence();                                               // what that one wrote, and not what an L1 still holds
   auto s_tmem = [&](int tile, int buffer) { return tmem_base + (uint32_t)((tile * 2 + buffer) * BKV); };
   auto o_tmem = [&](int tile) { return tmem_base + (uint32_t)(2 * QTILES * BKV + tile * HD); };
 
@@ -392,6 +394,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc2_kernel(
     fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS) : "memory");
   }
+  if (p.beside) pdl_wait();                                           // who follows this kernel finds the one in front done as well
 }
 
 }  // namespace tc2
