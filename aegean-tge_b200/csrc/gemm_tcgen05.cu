@@ -48,6 +48,10 @@ constexpr int A_STAGE_BYTES = BM * BK * 2;
 constexpr int MAX_STAGES = 8;
 constexpr int EPI_WARPS = 8;              // two per 32-lane quarter of tensor memory, each taking half the columns
 constexpr int NUM_THREADS = (2 + EPI_WARPS) * 32;
+// Pairs of SMs run wide tiles, whose last epilogue nothing hides: four warps to a quarter.  (Not on one SM alone: what runs there are mostly
+// a few tokens, and the registers of so many threads would keep the next product's block from starting beside a small kernel.)
+constexpr int PAIR_EPI_WARPS = 16;
+constexpr int PAIR_THREADS = (2 + PAIR_EPI_WARPS) * 32;
 constexpr int SMEM_LIMIT = 227 * 1024;
 
 struct GemmParams {
@@ -74,6 +78,15 @@ struct GemmParams {
 constexpr int DEFER_MAX_TOKENS = 128;
 
 __device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.0f + expf(-g)) * u; }
+// The same for results that are rounded to bfloat16: exp as a base-2 exponential, the division as a product with the reciprocal, both
+// approximate as __expf and __fdividef are, without care for subnormal numbers (1 + e^-g is none, and an e^-g that small adds
+// nothing to it).
+__device__ __forceinline__ float gate_mul(float g, float u) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(e) : "f"(g * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(1.0f + e));
+  return g * r * u;
+}
 // the clamped gate: g <- min(g, L), u <- clamp(u, -L, L), g sigmoid(1.702 g) (u + 1)
 __device__ __forceinline__ float clamped_gate_mul(float g, float u, float limit) {
   g = fminf(g, limit);
@@ -95,6 +108,15 @@ __device__ __forceinline__ float row_factor_of(const float* __restrict__ ss, int
     for (int i = 0; i < 8; ++i) sum += part[i];
   }
   return 1.0f / sqrtf(sum / (float)width + eps);
+}
+
+// The columns of a tile that the `part`-th of a quarter's epilogue warps takes: groups of 16, shared out evenly.
+template <int WARPS>
+__device__ __forceinline__ void epilogue_columns(int bn, int part, int& begin, int& end) {
+  constexpr int PARTS = WARPS / 4;
+  const int groups = bn / 16;
+  begin = groups * part / PARTS * 16;
+  end = groups * (part + 1) / PARTS * 16;
 }
 
 // What a finished tile's epilogue needs besides the accumulator, asked for while the tensor cores still work on the tile:
@@ -185,7 +207,7 @@ __device__ __forceinline__ void store_gated(const GemmParams& p, int lane, int n
   for (int j = 0; j < 8; ++j) {
     const float got = __shfl_xor_sync(0xffffffffu, odd ? v[2 * j] : v[2 * j + 1], 1);
     const float g = odd ? got : v[2 * j], u = odd ? v[2 * j + 1] : got;
-    x[j] = CLAMPED ? clamped_gate_mul(g, u, p.alpha) : __fdividef(g, 1.0f + __expf(-g)) * u;
+    x[j] = CLAMPED ? clamped_gate_mul(g, u, p.alpha) : gate_mul(g, u);
   }
   __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out);
   if (!pairs) {
@@ -419,10 +441,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   } else {
     // ------------------------------- epilogue -------------------------------
     const int quarter = warp & 3;            // tensor-memory lanes this warp may read
-    const int column_half = (warp - 2) >> 2; // which half of the token columns it takes
-    const int first_half = ((p.bn / 16 + 1) / 2) * 16;   // groups of 16 columns, the odd one to the first half
-    const int c_begin = column_half == 0 ? 0 : first_half;
-    const int c_end = column_half == 0 ? first_half : p.bn;
+    int c_begin, c_end;
+    epilogue_columns<EPI_WARPS>(p.bn, (warp - 2) >> 2, c_begin, c_end);
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
@@ -502,7 +522,7 @@ __device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t desc_a, ui
 
 constexpr int PAIR_BM = 2 * BM;          // weight rows per tile of a pair
 
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                          const GemmParams p) {
   extern __shared__ unsigned char smem_raw[];
@@ -531,7 +551,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(tfull_bar(s), 1);
-      mbar_init(tempty_bar(s), 2 * EPI_WARPS);                          // used in the even block only
+      mbar_init(tempty_bar(s), 2 * PAIR_EPI_WARPS);                          // used in the even block only
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -640,10 +660,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
   } else {
     // ------------------------------- epilogue (both blocks) -------------------------------
     const int quarter = warp & 3;
-    const int column_half = (warp - 2) >> 2;
-    const int first_half = ((p.bn / 16 + 1) / 2) * 16;
-    const int c_begin = column_half == 0 ? 0 : first_half;
-    const int c_end = column_half == 0 ? first_half : p.bn;
+    int c_begin, c_end;
+    epilogue_columns<PAIR_EPI_WARPS>(p.bn, (warp - 2) >> 2, c_begin, c_end);
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
@@ -908,7 +926,7 @@ int pair_capacity() {
   }
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(sm_count() / 2 * 2);
-  config.blockDim = dim3(NUM_THREADS);
+  config.blockDim = dim3(PAIR_THREADS);
   config.dynamicSmemBytes = SMEM_LIMIT;
   cudaLaunchAttribute attribute[1];
   attribute[0].id = cudaLaunchAttributeClusterDimension;
@@ -1082,7 +1100,7 @@ int launch_product(const void* x, long long ldx, const void* w, long long ldw, c
     const long long total = (long long)p.tiles_w * p.tiles_t * p.splits;
     const int pairs = pair_capacity();
     const int grid = 2 * (int)(total < pairs ? total : pairs);
-    tge_launch_clusters(gemm_tcgen05_pair_kernel, grid, NUM_THREADS, smem, 2, stream, map_w, map_x, p);
+    tge_launch_clusters(gemm_tcgen05_pair_kernel, grid, PAIR_THREADS, smem, 2, stream, map_w, map_x, p);
     rc = tge_check_launch("gemm_tcgen05_pair");
     if (rc != 0) return rc;
     *splits_out = pair_partial ? pair_plan.splits : 0;
