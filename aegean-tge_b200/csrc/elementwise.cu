@@ -90,7 +90,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* dst, float a, float b, flo
 // ROWS rows at a time, their loads on their way together: where rows are many, a block of one row waits for its load, its sum and its
 // store in turn, and few blocks fit beside it.  A row's sum is added in the same order whatever ROWS is.
 template <typename TOut, int ROWS>
-__global__ void __launch_bounds__(512) rmsnorm_vec_kernel(const float* __restrict__ x, const float* __restrict__ weight,
+__global__ void __launch_bounds__(512) rmsnorm_vec_kernel(const float* x, const float* __restrict__ weight,
                                                           const int* __restrict__ rows, TOut* __restrict__ out,
                                                           int hidden, int out_rows, int src_rows, float eps, int* status) {
   __shared__ float scratch[ROWS][32];

@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(256) decay_prepare_vec_kernel(
 // token (everything a multiple of eight).  Bound by its bytes, two thirds of them the float32 results (88 MB for 2,048 tokens of 28 heads
 // of 128, where the kernel above takes 32 us).
 __global__ void __launch_bounds__(256) decay_prepare_eights_kernel(
-    const __nv_bfloat16* __restrict__ rows, long long ld, int q_off, int k_off, int heads, int dim, int activation,
+    const __nv_bfloat16* rows, long long ld, int q_off, int k_off, int heads, int dim, int activation,
     const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary,
     float k_scale, const int* __restrict__ positions, float* __restrict__ prepared, int* status) {
   pdl_trigger();
@@ -940,7 +940,7 @@ __global__ void __launch_bounds__(256) gated_norm_vec_kernel(const float* __rest
 // Groups of up to 128 numbers, four to a warp, so that four rows' loads are on their way together (with a group to a warp each waited
 // for one: 2,048 tokens, 28 groups of 128, 22 us); a group's sum is the kernel's above.
 constexpr int GATED_EACH = 4;
-__global__ void __launch_bounds__(256) gated_norm_small_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ gate, long long ld_gate,
+__global__ void __launch_bounds__(256) gated_norm_small_kernel(const float* o, const __nv_bfloat16* gate, long long ld_gate,
                                                                const float* __restrict__ weight, __nv_bfloat16* __restrict__ out, long long ld_out,
                                                                int tokens, int groups, int size, float eps, int act) {
   pdl_trigger();
@@ -1139,8 +1139,8 @@ constexpr int POOL_AHEAD = 16, POOL_THREADS = 256;
 // of 128, blocks of 64: 69 us one position after the other; 34 eight at a time, a block of threads per token (63 of 64 only left).
 template <typename T>
 __global__ void __launch_bounds__(POOL_THREADS) pool_kv_kernel(
-    const T* __restrict__ k_pages, const T* __restrict__ v_pages, const int* __restrict__ block_table, int max_pages,
-    int num_pages, T* __restrict__ kp_pages, T* __restrict__ vp_pages, const int* __restrict__ pool_table,
+    const T* k_pages, const T* v_pages, const int* __restrict__ block_table, int max_pages,
+    int num_pages, T* kp_pages, T* vp_pages, const int* __restrict__ pool_table,
     int pool_max_pages, int pool_num_pages, int page_size, const int* __restrict__ positions,
     const int* __restrict__ seq_of_token, int tokens, int kv_heads, int dim, int vdim, int pool, int* status) {
   pdl_trigger();
@@ -1533,7 +1533,7 @@ __device__ __forceinline__ void unpack_eight(const uint4& raw, float f[8]) {
 
 template <int TAPS>
 __global__ void __launch_bounds__(CONV_THREADS) conv_norm_rope_store_vec_kernel(
-    const __nv_bfloat16* __restrict__ raw, long long ld, const float* __restrict__ conv_w, const float* __restrict__ conv_state,
+    const __nv_bfloat16* raw, long long ld, const float* __restrict__ conv_w, const float* conv_state,
     const int* __restrict__ slots, const int* __restrict__ q_start, const float* __restrict__ q_norm, const float* __restrict__ k_norm,
     float eps, const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary,
     const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int max_pages,
