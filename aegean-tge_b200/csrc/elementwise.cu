@@ -87,64 +87,46 @@ __device__ __forceinline__ void store4(__nv_bfloat16* dst, float a, float b, flo
   *reinterpret_cast<uint2*>(dst) = packed;
 }
 
-// ROWS rows at a time, their loads on their way together: where rows are many, a block of one row waits for its load, its sum and its
-// store in turn, and few blocks fit beside it.  A row's sum is added in the same order whatever ROWS is.
-template <typename TOut, int ROWS>
+template <typename TOut>
 __global__ void __launch_bounds__(512) rmsnorm_vec_kernel(const float* x, const float* __restrict__ weight,
                                                           const int* __restrict__ rows, TOut* __restrict__ out,
-                                                          int hidden, int out_rows, int src_rows, float eps, int* status) {
-  __shared__ float scratch[ROWS][32];
+                                                          int hidden, int src_rows, float eps, int* status) {
+  __shared__ float scratch[32];
   pdl_trigger();
-  const int quads = hidden >> 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
-  float4 gain[NORM_VEC_ITERS], value[ROWS][NORM_VEC_ITERS];
+  const int quads = hidden >> 2;
+  float4 gain[NORM_VEC_ITERS], value[NORM_VEC_ITERS];
 #pragma unroll
   for (int k = 0; k < NORM_VEC_ITERS; ++k) {      // constants of the model: before the wait
     const int i = threadIdx.x + k * blockDim.x;
     gain[k] = i < quads ? reinterpret_cast<const float4*>(weight)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   pdl_wait();
-  const int r0 = blockIdx.x * ROWS;
-#pragma unroll
-  for (int n = 0; n < ROWS; ++n) {
-    const int r = min(r0 + n, out_rows - 1);
-    int src = rows ? rows[r] : r;
-    if (src < 0 || src >= src_rows) {
-      if (threadIdx.x == 0) atomicOr(status, TGE_STATUS_BAD_ROW);
-      src = 0;
-    }
-    const float4* in = reinterpret_cast<const float4*>(x + (size_t)src * hidden);
-#pragma unroll
-    for (int k = 0; k < NORM_VEC_ITERS; ++k) {
-      const int i = threadIdx.x + k * blockDim.x;
-      value[n][k] = i < quads ? in[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+  const int r = blockIdx.x;
+  int src = rows ? rows[r] : r;
+  if (src < 0 || src >= src_rows) {
+    if (threadIdx.x == 0) atomicOr(status, TGE_STATUS_BAD_ROW);
+    src = 0;
   }
+  const float4* in = reinterpret_cast<const float4*>(x + (size_t)src * hidden);
+  float sum = 0.0f;
 #pragma unroll
-  for (int n = 0; n < ROWS; ++n) {
-    float sum = 0.0f;
-#pragma unroll
-    for (int k = 0; k < NORM_VEC_ITERS; ++k) {
-      sum = fmaf(value[n][k].x, value[n][k].x, sum);
-      sum = fmaf(value[n][k].y, value[n][k].y, sum);
-      sum = fmaf(value[n][k].z, value[n][k].z, sum);
-      sum = fmaf(value[n][k].w, value[n][k].w, sum);
-    }
-    sum = warp_sum(sum);
-    if (lane == 0) scratch[n][warp] = sum;
+  for (int k = 0; k < NORM_VEC_ITERS; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    value[k] = i < quads ? in[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    sum = fmaf(value[k].x, value[k].x, sum);
+    sum = fmaf(value[k].y, value[k].y, sum);
+    sum = fmaf(value[k].z, value[k].z, sum);
+    sum = fmaf(value[k].w, value[k].w, sum);
   }
-  __syncthreads();
+  sum = block_sum(sum, scratch);
+  const float scale = 1.0f / sqrtf(sum / (float)hidden + eps);
+  TOut* dst = out + (size_t)r * hidden;
 #pragma unroll
-  for (int n = 0; n < ROWS; ++n) {
-    if (r0 + n >= out_rows) break;
-    const float scale = 1.0f / sqrtf(warp_sum(lane < warps ? scratch[n][lane] : 0.0f) / (float)hidden + eps);
-    TOut* dst = out + (size_t)(r0 + n) * hidden;
-#pragma unroll
-    for (int k = 0; k < NORM_VEC_ITERS; ++k) {
-      const int i = threadIdx.x + k * blockDim.x;
-      if (i < quads)
-        store4(dst + 4 * (size_t)i, value[n][k].x * scale * gain[k].x, value[n][k].y * scale * gain[k].y,
-               value[n][k].z * scale * gain[k].z, value[n][k].w * scale * gain[k].w);
-    }
+  for (int k = 0; k < NORM_VEC_ITERS; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    if (i < quads)
+      store4(dst + 4 * (size_t)i, value[k].x * scale * gain[k].x, value[k].y * scale * gain[k].y,
+             value[k].z * scale * gain[k].z, value[k].w * scale * gain[k].w);
   }
 }
 
@@ -156,17 +138,12 @@ TGE_API int tge_rmsnorm(const float* x, const float* weight, const int* rows, vo
   int threads = hidden >= 2048 ? 512 : 256;
   const bool aligned = ((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out) % 16 == 0;
   if (hidden % 4 == 0 && hidden / 4 <= NORM_VEC_ITERS * threads && aligned) {
-    // more and smaller blocks per SM keep more loads in flight while others sit in their reduction; two rows to a block once such
-    // blocks no longer find room at the same time
+    // more and smaller blocks per SM keep more loads in flight while others sit in their reduction
     if (hidden / 4 <= NORM_VEC_ITERS * 256) threads = 256;
-    auto run = [&](auto one, auto two, auto* to) {
-      if (out_rows >= 4 * tge_sm_count())
-        tge_launch(two, (out_rows + 1) / 2, threads, 0, stream, x, weight, rows, to, hidden, out_rows, src_rows, eps, status);
-      else
-        tge_launch(one, out_rows, threads, 0, stream, x, weight, rows, to, hidden, out_rows, src_rows, eps, status);
-    };
-    if (out_is_bf16) run(rmsnorm_vec_kernel<__nv_bfloat16, 1>, rmsnorm_vec_kernel<__nv_bfloat16, 2>, (__nv_bfloat16*)out);
-    else run(rmsnorm_vec_kernel<float, 1>, rmsnorm_vec_kernel<float, 2>, (float*)out);
+    if (out_is_bf16)
+      tge_launch(rmsnorm_vec_kernel<__nv_bfloat16>, out_rows, threads, 0, stream, x, weight, rows, (__nv_bfloat16*)out, hidden, src_rows, eps, status);
+    else
+      tge_launch(rmsnorm_vec_kernel<float>, out_rows, threads, 0, stream, x, weight, rows, (float*)out, hidden, src_rows, eps, status);
     return tge_launched("rmsnorm", 1);
   }
   if (out_is_bf16)
@@ -288,6 +265,7 @@ __global__ void rope_kv_store_vec_kernel(__nv_bfloat16* __restrict__ qkv, int ro
                                          int num_pages, int page_size, int heads, int kv_heads, int head_dim, int rotary,
                                          int store_kv, int* status) {
   pdl_trigger();
+  pdl_wait();
   const int t = blockIdx.x;
   __nv_bfloat16* row = qkv + (size_t)t * row_stride;
   const int half = rotary / 2;
@@ -299,7 +277,8 @@ __global__ void rope_kv_store_vec_kernel(__nv_bfloat16* __restrict__ qkv, int ro
   const int rotations = q_units + k_rot_units;
   const int total = rotations + k_tail_units + v_units;
   for (int u = threadIdx.x; u < total; u += blockDim.x) {
-    // the chain position -> page and angles is walked while the kernel in front still runs
+    // where the unit comes from depends on nothing that has to be looked up: ask for the data first,
+    // then walk the chain position -> page
     int h, d;
     const __nv_bfloat16* src;
     __nv_bfloat16* page_base;      // k or v pages for units that go to the cache
@@ -320,6 +299,9 @@ __global__ void rope_kv_store_vec_kernel(__nv_bfloat16* __restrict__ qkv, int ro
       src = row + (size_t)(heads + kv_heads + h) * head_dim + d;
       page_base = v_pages;
     }
+    const uint4 first = *reinterpret_cast<const uint4*>(src);
+    uint4 second = first;
+    if (rotation) second = *reinterpret_cast<const uint4*>(src + half);
     const int pos = positions[t];
     if (rotation && (pos < 0 || pos >= table_rows)) {
       atomicOr(status, TGE_STATUS_BAD_ROW);
@@ -334,22 +316,17 @@ __global__ void rope_kv_store_vec_kernel(__nv_bfloat16* __restrict__ qkv, int ro
       }
       dst = page_base + (((size_t)page * kv_heads + h) * page_size + pos % page_size) * head_dim + d;
     }
-    float lo[8], hi[8], c[8], s[8], out_lo[8], out_hi[8];
-    if (rotation) {
-      const float* cs = cos_table + (size_t)pos * half + d;
-      const float* sn = sin_table + (size_t)pos * half + d;
-      *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(cs);
-      *reinterpret_cast<float4*>(c + 4) = *reinterpret_cast<const float4*>(cs + 4);
-      *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(sn);
-      *reinterpret_cast<float4*>(s + 4) = *reinterpret_cast<const float4*>(sn + 4);
-    }
-    pdl_wait();
-    const uint4 first = *reinterpret_cast<const uint4*>(src);
     if (!rotation) {
       *reinterpret_cast<uint4*>(dst) = first;
       continue;
     }
-    const uint4 second = *reinterpret_cast<const uint4*>(src + half);
+    const float* cs = cos_table + (size_t)pos * half + d;
+    const float* sn = sin_table + (size_t)pos * half + d;
+    float lo[8], hi[8], c[8], s[8], out_lo[8], out_hi[8];
+    *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(cs);
+    *reinterpret_cast<float4*>(c + 4) = *reinterpret_cast<const float4*>(cs + 4);
+    *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(sn);
+    *reinterpret_cast<float4*>(s + 4) = *reinterpret_cast<const float4*>(sn + 4);
     unpack8(first, lo);
     unpack8(second, hi);
 #pragma unroll

@@ -55,17 +55,6 @@ def test_rmsnorm(ops, out_dtype, rows, hidden, eps):
     ops.check_status()
 
 
-@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("rows,hidden", [(593, 64), (1001, 3584), (700, 5120), (640, 8192)])
-def test_rmsnorm_two_rows_to_a_block_have_the_bits_of_one(ops, out_dtype, rows, hidden):
-    x, w = torch.randn(rows, hidden, device=DEV), torch.randn(hidden, device=DEV)
-    pick = torch.randperm(rows, device=DEV).to(torch.int32)
-    many = ops.rmsnorm(x, w, 1e-6, out_dtype, rows=pick)
-    few = torch.cat([ops.rmsnorm(x, w, 1e-6, out_dtype, rows=part.contiguous()) for part in pick.split(100)])
-    ops.check_status()
-    assert torch.equal(many, few) and torch.equal(ops.rmsnorm(x, w, 1e-6, out_dtype)[pick.long()], many)
-
-
 def test_rmsnorm_eps_matters(ops):
     """Tiny inputs make eps dominate: a wrong or ignored eps shows at once."""
     x = torch.full((1, 64), 1e-4)
