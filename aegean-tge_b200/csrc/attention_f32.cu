@@ -6,7 +6,7 @@
 // tokens at 28 heads over 4 of 128 took 1,403 us a layer, against 5 us for its 33 MB of keys and values.  Here
 //   * a block owns up to 16, 32 or 64 rows, (query, head of the group) pairs of one request and kv head, and 64 keys at a time
 //     lie in shared memory for all of them, the next 64 under way (cp.async, two buffers);
-//   * 16 threads to a row hold the scores as a matrix product does (rows by 4 keys each, paired float32 FMAs over the head),
+//   * 16 x 16 threads hold the scores as a matrix product does (rows by 4 keys each, paired float32 FMAs over the head),
 //     so a tile costs one round of maxima, exponentials and sums, not 64;
 //   * where the rows are few the keys are cut into runs, each a block of its own, merged by a second kernel.
 // Measured in place (B200, float32): that step 1,403 -> 25 us a layer, 512 prompt tokens 639 -> 122 us; 100 prompt tokens at 12
@@ -23,10 +23,8 @@ namespace {
 
 constexpr int TILE_KEYS = 64;
 constexpr int RUN_KEYS = 256;          // four tiles: long enough that merging costs little, short enough to fill the chip
-constexpr int MAX_ROWS = 64;
-// Threads of a block of so many rows: sixteen to a row, two rows to a thread in the largest.
-template <int ROWS>
-constexpr int THREADS_OF = ROWS <= 32 ? 256 : 512;
+constexpr int THREADS = 256;
+constexpr int MAX_ROWS_PER_THREAD = 4;
 
 struct F32AttnParams {
   const float* q;
@@ -71,16 +69,16 @@ __device__ __forceinline__ float merge_sum(float all, float run, float keep, flo
   return __fmaf_rn(run, take, __fmul_rn(all, keep));
 }
 
-template <int HD, int ROWS>
+template <int HD, int TR>
 constexpr size_t f32_attn_smem() {
-  return sizeof(float) * ((size_t)ROWS * (HD + 4) + 2 * (size_t)TILE_KEYS * (HD + 4) + 2 * (size_t)TILE_KEYS * HD +
-                          (size_t)ROWS * (TILE_KEYS + 4));
+  return sizeof(float) * ((size_t)16 * TR * (HD + 4) + 2 * (size_t)TILE_KEYS * (HD + 4) + 2 * (size_t)TILE_KEYS * HD +
+                          (size_t)16 * TR * (TILE_KEYS + 4));
 }
 
-// Rows r = ty + TY i of the block, keys tx + 16 j of the tile, columns of the output in groups of VEC from tx * VEC.
-template <int HD, int ROWS>
-__global__ void __launch_bounds__(THREADS_OF<ROWS>) attention_f32_kernel(const F32AttnParams p) {
-  constexpr int THREADS = THREADS_OF<ROWS>, TY = THREADS / 16, TR = ROWS / TY, KP = HD + 4, PP = TILE_KEYS + 4;
+// Rows r = ty + 16 i of the block, keys tx + 16 j of the tile, columns of the output in groups of VEC from tx * VEC.
+template <int HD, int TR>
+__global__ void __launch_bounds__(THREADS) attention_f32_kernel(const F32AttnParams p) {
+  constexpr int ROWS = 16 * TR, KP = HD + 4, PP = TILE_KEYS + 4;
   constexpr int COLS = HD / 16, VEC = COLS < 4 ? COLS : 4, GROUPS = COLS / VEC;
   extern __shared__ __align__(16) float smem_f32[];
   float* q_s = smem_f32;                               // [ROWS][KP]
@@ -142,7 +140,7 @@ __global__ void __launch_bounds__(THREADS_OF<ROWS>) attention_f32_kernel(const F
   bool row_ok[TR];
 #pragma unroll
   for (int i = 0; i < TR; ++i) {
-    const int r = ty + TY * i;
+    const int r = ty + 16 * i;
     row_ok[i] = r < q_count * p.group;
     row_pos[i] = row_ok[i] ? pos0 + r / p.group : -1;          // a row that is none sees no key
     row_first[i] = p.window > 0 ? max(row_pos[i] - p.window + 1, 0) : 0;
@@ -224,7 +222,7 @@ __global__ void __launch_bounds__(THREADS_OF<ROWS>) attention_f32_kernel(const F
       for (int d = 0; d < HD; d += 4) {
         ulonglong2 qv[TR], kv[J];
 #pragma unroll
-        for (int i = 0; i < TR; ++i) qv[i] = *reinterpret_cast<const ulonglong2*>(q_s + (ty + TY * i) * KP + d);
+        for (int i = 0; i < TR; ++i) qv[i] = *reinterpret_cast<const ulonglong2*>(q_s + (ty + 16 * i) * KP + d);
 #pragma unroll
         for (int j = 0; j < J; ++j) kv[j] = *reinterpret_cast<const ulonglong2*>(kt + (tx + 16 * j) * KP + d);
 #pragma unroll
@@ -262,7 +260,7 @@ __global__ void __launch_bounds__(THREADS_OF<ROWS>) attention_f32_kernel(const F
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float w = expf(s[j] - base);
-        p_s[(ty + TY * i) * PP + tx + 16 * j] = w;
+        p_s[(ty + 16 * i) * PP + tx + 16 * j] = w;
         sum += w;
       }
 #pragma unroll
@@ -278,7 +276,7 @@ __global__ void __launch_bounds__(THREADS_OF<ROWS>) attention_f32_kernel(const F
       for (int j = 0; j < held; j += 4) {
         float4 w[TR];
 #pragma unroll
-        for (int i = 0; i < TR; ++i) w[i] = *reinterpret_cast<const float4*>(p_s + (ty + TY * i) * PP + j);
+        for (int i = 0; i < TR; ++i) w[i] = *reinterpret_cast<const float4*>(p_s + (ty + 16 * i) * PP + j);
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
           const float* vrow = vt + (j + jj) * HD;
@@ -331,7 +329,7 @@ __global__ void __launch_bounds__(THREADS_OF<ROWS>) attention_f32_kernel(const F
 #pragma unroll
   for (int i = 0; i < TR; ++i) {
     if (!row_ok[i]) continue;
-    const int r = ty + TY * i;
+    const int r = ty + 16 * i;
     const int token = q_begin + q_first + r / p.group, head = kvh * p.group + r % p.group;
     if (one_run) {
       float* dst = p.partial + (((size_t)run_only * p.tokens + token) * p.heads + head) * (HD + 2);
@@ -396,32 +394,32 @@ int row_blocks(int tokens, int num_seqs, int max_q_len, int bq) {
 // blocks of that many still find an SM each, 64 otherwise: a block computes all its rows, in use or not, and while SMs are idle
 // smaller blocks finish sooner (us, 64 / 32 rows, 28 heads over 4 of 128: three prompt tokens 6.6 / 4.6,
 // seven 7.5 / 4.9, forty 11.5 / 8.1, a hundred 20.7 / 15.0; sixteen at 3,000 find no room: 47 / 66).
-int rows_per_block(int tokens, int num_seqs, int max_q_len, int max_ctx_len, int kv_heads, int group) {
+int rows_per_thread(int tokens, int num_seqs, int max_q_len, int max_ctx_len, int kv_heads, int group) {
   const long long rows = group * (long long)max_q_len, runs = (max_ctx_len + RUN_KEYS - 1) / RUN_KEYS;
-  if (rows <= 16) return 16;
-  if (rows <= 32 || (group <= 32 && row_blocks(tokens, num_seqs, max_q_len, 32 / group) * kv_heads * runs <= tge_sm_count())) return 32;
-  return MAX_ROWS;
+  if (rows <= 16) return 1;
+  if (rows <= 32 || (group <= 32 && row_blocks(tokens, num_seqs, max_q_len, 32 / group) * kv_heads * runs <= tge_sm_count())) return 2;
+  return MAX_ROWS_PER_THREAD;
 }
 
 // Runs that are blocks of their own, 1: none.  Only where the row blocks alone leave the chip half empty, and where the
 // states stay within 64 MB: a long portion deep in a long context has keys enough for every block.
 constexpr long long MAX_STATE_FLOATS = 16 << 20;
 int runs_of(int tokens, int num_seqs, int max_q_len, int max_ctx_len, int kv_heads, int group, int head_dim) {
-  const int bq = rows_per_block(tokens, num_seqs, max_q_len, max_ctx_len, kv_heads, group) / group;
+  const int bq = 16 * rows_per_thread(tokens, num_seqs, max_q_len, max_ctx_len, kv_heads, group) / group;
   const long long blocks = (long long)row_blocks(tokens, num_seqs, max_q_len, bq) * kv_heads;
   const int runs = (max_ctx_len + RUN_KEYS - 1) / RUN_KEYS;
   const bool fits = (long long)runs * tokens * kv_heads * group * (head_dim + 2) <= MAX_STATE_FLOATS;
   return blocks >= 2 * tge_sm_count() || !fits ? 1 : runs;
 }
 
-template <int HD, int ROWS>
+template <int HD, int TR>
 int launch(const F32AttnParams& p, int max_q_len, cudaStream_t stream) {
-  constexpr size_t smem = f32_attn_smem<HD, ROWS>();
+  constexpr size_t smem = f32_attn_smem<HD, TR>();
   static_assert(smem <= 227 * 1024, "a block's tiles fit its shared memory");
-  cudaError_t err = cudaFuncSetAttribute(attention_f32_kernel<HD, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t err = cudaFuncSetAttribute(attention_f32_kernel<HD, TR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err == cudaSuccess)
-    err = tge_launch(attention_f32_kernel<HD, ROWS>, dim3(row_blocks(p.tokens, p.num_seqs, max_q_len, ROWS / p.group), p.kv_heads, p.runs),
-                     dim3(THREADS_OF<ROWS>), smem, stream, p);
+    err = tge_launch(attention_f32_kernel<HD, TR>, dim3(row_blocks(p.tokens, p.num_seqs, max_q_len, 16 * TR / p.group), p.kv_heads, p.runs),
+                     dim3(THREADS), smem, stream, p);
   if (err == cudaSuccess && p.runs > 1)
     err = tge_launch(attention_f32_merge_kernel<HD>, dim3(p.tokens, (p.heads + 128 / HD - 1) / (128 / HD)), dim3(128), 0, stream, p);
   if (err != cudaSuccess) {
@@ -434,12 +432,12 @@ int launch(const F32AttnParams& p, int max_q_len, cudaStream_t stream) {
 
 template <int HD>
 int launch_rows(const F32AttnParams& p, int max_q_len, int max_ctx_len, cudaStream_t stream) {
-  const int rows = rows_per_block(p.tokens, p.num_seqs, max_q_len, max_ctx_len, p.kv_heads, p.group);
-  return rows == 16 ? launch<HD, 16>(p, max_q_len, stream) : rows == 32 ? launch<HD, 32>(p, max_q_len, stream) : launch<HD, MAX_ROWS>(p, max_q_len, stream);
+  const int rows = rows_per_thread(p.tokens, p.num_seqs, max_q_len, max_ctx_len, p.kv_heads, p.group);
+  return rows == 1 ? launch<HD, 1>(p, max_q_len, stream) : rows == 2 ? launch<HD, 2>(p, max_q_len, stream) : launch<HD, MAX_ROWS_PER_THREAD>(p, max_q_len, stream);
 }
 
 bool f32_attention_takes(int heads, int kv_heads, int head_dim) {
-  return kv_heads > 0 && heads > 0 && heads % kv_heads == 0 && heads / kv_heads <= MAX_ROWS && kv_heads <= 65535 &&
+  return kv_heads > 0 && heads > 0 && heads % kv_heads == 0 && heads / kv_heads <= 16 * MAX_ROWS_PER_THREAD && kv_heads <= 65535 &&
          (head_dim == 16 || head_dim == 32 || head_dim == 64 || head_dim == 128);
 }
 
