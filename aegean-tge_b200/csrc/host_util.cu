@@ -76,6 +76,16 @@ TGE_API int tge_copy(void* dst, const void* src, long long bytes, cudaStream_t s
   return checked("copy", cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyDefault, stream));
 }
 
+// A captured step's replay as one call: the step's index arrays go to the device (`copied` is recorded behind that copy), token ids that are
+// on the device already go over them, the graph is launched.
+TGE_API int tge_replay_step(void* dev, const void* host, long long bytes, void* copied, void* tokens_at, const void* tokens, long long token_bytes,
+                            void* graph, cudaStream_t stream) {
+  int rc = checked("copy of a step", cudaMemcpyAsync(dev, host, (size_t)bytes, cudaMemcpyHostToDevice, stream));
+  if (rc == 0) rc = checked("event record", cudaEventRecord((cudaEvent_t)copied, stream));
+  if (rc == 0 && token_bytes > 0) rc = checked("copy of a step's tokens", cudaMemcpyAsync(tokens_at, tokens, (size_t)token_bytes, cudaMemcpyDeviceToDevice, stream));
+  return rc != 0 ? rc : checked("graph launch", cudaGraphLaunch((cudaGraphExec_t)graph, stream));
+}
+
 TGE_API const char* tge_last_error() { return g_error; }
 
 TGE_API int tge_abi_version() { return 1; }

@@ -212,3 +212,18 @@ TGE_API int tge_sample(const float* logits, long long row_stride, const float* t
   TGE_REQUIRE(err == cudaSuccess, "sample: launch failed: %s", cudaGetErrorString(err));
   return tge_launched("sample", 1);
 }
+
+// tge_sample, the copy of its ids to pinned host memory, and an event behind that copy.
+TGE_API int tge_sample_to_host(const float* logits, long long row_stride, const float* temperature, const float* uniform, int* out, int rows,
+                               int vocab, int* host, void* event, cudaStream_t stream) {
+  const int launched = tge_sample(logits, row_stride, temperature, uniform, out, rows, vocab, stream);
+  if (launched < 0) return launched;
+  cudaError_t err = cudaMemcpyAsync(host, out, (size_t)rows * sizeof(int), cudaMemcpyDeviceToHost, stream);
+  if (err == cudaSuccess) err = cudaEventRecord((cudaEvent_t)event, stream);
+  if (err != cudaSuccess) {
+    cudaGetLastError();
+    tge_set_error("sample: the ids' way to the host: %s", cudaGetErrorString(err));
+    return -2;
+  }
+  return launched;
+}

@@ -85,6 +85,7 @@ class ModelRunner:
         self._graphs: Dict[tuple, "DecodeGraph"] = {}          # in order of last use
         self._graph_pool = None
         self._capture_stream = None
+        self._zeros: Dict[int, tuple] = {}                     # by batch size, at most max_graph_batch of them
         self.graphs_captured = 0
         self.graph_replays = 0
         self.model = model
@@ -145,7 +146,8 @@ class ModelRunner:
     def step_plan(self, plan) -> Optional[torch.Tensor]:
         """Runs a scheduler's plan: the same step, packed from the scheduler's own copies of the tokens.
 
-        Pages were reserved when the plan was made, and the scheduler records progress in ``update``.
+        Pages were reserved when the plan was made, and the scheduler records progress in ``update``.  The logits are
+        valid for what is queued on them before the next step.
         """
         items = plan.items
         if not items:
@@ -156,7 +158,7 @@ class ModelRunner:
         tokens = sum(item.count for item in items)
         wanted = [i for i, item in enumerate(items) if item.samples]
         return self._run(lambda width, pad_rows, out, layout: plan.pack(vocab, width, pad_rows, out, layout),
-                         len(items), tokens, single, max_ctx, wanted, None)
+                         len(items), tokens, single, max_ctx, wanted, None, lend=True)
 
     def can_step_ahead(self, batch: int) -> bool:
         return self.use_graphs and batch <= self.max_graph_batch
@@ -166,28 +168,33 @@ class ModelRunner:
         token ids taken from ``token_ids`` on the device: the step can be queued before the host has seen them.
 
         Pages are reserved all or nothing (PoolExhausted if they do not fit); progress is not recorded.
-        Returns the logits of every row.
+        Returns the logits of every row, valid for what is queued on them before the next step.
         """
         cache, lib = self.cache, self._lib
         count = len(requests)
         handles = (ctypes.c_int64 * count)(*[cache.handle_of(r) for r in requests])
-        dummy = np.zeros(count, dtype=np.int32)
-        want = np.zeros(count, dtype=np.int32)
-        token_ptrs = (ctypes.c_void_p * count)(*[dummy.ctypes.data + 4 * i for i in range(count)])
-        want_ptrs = (ctypes.c_void_p * count)(*[want.ctypes.data + 4 * i for i in range(count)])
-        ones = (ctypes.c_int * count)(*([1] * count))
+        _zeros, zero_ptrs, ones = self._placeholders(count)
         vocab = self.model.spec.vocab_size
 
         def pack(width: int, pad_rows: int, out: np.ndarray, layout) -> int:
-            return _rt.check(lib.tge_rt_step_pack(cache.native, count, handles, token_ptrs, ones, want_ptrs, ones, vocab,
+            return _rt.check(lib.tge_rt_step_pack(cache.native, count, handles, zero_ptrs, ones, zero_ptrs, ones, vocab,
                                                   self.max_model_len, width, pad_rows, out.ctypes.data, out.size,
                                                   ctypes.byref(layout)))
 
         max_ctx = lib.tge_rt_cache_max_context(cache.native, handles, ones, count)
-        return self._run(pack, count, count, True, max_ctx, list(range(count)), None, device_tokens=token_ids)
+        return self._run(pack, count, count, True, max_ctx, list(range(count)), None, device_tokens=token_ids, lend=True)
+
+    def _placeholders(self, count: int) -> tuple:
+        """One token of id 0 and one wanted place 0 for each of ``count`` portions, as the packer reads them (never written)."""
+        if count not in self._zeros:
+            zeros = np.zeros(1, dtype=np.int32)
+            self._zeros[count] = (zeros, (ctypes.c_void_p * count)(*([zeros.ctypes.data] * count)), (ctypes.c_int * count)(*([1] * count)))
+        return self._zeros[count]
 
     def _run(self, pack: Packer, batch: int, tokens: int, single: bool, max_ctx: int, wanted: List[int],
-             packed: Optional[Callable[[], None]], device_tokens: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+             packed: Optional[Callable[[], None]], device_tokens: Optional[torch.Tensor] = None,
+             lend: bool = False) -> Optional[torch.Tensor]:
+        """``lend``: the logits may lie in a buffer that the next step overwrites (who queues all use of them first needs no copy)."""
         groups = len(self.cache.groups)
         if self.use_graphs and single and batch <= self.max_graph_batch:
             bound = 1024
@@ -213,7 +220,7 @@ class ModelRunner:
             elif len(wanted) != batch:
                 logits = logits[torch.tensor(wanted, device=self.device)]
             else:
-                logits = logits[:batch].clone()  # the graph's own buffer is overwritten by the next replay
+                logits = logits[:batch] if lend else logits[:batch].clone()  # the next replay overwrites the graph's own buffer
         else:
             need = 4 * tokens + 4 * batch + 1 + groups * batch * self._widest
             if self._staging is None:
@@ -298,6 +305,7 @@ class DecodeGraph:
             torch.cuda.empty_cache()
             self.graph = torch.cuda.CUDAGraph()
             self._capture(runner, side)
+        self.exec = self.graph.raw_cuda_graph_exec()
         self.kernels = ops.launches - before
         ops.launches = before
 
@@ -325,9 +333,6 @@ class DecodeGraph:
             raise RuntimeError("decode graph: the packed step does not have the captured layout")
         if packed is not None:
             packed()
-        staging.send(turn, total, self.dev)
-        if device_tokens is not None:      # the token ids are still on the device: they overwrite the packed placeholders
-            first = self.layout.token_ids
-            self.dev[first:first + device_tokens.numel()].copy_(device_tokens, non_blocking=True)
-        self.graph.replay()
+        # token ids that are still on the device overwrite the packed placeholders
+        _ops.replay_step(self.exec, self.dev, staging.hosts[turn], total, staging.copied[turn], device_tokens, self.layout.token_ids)
         return self.logits

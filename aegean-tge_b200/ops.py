@@ -63,6 +63,7 @@ def core() -> ctypes.CDLL:
         _declare(lib, "tge_event_wait", [_c_ptr, _c_ptr])
         _declare(lib, "tge_event_destroy", [_c_ptr])
         _declare(lib, "tge_copy", [_c_ptr, _c_ptr, _c_ll, _c_ptr])
+        _declare(lib, "tge_replay_step", [_c_ptr, _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ptr, _c_ll, _c_ptr, _c_ptr])
         _declare(lib, "tge_embedding", [_c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_ptr])
         _declare(lib, "tge_rmsnorm", [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_float,
                                       _c_ptr, _c_ptr])
@@ -180,6 +181,7 @@ def core() -> ctypes.CDLL:
                                                _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int,
                                                _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr])
         _declare(lib, "tge_soft_cap", [_c_ptr, _c_ll, _c_int, _c_int, _c_float, _c_ptr])
+        _declare(lib, "tge_sample_to_host", [_c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr])
         _declare(lib, "tge_sample", [_c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr])
         _declare(lib, "tge_apply_penalty", [_c_ptr, _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr])
         _declare(lib, "tge_sample_cuts", [_c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr,
@@ -311,6 +313,23 @@ def copy_bytes(dst: torch.Tensor, src: torch.Tensor, count: int) -> None:
         raise KernelError(f"copy: {count} bytes between tensors of {src.nbytes} and {dst.nbytes}")
     lib = core()
     _check(lib.tge_copy(dst.data_ptr(), src.data_ptr(), count, _stream()), lib)
+
+
+def replay_step(graph: int, dev: torch.Tensor, host: torch.Tensor, ints: int, copied: StepEvent, tokens: Optional[torch.Tensor],
+                tokens_at: int) -> None:
+    """Queues a captured step on the current stream: the first ``ints`` of ``host`` (pinned int32) to ``dev``, then ``copied``;
+    ``tokens`` (int32 on the device, None: none) over ``dev`` from ``tokens_at`` on; the launch of ``graph`` (an executable graph's handle).
+    The caller keeps all of them alive, ``host`` unchanged until ``copied``."""
+    count = 0
+    if tokens is not None:
+        _want(tokens, "token ids", torch.int32)
+        count = tokens.numel()
+    if ints > dev.numel() or ints > host.numel() or tokens_at + count > dev.numel():
+        raise KernelError(f"replay: {ints} index entries and {count} tokens from {tokens_at} on in buffers of {host.numel()} and {dev.numel()}")
+    at, lib = dev.data_ptr(), core()
+    _check(lib.tge_replay_step(at, host.data_ptr(), 4 * ints, copied._handle, at + 4 * tokens_at, None if tokens is None else tokens.data_ptr(),
+                               4 * count, graph, _stream()), lib)
+    copied._recorded = True
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -1306,6 +1325,23 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, uniform: torch.Tenso
     _check(lib.tge_sample(logits.data_ptr(), stride, temperature.data_ptr(), uniform.data_ptr(), out.data_ptr(), rows,
                           vocab, _stream()), lib)
     return out
+
+
+def sample_to_host(logits: torch.Tensor, temperature: torch.Tensor, uniform: torch.Tensor, out: torch.Tensor, host: torch.Tensor,
+                   event: StepEvent) -> None:
+    """:func:`sample` into ``out`` (int32 [R]), the ids' copy to ``host`` (pinned int32 [R]), and ``event`` recorded behind it."""
+    _want(logits, "logits", torch.float32, contiguous=False)
+    rows, vocab = logits.shape
+    for name, t, dtype in (("temperature", temperature, torch.float32), ("uniform draws", uniform, torch.float32), ("sampled ids", out, torch.int32)):
+        _want(t, name, dtype)
+        if t.numel() != rows:
+            raise KernelError(f"sample: {t.numel()} numbers of {name} for {rows} rows")
+    if host.dtype != torch.int32 or host.numel() != rows or not host.is_contiguous():
+        raise KernelError(f"sample: the ids of {rows} rows need as many int32 on the host")
+    lib = core()
+    _check(lib.tge_sample_to_host(logits.data_ptr(), _rows_2d(logits, "logits"), temperature.data_ptr(), uniform.data_ptr(), out.data_ptr(), rows,
+                                  vocab, host.data_ptr(), event._handle, _stream()), lib)
+    event._recorded = True
 
 
 def apply_penalty(logits: torch.Tensor, history: torch.Tensor, history_start: torch.Tensor,

@@ -38,13 +38,17 @@ class Sampler:
         the top-k / top-p / min-p cuts are all settled by kernels that read only what is on the device."""
         return all(not p.has_penalty for p in params)
 
+    def _greedy(self, rows: int) -> torch.Tensor:
+        """Temperatures and draws [2, rows] of rows that take the first maximum."""
+        if rows not in self._zeros:
+            self._zeros[rows] = torch.zeros((2, rows), dtype=torch.float32, device=self.device)
+        return self._zeros[rows]
+
     def _draw(self, scores: torch.Tensor, params: Sequence[SamplingParams], rngs: Sequence[XorShift32]) -> torch.Tensor:
         """Token ids on the device for rows of scores: one kernel for all rows, one more for the rows with cuts."""
         rows = scores.shape[0]
         if all(p.greedy for p in params):
-            if rows not in self._zeros:
-                self._zeros[rows] = torch.zeros((2, rows), dtype=torch.float32, device=self.device)
-            floats = self._zeros[rows]
+            floats = self._greedy(rows)
             return self.ops.sample(scores, floats[0], floats[1])
         cuts = any(p.has_cuts and not p.greedy for p in params)
         table = [[max(float(p.temperature), 0.0) for p in params],
@@ -64,11 +68,15 @@ class Sampler:
         """Like :meth:`sample` for rows that stay on the device, without waiting: returns the ids on the
         device, their copy in pinned host memory, and the event after which that copy is complete."""
         rows = logits.shape[0]
-        ids = self._draw(logits, params, rngs)
         turn = self._turn = (getattr(self, "_turn", -1) + 1) % 4
         if rows not in self._pinned:
             self._pinned[rows] = [(torch.empty(rows, dtype=torch.int32).pin_memory(), self.ops.StepEvent()) for _ in range(4)]
         host, event = self._pinned[rows][turn]
+        if all(p.greedy for p in params):         # kernel, copy and event in one call
+            floats, ids = self._greedy(rows), torch.empty(rows, dtype=torch.int32, device=self.device)
+            self.ops.sample_to_host(logits, floats[0], floats[1], ids, host, event)
+            return ids, host, event
+        ids = self._draw(logits, params, rngs)
         self.ops.copy_bytes(host, ids, 4 * rows)
         event.record()
         return ids, host, event
