@@ -1516,11 +1516,12 @@ __global__ void __launch_bounds__(NRV_THREADS) norm_rope_store_vec_kernel(
 }
 
 // With a convolution of two to four taps, eight bfloat16 channels to a lane (sizes and strides as above): a group of `lanes` lanes takes a
-// head of q, k or v for CONV_TOKENS neighbouring tokens, whose rows and the taps before them are asked for at once and
-// serve every token they reach; places, pages and angles are looked up while the kernel in front still runs.  Bound by its bytes (q and k
-// and v read and written once) and by one round trip a block; a warp per (token, head) with two-byte loads of every tap, one behind
-// the other, took 86 us for 2,048 tokens of 28 heads over 4 of 128, with each token's look-ups behind the last one's stores 57.
-constexpr int CONV_TOKENS = 4, CONV_THREADS = 256, CONV_VEC_TOKENS = 16;
+// head of q, k or v for CONV_TOKENS neighbouring tokens, one after the other with the next one's row on its way; the taps before a token
+// stay in registers.  Places, pages and angles are looked up into shared memory while the kernel in front still runs.  Bound by its
+// instructions (about 250 a warp and token), not by its bytes (38 MB for 2,048 tokens of 28 heads over 4 of 128): a warp per (token, head) with
+// two-byte loads of every tap, one behind the other, took 86 us there; four tokens unrolled with their rows and taps in registers 62 (a
+// quarter of an SM's warps, 1,800 instructions each, waits for the instructions themselves).
+constexpr int CONV_TOKENS = 8, CONV_THREADS = 256, CONV_VEC_TOKENS = 16;
 
 __device__ __forceinline__ void unpack_eight(const uint4& raw, float f[8]) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -1533,17 +1534,40 @@ __device__ __forceinline__ void unpack_eight(const uint4& raw, float f[8]) {
 
 template <int TAPS>
 __global__ void __launch_bounds__(CONV_THREADS) conv_norm_rope_store_vec_kernel(
-    const __nv_bfloat16* raw, long long ld, const float* __restrict__ conv_w, const float* conv_state,
-    const int* __restrict__ slots, const int* __restrict__ q_start, const float* __restrict__ q_norm, const float* __restrict__ k_norm,
-    float eps, const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary,
+    const __nv_bfloat16* raw, long long ld, const float* __restrict__ conv_w, const float* conv_state, const int* __restrict__ slots,
+    const int* __restrict__ q_start, const float* __restrict__ q_norm, const float* __restrict__ k_norm, float eps,
+    const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary,
     const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int max_pages,
     __nv_bfloat16* __restrict__ k_pages, __nv_bfloat16* __restrict__ v_pages, int num_pages, int page_size,
     __nv_bfloat16* __restrict__ q_out, long long ld_q, int tokens, int heads, int kv_heads, int dim, int vdim, int store, int norm_last,
     int lanes, int* status) {
-  constexpr int ROWS = CONV_TOKENS + TAPS - 1;
   extern __shared__ __align__(16) float angles[];        // [CONV_TOKENS][2][half]: cosines, then sines
+  __shared__ int locals[CONV_TOKENS], states[CONV_TOKENS], pages[CONV_TOKENS], places[CONV_TOKENS], at_angle[CONV_TOKENS];
   pdl_trigger();
-  const int t0 = blockIdx.x * CONV_TOKENS;
+  const int t0 = blockIdx.x * CONV_TOKENS, count = min(CONV_TOKENS, tokens - t0), half = rotary >> 1;
+  // what the step was given, and the angles, while the kernel in front still runs
+  if ((int)threadIdx.x < count) {
+    const int i = threadIdx.x, t = t0 + i, seq = seq_of_token[t], position = positions[t];
+    locals[i] = t - q_start[seq];                          // the token's index in its portion
+    states[i] = slots[seq];
+    int page = -1, place = 0;
+    if (store) {
+      const int page_index = position / page_size;
+      place = position - page_index * page_size;
+      if (position >= 0 && page_index < max_pages) page = block_table[(size_t)seq * max_pages + page_index];
+      if (page >= num_pages) page = -1;
+    }
+    pages[i] = page;
+    places[i] = place;
+    const bool known = position >= 0 && position < table_positions;
+    if (rotary > 0 && !known) atomicOr(status, TGE_STATUS_BAD_ROW);
+    at_angle[i] = known ? position : 0;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < count * rotary; e += CONV_THREADS) {
+    const int i = e / rotary, n = e - i * rotary;
+    angles[e] = (n < half ? cos_table : sin_table)[(size_t)at_angle[i] * half + (n < half ? n : n - half)];
+  }
   const int mine = threadIdx.x & (lanes - 1), unit = blockIdx.y * (CONV_THREADS / lanes) + (int)threadIdx.x / lanes;
   const int kind = unit < heads ? 0 : (unit < heads + kv_heads ? 1 : 2);        // q, k, v
   const int head = kind == 0 ? unit : (kind == 1 ? unit - heads : unit - heads - kv_heads);
@@ -1551,87 +1575,75 @@ __global__ void __launch_bounds__(CONV_THREADS) conv_norm_rope_store_vec_kernel(
   const bool valid = unit < heads + 2 * kv_heads && mine * 8 < size;
   const int channels = (heads + kv_heads) * dim + kv_heads * vdim;
   const int c = (kind == 0 ? head * dim : (kind == 1 ? (heads + head) * dim : (heads + kv_heads) * dim + head * vdim)) + mine * 8;
-  // what the step was given, and the angles, while the kernel in front still runs
-  int local[CONV_TOKENS], slot[CONV_TOKENS], page[CONV_TOKENS], place[CONV_TOKENS];
-  const int half = rotary >> 1;
+  const float* norm_w = kind == 0 ? q_norm : (kind == 1 ? k_norm : nullptr);
+  float gain[8];
 #pragma unroll
-  for (int i = 0; i < CONV_TOKENS; ++i) {
-    const int t = min(t0 + i, tokens - 1), seq = seq_of_token[t], position = positions[t];
-    local[i] = t - q_start[seq];                           // the token's index in its portion
-    slot[i] = slots[seq];
-    page[i] = -1;
-    place[i] = 0;
-    if (store) {
-      const int page_index = position / page_size;
-      place[i] = position - page_index * page_size;
-      if (position >= 0 && page_index < max_pages) page[i] = block_table[(size_t)seq * max_pages + page_index];
-    }
-    if (rotary > 0) {
-      const bool known = position >= 0 && position < table_positions;
-      if (!known && threadIdx.x == 0) atomicOr(status, TGE_STATUS_BAD_ROW);
-      for (int e = threadIdx.x; e < 2 * half; e += CONV_THREADS)
-        angles[i * 2 * half + e] = (e < half ? cos_table : sin_table)[(size_t)(known ? position : 0) * half + (e < half ? e : e - half)];
-    }
-  }
+  for (int e = 0; e < 8; ++e) gain[e] = valid && norm_w != nullptr ? norm_w[mine * 8 + e] : 1.0f;
+  const int away = half >> 3;
+  const bool turns = kind != 2 && mine * 8 < rotary, low = mine < away;
+  const int from = ((threadIdx.x & 31) & ~(lanes - 1)) + (turns ? (low ? mine + away : mine - away) : mine);
+  const bool norm_first = !norm_last && (q_norm != nullptr || k_norm != nullptr);      // the same for the whole block
   __syncthreads();
   pdl_wait();
-  uint4 rows[ROWS];                    // tokens t0 - (TAPS - 1) ... t0 + CONV_TOKENS - 1
+  auto row_of = [&](int t) { return valid && t >= 0 ? *reinterpret_cast<const uint4*>(raw + (size_t)t * ld + c) : make_uint4(0u, 0u, 0u, 0u); };
+  uint4 ahead = row_of(t0);
+  float past[TAPS - 1][8];             // the rows before this token's, the oldest first
 #pragma unroll
-  for (int r = 0; r < ROWS; ++r) {
-    const int t = t0 - (TAPS - 1) + r;
-    rows[r] = valid && t >= 0 && t < tokens ? *reinterpret_cast<const uint4*>(raw + (size_t)t * ld + c) : make_uint4(0u, 0u, 0u, 0u);
-  }
+  for (int j = 0; j < TAPS - 1; ++j) unpack_eight(row_of(t0 - (TAPS - 1) + j), past[j]);
   float w[8 * TAPS];                   // [channel][tap], as they lie
 #pragma unroll
   for (int i = 0; i < 8 * TAPS; i += 4) {
     const float4 four = valid ? *reinterpret_cast<const float4*>(conv_w + (size_t)c * TAPS + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     w[i] = four.x; w[i + 1] = four.y; w[i + 2] = four.z; w[i + 3] = four.w;
   }
-  const float* norm_w = kind == 0 ? q_norm : (kind == 1 ? k_norm : nullptr);
-  const int away = half >> 3;
-  const bool turns = kind != 2 && mine * 8 < rotary, low = mine < away;
-  const int group_first = (threadIdx.x & 31) & ~(lanes - 1);
-  const int from = group_first + (turns ? (low ? mine + away : mine - away) : mine);
+#pragma unroll 1
+  for (int i = 0; i < count; ++i) {
+    const int t = t0 + i, local = locals[i];
+    float now[8], f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    unpack_eight(ahead, now);
+    if (i + 1 < count) ahead = row_of(t + 1);
+    if (local < TAPS - 1) {            // taps from before the portion: the request's state
 #pragma unroll
-  for (int i = 0; i < CONV_TOKENS; ++i) {
-    const int t = t0 + i;
-    if (t >= tokens) break;                                // the same for the whole block
-    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int j = 0; j < TAPS; ++j) {
-      const int back = TAPS - 1 - j;                       // how many tokens before this one
-      float u[8];
-      unpack_eight(rows[i + j], u);
-      if (local[i] < back) {                               // from before the portion: the request's state
-        const float* at = conv_state + ((size_t)slot[i] * (TAPS - 1) + (TAPS - 1 + local[i] - back)) * channels + c;
+      for (int j = 0; j < TAPS - 1; ++j) {
+        if (local >= TAPS - 1 - j) continue;
+        const float* at = conv_state + ((size_t)states[i] * (TAPS - 1) + local + j) * channels + c;
 #pragma unroll
         for (int e = 0; e < 8; e += 4) {
           const float4 four = valid ? *reinterpret_cast<const float4*>(at + e) : make_float4(0.f, 0.f, 0.f, 0.f);
-          u[e] = four.x; u[e + 1] = four.y; u[e + 2] = four.z; u[e + 3] = four.w;
+          past[j][e] = four.x; past[j][e + 1] = four.y; past[j][e + 2] = four.z; past[j][e + 3] = four.w;
         }
       }
+    }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] = fmaf(w[e * TAPS + j], u[e], f[e]);
+    for (int j = 0; j < TAPS - 1; ++j)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = fmaf(w[e * TAPS + j], past[j][e], f[e]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      f[e] = fmaf(w[e * TAPS + TAPS - 1], now[e], f[e]);
+#pragma unroll
+      for (int j = 0; j + 1 < TAPS - 1; ++j) past[j][e] = past[j + 1][e];
+      past[TAPS - 2][e] = now[e];
     }
     auto norm = [&](bool wanted) {
       float sum = 0.0f;
 #pragma unroll
       for (int e = 0; e < 8; ++e) sum = fmaf(f[e], f[e], sum);
       for (int step = lanes >> 1; step > 0; step >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, step);
-      const float scale = 1.0f / sqrtf(sum / (float)size + eps);
-      if (wanted && valid) {
+      const float scale = wanted ? 1.0f / sqrtf(sum / (float)size + eps) : 1.0f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] *= scale * (norm_w != nullptr ? norm_w[mine * 8 + e] : 1.0f);
-      }
+      for (int e = 0; e < 8; ++e) f[e] *= scale * gain[e];
     };
-    if (!norm_last && (q_norm != nullptr || k_norm != nullptr)) norm(norm_w != nullptr);      // the same for the whole block
+    if (norm_first) norm(norm_w != nullptr);
     if (rotary > 0) {
-      const float* cs = angles + i * 2 * half + (low ? mine : mine - away) * 8;
-      const float* sn = cs + half;
+      const float4* cs = reinterpret_cast<const float4*>(angles + i * rotary + (turns ? (low ? mine : mine - away) * 8 : 0));
+      const float4* sn = cs + (half >> 2);
+      const float4 c0 = cs[0], c1 = cs[1], s0 = sn[0], s1 = sn[1];
+      const float cc[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, ss[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float other = __shfl_sync(0xffffffffu, f[e], from);
-        if (turns) f[e] = low ? f[e] * cs[e] - other * sn[e] : f[e] * cs[e] + other * sn[e];
+        if (turns) f[e] = low ? f[e] * cc[e] - other * ss[e] : f[e] * cc[e] + other * ss[e];
       }
     }
     if (norm_last) norm(kind != 2);
@@ -1639,11 +1651,11 @@ __global__ void __launch_bounds__(CONV_THREADS) conv_norm_rope_store_vec_kernel(
     __nv_bfloat16* dst = q_out + (size_t)t * ld_q + (size_t)head * dim;
     if (kind != 0) {
       if (!store) continue;
-      if (page[i] < 0 || page[i] >= num_pages) {
+      if (pages[i] < 0) {
         if (mine == 0) atomicOr(status, TGE_STATUS_BAD_PAGE);
         continue;
       }
-      dst = (kind == 1 ? k_pages : v_pages) + (((size_t)page[i] * kv_heads + head) * page_size + place[i]) * size;
+      dst = (kind == 1 ? k_pages : v_pages) + (((size_t)pages[i] * kv_heads + head) * page_size + places[i]) * size;
     }
     uint4 packed;
     __nv_bfloat162* two = reinterpret_cast<__nv_bfloat162*>(&packed);
