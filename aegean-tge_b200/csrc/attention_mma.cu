@@ -1690,7 +1690,7 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
 // bring one token each (0: unknown or none).  They then go to the split-key decode kernel, which reads each
 // sequence's keys once for all query heads of a kv head, instead of filling one 128-row query tile of the
 // prefill kernel each; the other sequences follow in a second launch.  A row's value does not depend on the
-// route beyond rounding.
+// route beyond rounding.  `rest_ctx_len`: a bound on those others' contexts (0: max_ctx_len).
 // `dist_bias` (float32 [heads, dist_span], or null): a learned bias by distance, added unscaled to the scaled score of the
 // key n positions back, entry min(n, dist_span - 1) of the head's row; every kernel adds it where it scales its scores.
 // `keep_first` (with a window): the first so many positions stay visible beside the window.  `gate` (bfloat16 [tokens,
@@ -1705,7 +1705,7 @@ TGE_API int tge_attention_mma(const void* q, int q_stride, const void* k_pages, 
                               int kv_heads, float scale, int window, int split_tokens, float* scratch, int* status,
                               int decode_prefix, int prefix_split_tokens, const float* sink, int leave_states,
                               int v_pitch, const float* dist_bias, int dist_span, int keep_first, const void* gate,
-                              int gate_stride, int gate_elements, int shared_keys, cudaStream_t stream) {
+                              int gate_stride, int gate_elements, int shared_keys, int rest_ctx_len, cudaStream_t stream) {
   TGE_REQUIRE(decode_prefix >= 0 && decode_prefix <= num_seqs, "attention_mma: %d leading single tokens of %d sequences",
               decode_prefix, num_seqs);
   TGE_REQUIRE(prefix_split_tokens >= 0 && prefix_split_tokens % BKV == 0,
@@ -1716,7 +1716,8 @@ TGE_API int tge_attention_mma(const void* q, int q_stride, const void* k_pages, 
                               window, split_tokens, scratch, status, 0, sink, leave_states, v_pitch, dist_bias, dist_span, keep_first, gate, gate_stride, gate_elements, shared_keys, stream);
   // Side by side where nothing but keys, queries and constants is read (gates may be the kernel in front's work) and where the
   // scratch memory holds the states of one of the two calls only.
-  const bool rest_cut = split_tokens > 0 && max_ctx_len > split_tokens, lead_cut = prefix_split_tokens > 0 && max_ctx_len > prefix_split_tokens;
+  const int rest_ctx = rest_ctx_len > 0 && rest_ctx_len < max_ctx_len ? rest_ctx_len : max_ctx_len;
+  const bool rest_cut = split_tokens > 0 && rest_ctx > split_tokens, lead_cut = prefix_split_tokens > 0 && max_ctx_len > prefix_split_tokens;
   LeadingTokens lead;
   LeadingTokens* const ask = gate == nullptr && !leave_states && !(rest_cut && lead_cut) ? &lead : nullptr;
   const int first = attention_dispatch(q, q_stride, k_pages, v_pages, block_table, max_pages, num_pages, page_size, q_start,
@@ -1726,7 +1727,7 @@ TGE_API int tge_attention_mma(const void* q, int q_stride, const void* k_pages, 
   if (first < 0) return first;
   int rest = attention_dispatch(q, q_stride, k_pages, v_pages, block_table + (size_t)decode_prefix * max_pages, max_pages,
                                 num_pages, page_size, q_start + decode_prefix, start_pos + decode_prefix, positions,
-                                num_seqs - decode_prefix, tokens, max_q_len, max_ctx_len, out, out_stride, heads,
+                                num_seqs - decode_prefix, tokens, max_q_len, rest_ctx, out, out_stride, heads,
                                 kv_heads, scale, window, split_tokens, scratch, status, decode_prefix, sink, leave_states, v_pitch, dist_bias,
                                 dist_span, keep_first, gate, gate_stride, gate_elements, shared_keys, stream, nullptr, lead.late);
   if (rest < 0) return rest;

@@ -78,13 +78,17 @@ def context_from_packed(dev: torch.Tensor, host: np.ndarray, layout: "_rt.StepLa
     # decoding requests usually come first in a step (the scheduler plans running requests before new ones)
     longer = np.flatnonzero(q_lens != 1)
     decode_prefix = int(longer[0]) if longer.size else 0
+    starts = host[L.start_pos:L.start_pos + S]
+    lead = starts[:decode_prefix] + 1
     ctx = StepContext(
         num_tokens=T, num_seqs=S, token_ids=take(L.token_ids, T), positions=take(L.positions, T),
         seq_of_token=take(L.seq_of_token, T), q_start=take(L.q_start, S + 1), start_pos=take(L.start_pos, S),
         ctx_len=take(L.ctx_len, S), slots=take(L.slots, S),
         block_tables=[take(L.table[g], S * L.width[g]).view(S, L.width[g]) for g in range(groups)],
         max_q_len=L.max_q_len, max_ctx_len=L.max_ctx_len if max_ctx_len is None else max_ctx_len,
-        typical_ctx_len=typical_ctx_len, decode_prefix=decode_prefix, host_q_lens=q_lens.tolist(),
-        host_start_pos=host[L.start_pos:L.start_pos + S].tolist(), host_slots=host[L.slots:L.slots + S].tolist())
+        typical_ctx_len=typical_ctx_len, decode_prefix=decode_prefix,
+        lead_keys=int(lead.sum()) if decode_prefix else 0, lead_longest=int(lead.max()) if decode_prefix else 0,
+        rest_ctx_len=int((starts[decode_prefix:] + q_lens[decode_prefix:]).max()) if decode_prefix else 0, host_q_lens=q_lens.tolist(),
+        host_start_pos=starts.tolist(), host_slots=host[L.slots:L.slots + S].tolist())
     rows = take(L.logit_rows, R) if R else None
     return ctx, rows

@@ -218,7 +218,7 @@ def attention_lib(head_dim: int, value_dim: int = 0) -> ctypes.CDLL:
         _declare(lib, "tge_attention_mma", [_c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_ptr,
                                             _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_int, _c_int,
                                             _c_int, _c_float, _c_int, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr,
-                                            _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_ptr])
+                                            _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_ptr])
         lib.tge_attention_mma_scratch_floats.argtypes = [_c_int, _c_int, _c_int]
         lib.tge_attention_mma_scratch_floats.restype = _c_ll
         if lib.tge_attention_mma_head_dim() != head_dim or lib.tge_attention_mma_value_dim() != value_dim:
@@ -887,7 +887,7 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
               pooled_v: Optional[torch.Tensor] = None, pool_table: Optional[torch.Tensor] = None,
               values_in_keys: int = 0, dist_bias: Optional[torch.Tensor] = None, keep_first: int = 0,
               gate: Optional[torch.Tensor] = None,
-              shared_keys: bool = False) -> torch.Tensor:
+              shared_keys: bool = False, lead_keys: int = 0, lead_longest: int = 0, rest_ctx_len: int = 0) -> torch.Tensor:
     """Paged causal attention of a flat batch of portions.
 
     q: [T, >= heads*head_dim] (dense rows, any row stride) holding rotated queries;
@@ -899,6 +899,8 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
     that are attended in parallel and merged; 0 picks a value from the batch shape.
     ``decode_prefix``: how many sequences at the head of the batch are known to bring one token each
     while others bring more (0: unknown); the tensor-core path then serves them with its decode kernel.
+    ``lead_keys`` / ``lead_longest``: how many keys those see together and at most, ``rest_ctx_len``: a bound on the contexts of the
+    others (0: unknown; all three tune how keys are cut and which kernels serve them).
     ``pool`` > 0 (with a window): beside the last ``window`` tokens a query sees one pooled key and value for
     every block of ``pool`` positions that lies wholly before them, in the same softmax; ``pooled_k`` /
     ``pooled_v`` are pages shaped like the keys' and values', entry b of a request where position b would be, found
@@ -987,7 +989,7 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
         raise KernelError("attention: runs of heads over the same keys are for single tokens on the tensor-core kernels")
     if use_mma:
         lib = attention_lib(head_dim, value_dim)
-        prefix = decode_prefix if decode_prefix >= MIN_DECODE_PREFIX and max_q_len > 1 and not pool else 0
+        prefix = decode_prefix if decode_prefix >= MIN_DECODE_PREFIX and max_q_len > 1 and not pool and heads // kv_heads <= 16 else 0
         prefix_split = split_tokens
         if pool:
             # The window's tokens go through the tensor-core kernels with their keys cut into at least two runs, so
@@ -1001,17 +1003,23 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
                 # request's keys holds nothing and is never read)
                 max_ctx_len = max(max_ctx_len, 128)
                 split_tokens = 64 * -(-max_ctx_len // 128)
+        rest_ctx = min(rest_ctx_len or max_ctx_len, max_ctx_len) if prefix else max_ctx_len
         if split_tokens == 0:
-            split_tokens = choose_attention_split(tokens, num_seqs, max_q_len, min(typical_ctx_len or max_ctx_len, span),
-                                                  heads, kv_heads, bound=span)
+            own = min(typical_ctx_len or max_ctx_len, span, rest_ctx)
+            split_tokens = choose_attention_split(tokens - prefix, num_seqs - prefix, max_q_len, own, heads, kv_heads, bound=min(span, rest_ctx))
             # the single tokens at the head of a mixed step are a decode batch of their own: a few of them deep in
             # long contexts want their keys cut although the portions beside them do not
-            prefix_split = choose_attention_split(prefix, prefix, 1, span, heads, kv_heads, bound=span) if prefix else 0
+            if prefix and lead_keys > 0 and span >= max_ctx_len:
+                prefix_split = choose_leading_split(lead_keys, lead_longest, kv_heads)
+            elif prefix:
+                prefix_split = choose_attention_split(prefix, prefix, 1, span, heads, kv_heads, bound=span)
+            else:
+                prefix_split = 0
         # single tokens over a window cut the window's span (from its first tile on), everything else the whole context
         narrow = heads // kv_heads <= 16 and window > 0 and keep_first == 0 and not pool
         one_window = min(max_ctx_len, window + 63) if narrow else max_ctx_len
         count = lambda split, reach: 1 if split == 0 or reach <= split else -(-reach // split)
-        splits = max(count(split_tokens, one_window if max_q_len <= 1 else max_ctx_len), count(prefix_split, one_window) if prefix else 1)
+        splits = max(count(split_tokens, one_window if max_q_len <= 1 else rest_ctx), count(prefix_split, one_window) if prefix else 1)
         need = lib.tge_attention_mma_scratch_floats(tokens, heads, splits)
         scratch = scratch_floats(need) if need > 0 else None
         _check(lib.tge_attention_mma(q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(),
@@ -1020,7 +1028,7 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
                                      max_ctx_len, out.data_ptr(), out_stride, heads, kv_heads, float(scale), window,
                                      split_tokens, _ptr(scratch), status_word().data_ptr(), prefix, prefix_split,
                                      _ptr(sink), int(bool(pool)), v_pitch, _ptr(dist_bias), dist_span,
-                                     keep_first, _ptr(gate), gate_stride, gate_elements, int(shared_keys), _stream()), lib)
+                                     keep_first, _ptr(gate), gate_stride, gate_elements, int(shared_keys), rest_ctx, _stream()), lib)
         if pool:
             core_lib = core()
             states = scratch.data_ptr()
@@ -1306,6 +1314,19 @@ def choose_attention_split(tokens: int, num_seqs: int, max_q_len: int, max_ctx_l
     if want_splits <= 1 and 2 * blocks <= 2 * sms and max_ctx_len >= 4096:
         want_splits = 2
     return keys_per_split(want_splits) if want_splits > 1 else 0
+
+
+def choose_leading_split(keys: int, longest: int, kv_heads: int) -> int:
+    """Keys per split for the single tokens at a mixed step's head, whose contexts are known: ``keys`` together, ``longest`` at most.
+
+    The prompt's kernel runs beside theirs and fills the SMs that they leave, so they are cut only where the longest would outlast
+    all of an SM's share of the work by more than the merging kernel costs (a block takes about 18 ns a key, so 512 keys 9 us).  Measured (us a
+    layer, uncut / cut at an SM's share): 28 heads over 4, 40 requests of up to 4,000 beside 300 tokens 80 / 56, 8 of up to 4,096
+    beside 512 43 / 30; left alone: 31 of up to 4,096 beside 1,187 at 40 over 8 100 / 106, 31 of 2,048 beside 512 44 / 48,
+    20 of up to 800 beside 700 31 / 40."""
+    share = -(-keys * kv_heads // core().tge_device_sm_count())
+    cut = max(512, -(-share // 64) * 64)
+    return cut if longest - cut >= 512 else 0
 
 
 def sample(logits: torch.Tensor, temperature: torch.Tensor, uniform: torch.Tensor,

@@ -334,7 +334,8 @@ class GQAttention(Mixer):
         return ops.attention(qk[:, :self.q_dim], k_pages, v_pages, table, ctx.q_start, ctx.start_pos, ctx.positions,
                              ctx.seq_of_token, ctx.num_seqs, ctx.max_q_len, ctx.max_ctx_len, self.heads, self.kv_heads,
                              self.head_dim, self.scale, window=int(self.window or 0), split_tokens=ctx.attn_split_tokens,
-                             typical_ctx_len=ctx.typical_ctx_len, decode_prefix=ctx.decode_prefix, sink=self.sink, out=out,
+                             typical_ctx_len=ctx.typical_ctx_len, decode_prefix=ctx.decode_prefix, lead_keys=ctx.lead_keys,
+                             lead_longest=ctx.lead_longest, rest_ctx_len=ctx.rest_ctx_len, sink=self.sink, out=out,
                              dist_bias=self.dist_table)
 
     def attend_separate(self, h, ctx: StepContext, cache: LayerCache, out: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -360,7 +361,8 @@ class GQAttention(Mixer):
         return ops.attention(rows[:, :self.q_dim], k_pages, v_pages, table, ctx.q_start, ctx.start_pos, ctx.positions,
                              ctx.seq_of_token, ctx.num_seqs, ctx.max_q_len, ctx.max_ctx_len, self.heads, self.kv_heads,
                              self.head_dim, self.scale, window=int(self.window or 0), split_tokens=ctx.attn_split_tokens,
-                             typical_ctx_len=ctx.typical_ctx_len, decode_prefix=ctx.decode_prefix, sink=self.sink, out=out,
+                             typical_ctx_len=ctx.typical_ctx_len, decode_prefix=ctx.decode_prefix, lead_keys=ctx.lead_keys,
+                             lead_longest=ctx.lead_longest, rest_ctx_len=ctx.rest_ctx_len, sink=self.sink, out=out,
                              dist_bias=self.dist_table, keep_first=self.keep_first, gate=gate)
 
     def cache_spec(self) -> Optional[PagedCacheSpec]:
@@ -406,7 +408,8 @@ class GQAttention(Mixer):
         return ops.attention(q, k_pages, v_pages, table, ctx.q_start, ctx.start_pos, ctx.positions, ctx.seq_of_token,
                              ctx.num_seqs, ctx.max_q_len, ctx.max_ctx_len, self.heads, self.kv_heads, self.head_dim,
                              self.scale, window=int(self.window or 0), split_tokens=ctx.attn_split_tokens,
-                             typical_ctx_len=ctx.typical_ctx_len, decode_prefix=ctx.decode_prefix, sink=self.sink,
+                             typical_ctx_len=ctx.typical_ctx_len, decode_prefix=ctx.decode_prefix, lead_keys=ctx.lead_keys,
+                             lead_longest=ctx.lead_longest, rest_ctx_len=ctx.rest_ctx_len, sink=self.sink,
                              out=out, gate=gate, **pooled)
 
     def share_input_projection(self, rows: torch.Tensor) -> Optional[torch.Tensor]:
@@ -502,7 +505,8 @@ class GQAttention(Mixer):
                           ctx.seq_of_token, ctx.num_seqs, ctx.max_q_len, ctx.max_ctx_len, self.heads,
                           self.kv_heads, self.head_dim, self.scale, window=int(self.window or 0),
                           split_tokens=ctx.attn_split_tokens, typical_ctx_len=ctx.typical_ctx_len,
-                          decode_prefix=ctx.decode_prefix, sink=self.sink, out=out)
+                          decode_prefix=ctx.decode_prefix, lead_keys=ctx.lead_keys,
+                          lead_longest=ctx.lead_longest, rest_ctx_len=ctx.rest_ctx_len, sink=self.sink, out=out)
         return a if beside is None else (a, did_beside)
 
     def inner(self, h, ctx: StepContext, cache: LayerCache, out: Optional[torch.Tensor] = None, beside=None):

@@ -139,6 +139,9 @@ class StepContext:
     host_slots: List[int] = field(default_factory=list)
     attn_split_tokens: int = 0         # 0 = let the kernel wrapper decide
     decode_prefix: int = 0             # in a step with longer portions: how many leading portions are single tokens
+    lead_keys: int = 0                 # what those hold together with their own tokens,
+    lead_longest: int = 0              # the most that one of them does (0: unknown),
+    rest_ctx_len: int = 0              # and the longest context of the portions behind them (0: unknown)
     scratch: Dict[str, Any] = field(default_factory=dict)
 
 

@@ -204,7 +204,8 @@ class LatentAttention(Mixer):
             ops.attention(queries[:, lo * self.entry:(lo + n) * self.entry], pages, None, table, ctx.q_start, ctx.start_pos,
                           ctx.positions, ctx.seq_of_token, ctx.num_seqs, ctx.max_q_len, ctx.max_ctx_len, n, runs if together else 1, self.entry,
                           self.scale, window=self.window or 0, split_tokens=split, typical_ctx_len=ctx.typical_ctx_len,
-                          decode_prefix=ctx.decode_prefix, values_in_keys=self.kv_rank, shared_keys=together,
+                          decode_prefix=ctx.decode_prefix, lead_keys=ctx.lead_keys,
+                          lead_longest=ctx.lead_longest, rest_ctx_len=ctx.rest_ctx_len, values_in_keys=self.kv_rank, shared_keys=together,
                           out=attended[:, lo * self.kv_rank:(lo + n) * self.kv_rank])
         if out is None:
             out = torch.empty((tokens, self.heads * self.vdim), dtype=dtype, device=h.device)
@@ -272,7 +273,8 @@ class LatentAttention(Mixer):
         attended = ops.attention(queries, keys, values, own_table, ctx.q_start, ctx.start_pos, ctx.positions, ctx.seq_of_token,
                                  ctx.num_seqs, ctx.max_q_len, ctx.max_ctx_len, self.heads, self.heads, per, self.scale,
                                  window=self.window or 0, split_tokens=ctx.attn_split_tokens, typical_ctx_len=ctx.typical_ctx_len,
-                                 decode_prefix=ctx.decode_prefix, out=out)
+                                 decode_prefix=ctx.decode_prefix, lead_keys=ctx.lead_keys,
+                                 lead_longest=ctx.lead_longest, rest_ctx_len=ctx.rest_ctx_len, out=out)
         mode = {"none": 0, "head": 1, "element": 2}[self.gate]
         return ops.gate_rows(attended, gate, self.heads, mode) if mode else attended
 

@@ -608,7 +608,7 @@ def test_linear_qkv_rope_store(ops, heads, kv_heads, head_dim, rotary, hidden, q
 # attention
 # ---------------------------------------------------------------------------
 def _attention_case(ops, dtype, heads, kv_heads, head_dim, q_lens, starts, window=0, split=0, force_simt=False,
-                    page_size=16, spike=None, decode_prefix=0):
+                    page_size=16, spike=None, decode_prefix=0, known=None):
     lengths = [s + n for s, n in zip(starts, q_lens)]
     k_pages, v_pages, table, k_list, v_list = paged_cache(lengths, kv_heads, head_dim, page_size, dtype, DEV, seed=9)
     positions, seq_of_token, q_start, start_pos = batch_index(q_lens, starts, DEV)
@@ -626,7 +626,7 @@ def _attention_case(ops, dtype, heads, kv_heads, head_dim, q_lens, starts, windo
     dq = buf.to(DEV)
     out = ops.attention(dq[:, :heads * head_dim], k_pages, v_pages, table, q_start, start_pos, positions,
                         seq_of_token, len(q_lens), max(q_lens), max(lengths), heads, kv_heads, head_dim, scale,
-                        window=window, split_tokens=split, force_simt=force_simt, decode_prefix=decode_prefix)
+                        window=window, split_tokens=split, force_simt=force_simt, decode_prefix=decode_prefix, **(known or {}))
     ops.check_status()
     q = buf[:, :heads * head_dim].view(T, heads, head_dim)
     refs = []
@@ -728,6 +728,42 @@ def test_leading_single_tokens_deep_in_long_contexts_get_splits_of_their_own(ops
     err, _, _ = _attention_case(ops, torch.bfloat16, 14, 2, 128, [1] * 9 + [1500], starts, decode_prefix=9, spike=(0, 123))
     assert err < TOL[torch.bfloat16]
     assert ops.choose_attention_split(1509, 10, 1500, 4400, 14, 2, bound=4400) == 0  # whose keys are not cut
+
+
+@pytest.mark.parametrize("heads,kv_heads,head_dim,window", [(14, 2, 128, 0), (8, 2, 64, 0), (6, 2, 48, 0), (20, 1, 128, 0), (14, 2, 128, 300)])
+@pytest.mark.parametrize("lead,portions,starts", [
+    ([1800, 3, 900, 64, 63, 1200, 65, 5], [70], [0]), ([40, 30, 20, 10, 5, 4, 3, 2], [200, 3], [0, 700]), ([1500] * 9, [17, 300], [128, 0])])
+def test_mixed_steps_whose_lengths_are_known(ops, heads, kv_heads, head_dim, window, lead, portions, starts):
+    """Single tokens cut at an SM's share of their keys or not at all, beside portions that are served by their own longest context: the
+    longest request among the single tokens, among the portions, all alike; a group too large for the decode kernel, pages of a
+    head size that goes without tensor maps, a window."""
+    q_lens, begins = [1] * len(lead) + portions, lead + starts
+    known = dict(lead_keys=sum(lead) + len(lead), lead_longest=max(lead) + 1, rest_ctx_len=max(s + n for s, n in zip(starts, portions)))
+    err, _, _ = _attention_case(ops, torch.bfloat16, heads, kv_heads, head_dim, q_lens, begins, window=window, decode_prefix=len(lead), known=known,
+                                spike=(0, lead[0] - 1))
+    assert err < TOL[torch.bfloat16]
+
+
+def test_side_by_side_attention_is_done_before_what_follows(ops):
+    """The two attention kernels of a mixed step run side by side; the kernels behind them (here products over their rows, and the next step's
+    attention into the same buffer) find both done, every time."""
+    lead = [int(n) for n in torch.randint(50, 3000, (40,), generator=torch.Generator().manual_seed(1))]
+    q_lens, starts = [1] * len(lead) + [90], lead + [0]
+    k_pages, v_pages, table, _k, _v = paged_cache([a + n for a, n in zip(starts, q_lens)], 4, 128, 64, torch.bfloat16, DEV, seed=5)
+    positions, seq_of_token, q_start, start_pos = batch_index(q_lens, starts, DEV)
+    gen = torch.Generator().manual_seed(6)
+    q = [torch.randn(sum(q_lens), 28 * 128, generator=gen).to(torch.bfloat16).to(DEV) for _ in range(2)]
+    w = (torch.randn(256, 28 * 128, generator=gen) * 0.02).to(torch.bfloat16).to(DEV)
+    out = torch.zeros_like(q[0])
+    first = [None, None]
+    for i in range(40):
+        ops.attention(q[i % 2], k_pages, v_pages, table, q_start, start_pos, positions, seq_of_token, len(q_lens), 90, max(lead) + 1, 28, 4, 128,
+                      128 ** -0.5, decode_prefix=len(lead), lead_keys=sum(lead) + 40, lead_longest=max(lead) + 1, rest_ctx_len=90, out=out)
+        rows = ops.linear(out, w, None, ops.GEMM_STORE_F32, settled=True)
+        if first[i % 2] is None:
+            first[i % 2] = rows
+        assert torch.equal(rows, first[i % 2]), i
+    ops.check_status()
 
 
 def test_leading_single_tokens_that_fill_the_chip_are_not_cut(ops, monkeypatch):
