@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(256) decay_prepare_vec_kernel(
 
 // The same eight numbers at a time, sixteen where a unit is turned (eight of the lower half and the eight they are paired with), a block per
 // token (everything a multiple of eight).  Bound by its bytes, two thirds of them the float32 results (88 MB for 2,048 tokens of 28 heads
-// of 128, where the kernel above takes 32 us).
+// of 128: 23 us, the kernel above 32).
 __global__ void __launch_bounds__(256) decay_prepare_eights_kernel(
     const __nv_bfloat16* rows, long long ld, int q_off, int k_off, int heads, int dim, int activation,
     const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary,
@@ -938,7 +938,7 @@ __global__ void __launch_bounds__(256) gated_norm_vec_kernel(const float* __rest
 }
 
 // Groups of up to 128 numbers, four to a warp, so that four rows' loads are on their way together (with a group to a warp each waited
-// for one: 2,048 tokens, 28 groups of 128, 22 us); a group's sum is the kernel's above.
+// for one: 2,048 tokens, 28 groups of 128, 22 us; this 19, bound by its instructions); a group's sum is the kernel's above.
 constexpr int GATED_EACH = 4;
 __global__ void __launch_bounds__(256) gated_norm_small_kernel(const float* o, const __nv_bfloat16* gate, long long ld_gate,
                                                                const float* __restrict__ weight, __nv_bfloat16* __restrict__ out, long long ld_out,
@@ -1136,7 +1136,7 @@ constexpr int POOL_AHEAD = 16, POOL_THREADS = 256;
 // threads per (32 tokens, kv head), which looks for the tokens at a block's last position among them.  The means are taken over the
 // keys and values as their pages hold them, and entry b of a request lies where position b would in the pooled pages.
 // Bound by round trips: POOL_AHEAD positions' pages, then their numbers, are on their way together, added in order.  2,048 tokens, 4 kv heads
-// of 128, blocks of 64: 69 us one position after the other; 34 eight at a time, a block of threads per token (63 of 64 only left).
+// of 128, blocks of 64: 69 us one position after the other; 34 eight at a time, a block of threads per token (63 of 64 only left); this 23.
 template <typename T>
 __global__ void __launch_bounds__(POOL_THREADS) pool_kv_kernel(
     const T* k_pages, const T* v_pages, const int* __restrict__ block_table, int max_pages,
@@ -1520,7 +1520,7 @@ __global__ void __launch_bounds__(NRV_THREADS) norm_rope_store_vec_kernel(
 // stay in registers.  Places, pages and angles are looked up into shared memory while the kernel in front still runs.  Bound by its
 // instructions (about 250 a warp and token), not by its bytes (38 MB for 2,048 tokens of 28 heads over 4 of 128): a warp per (token, head) with
 // two-byte loads of every tap, one behind the other, took 86 us there; four tokens unrolled with their rows and taps in registers 62 (a
-// quarter of an SM's warps, 1,800 instructions each, waits for the instructions themselves).
+// quarter of an SM's warps, 1,800 instructions each, waits for the instructions themselves), this 47.
 constexpr int CONV_TOKENS = 8, CONV_THREADS = 256, CONV_VEC_TOKENS = 16;
 
 __device__ __forceinline__ void unpack_eight(const uint4& raw, float f[8]) {
