@@ -48,8 +48,8 @@ constexpr int A_STAGE_BYTES = BM * BK * 2;
 constexpr int MAX_STAGES = 8;
 constexpr int EPI_WARPS = 8;              // two per 32-lane quarter of tensor memory, each taking half the columns
 constexpr int NUM_THREADS = (2 + EPI_WARPS) * 32;
-// Pairs of SMs run wide tiles, whose last epilogue nothing hides: four warps to a quarter.  (Not on one SM alone: what runs there are mostly
-// a few tokens, and the registers of so many threads would keep the next product's block from starting beside a small kernel.)
+// Pairs of SMs run wide tiles, whose last epilogue nothing hides: four warps to a quarter.  (An SM alone runs a few tokens mostly, one or two
+// groups of sixteen columns to a tile, which eight warps share as well.)
 constexpr int PAIR_EPI_WARPS = 16;
 constexpr int PAIR_THREADS = (2 + PAIR_EPI_WARPS) * 32;
 constexpr int SMEM_LIMIT = 227 * 1024;
