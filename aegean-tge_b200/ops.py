@@ -1019,8 +1019,10 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
         narrow = heads // kv_heads <= 16 and window > 0 and keep_first == 0 and not pool
         one_window = min(max_ctx_len, window + 63) if narrow else max_ctx_len
         count = lambda split, reach: 1 if split == 0 or reach <= split else -(-reach // split)
-        splits = max(count(split_tokens, one_window if max_q_len <= 1 else rest_ctx), count(prefix_split, one_window) if prefix else 1)
-        need = lib.tge_attention_mma_scratch_floats(tokens, heads, splits)
+        splits = count(split_tokens, one_window if max_q_len <= 1 else rest_ctx)
+        # the single tokens' states are laid out for themselves alone
+        need = max(lib.tge_attention_mma_scratch_floats(tokens, heads, splits),
+                   lib.tge_attention_mma_scratch_floats(prefix, heads, count(prefix_split, one_window)) if prefix else 0)
         scratch = scratch_floats(need) if need > 0 else None
         _check(lib.tge_attention_mma(q.data_ptr(), q_stride, k_pages.data_ptr(), v_pages.data_ptr(),
                                      block_table.data_ptr(), max_pages, num_pages, page_size, q_start.data_ptr(),
