@@ -1293,11 +1293,11 @@ const CUtensorMap* pool_map(const void* pages, int num_pages, int kv_heads, int 
 // request of 2,048 tokens in 17 splits 8.5 us a layer and now 5.9, eight in 8 splits 4.9 and 4.8 (7B shape, in place).
 constexpr int MERGE_LANES = 4;                                          // splits per lane at most: 128 in all
 constexpr int MERGE_BATCH = 16;                                         // states on their way together
-__global__ void attention_merge_kernel(const float* __restrict__ partial_o, const float* __restrict__ partial_ml,
+__global__ void attention_merge_kernel(const float* partial_o, const float* partial_ml,
                                        const int* __restrict__ positions, __nv_bfloat16* __restrict__ out,
                                        int out_stride, int total_tokens, int heads, int window, int split_tokens,
                                        int num_splits, int first_token, const float* __restrict__ sink, int keep_first,
-                                       const __nv_bfloat16* __restrict__ gate, int gate_stride, int gate_elements,
+                                       const __nv_bfloat16* gate, int gate_stride, int gate_elements,
                                        int window_runs) {
   pdl_trigger();
   const int t = blockIdx.x + first_token, h = blockIdx.y, lane = threadIdx.x & 31;

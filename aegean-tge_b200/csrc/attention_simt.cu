@@ -166,10 +166,10 @@ __global__ void __launch_bounds__(128) attention_simt_kernel(
 // output.  One warp per (token, head): the pooled state never leaves its registers.
 template <typename T>
 __global__ void __launch_bounds__(128) attention_pooled_merge_kernel(
-    const T* __restrict__ q, int q_stride, const T* __restrict__ kp_pages, const T* __restrict__ vp_pages,
+    const T* q, int q_stride, const T* kp_pages, const T* vp_pages,
     const int* __restrict__ pool_table, int pool_max_pages, int pool_num_pages, int page_size,
-    const int* __restrict__ positions, const int* __restrict__ seq_of_token, const float* __restrict__ partial_o,
-    const float* __restrict__ partial_ml, int total_tokens, int num_runs, int run_tokens, T* __restrict__ out,
+    const int* __restrict__ positions, const int* __restrict__ seq_of_token, const float* partial_o,
+    const float* partial_ml, int total_tokens, int num_runs, int run_tokens, T* __restrict__ out,
     int out_stride, int heads, int kv_heads, int head_dim, int value_dim, float scale_log2, int window, int pool,
     const float* __restrict__ sink, int* status) {
   pdl_trigger();

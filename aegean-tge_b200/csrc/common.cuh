@@ -46,8 +46,11 @@ constexpr int TGE_UNSUPPORTED = -100;  // shape outside what the kernel takes; n
 // the stream may then be scheduled and run its own set-up) and pdl_wait() before it first touches global
 // memory that an earlier kernel writes or reads: the wait returns once the preceding kernel has finished
 // and its writes are visible.  Without the launch attribute both are no-ops.
-// A kernel with work in front of its wait takes what the kernel before it writes through pointers without __restrict__: loads through a
-// const __restrict__ pointer count as loads of what never changes, and the compiler may move them ahead of the wait.
+// A kernel that waits takes everything an earlier kernel may have written or read (results, rows updated in place, states) through
+// pointers without __restrict__: loads through a const __restrict__ pointer count as loads of what never changes, and those
+// through any __restrict__ pointer as loads that the wait cannot touch, so the compiler may move them ahead of it, whether
+// other work stands there or not.  __restrict__ is for the model's constants, for what the host gave the step (positions, tables), and
+// for results that the kernel writes and does not read before it has written them.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 

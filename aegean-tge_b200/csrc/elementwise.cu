@@ -48,7 +48,7 @@ TGE_API int tge_embedding(const void* table, int is_bf16, const int* ids, float*
 // One block per output row; optional row gather (rows[r] = source row).
 // ---------------------------------------------------------------------------
 template <typename TOut>
-__global__ void rmsnorm_kernel(const float* __restrict__ x, const float* __restrict__ weight,
+__global__ void rmsnorm_kernel(const float* x, const float* __restrict__ weight,
                                const int* __restrict__ rows, TOut* __restrict__ out, int hidden,
                                int src_rows, float eps, int* status) {
   __shared__ float scratch[32];
@@ -183,7 +183,7 @@ TGE_API int tge_add_to_stream(float* x, const void* y, int y_is_bf16, long long 
 // the cache, v is copied.  A page is [kv_heads, page_size, head_dim].
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void rope_kv_store_kernel(T* __restrict__ qkv, int row_stride, const float* __restrict__ cos_table,
+__global__ void rope_kv_store_kernel(T* qkv, int row_stride, const float* __restrict__ cos_table,
                                      const float* __restrict__ sin_table, int table_rows,
                                      const int* __restrict__ positions, const int* __restrict__ seq_of_token,
                                      const int* __restrict__ block_table, int max_pages, T* __restrict__ k_pages,
@@ -257,7 +257,7 @@ __device__ __forceinline__ uint4 pack8(const float f[8]) {
   return raw;
 }
 
-__global__ void rope_kv_store_vec_kernel(__nv_bfloat16* __restrict__ qkv, int row_stride, const float* __restrict__ cos_table,
+__global__ void rope_kv_store_vec_kernel(__nv_bfloat16* qkv, int row_stride, const float* __restrict__ cos_table,
                                          const float* __restrict__ sin_table, int table_rows,
                                          const int* __restrict__ positions, const int* __restrict__ seq_of_token,
                                          const int* __restrict__ block_table, int max_pages,
@@ -379,7 +379,7 @@ TGE_API int tge_rope_kv_store(void* qkv, int is_bf16, int row_stride, const floa
 // out[m, n] = rows[m, n] / sqrt(sum over slices of sums[slice][m] / width + eps), bfloat16: completes rows that
 // travelled without their RMSNorm factor, for a taker that cannot apply it itself.
 namespace {
-__global__ void scale_rows_kernel(const __nv_bfloat16* __restrict__ rows, long long ld_rows, const float* __restrict__ sums,
+__global__ void scale_rows_kernel(const __nv_bfloat16* rows, long long ld_rows, const float* sums,
                                   int slices, int width, float eps, __nv_bfloat16* __restrict__ out, long long ld_out,
                                   int m_rows, int n_cols) {
   pdl_trigger();
@@ -415,8 +415,8 @@ TGE_API int tge_scale_rows(const void* rows, long long ld_rows, const float* sum
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256) qk_norm_kv_store_kernel(
-    T* __restrict__ qkv, int row_stride, const float* __restrict__ q_weight, const float* __restrict__ k_weight,
-    float eps, int per_head, const T* __restrict__ v_other, int v_other_stride, const float* __restrict__ blend,
+    T* qkv, int row_stride, const float* __restrict__ q_weight, const float* __restrict__ k_weight,
+    float eps, int per_head, const T* v_other, int v_other_stride, const float* __restrict__ blend,
     const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table,
     int max_pages, T* __restrict__ k_pages, T* __restrict__ v_pages, int num_pages, int page_size, int heads,
     int kv_heads, int head_dim, int value_dim, int store_kv, int* status) {
@@ -517,8 +517,8 @@ constexpr int QKN_UNITS = 12;          // most units per thread: rows of up to 2
 // blocks on an SM; with 12 for every row a 2,048-token step took 28 us where the rotate-and-store kernel takes 10).
 template <int UNITS>
 __global__ void __launch_bounds__(QKN_THREADS) qk_norm_kv_store_vec_kernel(
-    __nv_bfloat16* __restrict__ qkv, int row_stride, const float* __restrict__ q_weight, const float* __restrict__ k_weight,
-    float eps, const __nv_bfloat16* __restrict__ v_other, int v_other_stride, const float* __restrict__ blend,
+    __nv_bfloat16* qkv, int row_stride, const float* __restrict__ q_weight, const float* __restrict__ k_weight,
+    float eps, const __nv_bfloat16* v_other, int v_other_stride, const float* __restrict__ blend,
     const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table,
     int max_pages, __nv_bfloat16* __restrict__ k_pages, __nv_bfloat16* __restrict__ v_pages, int num_pages, int page_size,
     int heads, int kv_heads, int head_dim, int value_dim, int store_kv, int* status) {
@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(QKN_THREADS) qk_norm_kv_store_vec_kernel(
 // The same for the norm over each head: `lanes` lanes (a power of two, one per 16 bytes of a head) share a head, which
 // stays in registers between its sum of squares and its scaling.
 __global__ void __launch_bounds__(QKN_THREADS) qk_head_norm_kv_store_vec_kernel(
-    __nv_bfloat16* __restrict__ qkv, int row_stride, const float* __restrict__ q_weight, const float* __restrict__ k_weight,
+    __nv_bfloat16* qkv, int row_stride, const float* __restrict__ q_weight, const float* __restrict__ k_weight,
     float eps, const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table,
     int max_pages, __nv_bfloat16* __restrict__ k_pages, __nv_bfloat16* __restrict__ v_pages, int num_pages, int page_size,
     int heads, int kv_heads, int head_dim, int value_dim, int store_kv, int lanes, int* status) {
@@ -736,7 +736,7 @@ TGE_API int tge_qk_norm_kv_store(void* qkv, int is_bf16, int row_stride, const f
 // ---------------------------------------------------------------------------
 // Soft cap of float32 scores, in place: z <- cap * tanh(z / cap).
 // ---------------------------------------------------------------------------
-__global__ void soft_cap_kernel(float* __restrict__ z, long long ld, int rows, int cols, float cap) {
+__global__ void soft_cap_kernel(float* z, long long ld, int rows, int cols, float cap) {
   pdl_trigger();
   pdl_wait();
   const size_t count = (size_t)rows * cols;

@@ -28,8 +28,8 @@ constexpr int GP_MAX_TAPS = 16;
 
 // One convolved and activated channel of token t.  `raw` row t holds the step's inputs; inputs from before the portion
 // come from the request's tail [taps-1, channels] (oldest first), zeros for a request that starts.
-__device__ __forceinline__ float conv_channel(const float* __restrict__ raw, long long ld, int conv_off, int c, int t,
-                                              int first, const float* __restrict__ tail, int channels,
+__device__ __forceinline__ float conv_channel(const float* raw, long long ld, int conv_off, int c, int t,
+                                              int first, const float* tail, int channels,
                                               const float* __restrict__ w, const float* __restrict__ bias, int taps) {
   float acc = bias != nullptr ? bias[c] : 0.0f;
   const int keep = taps - 1;
@@ -49,8 +49,8 @@ __device__ __forceinline__ float conv_channel(const float* __restrict__ raw, lon
 //   qk[t, g] = (C, B), v[t, h] = x, gates[t, h] = (exp(-exp(A_h) dt), dt) with dt = softplus(dt + dt_bias_h).
 // One block per token (several for a step of few tokens); its warps take the units (q/k groups, value heads) in turn.
 __global__ void __launch_bounds__(128) gated_prepare_kernel(
-    const float* __restrict__ raw, long long ld, int mode, int groups, int heads, int dim, int vdim, int taps,
-    const float* __restrict__ conv_w, const float* __restrict__ conv_b, const float* __restrict__ tails,
+    const float* raw, long long ld, int mode, int groups, int heads, int dim, int vdim, int taps,
+    const float* __restrict__ conv_w, const float* __restrict__ conv_b, const float* tails,
     const int* __restrict__ slots, const int* __restrict__ q_start, const int* __restrict__ seq_of_token,
     const float* __restrict__ a_log, const float* __restrict__ dt_bias, float unit_eps, float q_scale,
     float* __restrict__ qk, float* __restrict__ v, float* __restrict__ gates) {
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(128) gated_prepare_kernel(
 
 // The convolution's tail after the step: the last taps-1 inputs of each request, oldest first.  One thread per
 // (request, channel) reads what it needs before it writes, so a portion shorter than the tail shifts it.
-__global__ void conv_tail_update_kernel(const float* __restrict__ raw, long long ld, int conv_off, float* __restrict__ tails,
+__global__ void conv_tail_update_kernel(const float* raw, long long ld, int conv_off, float* tails,
                                         const int* __restrict__ slots, const int* __restrict__ q_start, int taps,
                                         int channels) {
   pdl_trigger();
@@ -148,8 +148,8 @@ constexpr int GR_COLS = GR_WARPS * 4;       // columns of a block
 
 template <int ROWS, bool DELTA>
 __global__ void __launch_bounds__(GR_WARPS * 32) gated_rule_scan_kernel(
-    const float* __restrict__ qk, const float* __restrict__ v, const float* __restrict__ gates,
-    const float* __restrict__ skip, int heads, int groups, int dim, int vdim, float* __restrict__ state,
+    const float* qk, const float* v, const float* gates,
+    const float* __restrict__ skip, int heads, int groups, int dim, int vdim, float* state,
     const int* __restrict__ slots, const int* __restrict__ q_start, float* __restrict__ out) {
   pdl_trigger();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -242,8 +242,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 
 template <int ROWS, int PARTS, bool DELTA>
 __global__ void __launch_bounds__(GR_WARPS * 32) gated_rule_scan_staged_kernel(
-    const float* __restrict__ qk, const float* __restrict__ v, const float* __restrict__ gates,
-    const float* __restrict__ skip, int heads, int groups, int vdim, float* __restrict__ state,
+    const float* qk, const float* v, const float* gates,
+    const float* __restrict__ skip, int heads, int groups, int vdim, float* state,
     const int* __restrict__ slots, const int* __restrict__ q_start, float* __restrict__ out) {
   constexpr int DIM = ROWS * PARTS;
   constexpr int GS_COLS = GR_WARPS * 2 * (32 / PARTS); // columns of a block
@@ -407,7 +407,7 @@ int launch_gated_rule_scan(const float* qk, const float* v, const float* gates, 
 }
 
 // x[t] += alpha * y[t] / sqrt(mean(y[t]^2) + eps) * w; one block per token.
-__global__ void __launch_bounds__(256) norm_scale_add_kernel(float* __restrict__ x, const float* __restrict__ y, long long ldy,
+__global__ void __launch_bounds__(256) norm_scale_add_kernel(float* x, const float* y, long long ldy,
                                                              const float* __restrict__ weight, int width, float alpha,
                                                              float eps) {
   __shared__ float scratch[32];
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(256) norm_scale_add_kernel(float* __restrict__
 // its pages.  One block per token, a warp per head.
 template <typename T>
 __global__ void __launch_bounds__(256) qk_temp_store_kernel(
-    T* __restrict__ qk, int row_stride, const float* __restrict__ q_weight, const float* __restrict__ k_weight, float eps,
+    T* qk, int row_stride, const float* __restrict__ q_weight, const float* __restrict__ k_weight, float eps,
     float temp_coef, int temp_every, const int* __restrict__ positions, const int* __restrict__ seq_of_token,
     const int* __restrict__ block_table, int max_pages, T* __restrict__ k_pages, T* __restrict__ v_pages, int num_pages,
     int page_size, int heads, int kv_heads, int head_dim, int store_kv, int* status) {
@@ -475,7 +475,7 @@ __global__ void __launch_bounds__(256) qk_temp_store_kernel(
 // rows [T, 2 * inner] float32 with (g_i, u_i) side by side -> out [T, inner]:
 // g <- min(g, L); u <- clamp(u, -L, L); out = g sigmoid(alpha g) (u + offset).
 template <typename T>
-__global__ void __launch_bounds__(256) gated_clamp_act_kernel(const float* __restrict__ rows, long long ld, T* __restrict__ out,
+__global__ void __launch_bounds__(256) gated_clamp_act_kernel(const float* rows, long long ld, T* __restrict__ out,
                                                               long long ld_out, int tokens, int inner, float limit,
                                                               float alpha, float offset) {
   pdl_trigger();
@@ -492,7 +492,7 @@ __global__ void __launch_bounds__(256) gated_clamp_act_kernel(const float* __res
 
 // out[t] = [a[t] | b[t]] in the products' number format.
 template <typename T>
-__global__ void __launch_bounds__(256) concat_rows_kernel(const float* __restrict__ a, const float* __restrict__ b,
+__global__ void __launch_bounds__(256) concat_rows_kernel(const float* a, const float* b,
                                                           T* __restrict__ out, int tokens, int width) {
   pdl_trigger();
   pdl_wait();

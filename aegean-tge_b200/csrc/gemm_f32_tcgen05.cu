@@ -116,7 +116,7 @@ __device__ __forceinline__ void finish(const F32GemmParams& p, float v, int m, i
 }
 
 // ---- the token rows in three parts: planes [3][M][Kp] of bfloat16, zeros behind column K ----
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, long long ldx, __nv_bfloat16* __restrict__ planes,
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* x, long long ldx, __nv_bfloat16* __restrict__ planes,
                                                          int M, int K, int Kp, int vec) {
   // Trigger behind the wait: the product then starts once whatever came before this call is done, so its loader may ask for the
   // weights, and the kernel that adds the cuts for the bias, ahead of their own waits, whoever wrote those.

@@ -164,8 +164,8 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool live) 
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(to), "l"(src), "r"(bytes) : "memory");
 }
 
-__global__ void __launch_bounds__(128) gemm_skinny_kernel(const float* __restrict__ x, size_t ldx, const float* __restrict__ w, size_t ldw,
-                                                          const float* __restrict__ bias, float* __restrict__ out, size_t ldo, int M,
+__global__ void __launch_bounds__(128) gemm_skinny_kernel(const float* x, size_t ldx, const float* w, size_t ldw,
+                                                          const float* bias, float* __restrict__ out, size_t ldo, int M,
                                                           int N, int K, int epilogue, float alpha, int act_from) {
   extern __shared__ __align__(16) float ring[];
   pdl_trigger();

@@ -97,7 +97,7 @@ __device__ __forceinline__ bool gated_epilogue(int epilogue) { return epilogue =
 
 // 1 / sqrt(mean square of the row + eps) from the row's sums of squares in slices (added in slice order; the
 // loads of eight slices are in flight together)
-__device__ __forceinline__ float row_factor_of(const float* __restrict__ ss, int slices, int width, float eps, int m_tok, int m) {
+__device__ __forceinline__ float row_factor_of(const float* ss, int slices, int width, float eps, int m_tok, int m) {
   if (ss == nullptr) return 1.0f;
   float sum = 0.0f;
   for (int first = 0; first < slices; first += 8) {
@@ -692,9 +692,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
 }
 
 // Adds the k-splits in split order and applies the epilogue.
-__global__ void splitk_epilogue_kernel(const float* __restrict__ partial, const float* __restrict__ bias, void* out,
+__global__ void splitk_epilogue_kernel(const float* partial, const float* __restrict__ bias, void* out,
                                        long long ldo, int m_tok, int n_w, int splits, int epilogue,
-                                       const float* __restrict__ ss, int ss_slices, int ss_width, float ss_eps,
+                                       const float* ss, int ss_slices, int ss_width, float ss_eps,
                                        float alpha, int act_from) {
   pdl_trigger();
   pdl_wait();
@@ -741,9 +741,9 @@ __global__ void splitk_epilogue_kernel(const float* __restrict__ partial, const 
 // and by one round trip; the kernel above divides an index per element and loads four bytes at a time:
 // 193 tokens of the 7B shape (q/k/v in 3 cuts, o in 4, down in 5) 8.8 us a launch, now 3.3.
 constexpr int QUAD_THREADS = 128;
-__global__ void __launch_bounds__(QUAD_THREADS) splitk_epilogue_quad_kernel(const float* __restrict__ partial, const float* __restrict__ bias, void* out,
+__global__ void __launch_bounds__(QUAD_THREADS) splitk_epilogue_quad_kernel(const float* partial, const float* __restrict__ bias, void* out,
                                                                             long long ldo, int m_tok, int n_w, int splits, int epilogue,
-                                                                            const float* __restrict__ ss, int ss_slices, int ss_width, float ss_eps,
+                                                                            const float* ss, int ss_slices, int ss_width, float ss_eps,
                                                                             float alpha, int act_from) {
   pdl_trigger();
   const int m = blockIdx.y, n = ((int)blockIdx.x * QUAD_THREADS + (int)threadIdx.x) * 4;
@@ -1153,7 +1153,7 @@ constexpr int NORM_THREADS = 1024;
 constexpr int NORM_PER_THREAD = 8;               // columns per thread: rows up to 1024 * 8 = 8192 wide
 
 __global__ void __launch_bounds__(NORM_THREADS)
-splitk_add_norm_kernel(const float* __restrict__ partial, const float* __restrict__ bias, float* __restrict__ stream,
+splitk_add_norm_kernel(const float* partial, const float* __restrict__ bias, float* stream,
                        long long ld_stream, const float* __restrict__ norm_weight, float eps,
                        __nv_bfloat16* __restrict__ norm_out, long long ld_norm, int m_tok, int n_w, int splits,
                        float alpha) {
@@ -1181,10 +1181,14 @@ splitk_add_norm_kernel(const float* __restrict__ partial, const float* __restric
 #pragma unroll 4
       for (int s = 0; s < splits; ++s) acc += src[s * plane];
       const float v = stream[(size_t)t * ld_stream + n] + alpha * (acc + add[i]);
-      stream[(size_t)t * ld_stream + n] = v;
       value[i] = v;
       sum = fmaf(v, v, sum);
     }
+  }
+#pragma unroll
+  for (int i = 0; i < NORM_PER_THREAD; ++i) {      // behind every load: a store in between would keep the next column's loads behind it
+    const int n = threadIdx.x + i * NORM_THREADS;
+    if (n < n_w) stream[(size_t)t * ld_stream + n] = value[i];
   }
   sum = block_sum(sum, scratch);
   const float scale = 1.0f / sqrtf(sum / (float)n_w + eps);
@@ -1198,7 +1202,7 @@ splitk_add_norm_kernel(const float* __restrict__ partial, const float* __restric
 // One block per (token, head): the head's q, k or v values = sum of the partial sums + bias; a query head is
 // rotated into the qkv buffer, a key head rotated into its page, a value head copied into its page
 // (formulas as in the stand-alone rotate-and-store kernel).
-__global__ void splitk_qkv_rope_store_kernel(const float* __restrict__ partial, const float* __restrict__ bias,
+__global__ void splitk_qkv_rope_store_kernel(const float* partial, const float* __restrict__ bias,
                                              __nv_bfloat16* __restrict__ qkv, long long ld_qkv, int m_tok, int n_w,
                                              int splits, const float* __restrict__ cos_table,
                                              const float* __restrict__ sin_table, int table_rows, int rotary,
@@ -1206,7 +1210,7 @@ __global__ void splitk_qkv_rope_store_kernel(const float* __restrict__ partial, 
                                              const int* __restrict__ block_table, int max_pages,
                                              __nv_bfloat16* __restrict__ k_pages, __nv_bfloat16* __restrict__ v_pages,
                                              int num_pages, int page_size, int heads, int kv_heads, int head_dim,
-                                             int* status, const float* __restrict__ ss, int ss_slices, int ss_width,
+                                             int* status, const float* ss, int ss_slices, int ss_width,
                                              float ss_eps) {
   extern __shared__ float head_values[];
   pdl_trigger();
@@ -1301,15 +1305,15 @@ constexpr int ACT_PER_THREAD = 4;
 constexpr int QKV_ACT_SLICE = QKV_ACT_THREADS * ACT_PER_THREAD;      // up columns per block
 
 __global__ void __launch_bounds__(QKV_ACT_THREADS)
-splitk_qkv_norm_act_store_kernel(const float* __restrict__ partial, int m_tok, int n_w, int splits,
+splitk_qkv_norm_act_store_kernel(const float* partial, int m_tok, int n_w, int splits,
                                  __nv_bfloat16* __restrict__ qkv, long long ld_qkv, __nv_bfloat16* __restrict__ act_out,
                                  long long ld_act, int activation, const float* __restrict__ q_weight,
-                                 const float* __restrict__ k_weight, float eps, const __nv_bfloat16* __restrict__ v_other,
+                                 const float* __restrict__ k_weight, float eps, const __nv_bfloat16* v_other,
                                  long long ld_other, const float* __restrict__ blend, const int* __restrict__ positions,
                                  const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int max_pages,
                                  __nv_bfloat16* __restrict__ k_pages, __nv_bfloat16* __restrict__ v_pages, int num_pages,
                                  int page_size, int heads, int kv_heads, int head_dim, int value_dim, int store_kv,
-                                 int* status, const float* __restrict__ ss, int ss_slices, int ss_width, float ss_eps) {
+                                 int* status, const float* ss, int ss_slices, int ss_width, float ss_eps) {
   __shared__ float scratch[64];
   pdl_trigger();
   const int t = blockIdx.x;
@@ -1436,7 +1440,7 @@ splitk_qkv_norm_act_store_kernel(const float* __restrict__ partial, int m_tok, i
 constexpr int SCALE_SLICE = 256;
 
 __global__ void __launch_bounds__(SCALE_SLICE)
-splitk_add_scale_kernel(const float* __restrict__ partial, const float* __restrict__ bias, float* __restrict__ stream,
+splitk_add_scale_kernel(const float* partial, const float* __restrict__ bias, float* stream,
                         long long ld_stream, const float* __restrict__ norm_weight, __nv_bfloat16* __restrict__ scaled_out,
                         long long ld_scaled, float* __restrict__ ss_out, int m_tok, int n_w, int splits, float alpha) {
   __shared__ float scratch[32];

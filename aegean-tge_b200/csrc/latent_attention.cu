@@ -47,7 +47,7 @@ __device__ __forceinline__ float rotated_pair_element(const float* x, int e, int
 
 template <typename T>
 __global__ void __launch_bounds__(256) latent_prepare_kernel(
-    const float* __restrict__ raw, long long ld_raw, int q_rank, int kv_rank, int rot, int gate_n, int has_kv,
+    const float* raw, long long ld_raw, int q_rank, int kv_rank, int rot, int gate_n, int has_kv,
     const float* __restrict__ q_weight, const float* __restrict__ kv_weight, float eps, const float* __restrict__ cos_table,
     const float* __restrict__ sin_table, int rot_dims, int halves, int max_positions, const int* __restrict__ positions,
     const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int max_pages, int num_pages, int page_size,
@@ -106,8 +106,8 @@ constexpr int HL_ROWS_MAX_TOKENS = 16;     // steps of up to this many tokens ta
 // 2 x 2 patch, every output accumulated over k in ascending order (so a row's result does not depend on the batch).
 template <typename T>
 __global__ void __launch_bounds__(256) head_linear_kernel(
-    const T* __restrict__ x, long long x_row, long long x_head, const T* __restrict__ w, T* __restrict__ out,
-    long long out_row, long long out_head, const float* __restrict__ gate, int gate_mode, long long gate_row, int tokens,
+    const T* x, long long x_row, long long x_head, const T* __restrict__ w, T* __restrict__ out,
+    long long out_row, long long out_head, const float* gate, int gate_mode, long long gate_row, int tokens,
     int n_out, int k_in) {
   __shared__ float xs[HL_BM][HL_BK + 1];
   __shared__ float ws[HL_BN][HL_BK + 1];
@@ -159,8 +159,8 @@ __global__ void __launch_bounds__(256) head_linear_kernel(
 // sum depends on k_in alone.
 template <typename T>
 __global__ void __launch_bounds__(256) head_linear_rows_kernel(
-    const T* __restrict__ x, long long x_row, long long x_head, const T* __restrict__ w, T* __restrict__ out,
-    long long out_row, long long out_head, const float* __restrict__ gate, int gate_mode, long long gate_row, int tokens,
+    const T* x, long long x_row, long long x_head, const T* __restrict__ w, T* __restrict__ out,
+    long long out_row, long long out_head, const float* gate, int gate_mode, long long gate_row, int tokens,
     int n_out, int k_in) {
   pdl_trigger();
   pdl_wait();
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256) head_linear_rows_kernel(
 
 template <typename T>
 __global__ void __launch_bounds__(256) rotate_runs_kernel(
-    const T* __restrict__ src, long long src_row, long long src_head, T* __restrict__ dst, long long dst_row,
+    const T* src, long long src_row, long long src_head, T* __restrict__ dst, long long dst_row,
     long long dst_head, const float* __restrict__ cos_table, const float* __restrict__ sin_table, int rot_dims,
     int max_positions, const int* __restrict__ positions, int tokens, int heads, int width, int first, int halves, int* status) {
   pdl_trigger();
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256) rotate_runs_kernel(
 // The same on pairs of bfloat16 (every size, stride and the first rotated place even, rows on 4 bytes; of halves their
 // length even as well): a thread owns two neighbouring numbers, of halves it also reads the two they are rotated with.
 __global__ void __launch_bounds__(256) rotate_runs_pairs_kernel(
-    const __nv_bfloat16* __restrict__ src, long long src_row, long long src_head, __nv_bfloat16* __restrict__ dst,
+    const __nv_bfloat16* src, long long src_row, long long src_head, __nv_bfloat16* __restrict__ dst,
     long long dst_row, long long dst_head, const float* __restrict__ cos_table, const float* __restrict__ sin_table,
     int rot_dims, int max_positions, const int* __restrict__ positions, int tokens, int heads, int width, int first,
     int halves, int* status) {
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(256) rotate_runs_pairs_kernel(
 // page_seq[p] and is its page_idx[p]-th.  Positions beyond what the request holds give zeros.
 template <typename T>
 __global__ void __launch_bounds__(128) latent_gather_kernel(
-    const T* __restrict__ pages, const int* __restrict__ table, int max_pages, int num_pages, const int* __restrict__ page_seq,
+    const T* pages, const int* __restrict__ table, int max_pages, int num_pages, const int* __restrict__ page_seq,
     const int* __restrict__ page_idx, const int* __restrict__ ctx_len, int page_size, int kv_rank, int rot, int heads, int per,
     T* __restrict__ latents, T* __restrict__ keys, int* status) {
   pdl_trigger();
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(128) latent_gather_kernel(
 // expanded: [slots, ld] = per position [heads x dim plain key parts | heads x vdim values]; keys [pages, heads,
 // page_size, dim + rot], values [pages, heads, page_size, vdim].
 template <typename T>
-__global__ void __launch_bounds__(256) latent_scatter_kernel(const T* __restrict__ expanded, long long ld, int page_size,
+__global__ void __launch_bounds__(256) latent_scatter_kernel(const T* expanded, long long ld, int page_size,
                                                              int heads, int dim, int per, int vdim, T* __restrict__ keys,
                                                              T* __restrict__ values) {
   pdl_trigger();
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(256) latent_scatter_kernel(const T* __restrict
 
 // x[t, n, j] *= gate[t, n] (mode 1) or gate[t, n * vdim + j] (mode 2), in place.
 template <typename T>
-__global__ void __launch_bounds__(256) gate_rows_kernel(T* __restrict__ x, long long x_row, const float* __restrict__ gate,
+__global__ void __launch_bounds__(256) gate_rows_kernel(T* x, long long x_row, const float* gate,
                                                         long long gate_row, int mode, int heads, int vdim) {
   pdl_trigger();
   pdl_wait();

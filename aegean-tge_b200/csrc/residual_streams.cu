@@ -65,7 +65,7 @@ constexpr int block_limit(int streams) { return streams == 0 || streams > 4 ? 25
 // Shared memory: [width] the row's u (when it is normed), then the connection's numbers.
 template <int S, typename T, bool VEC>
 __global__ void __launch_bounds__(block_limit(S)) streams_rows_kernel(
-    float* __restrict__ x, int src_rows, int streams_arg, int width, const float* __restrict__ y, long long ld_y,
+    float* x, int src_rows, int streams_arg, int width, const float* y, long long ld_y,
     const float* __restrict__ mix, const float* __restrict__ out, const float* __restrict__ in, const float* __restrict__ gain,
     float eps, const int* __restrict__ rows, T* __restrict__ h, int* status) {
   extern __shared__ __align__(16) float streams_smem[];
@@ -170,8 +170,8 @@ constexpr int SLICE = 256;
 // partial: float32 [splits, tokens, width] (null: nothing is updated).  scaled: bfloat16 [tokens, width] = u * gain; sums:
 // float32 [slices, tokens], each slice's sum of u^2 (both null: only the update).
 template <int S>
-__global__ void __launch_bounds__(SLICE) streams_slices_kernel(float* __restrict__ x, int streams_arg, int width,
-                                                               const float* __restrict__ partial, int splits, int tokens,
+__global__ void __launch_bounds__(SLICE) streams_slices_kernel(float* x, int streams_arg, int width,
+                                                               const float* partial, int splits, int tokens,
                                                                const float* __restrict__ mix, const float* __restrict__ out,
                                                                const float* __restrict__ in, const float* __restrict__ gain,
                                                                __nv_bfloat16* __restrict__ scaled, float* __restrict__ sums) {

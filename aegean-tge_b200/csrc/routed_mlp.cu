@@ -47,7 +47,7 @@ __device__ __forceinline__ void warp_argmax(const float* values, int n, int lane
 // One warp per token.  Loops over the few outputs stay rolled: in a decode step the weights of a layer pass through the L2
 // between two launches, so every line of instructions is fetched from memory again.  Shared memory per warp: 4 arrays of `outputs` floats (scores, choice values, group maxima,
 // kept flags).
-__global__ void __launch_bounds__(128) router_topk_kernel(const float* __restrict__ logits, long long ld,
+__global__ void __launch_bounds__(128) router_topk_kernel(const float* logits, long long ld,
                                                           const float* __restrict__ correction, int tokens, int outputs,
                                                           int top, int group_count, int group_keep, int group_pairs,
                                                           int logistic, int over_sum, float factor, int* __restrict__ ids,
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(128) router_topk_kernel(const float* __restric
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) activation_kernel(T* __restrict__ rows, long long ld, int count, int width, int kind,
+__global__ void __launch_bounds__(256) activation_kernel(T* rows, long long ld, int count, int width, int kind,
                                                          const float* __restrict__ params) {
   pdl_trigger();
   pdl_wait();
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256) activation_kernel(T* __restrict__ rows, l
 }
 
 // The same on eight bfloat16 at a time: rows whose width and stride are multiples of 8 and that start on 16 bytes.
-__global__ void __launch_bounds__(256) activation_vec_kernel(__nv_bfloat16* __restrict__ rows, long long ld, int count, int width,
+__global__ void __launch_bounds__(256) activation_vec_kernel(__nv_bfloat16* rows, long long ld, int count, int width,
                                                              int kind, const float* __restrict__ params) {
   pdl_trigger();
   pdl_wait();
@@ -267,13 +267,13 @@ __global__ void __launch_bounds__(256) activation_vec_kernel(__nv_bfloat16* __re
 // sum_k a[k] * b[k] over a warp: every lane takes the elements lane, lane + 32, ... in ascending order and the lanes'
 // sums meet in a butterfly, so the order depends on nothing but n.
 template <typename T>
-__device__ __forceinline__ float warp_dot(const T* __restrict__ a, const T* __restrict__ b, int n, int lane) {
+__device__ __forceinline__ float warp_dot(const T* a, const T* b, int n, int lane) {
   float acc = 0.0f;
   for (int k = lane; k < n; k += 32) acc = fmaf(to_float<T>(a[k]), to_float<T>(b[k]), acc);
   return warp_sum(acc);
 }
 template <>
-__device__ __forceinline__ float warp_dot<__nv_bfloat16>(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
+__device__ __forceinline__ float warp_dot<__nv_bfloat16>(const __nv_bfloat16* a, const __nv_bfloat16* b,
                                                         int n, int lane) {
   float acc = 0.0f;
   if ((n & 7) == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0) {
@@ -319,8 +319,8 @@ __device__ __forceinline__ float clamped_gate(const ExpertAct& act, float g, flo
 // inner[pair, j] = relu(z_j)^2 or the gate on (z_2j, z_2j+1), z = w_up[expert] h[token] (times the pair's weight, if the
 // weight is the input's), for the pairs whose choice is an expert.
 template <typename T>
-__global__ void __launch_bounds__(256) expert_up_kernel(const T* __restrict__ h, long long ld_h, const T* __restrict__ w_up,
-                                                        const int* __restrict__ ids, const float* __restrict__ in_weights,
+__global__ void __launch_bounds__(256) expert_up_kernel(const T* h, long long ld_h, const T* __restrict__ w_up,
+                                                        const int* ids, const float* in_weights,
                                                         T* __restrict__ inner, int top, int experts, int width, int ff,
                                                         ExpertAct act) {
   pdl_trigger();
@@ -350,10 +350,10 @@ __global__ void __launch_bounds__(256) expert_up_kernel(const T* __restrict__ h,
 // x[token, n] <- gate * x[token, n] + sum over the token's choices, in their order, of weight * (w_down[expert][n, :] .
 // inner[pair, :]), or weight * h[token, n] for an identity expert; null weights and a null gate count as one.
 template <typename T>
-__global__ void __launch_bounds__(256) expert_down_add_kernel(const T* __restrict__ inner, const T* __restrict__ w_down,
-                                                              const T* __restrict__ h, long long ld_h,
-                                                              const int* __restrict__ ids, const float* __restrict__ weights,
-                                                              float* __restrict__ x, int top, int experts, int width, int ff,
+__global__ void __launch_bounds__(256) expert_down_add_kernel(const T* inner, const T* __restrict__ w_down,
+                                                              const T* h, long long ld_h,
+                                                              const int* ids, const float* weights,
+                                                              float* x, int top, int experts, int width, int ff,
                                                               long long down_expert, long long down_row, RowGate gate) {
   pdl_trigger();
   pdl_wait();
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(256) expert_down_add_kernel(const T* __restric
 
 // One block.  place[pair]: the pair's row in the buffer grouped by expert (-1 for an identity expert);
 // offsets[e] .. offsets[e + 1]: expert e's rows.
-__global__ void __launch_bounds__(1024) expert_sort_kernel(const int* __restrict__ ids, int pairs, int experts,
+__global__ void __launch_bounds__(1024) expert_sort_kernel(const int* ids, int pairs, int experts,
                                                            int* __restrict__ place, int* __restrict__ offsets) {
   extern __shared__ int sort_smem[];
   int* count = sort_smem;
@@ -408,8 +408,8 @@ __global__ void __launch_bounds__(1024) expert_sort_kernel(const int* __restrict
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) expert_gather_kernel(const T* __restrict__ h, long long ld_h, const int* __restrict__ place,
-                                                            const float* __restrict__ in_weights, T* __restrict__ grouped,
+__global__ void __launch_bounds__(256) expert_gather_kernel(const T* h, long long ld_h, const int* place,
+                                                            const float* in_weights, T* __restrict__ grouped,
                                                             int top, int width) {
   pdl_trigger();
   pdl_wait();
@@ -439,9 +439,9 @@ __global__ void __launch_bounds__(256) expert_gather_kernel(const T* __restrict_
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) expert_combine_add_kernel(const float* __restrict__ outputs, const int* __restrict__ place,
-                                                                 const float* __restrict__ weights, const T* __restrict__ h,
-                                                                 long long ld_h, float* __restrict__ x, int top, int width,
+__global__ void __launch_bounds__(256) expert_combine_add_kernel(const float* outputs, const int* place,
+                                                                 const float* weights, const T* h,
+                                                                 long long ld_h, float* x, int top, int width,
                                                                  RowGate gate) {
   pdl_trigger();
   pdl_wait();
@@ -464,9 +464,9 @@ __global__ void __launch_bounds__(256) expert_combine_add_kernel(const float* __
 // the down matrices side by side along k adds the weighted sum of the chosen experts.  Blocks with blockIdx.y ==
 // experts add the identity experts' share, weight * h, into the stream.
 template <typename T>
-__global__ void __launch_bounds__(256) expert_dense_weigh_kernel(T* __restrict__ z, const int* __restrict__ ids,
-                                                                 const float* __restrict__ weights, const T* __restrict__ h,
-                                                                 long long ld_h, float* __restrict__ x, int top, int experts,
+__global__ void __launch_bounds__(256) expert_dense_weigh_kernel(T* z, const int* ids,
+                                                                 const float* weights, const T* h,
+                                                                 long long ld_h, float* x, int top, int experts,
                                                                  int width, int ff) {
   pdl_trigger();
   pdl_wait();
@@ -502,8 +502,8 @@ __global__ void __launch_bounds__(256) expert_dense_weigh_kernel(T* __restrict__
 // the activated value.  `shared_ff` > 0: behind the experts' columns lie those of a feed-forward that every token uses
 // (2 shared_ff in z, shared_ff in out), its activated values times the token's gate; blocks with blockIdx.y == experts do it.
 template <typename T>
-__global__ void __launch_bounds__(256) expert_dense_gate_kernel(const T* __restrict__ z, const int* __restrict__ ids,
-                                                                const float* __restrict__ weights, T* __restrict__ out, int top,
+__global__ void __launch_bounds__(256) expert_dense_gate_kernel(const T* z, const int* ids,
+                                                                const float* weights, T* __restrict__ out, int top,
                                                                 int experts, int expert_ff, int weigh_input, ExpertAct act,
                                                                 int shared_ff, RowGate gate) {
   pdl_trigger();

@@ -29,7 +29,7 @@ __device__ __forceinline__ float warp_inclusive_scan(float v, int lane) {
 
 constexpr int MAX_CLUSTER = 8;
 
-__global__ void __launch_bounds__(1024) sample_kernel(const float* __restrict__ logits, long long row_stride,
+__global__ void __launch_bounds__(1024) sample_kernel(const float* logits, long long row_stride,
                                                       const float* __restrict__ temperature,
                                                       const float* __restrict__ uniform, int* __restrict__ out,
                                                       int vocab, int span) {

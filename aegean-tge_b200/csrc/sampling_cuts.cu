@@ -70,7 +70,7 @@ __device__ __forceinline__ int level_of_exponent(int d) { return d <= 0 ? 0 : (d
 // Calls visit(value, index) for every element of data[0, n), each thread of the block taking every 1024th group of
 // four (16-byte loads when the row starts on a 16-byte boundary, which keeps four times as many bytes in flight).
 template <typename Visit>
-__device__ __forceinline__ void for_each_element(const float* __restrict__ data, int n, Visit visit) {
+__device__ __forceinline__ void for_each_element(const float* data, int n, Visit visit) {
   const int tid = threadIdx.x;
   if ((reinterpret_cast<uintptr_t>(data) & 15u) == 0) {
     const int quads = n >> 2;

@@ -73,7 +73,7 @@ __device__ __forceinline__ void store_quad(__nv_bfloat16* dst, float4 v) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(1024) scale_add_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ y,
+__global__ void __launch_bounds__(1024) scale_add_norm_vec_kernel(float* x, const float* y,
                                                                   long long ldy, const float* __restrict__ weight,
                                                                   T* __restrict__ copy, int hidden, float alpha, float eps) {
   __shared__ float scratch[32];
@@ -126,9 +126,9 @@ constexpr int SCAN_WARPS = 4;
 
 template <typename T, int ROWS, int TOKENS>
 __global__ void __launch_bounds__(SCAN_WARPS * 32) decay_scan_kernel(
-    const T* __restrict__ rows, long long ld, int q_off, int k_off, int v_off, int heads, int dim, int vdim,
+    const T* rows, long long ld, int q_off, int k_off, int v_off, int heads, int dim, int vdim,
     int activation, const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions,
-    int rotary, float k_scale, const float* __restrict__ decay, float* __restrict__ state,
+    int rotary, float k_scale, const float* __restrict__ decay, float* state,
     const int* __restrict__ slots, const int* __restrict__ q_start, const int* __restrict__ positions,
     float* __restrict__ out, int* status) {
   pdl_trigger();
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(128) decay_prepare_kernel(
 // rotated numbers even).  Bound by its bytes: a block of 128 threads per (token, head) with two-byte loads took 40 us
 // for 2,048 tokens of 28 heads of 128, this 33.
 __global__ void __launch_bounds__(256) decay_prepare_vec_kernel(
-    const __nv_bfloat16* __restrict__ rows, long long ld, int q_off, int k_off, int heads, int dim, int activation,
+    const __nv_bfloat16* rows, long long ld, int q_off, int k_off, int heads, int dim, int activation,
     const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary,
     float k_scale, const int* __restrict__ positions, float* __restrict__ prepared, int* status) {
   pdl_trigger();
@@ -787,7 +787,7 @@ __global__ void __launch_bounds__(256) decay_scan_wide_kernel(
 // on the way in and the state it starts from on the way out; the request's slot gets the state after its last one.
 // Portions below `shortest` tokens have no segments; blockIdx.z counts the others (with a grid over all requests, blocks that only
 // left took 85 us of a step of 64 single tokens beside a prompt).  They are counted 32 requests at a time, one to a lane.
-__global__ void decay_segment_carry_kernel(float* __restrict__ carry, float* __restrict__ state, const float* __restrict__ decay,
+__global__ void decay_segment_carry_kernel(float* carry, float* state, const float* __restrict__ decay,
                                            const int* __restrict__ slots, const int* __restrict__ q_start, int num_seqs, int heads,
                                            int dim, int vdim, int segment, int shortest) {
   const int head = blockIdx.y;
@@ -850,7 +850,7 @@ __global__ void decay_segment_carry_kernel(float* __restrict__ carry, float* __r
 // (token, group).  weight may be null (no weight); act 0: silu, 1: sigmoid; act 2: the SiLU gate comes BEFORE the norm,
 // out = y / rms_g(y) * weight with y = o * silu(gate).
 template <typename T, typename TO = T>
-__global__ void __launch_bounds__(128) gated_norm_kernel(const float* __restrict__ o, const T* __restrict__ gate,
+__global__ void __launch_bounds__(128) gated_norm_kernel(const float* o, const T* gate,
                                                          long long ld_gate, const float* __restrict__ weight,
                                                          TO* __restrict__ out, long long ld_out, int tokens, int groups,
                                                          int size, float eps, int act) {
@@ -892,7 +892,7 @@ __global__ void __launch_bounds__(128) gated_norm_kernel(const float* __restrict
 // one group of 1,792 (a warp per token before) 33 us and 12.
 constexpr int GATED_QUADS = 4;            // per thread at most
 template <int UNIT>
-__global__ void __launch_bounds__(256) gated_norm_vec_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ gate, long long ld_gate,
+__global__ void __launch_bounds__(256) gated_norm_vec_kernel(const float* o, const __nv_bfloat16* gate, long long ld_gate,
                                                              const float* __restrict__ weight, __nv_bfloat16* __restrict__ out, long long ld_out,
                                                              int tokens, int groups, int size, float eps, int act) {
   __shared__ float scratch[32];
@@ -991,8 +991,8 @@ constexpr int MAX_TAPS = 16;
 
 template <typename T>
 __global__ void __launch_bounds__(128) conv_norm_rope_store_kernel(
-    const T* __restrict__ raw, long long ld, const float* __restrict__ conv_w, int taps,
-    const float* __restrict__ conv_state, const int* __restrict__ slots, const int* __restrict__ q_start,
+    const T* raw, long long ld, const float* __restrict__ conv_w, int taps,
+    const float* conv_state, const int* __restrict__ slots, const int* __restrict__ q_start,
     const float* __restrict__ q_norm, const float* __restrict__ k_norm, float eps,
     const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary,
     const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table,
@@ -1106,7 +1106,7 @@ __global__ void __launch_bounds__(128) conv_norm_rope_store_kernel(
 // The convolution state after the step: the last taps-1 projected rows of each request, oldest first.  One thread
 // per (request, channel) reads what it needs before it writes, so a portion shorter than the state shifts it.
 template <typename T>
-__global__ void conv_state_update_kernel(const T* __restrict__ raw, long long ld, float* __restrict__ conv_state,
+__global__ void conv_state_update_kernel(const T* raw, long long ld, float* conv_state,
                                          const int* __restrict__ slots, const int* __restrict__ q_start, int taps,
                                          int channels) {
   pdl_trigger();
@@ -1422,7 +1422,7 @@ constexpr int NRV_THREADS = 512;    // at most
 // numbers as well): `lanes` lanes (a power of two, one per 16 bytes of a head) share a head; the number a rotated one is
 // paired with comes from the lane half / 8 away.
 __global__ void __launch_bounds__(NRV_THREADS) norm_rope_store_vec_kernel(
-    const __nv_bfloat16* __restrict__ raw, long long ld, const float* __restrict__ q_norm, const float* __restrict__ k_norm,
+    const __nv_bfloat16* raw, long long ld, const float* __restrict__ q_norm, const float* __restrict__ k_norm,
     float eps, const float* __restrict__ cos_table, const float* __restrict__ sin_table, int table_positions, int rotary,
     const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int max_pages,
     __nv_bfloat16* __restrict__ k_pages, __nv_bfloat16* __restrict__ v_pages, int num_pages, int page_size,

@@ -54,8 +54,8 @@ __global__ void __launch_bounds__(256) group_norm_kernel(const float* x, const f
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) token_shift_kernel(const T* __restrict__ h, const float* __restrict__ mu,
-                                                          const float* __restrict__ state, const int* __restrict__ slots,
+__global__ void __launch_bounds__(256) token_shift_kernel(const T* h, const float* __restrict__ mu,
+                                                          const float* state, const int* __restrict__ slots,
                                                           int num_slots, const int* __restrict__ seq_of_token,
                                                           const int* __restrict__ q_start, const int* __restrict__ start_pos,
                                                           T* __restrict__ out, int tokens, int width, int* status) {
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(256) token_shift_kernel(const T* __restrict__ 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) shift_state_update_kernel(const T* __restrict__ h, float* __restrict__ state,
+__global__ void __launch_bounds__(256) shift_state_update_kernel(const T* h, float* state,
                                                                  const int* __restrict__ slots, int num_slots,
                                                                  const int* __restrict__ q_start, int width, int* status) {
   pdl_trigger();
