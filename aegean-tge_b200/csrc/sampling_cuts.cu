@@ -139,11 +139,15 @@ __device__ __forceinline__ void block_sums(float (&mass)[N], int (&count)[N], fl
 }
 
 __global__ void __launch_bounds__(THREADS, 1) sample_cuts_kernel(
-    const float* __restrict__ scores, long long row_stride, const float* __restrict__ temperature,
+    const float* scores, long long row_stride, const float* __restrict__ temperature,
     const int* __restrict__ top_k, const float* __restrict__ top_p, const float* __restrict__ min_p,
-    const float* __restrict__ uniform, float* __restrict__ sort_prob, int* __restrict__ sort_index, int padded,
-    int* __restrict__ out, int vocab, int skip_uncut, int span) {
+    const float* __restrict__ uniform, float* sort_prob, int* sort_index, int padded,
+    int* out, int vocab, int skip_uncut, int span) {
   namespace cg = cooperative_groups;
+  // The scores are the kernel in front's, and so is the id that an uncut row keeps: whoever follows finds it there, so every block
+  // waits, also one that has nothing else to do.
+  pdl_trigger();
+  pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   const int blocks = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int row = blockIdx.x / blocks;

@@ -16,7 +16,7 @@ SOURCES = sorted(CSRC.glob("*.cu")) + sorted(CSRC.glob("*.cuh"))
 CONSTANTS = set("""weight weight2 q_weight k_weight kv_weight norm_weight q_norm k_norm bias cos_table sin_table conv_w conv_b a_log dt_bias
                    skip decay sink blend correction params mu mix in gain w w_up w_down""".split())
 # what the host gave the step
-STEP = set("positions seq_of_token q_start start_pos slots block_table pool_table rows page_seq page_idx ctx_len temperature uniform".split())
+STEP = set("positions seq_of_token q_start start_pos slots block_table pool_table rows page_seq page_idx ctx_len temperature uniform top_k top_p min_p".split())
 # written, and not read before that
 RESULTS = set("""out copy k_pages v_pages pages keys values latents q_latent q_out qkv act_out norm_out scaled scaled_out ss_out sums planes
                  dst gate gates qk v h inner grouped ids weights place offsets prepared""".split())
@@ -66,3 +66,25 @@ def test_the_sources_are_read_as_they_are_meant_to_be():
     assert {"gemm_tcgen05_kernel", "gemm_tcgen05_pair_kernel", "splitk_epilogue_quad_kernel", "splitk_add_norm_kernel",
             "splitk_qkv_rope_store_kernel", "splitk_add_scale_kernel"} <= names
     assert sum(len(kernels(path)) for path in SOURCES) > 90
+
+
+def test_every_kernel_that_may_start_early_waits():
+    """``tge_launch`` lets a kernel start while the one in front still runs: it has to wait in its own body or in a function that it calls."""
+    defined, launched = {}, {}
+    for path in SOURCES:
+        for _kind, name, _head, body in functions(path):
+            defined[name] = body
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for name in re.findall(r"tge_launch(?:_clusters)?\(\s*(?:\w+::)*(\w+)", text):
+            launched.setdefault(name, path.name)
+        # kernels that a launch gets through a variable or a lambda's argument
+        for name in re.findall(r"(?:auto kernel =|run\(|launch\(|\?|:)\s*(\w+_kernel)\b", text):
+            launched.setdefault(name, path.name)
+
+    def waits(name):
+        body = defined[name]
+        return "pdl_wait(" in body or any(re.search(rf"\b{helper}(<[^;]*?>)?\(", body) and "pdl_wait(" in text for helper, text in defined.items())
+
+    names = [name for name in launched if name in defined and name != "attention_simt_kernel"]      # that one is launched with <<< >>>
+    assert len(names) > 70
+    assert [name for name in names if not waits(name)] == []

@@ -186,3 +186,29 @@ def test_the_event_of_a_draw_on_its_way_can_be_asked_and_waited_for(ops):
         assert event.query() and host.tolist() == best and ops.launches == before
         side.synchronize()
         assert seen.tolist() == best
+
+
+def test_cuts_wait_for_the_scores_and_for_the_ids_of_uncut_rows(ops):
+    """The head's product, the draw and the cuts one behind the other with nothing in between: the cuts see that product's scores, and a row
+    without cuts keeps the id that the draw in front has just written."""
+    gen = torch.Generator().manual_seed(4)
+    rows, vocab = 6, 40000
+    hidden = [torch.randn(rows, 512, generator=gen).to(torch.bfloat16).to(DEV) for _ in range(2)]
+    head = (torch.randn(vocab, 512, generator=gen) * 0.05).to(torch.bfloat16).to(DEV)
+    mk = lambda values, dtype: torch.tensor(values, dtype=dtype, device=DEV)
+    temps, uniform = mk([1.0] * rows, torch.float32), mk([0.1, 0.3, 0.5, 0.7, 0.9, 0.2], torch.float32)
+    cuts = mk([40, 0, 5, 0, 0, 300], torch.int32), mk([0.9, 1.0, 1.0, 1.0, 0.5, 1.0], torch.float32), mk([0.0] * rows, torch.float32)
+    logits = torch.zeros(rows, vocab, device=DEV)
+    wanted = []
+    for h in hidden:
+        ops.linear(h, head, None, ops.GEMM_STORE_F32, out=logits)
+        torch.cuda.synchronize()
+        ids = ops.sample(logits, temps, uniform)
+        torch.cuda.synchronize()
+        wanted.append(ops.sample_cuts(logits, temps, *cuts, uniform, out=ids).tolist())
+    got = []
+    for turn in range(20):
+        ops.linear(hidden[turn % 2], head, None, ops.GEMM_STORE_F32, out=logits)
+        ids = ops.sample(logits, temps, uniform)
+        got.append(ops.sample_cuts(logits, temps, *cuts, uniform, out=ids))
+    assert [ids.tolist() for ids in got] == wanted * 10
