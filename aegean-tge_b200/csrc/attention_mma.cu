@@ -22,6 +22,7 @@
 
 #include <stdlib.h>
 
+#include <atomic>
 #include <map>
 #include <tuple>
 
@@ -79,11 +80,34 @@ struct AttnParams {
   int gate_stride;
   int gate_elements;         // the logits are [tokens, heads * DV] instead: one gate per number of a head's output
   // The single tokens at the head of a step and the longer portions behind them share nothing, so their two kernels may run side by
-  // side: the first one lets its dependents start only behind its own wait (trigger_late), the second one then needs
-  // nothing of the kernel in front and waits for it at its very end alone (beside), so that whoever follows finds both done.
+  // side: the first one lets its dependents start only behind its own wait (trigger_late) and leaves `ticket` for them there, the
+  // second one (beside) takes the ticket in place of a wait, and waits for the first one at its very end, so that whoever
+  // follows finds both done.
   int trigger_late, beside;
+  unsigned long long ticket;
   float scale_log2;
 };
+
+// Tickets of side-by-side launches: a number of its own for every such pair of launches, in the place that it falls on.  The first
+// kernel writes it behind its wait, where it sees all that came before; the second one acquires it and so sees that as well (a wait
+// of its own would wait for the whole first kernel).  Nobody waits for a ticket: a block that does not find its number, because it is not
+// there yet or a later pair has overwritten it, waits for the first kernel instead.
+constexpr int TICKETS = 1024;
+__device__ unsigned long long g_tickets[TICKETS];
+
+__device__ __forceinline__ void leave_ticket(unsigned long long ticket) {
+  __threadfence();
+  asm volatile("st.release.gpu.global.u64 [%0], %1;\n" ::"l"(&g_tickets[ticket % TICKETS]), "l"(ticket) : "memory");
+}
+
+// In every thread that reads what the kernels in front wrote, by loads or by copies.
+__device__ __forceinline__ void wait_or_take_ticket(const AttnParams& p) {
+  unsigned long long found = 0;
+  if (p.beside) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];\n" : "=l"(found) : "l"(&g_tickets[p.ticket % TICKETS]) : "memory");
+  if (p.beside && found == p.ticket) asm volatile("fence.proxy.async;\n" ::: "memory");      // for copies by TMA as for loads
+  else pdl_wait();
+  __syncwarp();
+}
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -797,7 +821,11 @@ __global__ void __launch_bounds__((4 * GROUPS + 1) * 32) attention_decode_tma_ke
     }
   }
   pdl_wait();
-  if (p.trigger_late) pdl_trigger();
+  if (p.trigger_late && warp == 0) {                     // the first call in a block counts
+    if (lane == 0 && seq == 0 && kvh == 0 && split == 0) leave_ticket(p.ticket);
+    __syncwarp();
+    pdl_trigger();
+  }
 
   uint32_t qf[HD / 16][4];
 #pragma unroll
@@ -1413,7 +1441,8 @@ TGE_API long long tge_attention_mma_scratch_floats(int tokens, int heads, int nu
 
 // What a call for the single tokens at a step's head leaves for its caller to do.
 struct LeadingTokens {
-  bool late = false;         // the decode kernel ran and triggers behind its wait
+  unsigned long long ticket = 0;     // what the decode kernel is to leave
+  bool late = false;         // the decode kernel ran, triggers behind its wait and leaves the ticket there
   bool unmerged = false;     // the key runs' states wait for launch_merge(p, ...)
   AttnParams p;
 };
@@ -1424,8 +1453,8 @@ struct LeadingTokens {
 // split_tokens: 0 = one split; else a multiple of 64 (keys per split).  scratch: see above.
 // `first_token`: the sequences given here start at this token of the step (earlier tokens belong to sequences
 // that another launch serves); q, out, positions and the scratch layout stay those of the whole step.
-// `lead`: the call is for such earlier tokens (not null: their kernel triggers late where it can); `beside`: the call follows one whose
-// kernel did.
+// `lead`: the call is for such earlier tokens (not null: their kernel triggers late where it can); `beside` (0: none): the call follows one
+// whose kernel did, and this is the ticket that it leaves.
 static int attention_dispatch(const void* q, int q_stride, const void* k_pages, const void* v_pages,
                               const int* block_table, int max_pages, int num_pages, int page_size,
                               const int* q_start, const int* start_pos, const int* positions, int num_seqs,
@@ -1433,7 +1462,7 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
                               int kv_heads, float scale, int window, int split_tokens, float* scratch, int* status,
                               int first_token, const float* sink, int leave_states, int v_pitch, const float* dist_bias,
                               int dist_span, int keep_first, const void* gate, int gate_stride, int gate_elements,
-                              int shared_keys, cudaStream_t stream, LeadingTokens* lead = nullptr, bool beside = false) {
+                              int shared_keys, cudaStream_t stream, LeadingTokens* lead = nullptr, unsigned long long beside = 0) {
   TGE_REQUIRE(tokens >= 0 && num_seqs >= 0, "attention_mma: negative sizes");
   TGE_REQUIRE(dist_bias == nullptr || (dist_span > 0 && scale != 0.0f), "attention_mma: a bias by distance needs its span");
   TGE_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0,
@@ -1470,7 +1499,8 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
   TGE_REQUIRE(!shared_keys || (single && p.v_in_keys), "attention_mma: runs of heads over the same keys are for single tokens and values inside the keys");
   p.kv_pool = shared_keys ? 1 : kv_heads;
   p.trigger_late = 0;
-  p.beside = beside ? 1 : 0;
+  p.beside = beside != 0;
+  p.ticket = beside;
   p.q_stride = q_stride; p.out_stride = out_stride;
   p.max_pages = max_pages; p.num_pages = num_pages; p.page_size = page_size;
   p.page_shift = 0;
@@ -1524,7 +1554,10 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
     }
     p.bq = 1;
     p.early_tiles = p.early_tiles ? stages : 0;
-    p.trigger_late = lead != nullptr ? 1 : 0;
+    if (lead != nullptr) {
+      p.trigger_late = 1;
+      p.ticket = lead->ticket;
+    }
     dim3 grid(num_seqs, kv_heads, num_splits);
     if (two_groups) tge_launch(attention_decode_tma_kernel<2>, grid, 9 * 32, smem, stream, *map_k, *map_v, p);
     else tge_launch(attention_decode_tma_kernel<1>, grid, DEC_TMA_THREADS, smem, stream, *map_k, *map_v, p);
@@ -1720,7 +1753,18 @@ TGE_API int tge_attention_mma(const void* q, int q_stride, const void* k_pages, 
   const int rest_ctx = rest_ctx_len > 0 && rest_ctx_len < max_ctx_len ? rest_ctx_len : max_ctx_len;
   const bool rest_cut = split_tokens > 0 && rest_ctx > split_tokens, lead_cut = prefix_split_tokens > 0 && max_ctx_len > prefix_split_tokens;
   LeadingTokens lead;
-  LeadingTokens* const ask = gate == nullptr && !leave_states && !(rest_cut && lead_cut) ? &lead : nullptr;
+  LeadingTokens* ask = nullptr;
+  if (gate == nullptr && !leave_states && !(rest_cut && lead_cut)) {
+    // not in a captured graph, whose replays would all find the ticket of the first one
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+      static std::atomic<unsigned long long> tickets{0};
+      lead.ticket = ++tickets;
+      ask = &lead;
+    } else {
+      cudaGetLastError();
+    }
+  }
   const int first = attention_dispatch(q, q_stride, k_pages, v_pages, block_table, max_pages, num_pages, page_size, q_start,
                                        start_pos, positions, decode_prefix, decode_prefix, 1, max_ctx_len, out, out_stride,
                                        heads, kv_heads, scale, window, prefix_split_tokens, scratch, status, 0, sink, leave_states, v_pitch, dist_bias,
@@ -1730,7 +1774,7 @@ TGE_API int tge_attention_mma(const void* q, int q_stride, const void* k_pages, 
                                 num_pages, page_size, q_start + decode_prefix, start_pos + decode_prefix, positions,
                                 num_seqs - decode_prefix, tokens, max_q_len, rest_ctx, out, out_stride, heads,
                                 kv_heads, scale, window, split_tokens, scratch, status, decode_prefix, sink, leave_states, v_pitch, dist_bias,
-                                dist_span, keep_first, gate, gate_stride, gate_elements, shared_keys, stream, nullptr, lead.late);
+                                dist_span, keep_first, gate, gate_stride, gate_elements, shared_keys, stream, nullptr, lead.late ? lead.ticket : 0);
   if (rest < 0) return rest;
   if (lead.unmerged) {
     launch_merge(lead.p, positions, 0, stream);

@@ -141,9 +141,8 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc2_kernel(
   pdl_trigger();                                                      // tensor memory is held: the next kernel may be scheduled
   // Everything above read what the step was given (lengths, positions, the block table) and set up this block's own
   // memory, while the kernel before this one was still running; the queries and the newest keys are its work (or
-  // that of the kernel before it: p.beside).
-  if (!p.beside) pdl_wait();
-  else __threadfence();                                               // what that one wrote, and not what an L1 still holds
+  // that of the kernel before it, whose ticket says so: p.beside).
+  wait_or_take_ticket(p);
   auto s_tmem = [&](int tile, int buffer) { return tmem_base + (uint32_t)((tile * 2 + buffer) * BKV); };
   auto o_tmem = [&](int tile) { return tmem_base + (uint32_t)(2 * QTILES * BKV + tile * HD); };
 
