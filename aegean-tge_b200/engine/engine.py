@@ -160,7 +160,7 @@ class Engine:
                 self.ahead_dropped += 1
         sampling_items = [item for item in plan.items if item.samples]
         if pending is None:
-            logits = self.runner.step_plan(plan)
+            logits = self.runner.step_plan(plan, lend=True)          # all use of them is queued below
             if sampling_items:
                 params = [item.request.sampling for item in sampling_items]
                 if self.run_ahead and Sampler.stays_on_device(params):
@@ -209,7 +209,7 @@ class Engine:
         snapshot = (self.cache.snapshot_state([self.cache.slot_of(name) for name in names])
                     if self.cache.state_storage else None)
         try:
-            logits = self.runner.step_ahead(names, ids)
+            logits = self.runner.step_ahead(names, ids, lend=True)
         except PoolExhausted:
             return None
         result = self.sampler.sample_async(logits, [r.sampling for r in requests], [r.rng for r in requests])

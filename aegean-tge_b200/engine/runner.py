@@ -143,11 +143,11 @@ class ModelRunner:
         _rt.check(lib.tge_rt_cache_advance(cache.native, arrays.handles, arrays.token_counts, arrays.count))
         return logits
 
-    def step_plan(self, plan) -> Optional[torch.Tensor]:
+    def step_plan(self, plan, lend: bool = False) -> Optional[torch.Tensor]:
         """Runs a scheduler's plan: the same step, packed from the scheduler's own copies of the tokens.
 
-        Pages were reserved when the plan was made, and the scheduler records progress in ``update``.  The logits are
-        valid for what is queued on them before the next step.
+        Pages were reserved when the plan was made, and the scheduler records progress in ``update``.  ``lend``: the logits may be
+        a buffer that the next step overwrites, for a caller that queues all use of them before it.
         """
         items = plan.items
         if not items:
@@ -158,17 +158,17 @@ class ModelRunner:
         tokens = sum(item.count for item in items)
         wanted = [i for i, item in enumerate(items) if item.samples]
         return self._run(lambda width, pad_rows, out, layout: plan.pack(vocab, width, pad_rows, out, layout),
-                         len(items), tokens, single, max_ctx, wanted, None, lend=True)
+                         len(items), tokens, single, max_ctx, wanted, None, lend=lend)
 
     def can_step_ahead(self, batch: int) -> bool:
         return self.use_graphs and batch <= self.max_graph_batch
 
-    def step_ahead(self, requests: Sequence[Hashable], token_ids: torch.Tensor) -> torch.Tensor:
+    def step_ahead(self, requests: Sequence[Hashable], token_ids: torch.Tensor, lend: bool = False) -> torch.Tensor:
         """One more token for each of ``requests`` (each already advanced past its previous step), the
         token ids taken from ``token_ids`` on the device: the step can be queued before the host has seen them.
 
         Pages are reserved all or nothing (PoolExhausted if they do not fit); progress is not recorded.
-        Returns the logits of every row, valid for what is queued on them before the next step.
+        Returns the logits of every row (``lend``: as in :meth:`step_plan`).
         """
         cache, lib = self.cache, self._lib
         count = len(requests)
@@ -182,7 +182,7 @@ class ModelRunner:
                                                   ctypes.byref(layout)))
 
         max_ctx = lib.tge_rt_cache_max_context(cache.native, handles, ones, count)
-        return self._run(pack, count, count, True, max_ctx, list(range(count)), None, device_tokens=token_ids, lend=True)
+        return self._run(pack, count, count, True, max_ctx, list(range(count)), None, device_tokens=token_ids, lend=lend)
 
     def _placeholders(self, count: int) -> tuple:
         """One token of id 0 and one wanted place 0 for each of ``count`` portions, as the packer reads them (never written)."""

@@ -419,6 +419,32 @@ def test_steps_queued_ahead_change_nothing(model_dirs, tmp_path):
     assert ahead == plain and reasons_ahead == reasons and counts["dropped"] >= 1 and counts["used"] > 5
 
 
+def test_logits_of_a_step_outlive_the_next_one(model_dirs):
+    """Steps that replay a graph hand out logits of their own unless the caller asks for the graph's: two steps of a plan and two queued ahead
+    of them, all kept, and the graph's buffer where it is asked for."""
+    engine = _engine(model_dirs, "A", "bfloat16", run_ahead=False)
+    for n in (9, 14):
+        engine.add_request(_tokens("A", n, salt=n), 20)
+    engine.step()
+    runner, scheduler = engine.runner, engine.scheduler
+    kept, copies, requests = [], [], None
+    for _ in range(2):
+        plan = scheduler.schedule()
+        requests = [item.request for item in plan.items]
+        kept.append(runner.step_plan(plan))
+        copies.append(kept[-1].clone())
+        scheduler.update(plan, copies[-1].argmax(-1).tolist())
+    for _ in range(2):
+        ids = copies[-1].argmax(-1).int()
+        kept.append(runner.step_ahead([r.id for r in requests], ids))
+        copies.append(kept[-1].clone())
+        for request in requests:
+            engine.cache.set_computed(request.id, engine.cache.computed(request.id) + 1)
+    assert all(torch.equal(a, b) for a, b in zip(kept, copies)) and not torch.equal(copies[0], copies[1])
+    lent = runner.step_ahead([r.id for r in requests], ids, lend=True)
+    assert lent.data_ptr() in [graph.logits.data_ptr() for graph in runner._graphs.values()]
+
+
 def test_decode_graphs_are_capped_and_share_a_pool(model_dirs, oracle):
     """Decode steps at several batch sizes capture a graph for each size class (1, 2, 4, ...); only the most
     recently used ones are kept, they allocate from one pool, and a graph that was dropped is simply captured
