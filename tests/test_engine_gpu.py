@@ -445,6 +445,17 @@ def test_logits_of_a_step_outlive_the_next_one(model_dirs):
     assert lent.data_ptr() in [graph.logits.data_ptr() for graph in runner._graphs.values()]
 
 
+def test_token_ids_of_any_integer_type_and_place_go_into_a_step_queued_ahead(model_dirs):
+    engine = _engine(model_dirs, "A", "bfloat16", run_ahead=False)
+    names = [engine.add_request(_tokens("A", n, salt=n), 20) for n in (9, 14)]
+    engine.step()
+    engine.step()
+    ids = torch.tensor([7, 11], dtype=torch.int32, device="cuda")
+    wanted = engine.runner.step_ahead(names, ids)
+    for other in (ids.long(), ids.cpu(), torch.stack([ids, ids + 1], 1)[:, 0]):
+        assert torch.equal(engine.runner.step_ahead(names, other), wanted)
+
+
 def test_decode_graphs_are_capped_and_share_a_pool(model_dirs, oracle):
     """Decode steps at several batch sizes capture a graph for each size class (1, 2, 4, ...); only the most
     recently used ones are kept, they allocate from one pool, and a graph that was dropped is simply captured
