@@ -336,5 +336,5 @@ class DecodeGraph:
         # token ids that are still on the device overwrite the packed placeholders
         if device_tokens is not None and not (device_tokens.device == self.dev.device and device_tokens.dtype == torch.int32 and device_tokens.is_contiguous()):
             device_tokens = device_tokens.to(self.dev.device, torch.int32).contiguous()
-        _ops.replay_step(self.exec, self.dev, staging.hosts[turn], total, staging.copied[turn], device_tokens, self.layout.token_ids)
+        _ops.replay_step(self.exec, self.dev, staging.hosts[turn], total, staging.copied[turn], device_tokens, self.layout.token_ids, self.batch)
         return self.logits

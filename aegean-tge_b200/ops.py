@@ -316,20 +316,21 @@ def copy_bytes(dst: torch.Tensor, src: torch.Tensor, count: int) -> None:
 
 
 def replay_step(graph: int, dev: torch.Tensor, host: torch.Tensor, ints: int, copied: StepEvent, tokens: Optional[torch.Tensor],
-                tokens_at: int) -> None:
+                tokens_at: int, token_rows: int) -> None:
     """Queues a captured step on the current stream: the first ``ints`` of ``host`` (pinned int32) to ``dev``, then ``copied``;
-    ``tokens`` (int32 on the device, None: none) over ``dev`` from ``tokens_at`` on; the launch of ``graph`` (an executable graph's handle).
-    The caller keeps all of them alive, ``host`` unchanged until ``copied``."""
+    ``tokens`` (int32 on the device, at most ``token_rows``; None: none) over ``dev`` from ``tokens_at`` on; the launch of ``graph`` (an
+    executable graph's handle).  The caller keeps all of them alive, ``host`` unchanged until ``copied``."""
     count = 0
     if tokens is not None:
         _want(tokens, "token ids", torch.int32)
         count = tokens.numel()
-    if ints > dev.numel() or ints > host.numel() or tokens_at + count > dev.numel():
-        raise KernelError(f"replay: {ints} index entries and {count} tokens from {tokens_at} on in buffers of {host.numel()} and {dev.numel()}")
+    if ints > dev.numel() or ints > host.numel() or count > token_rows or tokens_at + token_rows > dev.numel():
+        raise KernelError(f"replay: {ints} index entries and {count} tokens for {token_rows} places from {tokens_at} on in buffers of "
+                          f"{host.numel()} and {dev.numel()}")
     at, lib = dev.data_ptr(), core()
+    copied._recorded = True          # whatever fails behind the copy: it may be queued, and who takes the buffer next has to wait for it
     _check(lib.tge_replay_step(at, host.data_ptr(), 4 * ints, copied._handle, at + 4 * tokens_at, None if tokens is None else tokens.data_ptr(),
                                4 * count, graph, _stream()), lib)
-    copied._recorded = True
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
