@@ -47,3 +47,12 @@ def test_more_token_ids_than_the_captured_step_has_places_for_are_refused(librar
         with pytest.raises(ops.KernelError):
             _replay(_Tokens(count=count))
         assert not library.calls
+
+
+def test_a_replay_that_fails_half_way_leaves_its_buffer_in_use(library):
+    """The copy out of the pinned buffer may be queued when a later part of the call fails: whoever takes the buffer next waits."""
+    library.rc = -2
+    event = SimpleNamespace(_handle=None, _recorded=False)
+    with pytest.raises(ops.KernelError):
+        _replay(None, event)
+    assert event._recorded
