@@ -766,6 +766,74 @@ def test_side_by_side_attention_is_done_before_what_follows(ops):
     ops.check_status()
 
 
+@pytest.mark.parametrize("lead,portions,starts,lead_is_cut,rest_is_cut", [
+    (list(range(100, 4001, 100)), [90], [0], True, False),          # singles cut, their states merged behind both kernels
+    (list(range(60, 640, 20)), [64], [4000], False, True),          # the portion's keys cut beside them
+    (list(range(300, 940, 80)), [1187], [0], False, False)])      # a prompt for blocks of two query tiles, its rows from a kernel of another kind
+@pytest.mark.parametrize("captured", [False, True])
+def test_side_by_side_attention_sees_what_the_kernels_in_front_have_just_written(ops, lead, portions, starts, lead_is_cut, rest_is_cut, captured):
+    """Queries, keys and values come out of the product and store right in front, other ones in every turn.  Expected: the single tokens and the
+    portions in calls of their own, everything waited for.  In a captured graph, whose replays repeat one launch, the kernels wait."""
+    from aegean_tge_b200.parts.rope import rotary_tables
+    heads, kv_heads, head_dim, hidden, page_size = 28, 4, 128, 256, 64
+    q_lens, begins, n = [1] * len(lead) + portions, lead + starts, len(lead)
+    lengths = [a + m for a, m in zip(begins, q_lens)]
+    known = dict(lead_keys=sum(lengths[:n]), lead_longest=max(lengths[:n]), rest_ctx_len=max(lengths[n:]))
+    lead_cut = ops.choose_leading_split(known["lead_keys"], known["lead_longest"], kv_heads)
+    rest_cut = ops.choose_attention_split(sum(portions), len(portions), max(portions), known["rest_ctx_len"], heads, kv_heads, bound=known["rest_ctx_len"])
+    assert (lead_cut > 0) == lead_is_cut and (rest_cut > 0) == rest_is_cut
+    k_pages, v_pages, table, _k, _v = paged_cache(lengths, kv_heads, head_dim, page_size, torch.bfloat16, DEV, seed=5)
+    positions, seq_of_token, q_start, start_pos = batch_index(q_lens, begins, DEV)
+    cos, sin = (t.to(DEV) for t in rotary_tables(10000.0, head_dim, 4096))
+    gen = torch.Generator().manual_seed(6)
+    tokens, turns = sum(q_lens), 6
+    x = [torch.randn(tokens, hidden, generator=gen).to(torch.bfloat16).to(DEV) for _ in range(turns)]
+    w = (torch.randn((heads + 2 * kv_heads) * head_dim, hidden, generator=gen) * 0.1).to(torch.bfloat16).to(DEV)
+    w_o = (torch.randn(256, heads * head_dim, generator=gen) * 0.02).to(torch.bfloat16).to(DEV)
+    attended, results = torch.zeros(tokens, heads * head_dim, dtype=torch.bfloat16, device=DEV), torch.zeros(turns, tokens, 256, device=DEV)
+
+    def store(i):
+        return ops.linear_qkv_rope_store(x[i], w, None, cos, sin, head_dim, positions, seq_of_token, table, k_pages, v_pages, heads, kv_heads, head_dim)
+
+    def turn(i):
+        qkv = store(i)
+        ops.attention(qkv[:, :heads * head_dim], k_pages, v_pages, table, q_start, start_pos, positions, seq_of_token, len(q_lens), max(q_lens),
+                      max(lengths), heads, kv_heads, head_dim, head_dim ** -0.5, decode_prefix=n, out=attended, **known)
+        ops.linear(attended, w_o, None, ops.GEMM_STORE_F32, out=results[i])
+
+    # positions and q_start of a call count from the call's first token
+    wanted = []
+    rest = batch_index(portions, starts, DEV)
+    for i in range(turns):
+        qkv = store(i)
+        torch.cuda.synchronize()
+        rows = torch.zeros_like(attended)
+        ops.attention(qkv[:n, :heads * head_dim], k_pages, v_pages, table[:n].contiguous(), q_start[:n + 1], start_pos[:n], positions[:n],
+                      seq_of_token[:n], n, 1, known["lead_longest"], heads, kv_heads, head_dim, head_dim ** -0.5, out=rows[:n])
+        torch.cuda.synchronize()
+        ops.attention(qkv[n:, :heads * head_dim], k_pages, v_pages, table[n:].contiguous(), rest[2], rest[3], rest[0], rest[1], len(portions),
+                      max(portions), known["rest_ctx_len"], heads, kv_heads, head_dim, head_dim ** -0.5, out=rows[n:])
+        torch.cuda.synchronize()
+        wanted.append(ops.linear(rows, w_o, None, ops.GEMM_STORE_F32))
+        torch.cuda.synchronize()
+    if captured:
+        turn(0)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for i in range(turns):
+                turn(i)
+        run = graph.replay
+    else:
+        run = lambda: [turn(i) for i in range(turns)]
+    for _ in range(4):
+        results.zero_()
+        run()
+        for i in range(turns):
+            assert rel_error(results[i], wanted[i]) < TOL[torch.bfloat16], i
+    ops.check_status()
+
+
 def test_leading_single_tokens_that_fill_the_chip_are_not_cut(ops, monkeypatch):
     """A mixed step whose single tokens occupy the SMs as they are: cut, they would cost more states to write and to merge than
     the parallel runs give back, and with kept first tokens scratch memory for runs of the whole context.  They have the
@@ -844,74 +912,6 @@ def test_attention_mma_split_keys(ops, split, q_lens, starts):
 
 @pytest.mark.parametrize("heads,kv_heads,head_dim", [(28, 4, 128), (10, 2, 64), (16, 1, 128)])
 @pytest.mark.parametrize("split,window", [(128, 0), (512, 0), (256, 300), (64, 0), (192, 77)])
-@pytest.mark.parametrize("lead,portions,starts,lead_is_cut,rest_is_cut", [
-    (list(range(100, 4001, 100)), [90], [0], True, False),          # singles cut, their states merged behind both kernels
-    (list(range(60, 640, 20)), [64], [4000], False, True),          # the portion's keys cut beside them
-    (list(range(300, 940, 80)), [1187], [0], False, False)])      # a prompt for blocks of two query tiles, its rows from a kernel of another kind
-@pytest.mark.parametrize("captured", [False, True])
-def test_side_by_side_attention_sees_what_the_kernels_in_front_have_just_written(ops, lead, portions, starts, lead_is_cut, rest_is_cut, captured):
-    """Queries, keys and values come out of the product and store right in front, other ones in every turn.  Expected: the single tokens and the
-    portions in calls of their own, everything waited for.  In a captured graph, whose replays repeat one launch, the kernels wait."""
-    from aegean_tge_b200.parts.rope import rotary_tables
-    heads, kv_heads, head_dim, hidden, page_size = 28, 4, 128, 256, 64
-    q_lens, begins, n = [1] * len(lead) + portions, lead + starts, len(lead)
-    lengths = [a + m for a, m in zip(begins, q_lens)]
-    known = dict(lead_keys=sum(lengths[:n]), lead_longest=max(lengths[:n]), rest_ctx_len=max(lengths[n:]))
-    lead_cut = ops.choose_leading_split(known["lead_keys"], known["lead_longest"], kv_heads)
-    rest_cut = ops.choose_attention_split(sum(portions), len(portions), max(portions), known["rest_ctx_len"], heads, kv_heads, bound=known["rest_ctx_len"])
-    assert (lead_cut > 0) == lead_is_cut and (rest_cut > 0) == rest_is_cut
-    k_pages, v_pages, table, _k, _v = paged_cache(lengths, kv_heads, head_dim, page_size, torch.bfloat16, DEV, seed=5)
-    positions, seq_of_token, q_start, start_pos = batch_index(q_lens, begins, DEV)
-    cos, sin = (t.to(DEV) for t in rotary_tables(10000.0, head_dim, 4096))
-    gen = torch.Generator().manual_seed(6)
-    tokens, turns = sum(q_lens), 6
-    x = [torch.randn(tokens, hidden, generator=gen).to(torch.bfloat16).to(DEV) for _ in range(turns)]
-    w = (torch.randn((heads + 2 * kv_heads) * head_dim, hidden, generator=gen) * 0.1).to(torch.bfloat16).to(DEV)
-    w_o = (torch.randn(256, heads * head_dim, generator=gen) * 0.02).to(torch.bfloat16).to(DEV)
-    attended, results = torch.zeros(tokens, heads * head_dim, dtype=torch.bfloat16, device=DEV), torch.zeros(turns, tokens, 256, device=DEV)
-
-    def store(i):
-        return ops.linear_qkv_rope_store(x[i], w, None, cos, sin, head_dim, positions, seq_of_token, table, k_pages, v_pages, heads, kv_heads, head_dim)
-
-    def turn(i):
-        qkv = store(i)
-        ops.attention(qkv[:, :heads * head_dim], k_pages, v_pages, table, q_start, start_pos, positions, seq_of_token, len(q_lens), max(q_lens),
-                      max(lengths), heads, kv_heads, head_dim, head_dim ** -0.5, decode_prefix=n, out=attended, **known)
-        ops.linear(attended, w_o, None, ops.GEMM_STORE_F32, out=results[i])
-
-    # positions and q_start of a call count from the call's first token
-    wanted = []
-    rest = batch_index(portions, starts, DEV)
-    for i in range(turns):
-        qkv = store(i)
-        torch.cuda.synchronize()
-        rows = torch.zeros_like(attended)
-        ops.attention(qkv[:n, :heads * head_dim], k_pages, v_pages, table[:n].contiguous(), q_start[:n + 1], start_pos[:n], positions[:n],
-                      seq_of_token[:n], n, 1, known["lead_longest"], heads, kv_heads, head_dim, head_dim ** -0.5, out=rows[:n])
-        torch.cuda.synchronize()
-        ops.attention(qkv[n:, :heads * head_dim], k_pages, v_pages, table[n:].contiguous(), rest[2], rest[3], rest[0], rest[1], len(portions),
-                      max(portions), known["rest_ctx_len"], heads, kv_heads, head_dim, head_dim ** -0.5, out=rows[n:])
-        torch.cuda.synchronize()
-        wanted.append(ops.linear(rows, w_o, None, ops.GEMM_STORE_F32))
-        torch.cuda.synchronize()
-    if captured:
-        turn(0)
-        torch.cuda.synchronize()
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph):
-            for i in range(turns):
-                turn(i)
-        run = graph.replay
-    else:
-        run = lambda: [turn(i) for i in range(turns)]
-    for _ in range(4):
-        results.zero_()
-        run()
-        for i in range(turns):
-            assert rel_error(results[i], wanted[i]) < TOL[torch.bfloat16], i
-    ops.check_status()
-
-
 def test_attention_decode_splits(ops, heads, kv_heads, head_dim, split, window):
     """Single tokens with two to sixteen key splits, some of them without keys for the short requests."""
     err, _, _ = _attention_case(ops, torch.bfloat16, heads, kv_heads, head_dim, [1, 1, 1, 1, 1], [1000, 0, 511, 512, 130],
