@@ -31,7 +31,9 @@
 
 enum GemmEpilogue : int { GEMM_STORE = 0, GEMM_STORE_F32 = 1, GEMM_ADD_F32 = 2, GEMM_SWIGLU = 3, GEMM_GELU = 4,
                           GEMM_GELU_TANH = 5, GEMM_GLU_CLAMPED = 6 };
-// Added to the epilogue by a caller whose weights no kernel still in flight can have written (a model's, once it is loaded).
+// Added to the epilogue by a caller whose weights and bias no kernel still in flight can have written (a model's, once it is loaded): the
+// products then ask for weights ahead of their wait for the kernel in front.  Without it they let their dependents start only
+// behind that wait, so that the kernel that adds cuts may still ask for the bias ahead of its own.
 constexpr int GEMM_WEIGHTS_SETTLED = 256;
 // GEMM_GLU_CLAMPED: the gated epilogue with both halves clamped at L = `alpha`: g <- min(g, L), u <- clamp(u, -L, L),
 // out = g sigmoid(1.702 g) (u + 1).
@@ -73,7 +75,7 @@ struct GemmParams {
   float ss_eps;
   float alpha;         // multiplies acc + bias in the plain epilogues (1: none)
   int act_from;        // first weight row the GELU epilogues activate
-  int settled;         // the weights were there before any kernel that may still run: the pair kernel asks for them early
+  int settled;         // weights, bias and what the kernel that adds cuts takes of the model were there before any kernel that may still run
 };
 constexpr int DEFER_MAX_TOKENS = 128;
 
@@ -334,10 +336,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   const uint32_t tmem_base = *tmem_slot_ptr;
   // Only now may the next kernel be scheduled: this block already holds its tensor memory, so a block of
   // the next kernel that lands on the same SM can at worst wait for it, never starve it.
+  if (!p.settled) pdl_wait();
   pdl_trigger();
   // Set-up above overlapped the previous kernel; from here on its results are read.  The loading warp
-  // waits later: weights are nobody's result, so it first asks for a ring-full of weight tiles.
-  if (warp != 0) pdl_wait();
+  // waits later where weights are nobody's result: it first asks for a ring-full of weight tiles.
+  if (p.settled && warp != 0) pdl_wait();
 
   const int total_work = p.tiles_w * p.tiles_t * p.splits;
   float* row_factor = nullptr;
@@ -359,7 +362,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       int issued = 0;
       bool ok = true;
       int ahead = 0;      // stages of the first item whose weight tile is already on its way
-      if ((int)blockIdx.x < total_work) {
+      if (p.settled && (int)blockIdx.x < total_work) {
         const int split = (int)blockIdx.x % p.splits;
         const int tile_w = ((int)blockIdx.x / p.splits) / p.tiles_t;
         const int kb_begin = (int)((long long)split * p.k_blocks / p.splits);
@@ -567,10 +570,11 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
   cluster_sync_all();             // both blocks' barriers exist before either signals the other
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  if (!p.settled) pdl_wait();
   pdl_trigger();
   // Settled weights (the caller says so): their loader asks for a ring-full of them while the kernel in front still runs.
   // (193 tokens in three prompts, 12 layers of the 7B shape, with the shorter epilogue: 2,087 -> 1,955 us.)
-  if (warp != 0 || !p.settled) pdl_wait();
+  if (p.settled && warp != 0) pdl_wait();
 
   const int total_work = p.tiles_w * p.tiles_t * p.splits;
   const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
@@ -1058,7 +1062,7 @@ namespace {
 int launch_product(const void* x, long long ldx, const void* w, long long ldw, const float* bias, void* out,
                    long long ldo, int M, int N, int K, int epilogue, float* scratch, long long scratch_floats,
                    int force_bn, int force_splits, bool partial_always, int* status, cudaStream_t stream,
-                   int* splits_out, const RowSums& sums = RowSums(), float alpha = 1.0f, int act_from = 0, bool settled = false) {
+                   int* splits_out, bool settled, const RowSums& sums = RowSums(), float alpha = 1.0f, int act_from = 0) {
   if (K % 8 != 0 || ldx % 8 != 0 || ldw % 8 != 0 || (uintptr_t)x % 16 != 0 || (uintptr_t)w % 16 != 0) return TGE_UNSUPPORTED;
   if (scratch == nullptr) scratch_floats = 0;
   const Plan plan = make_plan(M, N, K, scratch_floats, force_bn, force_splits);
@@ -1123,7 +1127,7 @@ int launch_product(const void* x, long long ldx, const void* w, long long ldw, c
   p.to_partial = to_partial ? 1 : 0;
   p.bias = bias; p.out = out; p.ldo = ldo; p.partial = scratch; p.status = status;
   p.ss = sums.ss; p.ss_slices = sums.slices; p.ss_width = sums.width; p.ss_eps = sums.eps;
-  p.alpha = alpha; p.act_from = act_from; p.settled = 0;
+  p.alpha = alpha; p.act_from = act_from; p.settled = settled ? 1 : 0;
 
   const size_t smem = 1024 + (size_t)plan.stages * (A_STAGE_BYTES + plan.bn * BK * 2) + 8 * (2 * plan.stages + 4) + 16 +
                       DEFER_MAX_TOKENS * sizeof(float);
@@ -1493,7 +1497,7 @@ TGE_API int tge_gemm_tcgen05(const void* x, long long ldx, const void* w, long l
   RowSums sums;
   sums.ss = x_ss; sums.slices = x_ss_slices; sums.width = x_ss_width; sums.eps = x_ss_eps;
   int rc = launch_product(x, ldx, w, ldw, bias, out, ldo, M, N, K, epilogue, scratch, scratch_floats, force_bn,
-                          force_splits, false, status, stream, &splits, sums, alpha, act_from, settled);
+                          force_splits, false, status, stream, &splits, settled, sums, alpha, act_from);
   if (rc != 1) return rc;
   if (splits > 0) {
     // bytes of four columns of the result: two bfloat16 where they are gated, four bfloat16, or four float32
@@ -1516,6 +1520,7 @@ TGE_API int tge_gemm_tcgen05(const void* x, long long ldx, const void* w, long l
   return 1;
 }
 
+// `settled` of the entry points below: GEMM_WEIGHTS_SETTLED of the one above, norm weights and angles included.
 // As tge_gemm_tcgen05_add_norm below, but the norm's factor is left to whoever multiplies the result next:
 // stream [M, N] float32 += x . w^T (+ bias); scaled_out [M, N] bf16 = stream * norm_weight;
 // ss_out float32 [tge_gemm_tcgen05_defer_slices(N), M] = the rows' sums of squares, in slices.  At most 128 tokens.
@@ -1524,14 +1529,14 @@ TGE_API int tge_gemm_tcgen05_defer_slices(int N) { return (N + SCALE_SLICE - 1) 
 TGE_API int tge_gemm_tcgen05_add_defer(const void* x, long long ldx, const void* w, long long ldw, const float* bias,
                                        float* stream_out, long long ldo, int M, int N, int K, const float* norm_weight,
                                        void* scaled_out, long long ld_scaled, float* ss_out, float* scratch,
-                                       long long scratch_floats, int* status, float alpha, cudaStream_t stream) {
+                                       long long scratch_floats, int* status, float alpha, int settled, cudaStream_t stream) {
   TGE_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm+defer: bad sizes M=%d N=%d K=%d", M, N, K);
   TGE_REQUIRE(status != nullptr && norm_weight != nullptr && scaled_out != nullptr && ss_out != nullptr, "gemm+defer: bad arguments");
   if (M == 0) return 0;
   if (M > DEFER_MAX_TOKENS || scratch == nullptr) return TGE_UNSUPPORTED;
   int splits = 0;
   int rc = launch_product(x, ldx, w, ldw, nullptr, stream_out, ldo, M, N, K, GEMM_ADD_F32, scratch, scratch_floats, 0, 0,
-                          true, status, stream, &splits);
+                          true, status, stream, &splits, settled != 0);
   if (rc != 1) return rc;
   tge_launch(splitk_add_scale_kernel, dim3((N + SCALE_SLICE - 1) / SCALE_SLICE, M), SCALE_SLICE, 0, stream,
              (const float*)scratch, bias, stream_out, ldo, norm_weight, (__nv_bfloat16*)scaled_out, ld_scaled, ss_out, M, N,
@@ -1546,14 +1551,14 @@ TGE_API int tge_gemm_tcgen05_add_defer(const void* x, long long ldx, const void*
 TGE_API int tge_gemm_tcgen05_add_norm(const void* x, long long ldx, const void* w, long long ldw, const float* bias,
                                       float* stream_out, long long ldo, int M, int N, int K, const float* norm_weight,
                                       float eps, void* norm_out, long long ld_norm, float* scratch,
-                                      long long scratch_floats, int* status, float alpha, cudaStream_t stream) {
+                                      long long scratch_floats, int* status, float alpha, int settled, cudaStream_t stream) {
   TGE_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm+norm: bad sizes M=%d N=%d K=%d", M, N, K);
   TGE_REQUIRE(status != nullptr && norm_weight != nullptr && norm_out != nullptr && eps > 0.0f, "gemm+norm: bad arguments");
   if (M == 0) return 0;
   if (M > FUSED_MAX_TOKENS || N > NORM_THREADS * NORM_PER_THREAD || scratch == nullptr) return TGE_UNSUPPORTED;
   int splits = 0;
   int rc = launch_product(x, ldx, w, ldw, nullptr, stream_out, ldo, M, N, K, GEMM_ADD_F32, scratch, scratch_floats, 0, 0,
-                          true, status, stream, &splits);
+                          true, status, stream, &splits, settled != 0);
   if (rc != 1) return rc;
   tge_launch(splitk_add_norm_kernel, dim3(M), NORM_THREADS, 0, stream,
              (const float*)scratch, bias, stream_out, ldo, norm_weight, eps, (__nv_bfloat16*)norm_out, ld_norm, M, N,
@@ -1565,14 +1570,14 @@ TGE_API int tge_gemm_tcgen05_add_norm(const void* x, long long ldx, const void* 
 // N floats), for a kernel of the caller's that adds them in their order.  At most 256 tokens; same return codes.
 TGE_API int tge_gemm_tcgen05_partials(const void* x, long long ldx, const void* w, long long ldw, int M, int N, int K,
                                       float* scratch, long long scratch_floats, int* splits_out, int* status,
-                                      cudaStream_t stream) {
+                                      int settled, cudaStream_t stream) {
   TGE_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm partials: bad sizes M=%d N=%d K=%d", M, N, K);
   TGE_REQUIRE(status != nullptr && splits_out != nullptr, "gemm partials: bad arguments");
   *splits_out = 0;
   if (M == 0) return 0;
   if (M > FUSED_MAX_TOKENS || scratch == nullptr) return TGE_UNSUPPORTED;
   return launch_product(x, ldx, w, ldw, nullptr, scratch, N, M, N, K, GEMM_STORE_F32, scratch, scratch_floats, 0, 0, true,
-                        status, stream, splits_out);
+                        status, stream, splits_out, settled != 0);
 }
 
 // The fused q/k/v product of an attention layer for a small batch: qkv = x . w^T + bias, q rotated into
@@ -1584,7 +1589,7 @@ TGE_API int tge_gemm_tcgen05_qkv_rope(const void* x, long long ldx, const void* 
                                       const int* seq_of_token, const int* block_table, int max_pages, void* k_pages,
                                       void* v_pages, int num_pages, int page_size, int heads, int kv_heads,
                                       int head_dim, float* scratch, long long scratch_floats, int* status,
-                                      const float* x_ss, int x_ss_slices, int x_ss_width, float x_ss_eps,
+                                      const float* x_ss, int x_ss_slices, int x_ss_width, float x_ss_eps, int settled,
                                       cudaStream_t stream) {
   TGE_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm+rope: bad sizes M=%d N=%d K=%d", M, N, K);
   TGE_REQUIRE(N == (heads + 2 * kv_heads) * head_dim, "gemm+rope: %d weight rows are not (heads + 2 kv heads) * head_dim", N);
@@ -1594,7 +1599,7 @@ TGE_API int tge_gemm_tcgen05_qkv_rope(const void* x, long long ldx, const void* 
   if (M > FUSED_MAX_TOKENS || (size_t)N * sizeof(float) > 200 * 1024 || scratch == nullptr) return TGE_UNSUPPORTED;
   int splits = 0;
   int rc = launch_product(x, ldx, w, ldw, nullptr, qkv, ld_qkv, M, N, K, GEMM_STORE, scratch, scratch_floats, 0, 0, true,
-                          status, stream, &splits);
+                          status, stream, &splits, settled != 0);
   if (rc != 1) return rc;
   tge_launch(splitk_qkv_rope_store_kernel, dim3(M, heads + 2 * kv_heads), head_dim >= 128 ? 128 : 64,
              (size_t)head_dim * sizeof(float), stream, (const float*)scratch, bias, (__nv_bfloat16*)qkv, ld_qkv, M, N,
@@ -1617,7 +1622,7 @@ TGE_API int tge_gemm_tcgen05_qkv_norm_act(const void* x, long long ldx, const vo
                                           int max_pages, void* k_pages, void* v_pages, int num_pages, int page_size,
                                           int heads, int kv_heads, int head_dim, int value_dim, int store_kv,
                                           float* scratch, long long scratch_floats, int* status, const float* x_ss,
-                                          int x_ss_slices, int x_ss_width, float x_ss_eps, cudaStream_t stream) {
+                                          int x_ss_slices, int x_ss_width, float x_ss_eps, int settled, cudaStream_t stream) {
   TGE_REQUIRE(M >= 0 && N > 0 && K > 0, "gemm+qk-norm: bad sizes M=%d N=%d K=%d", M, N, K);
   const long long n_qkv = (long long)heads * head_dim + (long long)kv_heads * (head_dim + value_dim);
   TGE_REQUIRE(heads > 0 && kv_heads > 0 && head_dim > 0 && value_dim > 0 && n_qkv <= N,
@@ -1631,7 +1636,7 @@ TGE_API int tge_gemm_tcgen05_qkv_norm_act(const void* x, long long ldx, const vo
   if (M > FUSED_MAX_TOKENS || n_qkv > (long long)QKV_ACT_THREADS * QKV_PER_THREAD || scratch == nullptr) return TGE_UNSUPPORTED;
   int splits = 0;
   int rc = launch_product(x, ldx, w, ldw, nullptr, qkv, ld_qkv, M, N, K, GEMM_STORE, scratch, scratch_floats, 0, 0, true,
-                          status, stream, &splits);
+                          status, stream, &splits, settled != 0);
   if (rc != 1) return rc;
   const size_t smem = 0;
   const int act_blocks = (int)((N - n_qkv + QKV_ACT_SLICE - 1) / QKV_ACT_SLICE);

@@ -78,22 +78,22 @@ def core() -> ctypes.CDLL:
                                            _c_int, _c_float, _c_float, _c_int, _c_ptr])
         _declare(lib, "tge_gemm_tcgen05_add_defer", [_c_ptr, _c_ll, _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ll, _c_int,
                                                      _c_int, _c_int, _c_ptr, _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ll,
-                                                     _c_ptr, _c_float, _c_ptr])
+                                                     _c_ptr, _c_float, _c_int, _c_ptr])
         _declare(lib, "tge_gemm_tcgen05_defer_slices", [_c_int])
         _declare(lib, "tge_scale_rows", [_c_ptr, _c_ll, _c_ptr, _c_int, _c_int, _c_float, _c_ptr, _c_ll, _c_int,
                                          _c_int, _c_ptr])
         _declare(lib, "tge_gemm_tcgen05_add_norm", [_c_ptr, _c_ll, _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ll, _c_int, _c_int,
                                                     _c_int, _c_ptr, _c_float, _c_ptr, _c_ll, _c_ptr, _c_ll, _c_ptr,
-                                                    _c_float, _c_ptr])
+                                                    _c_float, _c_int, _c_ptr])
         _declare(lib, "tge_gemm_tcgen05_qkv_rope", [_c_ptr, _c_ll, _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ll, _c_int, _c_int,
                                                     _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr,
                                                     _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
-                                                    _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_int, _c_int, _c_float, _c_ptr])
+                                                    _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_int, _c_int, _c_float, _c_int, _c_ptr])
         _declare(lib, "tge_gemm_tcgen05_qkv_norm_act", [_c_ptr, _c_ll, _c_ptr, _c_ll, _c_ptr, _c_ll, _c_ptr, _c_ll, _c_int,
                                                         _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_float, _c_ptr, _c_ll,
                                                         _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int,
                                                         _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ll,
-                                                        _c_ptr, _c_ptr, _c_int, _c_int, _c_float, _c_ptr])
+                                                        _c_ptr, _c_ptr, _c_int, _c_int, _c_float, _c_int, _c_ptr])
         lib.tge_gemm_tcgen05_pair_mode.argtypes = [_c_int]
         lib.tge_gemm_tcgen05_pair_mode.restype = None
         lib.tge_gemm_tcgen05_scratch_floats.argtypes = [_c_int, _c_int, _c_int]
@@ -147,7 +147,7 @@ def core() -> ctypes.CDLL:
         _declare(lib, "tge_streams_update_defer", [_c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr,
                                                    _c_ptr, _c_ptr, _c_ptr, _c_ptr])
         _declare(lib, "tge_gemm_tcgen05_partials", [_c_ptr, _c_ll, _c_ptr, _c_ll, _c_int, _c_int, _c_int, _c_ptr, _c_ll,
-                                                    ctypes.POINTER(_c_int), _c_ptr, _c_ptr])
+                                                    ctypes.POINTER(_c_int), _c_ptr, _c_int, _c_ptr])
         _declare(lib, "tge_mlstm_step", [_c_ptr, _c_int, _c_ll, _c_ptr, _c_ll, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr,
                                          _c_ptr, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_float, _c_float,
                                          _c_ptr])
@@ -573,7 +573,8 @@ def linear_qkv_norm_act_store(x, w: torch.Tensor, heads: int, kv_heads: int, hea
                               positions: torch.Tensor, seq_of_token: torch.Tensor, block_table: Optional[torch.Tensor],
                               k_pages: Optional[torch.Tensor], v_pages: Optional[torch.Tensor],
                               v_other: Optional[torch.Tensor] = None, blend: Optional[torch.Tensor] = None,
-                              act_out: Optional[torch.Tensor] = None, activation: int = GEMM_GELU) -> Optional[torch.Tensor]:
+                              act_out: Optional[torch.Tensor] = None, activation: int = GEMM_GELU,
+                              settled: bool = False) -> Optional[torch.Tensor]:
     """For a small bfloat16 batch, the q/k/v product of a layer that normalises q and k over their whole
     projections, with what follows it in one kernel: the product's partial sums are added, q and k normalised
     (float32), the values blended with ``v_other`` and k and v stored (as :func:`qk_norm_kv_store` does).  The
@@ -635,7 +636,7 @@ def linear_qkv_norm_act_store(x, w: torch.Tensor, heads: int, kv_heads: int, hea
                                            max_pages, _ptr(k_pages), _ptr(v_pages), num_pages, page_size, heads, kv_heads,
                                            head_dim, value_dim, int(store), scratch.data_ptr(), scratch.numel(),
                                            status_word().data_ptr(),
-                                           *(_NO_FACTOR if deferred is None else deferred.factor_args()), _stream())
+                                           *(_NO_FACTOR if deferred is None else deferred.factor_args()), int(settled), _stream())
     return None if _check(rc, lib) == UNSUPPORTED else qkv
 
 
@@ -687,7 +688,7 @@ class DeferredRows:
 
 
 _NO_FACTOR = (None, 0, 0, 0.0)
-_SETTLED = 256          # added to the epilogue: GEMM_WEIGHTS_SETTLED of csrc/gemm_tcgen05.cu
+_SETTLED = 256          # added to the epilogue: GEMM_WEIGHTS_SETTLED of csrc/gemm_tcgen05.cu; ``settled`` of the calls below
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], epilogue: int,
@@ -706,8 +707,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], epilo
     ``alpha`` multiplies product + bias in the store and add epilogues (a residual multiplier, a logit scale).
     Both types go to their tcgen05 kernel when the shape allows TMA (float32, split into three bfloat16 numbers, from
     512 x 512 weights on), else to the CUDA-core kernel.
-    ``settled``: no kernel that may still run has written ``w`` (a loaded model's weights): they may be read before the kernel
-    in front is done.
+    ``settled``: no kernel that may still run has written ``w`` or ``bias`` (a loaded model's weights): they may be read before the
+    kernel in front is done.
     """
     deferred = x if isinstance(x, DeferredRows) else None
     if deferred is not None:
@@ -814,14 +815,14 @@ def linear_add_norm(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tenso
                                                 _rows_2d(w, "linear weight"), _ptr(bias), stream.data_ptr(),
                                                 _rows_2d(stream, "stream"), M, N, K, norm_weight.data_ptr(),
                                                 out.data_ptr(), N, sums.data_ptr(), scratch.data_ptr(),
-                                                scratch.numel(), status_word().data_ptr(), float(alpha), _stream())
+                                                scratch.numel(), status_word().data_ptr(), float(alpha), int(settled), _stream())
             if _check(rc, lib) != UNSUPPORTED:
                 return DeferredRows(out, sums, N, eps)
         rc = lib.tge_gemm_tcgen05_add_norm(x.data_ptr(), _rows_2d(x, "linear input"), w.data_ptr(),
                                            _rows_2d(w, "linear weight"), _ptr(bias), stream.data_ptr(),
                                            _rows_2d(stream, "stream"), M, N, K, norm_weight.data_ptr(), float(eps),
                                            out.data_ptr(), N, scratch.data_ptr(), scratch.numel(),
-                                           status_word().data_ptr(), float(alpha), _stream())
+                                           status_word().data_ptr(), float(alpha), int(settled), _stream())
         if _check(rc, lib) != UNSUPPORTED:
             return out
     linear(x, w, bias, GEMM_ADD_F32, out=stream, alpha=alpha, settled=settled)
@@ -870,7 +871,7 @@ def linear_qkv_rope_store(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch
                                            block_table.shape[1], k_pages.data_ptr(), v_pages.data_ptr(), num_pages,
                                            page_size, heads, kv_heads, head_dim, scratch.data_ptr(), scratch.numel(),
                                            status_word().data_ptr(),
-                                           *(_NO_FACTOR if deferred is None else deferred.factor_args()), _stream())
+                                           *(_NO_FACTOR if deferred is None else deferred.factor_args()), int(settled), _stream())
         if _check(rc, lib) != UNSUPPORTED:
             return qkv
     qkv = linear(x if deferred is None else deferred, w, bias, GEMM_STORE, settled=settled)
@@ -2137,7 +2138,7 @@ def streams_defer(x: torch.Tensor, following, partial: Optional[torch.Tensor] = 
     return DeferredRows(rows, sums, width, eps) if following is not None else None
 
 
-def linear_partials(x: torch.Tensor, w: torch.Tensor) -> Optional[Tuple[torch.Tensor, int]]:
+def linear_partials(x: torch.Tensor, w: torch.Tensor, settled: bool = False) -> Optional[Tuple[torch.Tensor, int]]:
     """x . w^T of a small bfloat16 batch as float32 partial sums [splits, M, N] in the scratch buffer, not yet added up:
     (buffer, splits), to be read by the next kernel of the stream.  None: not a product for this path."""
     M, K = x.shape
@@ -2152,5 +2153,5 @@ def linear_partials(x: torch.Tensor, w: torch.Tensor) -> Optional[Tuple[torch.Te
     scratch = scratch_floats(max(lib.tge_gemm_tcgen05_scratch_floats(M, N, K), M * N))
     splits = _c_int(0)
     rc = lib.tge_gemm_tcgen05_partials(x.data_ptr(), _rows_2d(x, "linear input"), w.data_ptr(), _rows_2d(w, "linear weight"), M, N, K,
-                                       scratch.data_ptr(), scratch.numel(), ctypes.byref(splits), status_word().data_ptr(), _stream())
+                                       scratch.data_ptr(), scratch.numel(), ctypes.byref(splits), status_word().data_ptr(), int(settled), _stream())
     return None if _check(rc, lib) == UNSUPPORTED else (scratch, splits.value)

@@ -460,7 +460,8 @@ class GQAttention(Mixer):
                     h, self.w_shared if shared else self.w_qkv, self.heads, self.kv_heads, self.head_dim, self.value_dim,
                     q_w, k_w, eps, ctx.positions, ctx.seq_of_token, table if store_here else None,
                     k_pages if store_here else None, v_pages if store_here else None, v_other=other, blend=blend,
-                    act_out=beside[0] if shared else None, activation=beside[1] if shared else ops.GEMM_GELU)
+                    act_out=beside[0] if shared else None, activation=beside[1] if shared else ops.GEMM_GELU,
+                    settled=True)
                 did_beside = shared and qkv is not None
             if qkv is None:
                 qkv = ops.linear(h, self.w_qkv, self.b_qkv, ops.GEMM_STORE, settled=True)

@@ -211,7 +211,7 @@ class RoutedExperts(FeedForward):
     def route(self, h):
         """(ids int32 [T, top], weights float32 [T, top], the gate logits of the shared feed-forward [T] or None); the logits
         are a float32 product of the rows as given, which may lack their norm's factor."""
-        logits = self.ops.linear(h, self.w_router, self.router_bias, self.ops.GEMM_STORE_F32)
+        logits = self.ops.linear(h, self.w_router, self.router_bias, self.ops.GEMM_STORE_F32, settled=True)
         ids, weights = self.ops.router_topk(logits, self.correction, self.top, self.group_count, self.group_keep,
                                             logistic=self.logistic, over_sum=self.over_sum, group_pairs=self.group_pairs,
                                             factor=self.weights_scale, outputs=self.outputs)
@@ -227,7 +227,7 @@ class RoutedExperts(FeedForward):
         if not self.takes_deferred_at(tokens):
             return None
         ids, weights, gate = self.route(h)
-        z = ops.linear(h, self.up_rows, None, ops.GEMM_STORE)
+        z = ops.linear(h, self.up_rows, None, ops.GEMM_STORE, settled=True)
         a = ops.experts_dense_gate(z, ids, weights, self.experts, self.gate, self.weigh_input, self.shared_inner, gate)
         return a, self.down_columns
 
@@ -251,14 +251,14 @@ class RoutedExperts(FeedForward):
         tokens = h.shape[0]
         few = ctx.max_q_len <= 1 or tokens <= DIRECT_MAX_TOKENS
         if self.dense(tokens) and self.gate is not None and x_gate is None:
-            z = ops.linear(h, self.w_up.view(self.experts * 2 * self.inner_size, self.hidden), None, ops.GEMM_STORE)
+            z = ops.linear(h, self.w_up.view(self.experts * 2 * self.inner_size, self.hidden), None, ops.GEMM_STORE, settled=True)
             a = ops.experts_dense_gate(z, ids, weights, self.experts, self.gate, self.weigh_input)
-            ops.linear(a, self.w_down.view(self.hidden, self.experts * self.inner_size), None, ops.GEMM_ADD_F32, out=x)
+            ops.linear(a, self.w_down.view(self.hidden, self.experts * self.inner_size), None, ops.GEMM_ADD_F32, out=x, settled=True)
             return h
         if self.dense(tokens) and self.gate is None and x_gate is None:
-            z = ops.linear(h, self.w_up.view(self.experts * self.inner_size, self.hidden), None, ops.GEMM_STORE)
+            z = ops.linear(h, self.w_up.view(self.experts * self.inner_size, self.hidden), None, ops.GEMM_STORE, settled=True)
             ops.experts_dense_weigh(z, ids, weights, h, x, self.experts)
-            ops.linear(z, self.w_down.view(self.hidden, self.experts * self.inner_size), None, ops.GEMM_ADD_F32, out=x)
+            ops.linear(z, self.w_down.view(self.hidden, self.experts * self.inner_size), None, ops.GEMM_ADD_F32, out=x, settled=True)
             return h
         if few or self.experts == 0:
             ops.experts_direct(h, self.w_up, self.w_down, ids, weights, x, gate=self.gate, weigh_input=self.weigh_input,
@@ -278,25 +278,25 @@ class RoutedExperts(FeedForward):
             if hi > lo:
                 if fused is not None:
                     ops.linear(grouped[lo:hi], self.w_up[e], None, fused, out=inner[lo:hi],
-                               alpha=self.gate[0] if fused == ops.GEMM_GLU_CLAMPED else 1.0)
+                               alpha=self.gate[0] if fused == ops.GEMM_GLU_CLAMPED else 1.0, settled=True)
                 elif self.gate is not None:
-                    both = ops.linear(grouped[lo:hi], self.w_up[e], None, ops.GEMM_STORE_F32)
+                    both = ops.linear(grouped[lo:hi], self.w_up[e], None, ops.GEMM_STORE_F32, settled=True)
                     ops.gated_clamp_act(both, *self.gate, self.env.dtype, out=inner[lo:hi])
                 else:
-                    ops.linear(grouped[lo:hi], self.w_up[e], None, ops.GEMM_STORE, out=inner[lo:hi])
+                    ops.linear(grouped[lo:hi], self.w_up[e], None, ops.GEMM_STORE, out=inner[lo:hi], settled=True)
         if rows and self.gate is None:
             ops.activation(inner[:rows], ops.ACT_RELU_SQUARED)
         for e in range(self.experts):
             lo, hi = bounds[e], bounds[e + 1]
             if hi > lo:
-                ops.linear(inner[lo:hi], self.w_down[:, e, :], None, ops.GEMM_STORE_F32, out=outputs[lo:hi])
+                ops.linear(inner[lo:hi], self.w_down[:, e, :], None, ops.GEMM_STORE_F32, out=outputs[lo:hi], settled=True)
         ops.experts_combine_add(outputs, place, None if self.weigh_input else weights, h, x, x_gate=x_gate)
         return h
 
     def forward_f32(self, h: torch.Tensor, ctx: StepContext) -> torch.Tensor:
         last = self.last_product(h, ctx) if self.shared_inner else None
         if last is not None:
-            return self.ops.linear(last[0], last[1], None, self.ops.GEMM_STORE_F32)
+            return self.ops.linear(last[0], last[1], None, self.ops.GEMM_STORE_F32, settled=True)
         if self.shared is not None:
             # the feed-forward every token uses writes the rows, the chosen experts add to them
             complete = getattr(h, "complete", None)

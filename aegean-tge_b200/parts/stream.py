@@ -55,7 +55,7 @@ class Reinject(StreamStep):
 
     def forward(self, x: torch.Tensor, x0: torch.Tensor, ctx: StepContext) -> None:
         both = self.ops.concat_rows(x, x0, self.env.dtype)
-        self.ops.linear(both, self.weight, self.step, self.ops.GEMM_STORE_F32, out=x)
+        self.ops.linear(both, self.weight, self.step, self.ops.GEMM_STORE_F32, out=x, settled=True)
 
 
 @NORMS.register("connected_rmsnorm")
@@ -126,9 +126,9 @@ class ConnectedRMSNorm(Norm):
     def update_product(self, x: torch.Tensor, rows: torch.Tensor, weight: torch.Tensor, following: Optional["ConnectedRMSNorm"],
                        defer: bool = False):
         """:meth:`update` with y = rows . weight^T; of few rows the product's partial sums go straight to the update."""
-        partial = self.ops.linear_partials(rows, weight) if self.few(x) else None
+        partial = self.ops.linear_partials(rows, weight, settled=True) if self.few(x) else None
         if partial is None:
-            return self.update(x, self.ops.linear(rows, weight, None, self.ops.GEMM_STORE_F32), following, defer)
+            return self.update(x, self.ops.linear(rows, weight, None, self.ops.GEMM_STORE_F32, settled=True), following, defer)
         reads = following.reads() if following is not None else None
         h = self.ops.streams_defer(x, reads, partial[0], partial[1], self.mix, self.out)
         return h if defer or h is None else h.complete()

@@ -458,6 +458,58 @@ def test_gemm_pair_settled_weights_change_no_bit(ops, pair_everywhere, M, N, K):
     assert torch.equal(results[0], results[1]) and bool(torch.isfinite(results[0]).all())
 
 
+@pytest.mark.parametrize("pair", [0, 2])
+@pytest.mark.parametrize("M", [4, 100, 200])
+def test_products_wait_for_weights_that_the_kernel_in_front_has_just_written(ops, pair, M):
+    """Weights and biases that come out of the kernel right in front, other ones in every turn: without ``settled`` a product on one SM or on
+    pairs, the kernel that adds its cuts, and the fused forms see them.  Expected: the same calls, everything waited for."""
+    gen = torch.Generator().manual_seed(M)
+    N, K, turns = 1536, 2048, 4
+    seeds = [(torch.randn(N, 256, generator=gen) * 0.1).to(torch.bfloat16).to(DEV) for _ in range(turns)]
+    basis = (torch.randn(K, 256, generator=gen) * 0.1).to(torch.bfloat16).to(DEV)
+    row = [torch.randn(1, 512, generator=gen).to(torch.bfloat16).to(DEV) for _ in range(turns)]
+    maker = (torch.randn(N, 512, generator=gen) * 0.1).to(torch.bfloat16).to(DEV)
+    x = torch.randn(M, K, generator=gen).to(torch.bfloat16).to(DEV)
+    w, bias = torch.zeros(N, K, dtype=torch.bfloat16, device=DEV), torch.zeros(1, N, device=DEV)
+    norm = 1.0 + 0.1 * torch.randn(N, generator=gen).to(DEV)
+
+    def turn(i, between):
+        results, stream = [], torch.ones(M, N, device=DEV)
+        ops.linear(row[i], maker, None, ops.GEMM_STORE_F32, out=bias)
+        between()
+        ops.linear(seeds[i], basis, None, ops.GEMM_STORE, out=w)
+        between()
+        results.append(ops.linear(x, w, bias[0], ops.GEMM_STORE_F32, force_splits=3))
+        between()
+        ops.linear(seeds[i - 1], basis, None, ops.GEMM_STORE, out=w)
+        between()
+        results.append(ops.linear(x, w, None, ops.GEMM_STORE))
+        between()
+        ops.linear(seeds[i], basis, None, ops.GEMM_STORE, out=w)
+        ops.linear(row[i - 1], maker, None, ops.GEMM_STORE_F32, out=bias)
+        between()
+        results.append(ops.linear(x, w, bias[0], ops.GEMM_STORE_F32))
+        between()
+        ops.linear(seeds[i - 1], basis, None, ops.GEMM_STORE, out=w)
+        between()
+        results += [ops.linear_add_norm(x, w, bias[0], stream, norm, 1e-5, torch.bfloat16), stream]
+        between()
+        return results
+
+    ops.set_pair_gemm(pair)
+    try:
+        wanted = [turn(i, torch.cuda.synchronize) for i in range(turns)]
+        for _ in range(6):
+            got = [turn(i, lambda: None) for i in range(turns)]
+            for i in range(turns):
+                assert all(torch.equal(a, b) for a, b in zip(got[i], wanted[i])), i
+        ops.check_status()
+    finally:
+        ops.set_pair_gemm(1)
+    assert rel_error(wanted[0][0], ops_plain.linear(x.cpu(), ops_plain.linear(seeds[0].cpu(), basis.cpu(), None).to(torch.bfloat16),
+                                                    ops_plain.linear(row[0].cpu(), maker.cpu(), None)[0])) < TOL[torch.bfloat16]
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 256, 128), (8, 3584, 512), (33, 520, 264), (128, 1024, 320), (140, 384, 192), (150, 384, 192)])
 @pytest.mark.parametrize("defer", [False, True])
 def test_linear_add_norm_and_rows_without_their_factor(ops, M, N, K, defer):
