@@ -80,15 +80,8 @@ struct GemmParams {
 constexpr int DEFER_MAX_TOKENS = 128;
 
 __device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.0f + expf(-g)) * u; }
-// The same for results that are rounded to bfloat16: exp as a base-2 exponential, the division as a product with the reciprocal, both
-// approximate as __expf and __fdividef are, without care for subnormal numbers (1 + e^-g is none, and an e^-g that small adds
-// nothing to it).
-__device__ __forceinline__ float gate_mul(float g, float u) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(e) : "f"(g * -1.4426950408889634f));
-  asm("rcp.approx.ftz.f32 %0, %1;\n" : "=f"(r) : "f"(1.0f + e));
-  return g * r * u;
-}
+// The same for results that are rounded to bfloat16, with CUDA's fast exponential and division.
+__device__ __forceinline__ float gate_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
 // the clamped gate: g <- min(g, L), u <- clamp(u, -L, L), g sigmoid(1.702 g) (u + 1)
 __device__ __forceinline__ float clamped_gate_mul(float g, float u, float limit) {
   g = fminf(g, limit);

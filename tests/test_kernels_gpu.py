@@ -441,6 +441,34 @@ def test_gemm_tcgen05_stores_of_any_width_hold_the_same(ops, pair, M, N, K):
         ops.set_pair_gemm(1)
 
 
+@pytest.mark.parametrize("pair,M", [(0, 3), (2, 150)])
+def test_gated_epilogue_over_the_whole_range_of_gates(ops, pair, M):
+    """g / (1 + exp(-g)) u where the product is zero and the bias holds g and u: gates from -1e4 to 1e4, where exp(-g) overflows and where a
+    quotient's divisor does, infinities and NaN.  2^-8: the rounding to bfloat16; 89 * 3 / 2^126, the largest |g u| over the smallest such
+    divisor: CUDA's fast division gives zero for divisors above 2^126, which |g| <= 89 reaches."""
+    edges = [0.0, -0.0, 1e-30, -1e-30, -87.0, -87.5, -88.0, -88.5, -88.8, -89.0, -103.0, -1e4, 88.0, 1e4, 3e38, -3e38, float("inf"), float("-inf"),
+             float("nan")]
+    gates = torch.cat([torch.tensor(edges), torch.linspace(-110.0, 110.0, 4001), torch.linspace(-4.0, 4.0, 1000)])
+    gates = torch.cat([gates, torch.zeros(-gates.numel() % 64)])
+    up = torch.where(torch.arange(gates.numel()) % 2 == 0, 1.0, -3.0)
+    bias = torch.stack([gates, up], 1).reshape(-1).to(DEV)
+    x = torch.zeros(M, 64, dtype=torch.bfloat16, device=DEV)
+    w = torch.randn(bias.numel(), 64, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).to(DEV)
+    ops.set_pair_gemm(pair)
+    try:
+        got = ops.linear(x, w, bias, ops.GEMM_SWIGLU).double().cpu()
+    finally:
+        ops.set_pair_gemm(1)
+    ops.check_status()
+    exact = (gates.double() / (1.0 + torch.exp(-gates.double())) * up.double())[None].expand(M, -1)
+    special = ~torch.isfinite(exact) | (exact.abs() > 3e38)
+    assert torch.equal(torch.isnan(got), torch.isnan(exact))
+    off = ((got - exact).abs() > 2.0 ** -8 * exact.abs() + 89 * 3 * 2.0 ** -126) & ~special
+    assert not bool(off.any()), gates[off[0]].tolist()
+    infinite = torch.isinf(exact)
+    assert torch.equal(got[infinite], exact[infinite])
+
+
 @pytest.mark.parametrize("M,N,K", [(150, 256, 64), (193, 3584, 704), (300, 4608, 512), (2048, 768, 1024)])
 def test_gemm_pair_settled_weights_change_no_bit(ops, pair_everywhere, M, N, K):
     """Weights asked for ahead of the kernel in front (fewer k-blocks than stages, cuts along k, several tiles to a pair), each product
