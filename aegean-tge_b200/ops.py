@@ -991,7 +991,7 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
         raise KernelError("attention: runs of heads over the same keys are for single tokens on the tensor-core kernels")
     if use_mma:
         lib = attention_lib(head_dim, value_dim)
-        prefix = decode_prefix if decode_prefix >= MIN_DECODE_PREFIX and max_q_len > 1 and not pool and heads // kv_heads <= 16 else 0
+        prefix = decode_prefix if MIN_DECODE_PREFIX <= decode_prefix < num_seqs and max_q_len > 1 and not pool and heads // kv_heads <= 16 else 0
         prefix_split = split_tokens
         if pool:
             # The window's tokens go through the tensor-core kernels with their keys cut into at least two runs, so

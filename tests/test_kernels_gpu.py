@@ -688,7 +688,7 @@ def test_linear_qkv_rope_store(ops, heads, kv_heads, head_dim, rotary, hidden, q
 # attention
 # ---------------------------------------------------------------------------
 def _attention_case(ops, dtype, heads, kv_heads, head_dim, q_lens, starts, window=0, split=0, force_simt=False,
-                    page_size=16, spike=None, decode_prefix=0, known=None):
+                    page_size=16, spike=None, decode_prefix=0, known=None, longest=0):
     lengths = [s + n for s, n in zip(starts, q_lens)]
     k_pages, v_pages, table, k_list, v_list = paged_cache(lengths, kv_heads, head_dim, page_size, dtype, DEV, seed=9)
     positions, seq_of_token, q_start, start_pos = batch_index(q_lens, starts, DEV)
@@ -705,7 +705,7 @@ def _attention_case(ops, dtype, heads, kv_heads, head_dim, q_lens, starts, windo
     scale = 1.0 / math.sqrt(head_dim)
     dq = buf.to(DEV)
     out = ops.attention(dq[:, :heads * head_dim], k_pages, v_pages, table, q_start, start_pos, positions,
-                        seq_of_token, len(q_lens), max(q_lens), max(lengths), heads, kv_heads, head_dim, scale,
+                        seq_of_token, len(q_lens), longest or max(q_lens), max(lengths), heads, kv_heads, head_dim, scale,
                         window=window, split_tokens=split, force_simt=force_simt, decode_prefix=decode_prefix, **(known or {}))
     ops.check_status()
     q = buf[:, :heads * head_dim].view(T, heads, head_dim)
@@ -844,6 +844,13 @@ def test_side_by_side_attention_is_done_before_what_follows(ops):
             first[i % 2] = rows
         assert torch.equal(rows, first[i % 2]), i
     ops.check_status()
+
+
+@pytest.mark.parametrize("tokens,longest", [(8, 4), (30, 2)])
+def test_a_step_of_single_tokens_whose_bound_says_more(ops, tokens, longest):
+    """All portions single tokens, as ``decode_prefix`` says, under a looser bound of their length: no portion is left behind them."""
+    err, _, _ = _attention_case(ops, torch.bfloat16, 14, 2, 128, [1] * tokens, [2300] + [40] * (tokens - 1), decode_prefix=tokens, longest=longest)
+    assert err < TOL[torch.bfloat16]
 
 
 @pytest.mark.parametrize("lead,portions,starts,lead_is_cut,rest_is_cut", [
