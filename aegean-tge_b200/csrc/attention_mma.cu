@@ -1439,6 +1439,31 @@ TGE_API long long tge_attention_mma_scratch_floats(int tokens, int heads, int nu
   return num_splits > 1 ? (long long)num_splits * tokens * heads * (DV + 2) : 0;
 }
 
+// Two query tiles to a block share K and V and one SM; where blocks are few or short, one tile to a block has the SMs'
+// tensor cores to itself and less to set up.  The lines, measured at 28 heads over 4, 40 over 8, 12 over 2, 32 over 8, 16 over 16
+// of 128 and 14 over 2 of 64 (two tiles / one, us).  Up to 320 keys, any number of blocks: unless the single tiles take twice
+// the waves (28/4: 16 x 64 13.4 / 14.0, 20 x 64 24.5 / 20.8; 12/2: 64 x 32 16.9 / 20.3, 12 x 100 13.6 / 10.3, 8 x 300 17.4 / 19.7;
+// 40/8: 6 x 128 14.8 / 16.9, 32 x 64 51.4 / 41.7), or tiles are whole ones of a head's queries (16/16: 8 x 200 19.1 / 17.0);
+// what still loses: 40/8 64 x 32, seven waves for four, 61.8 / 64.6.  More
+// keys: blocks for no more than the SMs and up to 1,024 (28/4: 1,024 tokens 30.5 / 27.8; 1,500 38.8 / 40.2; 12/2: 3 x 512 20.9 / 17.0), for half of
+// them and up to 4,096 (512 after 1,024: 36.8 / 34.3; 40/8: 512 after 3,000 70.4 / 75.4), for a quarter (12/2: 200 after 6,144 40.1 / 40.1).
+// The call's `num_seqs` portions bring the step's tokens from `first_token` on: the single tokens in front of it, which have a kernel
+// of their own, count in neither.
+static bool one_query_tile(int tokens, int first_token, int num_seqs, int bq, int group, int kv_heads, int num_splits, int max_ctx_len, int sms) {
+  const long long rows = tokens - first_token;
+  const long long own_tiles = ((rows + num_seqs - 1) / num_seqs + bq - 1) / bq;                                  // of a portion, were all alike
+  auto waves = [&](long long blocks) { return (blocks * num_seqs * kv_heads * num_splits + sms - 1) / sms; };
+  const long long pair_blocks = (((rows + bq - 1) / bq + 1) / 2 + num_seqs) * kv_heads * num_splits;
+  return max_ctx_len <= 320 ? group == 1 || waves(own_tiles) < 2 * waves((own_tiles + 1) / 2)
+                            : (pair_blocks <= sms && max_ctx_len <= 1024) || (2 * pair_blocks <= sms && max_ctx_len <= 4096) || 4 * pair_blocks <= sms;
+}
+
+// The choice for an SM count of the caller's, for tests.
+TGE_API int tge_attention_mma_one_query_tile(int tokens, int first_token, int num_seqs, int group, int kv_heads, int num_splits, int max_ctx_len,
+                                             int sms) {
+  return one_query_tile(tokens, first_token, num_seqs, 128 / group, group, kv_heads, num_splits, max_ctx_len, sms);
+}
+
 // What a call for the single tokens at a step's head leaves for its caller to do.
 struct LeadingTokens {
   unsigned long long ticket = 0;     // what the decode kernel is to leave
@@ -1614,22 +1639,7 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
         out_stride % 8 == 0 && (uintptr_t)out % 16 == 0) {
       // the tcgen05 kernels: 128 rows per query tile as well
       static const bool one_tile = getenv("TGE_ATTENTION_ONE_TILE") != nullptr && getenv("TGE_ATTENTION_ONE_TILE")[0] != '\0';
-      // Two query tiles to a block share K and V and one SM; where blocks are few or short, one tile to a block has the SMs'
-      // tensor cores to itself and less to set up.  The lines, measured at 28 heads over 4, 40 over 8, 12 over 2, 32 over 8, 16 over 16
-      // of 128 and 14 over 2 of 64 (two tiles / one, us).  Up to 320 keys, any number of blocks: unless the single tiles take twice
-      // the waves (28/4: 16 x 64 13.4 / 14.0, 20 x 64 24.5 / 20.8; 12/2: 64 x 32 16.9 / 20.3, 12 x 100 13.6 / 10.3, 8 x 300 17.4 / 19.7;
-      // 40/8: 6 x 128 14.8 / 16.9, 32 x 64 51.4 / 41.7), or tiles are whole ones of a head's queries (16/16: 8 x 200 19.1 / 17.0);
-      // what still loses: 40/8 64 x 32, seven waves for four, 61.8 / 64.6.  More
-      // keys: blocks for no more than the SMs and up to 1,024 (28/4: 1,024 tokens 30.5 / 27.8; 1,500 38.8 / 40.2; 12/2: 3 x 512 20.9 / 17.0), for half of
-      // them and up to 4,096 (512 after 1,024: 36.8 / 34.3; 40/8: 512 after 3,000 70.4 / 75.4), for a quarter (12/2: 200 after 6,144 40.1 / 40.1).
-      const int sms = tge_sm_count();
-      const long long portions = num_seqs > first_token ? num_seqs - first_token : 1;          // the single tokens at the head: one each
-      const long long own_tiles = ((tokens - first_token + portions - 1) / portions + p.bq - 1) / p.bq;      // of a portion, were all alike
-      auto waves = [&](long long blocks) { return (blocks * portions * kv_heads * num_splits + sms - 1) / sms; };
-      const long long pair_blocks = (long long)(((tokens - first_token + p.bq - 1) / p.bq + 1) / 2 + num_seqs) * kv_heads * num_splits;
-      const bool few = max_ctx_len <= 320 ? group == 1 || waves(own_tiles) < 2 * waves((own_tiles + 1) / 2)
-                                          : (pair_blocks <= sms && max_ctx_len <= 1024) || (2 * pair_blocks <= sms && max_ctx_len <= 4096) ||
-                                                4 * pair_blocks <= sms;
+      const bool few = one_query_tile(tokens, first_token, num_seqs, p.bq, group, kv_heads, num_splits, max_ctx_len, tge_sm_count());
       if (tc2::FITS && !one_tile && !few && tc2::smem_bytes(range >> p.page_shift) <= 227 * 1024) {
         // two query tiles per block, one block per SM
         const size_t smem2 = tc2::smem_bytes(range >> p.page_shift);
