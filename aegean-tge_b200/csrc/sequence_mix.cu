@@ -1133,19 +1133,19 @@ __global__ void conv_state_update_kernel(const T* raw, long long ld, float* conv
 constexpr int POOL_AHEAD = 16, POOL_THREADS = 256;
 
 // The mean key and mean value of every block of `pool` positions whose last token this step brings: one block of
-// threads per (32 tokens, kv head), which looks for the tokens at a block's last position among them.  The means are taken over the
+// threads per (`each` tokens, kv head), which looks for the tokens at a block's last position among them.  The means are taken over the
 // keys and values as their pages hold them, and entry b of a request lies where position b would in the pooled pages.
-// Bound by round trips: POOL_AHEAD positions' pages, then their numbers, are on their way together, added in order.  2,048 tokens, 4 kv heads
-// of 128, blocks of 64: 69 us one position after the other; 34 eight at a time, a block of threads per token (63 of 64 only left); this 23.
+// Bound by round trips: POOL_AHEAD positions' pages, then their numbers, are on their way together, added in order, about 11 us a mean of
+// 64; a block takes its means one after the other, so how many tokens are its own is the launch's choice (tge_pool_kv).
 template <typename T>
 __global__ void __launch_bounds__(POOL_THREADS) pool_kv_kernel(
     const T* k_pages, const T* v_pages, const int* __restrict__ block_table, int max_pages,
     int num_pages, T* kp_pages, T* vp_pages, const int* __restrict__ pool_table,
     int pool_max_pages, int pool_num_pages, int page_size, const int* __restrict__ positions,
-    const int* __restrict__ seq_of_token, int tokens, int kv_heads, int dim, int vdim, int pool, int* status) {
+    const int* __restrict__ seq_of_token, int tokens, int each, int kv_heads, int dim, int vdim, int pool, int* status) {
   pdl_trigger();
-  const int first = blockIdx.x * 32, head = blockIdx.y, lane = threadIdx.x & 31;
-  const int mine = first + lane < tokens ? positions[first + lane] : -1;
+  const int first = blockIdx.x * each, head = blockIdx.y, lane = threadIdx.x & 31;
+  const int mine = lane < each && first + lane < tokens ? positions[first + lane] : -1;
   unsigned ends = __ballot_sync(0xffffffffu, mine >= 0 && (mine + 1) % pool == 0);      // the same in every warp
   pdl_wait();
   for (; ends != 0; ends &= ends - 1) {
@@ -1745,19 +1745,24 @@ TGE_API int tge_conv_norm_rope_store(const void* raw, int is_bf16, long long ld,
 TGE_API int tge_pool_kv(const void* k_pages, const void* v_pages, int is_bf16, const int* block_table, int max_pages,
                         int num_pages, void* kp_pages, void* vp_pages, const int* pool_table, int pool_max_pages,
                         int pool_num_pages, int page_size, const int* positions, const int* seq_of_token, int tokens,
-                        int kv_heads, int dim, int vdim, int pool, int* status, cudaStream_t stream) {
+                        int requests, int kv_heads, int dim, int vdim, int pool, int* status, cudaStream_t stream) {
   TGE_REQUIRE(pool > 0 && kv_heads > 0 && dim > 0 && vdim > 0 && page_size > 0, "pool_kv: bad shape");
   if (tokens == 0) return 0;
-  dim3 grid((tokens + 31) / 32, kv_heads);
+  // Tokens to a block of threads.  A prompt ends a pooled block every `pool` tokens, so 32 neighbouring ones hold few ends; single tokens of
+  // many requests in lockstep may all end one, and then each wants a block of threads of its own.  (us a launch at 1 / 4 / 32 tokens
+  // to a block, 4 kv heads of 128, pooled blocks of 64: 64 requests that all end one 19 / 48 / 365, 256 44 / 74 / 369, none of 64
+  // 1.0 / 1.0 / 1.0, none of 256 2.0 / 1.0 / 1.0; prompts of 300 14.5 / 13.6 / 12.8, 2,048 25.7 / 20.7 / 19.0; 2,048 with pooled blocks of 4 33 / 25 / 41.)
+  const int each = requests <= 4 && pool >= 32 && tokens > 256 ? 32 : tokens <= 256 ? 1 : 4;
+  dim3 grid((tokens + each - 1) / each, kv_heads);
   if (is_bf16)
     tge_launch(pool_kv_kernel<__nv_bfloat16>, grid, dim3(POOL_THREADS), 0, stream,
         (const __nv_bfloat16*)k_pages, (const __nv_bfloat16*)v_pages, block_table, max_pages, num_pages,
         (__nv_bfloat16*)kp_pages, (__nv_bfloat16*)vp_pages, pool_table, pool_max_pages, pool_num_pages, page_size, positions,
-        seq_of_token, tokens, kv_heads, dim, vdim, pool, status);
+        seq_of_token, tokens, each, kv_heads, dim, vdim, pool, status);
   else
     tge_launch(pool_kv_kernel<float>, grid, dim3(POOL_THREADS), 0, stream, (const float*)k_pages, (const float*)v_pages, block_table, max_pages,
                                                      num_pages, (float*)kp_pages, (float*)vp_pages, pool_table,
-                                                     pool_max_pages, pool_num_pages, page_size, positions, seq_of_token, tokens,
+                                                     pool_max_pages, pool_num_pages, page_size, positions, seq_of_token, tokens, each,
                                                      kv_heads, dim, vdim, pool, status);
   return tge_launched("pool_kv", 1);
 }

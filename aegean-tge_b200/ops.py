@@ -175,7 +175,7 @@ def core() -> ctypes.CDLL:
                                                    _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_ll, _c_int,
                                                    _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr])
         _declare(lib, "tge_pool_kv", [_c_ptr, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int,
-                                      _c_int, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr,
+                                      _c_int, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr,
                                       _c_ptr])
         _declare(lib, "tge_qk_norm_kv_store", [_c_ptr, _c_int, _c_int, _c_ptr, _c_ptr, _c_float, _c_int, _c_ptr, _c_int,
                                                _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_int,
@@ -1263,7 +1263,7 @@ def pool_kv(k_pages: torch.Tensor, v_pages: torch.Tensor, block_table: torch.Ten
     _check(lib.tge_pool_kv(k_pages.data_ptr(), v_pages.data_ptr(), int(k_pages.dtype == torch.bfloat16),
                            block_table.data_ptr(), block_table.shape[1], num_pages, pooled_k.data_ptr(),
                            pooled_v.data_ptr(), pool_table.data_ptr(), pool_table.shape[1], pooled_k.shape[0], page_size,
-                           positions.data_ptr(), seq_of_token.data_ptr(), positions.numel(), kv_heads, dim, vdim, int(pool),
+                           positions.data_ptr(), seq_of_token.data_ptr(), positions.numel(), block_table.shape[0], kv_heads, dim, vdim, int(pool),
                            status_word().data_ptr(), _stream()), lib)
 
 

@@ -669,6 +669,37 @@ def test_gated_norm_four_groups_to_a_warp_has_the_bits_of_one(ops, tokens, group
     assert torch.equal(many, few)
 
 
+@pytest.mark.parametrize("q_lens,starts,pool", [([1] * 70, [63] * 70, 64), ([1] * 300, [7] * 300, 8), ([1] * 40 + [600], [31] * 40 + [5], 32), ([700], [3], 64), ([300, 9], [0, 120], 3)])
+def test_pooled_means_of_requests_in_lockstep_and_of_prompts(ops, q_lens, starts, pool):
+    """Many requests that end a pooled block in one step, beside a prompt, a prompt alone; blocks of threads for one, four and 32 tokens."""
+    kv_heads, dim, vdim, page_size = 2, 64, 32, 16
+    lengths = [a + n for a, n in zip(starts, q_lens)]
+    k_pages, table = _paged(lengths, kv_heads, dim, page_size, torch.bfloat16, 3)
+    v_pages, v_table = _paged(lengths, kv_heads, vdim, page_size, torch.bfloat16, 3)
+    pooled_k, pool_table = _paged([max(n // pool, 1) for n in lengths], kv_heads, dim, page_size, torch.bfloat16, 5)
+    pooled_v, _ = _paged([max(n // pool, 1) for n in lengths], kv_heads, vdim, page_size, torch.bfloat16, 5)
+    assert torch.equal(table, v_table)
+    gen = torch.Generator().manual_seed(9)
+    for pages in (k_pages, v_pages, pooled_k, pooled_v):
+        pages.copy_(torch.randn(pages.shape, generator=gen).to(torch.bfloat16))
+    positions, seq, _ = _steps(q_lens, starts)
+    before = [pooled_k.clone(), pooled_v.clone()]
+    ops.pool_kv(k_pages, v_pages, table, pooled_k, pooled_v, pool_table, positions, seq, pool)
+    ops.check_status()
+    wanted = [t.clone() for t in before]
+    for s, (start, n) in enumerate(zip(starts, q_lens)):
+        for end in range(start, start + n):
+            if (end + 1) % pool:
+                continue
+            entry, where = (end + 1) // pool - 1, torch.arange(end - pool + 1, end + 1, device=DEV)
+            for pages, out in ((k_pages, wanted[0]), (v_pages, wanted[1])):
+                rows = pages[table[s, where // page_size].long(), :, where % page_size].double()
+                out[int(pool_table[s, entry // page_size]), :, entry % page_size] = rows.mean(0).to(torch.bfloat16)
+    for got, want, old in zip((pooled_k, pooled_v), wanted, before):
+        assert rel_error(got, want) < 2.0 ** -8          # a float32 sum against a float64 one: a rounding step of bfloat16 at most
+        assert torch.equal(got[want == old], old[want == old])
+
+
 def _window_pool_case(ops, dtype, heads, kv_heads, dim, vdim, size, pool, lengths, tails, page_size, spike=None):
     """Requests of ``lengths`` whose last ``tails[s]`` tokens come in a second step (0: all at once).  Keys and
     values are stored and pooled by the kernels; the queries of both steps are checked.  ``spike`` = (request, key
