@@ -1521,7 +1521,8 @@ __global__ void __launch_bounds__(NRV_THREADS) norm_rope_store_vec_kernel(
 // instructions (about 250 a warp and token), not by its bytes (38 MB for 2,048 tokens of 28 heads over 4 of 128): a warp per (token, head) with
 // two-byte loads of every tap, one behind the other, took 86 us there; four tokens unrolled with their rows and taps in registers 62 (a
 // quarter of an SM's warps, 1,800 instructions each, waits for the instructions themselves), this 47.
-constexpr int CONV_TOKENS = 8, CONV_THREADS = 256, CONV_VEC_TOKENS = 16;
+constexpr int CONV_TOKENS = 8, CONV_THREADS = 256;
+constexpr long long CONV_VEC_UNITS = 96;      // (token, head)s to an SM from which on it is taken
 
 __device__ __forceinline__ void unpack_eight(const uint4& raw, float f[8]) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -1703,8 +1704,13 @@ TGE_API int tge_conv_norm_rope_store(const void* raw, int is_bf16, long long ld,
                dim, vdim, store, norm_last, lanes, status);
     return tge_launched("norm_rope_store_vec", 1);
   }
-  // eight channels at a time from a few tokens on: below, the warps of single heads are more and as fast
-  const bool eights = is_bf16 && taps >= 2 && taps <= 4 && tokens >= CONV_VEC_TOKENS && dim % 8 == 0 && vdim % 8 == 0 && rotary % 16 == 0 &&
+  // Eight channels at a time where there are many (token, head)s: below, a block of threads to four of them spreads a step over the chip,
+  // where this kernel's blocks take eight tokens in turn and wait for each request's state anew.  (Single channels / eights, us with the
+  // state's update, 28 heads over 4 of 128: single tokens of 16 requests 8.3 / 15.7, 64 12.6 / 18.4, 128 16.5 / 22.1, 260 26.6 / 29.8, 392 37.8 / 36.6, 524
+  // 49 / 44; a prompt of 64 9.4 / 13.0, 260 13.9 / 15.0, 392 18.2 / 14.7, 2,048 78 / 39.  40 over 8, 14 over 2 and 8 over 2 of 64, 4 over 1: the line
+  // lies at 64 to 128 (token, head)s to an SM as well.)
+  const bool eights = is_bf16 && taps >= 2 && taps <= 4 && (long long)tokens * units >= CONV_VEC_UNITS * tge_sm_count() && dim % 8 == 0 &&
+                      vdim % 8 == 0 && rotary % 16 == 0 &&
                       ld % 8 == 0 && ld_q % 8 == 0 &&
                       (((uintptr_t)raw | (uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)conv_w | (uintptr_t)conv_state) & 15) == 0;
   if (eights) {

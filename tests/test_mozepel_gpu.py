@@ -600,10 +600,11 @@ def test_convolution_norm_rotation_and_store(ops, dtype, heads, kv_heads, dim, v
 
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,taps,rotary", [(5, 1, 128, 128, 4, 64), (4, 2, 64, 32, 3, 64), (3, 1, 24, 40, 2, 16), (28, 4, 128, 128, 4, 0)])
 @pytest.mark.parametrize("norm_last", [0, 1])
-@pytest.mark.parametrize("q_lens", [[16], [1, 2, 3, 9, 2], [33, 1, 30]])
+@pytest.mark.parametrize("q_lens", [[16], [1, 2, 3, 9, 2], [33, 1, 30], [1, 2, 3, 3001, 33, 1, 2]])
 def test_convolution_by_eights_against_single_channels(ops, heads, kv_heads, dim, vdim, taps, rotary, norm_last, q_lens):
-    """The kernel for eight channels and four tokens at a time against the one for single channels (whose rows start on odd elements),
-    requests of fewer tokens than taps beside longer ones, each with a state: the sums of squares alone are added in another order."""
+    """The kernel for eight channels at a time, tokens one after the other, against the one for single channels (whose rows start on odd
+    elements), requests of fewer tokens than taps beside longer ones, each with a state: the sums of squares alone are added in another
+    order.  Few tokens take the single channels both ways; the last step has enough for the other one at every size here."""
     from aegean_tge_b200.parts.rope import rotary_tables
     gen = torch.Generator().manual_seed(dim + taps)
     channels, tokens = (heads + kv_heads) * dim + kv_heads * vdim, sum(q_lens)
@@ -612,7 +613,7 @@ def test_convolution_by_eights_against_single_channels(ops, heads, kv_heads, dim
     odd[:, 1:] = raw
     conv_w = torch.randn(channels, taps, generator=gen).to(DEV)
     q_norm, k_norm = (1.0 + 0.2 * torch.randn(dim, generator=gen).to(DEV) for _ in range(2))
-    cos, sin = (t.to(DEV) for t in rotary_tables(5000.0, max(rotary, 2), 256))
+    cos, sin = (t.to(DEV) for t in rotary_tables(5000.0, max(rotary, 2), 4096))
     starts = [7 * s for s in range(len(q_lens))]
     positions, seq, q_start = _steps(q_lens, starts)
     slots = _i32([(3 * s + 2) % 7 for s in range(len(q_lens))])
