@@ -937,8 +937,8 @@ __global__ void __launch_bounds__(256) gated_norm_vec_kernel(const float* o, con
   }
 }
 
-// Groups of up to 128 numbers, four to a warp, so that four rows' loads are on their way together (with a group to a warp each waited
-// for one: 2,048 tokens, 28 groups of 128, 22 us; this 19, bound by its instructions); a group's sum is the kernel's above.
+// Groups of 128 numbers, four to a warp, so that four rows' loads are on their way together (with a group to a warp each waits for one);
+// bound by its instructions; a group's sum is the kernel's above.
 constexpr int GATED_EACH = 4;
 __global__ void __launch_bounds__(256) gated_norm_small_kernel(const float* o, const __nv_bfloat16* gate, long long ld_gate,
                                                                const float* __restrict__ weight, __nv_bfloat16* __restrict__ out, long long ld_out,
@@ -1392,8 +1392,9 @@ TGE_API int tge_gated_norm(const float* o, const void* gate, int is_bf16, long l
   // four numbers at a time where the rows allow it: a warp to a group of up to 512 numbers, a block up to 4,096
   const bool quads = is_bf16 && size % 4 == 0 && ld_gate % 4 == 0 && ld_out % 4 == 0 && size <= 256 * 4 * GATED_QUADS && units <= 0x7fffffffll &&
                      (uintptr_t)o % 16 == 0 && (uintptr_t)gate % 8 == 0 && (uintptr_t)out % 8 == 0 && (uintptr_t)weight % 16 == 0;
-  // four groups to a warp where they fill the chip that way
-  if (quads && size <= 128 && units >= (long long)GATED_EACH * 32 * tge_sm_count())
+  // Four groups to a warp where there are many and each fills its warp's lanes.  (One / four, us: groups of 128, 19,000 of them 7.6 / 9.2,
+  // 38,000 13.7 / 14.2, 57,000 19.9 / 19.1, 150,000 53.6 / 44.6; groups of 100 or 64, 57,000 19.9 / 26.9, 150,000 54 / 64 and 50 / 63.)
+  if (quads && size == 32 * 4 && units >= 320ll * tge_sm_count())
     tge_launch(gated_norm_small_kernel, dim3((unsigned)((units + 8 * GATED_EACH - 1) / (8 * GATED_EACH))), dim3(256), 0, stream, o,
                (const __nv_bfloat16*)gate, ld_gate, weight, (__nv_bfloat16*)out, ld_out, tokens, groups, size, eps, act);
   else if (quads && size <= 32 * 4 * GATED_QUADS)

@@ -658,7 +658,7 @@ def test_decay_scan_prepares_by_eights_as_by_single_numbers(ops, heads, dim, rot
         assert rel_error(got, want.cpu().double()) < 1e-6
 
 
-@pytest.mark.parametrize("tokens,groups,size", [(1200, 16, 128), (700, 28, 100), (19000, 1, 4)])
+@pytest.mark.parametrize("tokens,groups,size", [(1200, 16, 128), (700, 28, 100), (19000, 1, 4), (3001, 16, 128), (1700, 28, 128), (47361, 1, 128)])
 @pytest.mark.parametrize("sigmoid,gate_first", [(False, False), (True, False), (False, True)])
 def test_gated_norm_four_groups_to_a_warp_has_the_bits_of_one(ops, tokens, groups, size, sigmoid, gate_first):
     gen = torch.Generator().manual_seed(size)
