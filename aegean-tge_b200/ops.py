@@ -1012,7 +1012,7 @@ def attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor, blo
             # the single tokens at the head of a mixed step are a decode batch of their own: a few of them deep in
             # long contexts want their keys cut although the portions beside them do not
             if prefix and lead_keys > 0 and span >= max_ctx_len:
-                prefix_split = choose_leading_split(lead_keys, lead_longest, kv_heads)
+                prefix_split = choose_leading_split(prefix, lead_keys, lead_longest, kv_heads, max_ctx_len)
             elif prefix:
                 prefix_split = choose_attention_split(prefix, prefix, 1, span, heads, kv_heads, bound=span)
             else:
@@ -1320,17 +1320,20 @@ def choose_attention_split(tokens: int, num_seqs: int, max_q_len: int, max_ctx_l
     return keys_per_split(want_splits) if want_splits > 1 else 0
 
 
-def choose_leading_split(keys: int, longest: int, kv_heads: int) -> int:
-    """Keys per split for the single tokens at a mixed step's head, whose contexts are known: ``keys`` together, ``longest`` at most.
+def choose_leading_split(count: int, keys: int, longest: int, kv_heads: int, bound: int) -> int:
+    """Keys per split for the ``count`` single tokens at a mixed step's head, whose contexts are known: ``keys`` together, ``longest`` at most;
+    ``bound``: the longest context of the step.
 
-    The prompt's kernel runs beside theirs and fills the SMs that they leave, so they are cut only where the longest would outlast
-    all of an SM's share of the work by more than the merging kernel costs (a block takes about 18 ns a key, so 512 keys 9 us).  Measured (us a
-    layer, uncut / cut at an SM's share): 28 heads over 4, 40 requests of up to 4,000 beside 300 tokens 80 / 56, 8 of up to 4,096
-    beside 512 43 / 30; left alone: 31 of up to 4,096 beside 1,187 at 40 over 8 100 / 106, 31 of 2,048 beside 512 44 / 48,
-    20 of up to 800 beside 700 31 / 40."""
-    share = -(-keys * kv_heads // core().tge_device_sm_count())
-    cut = max(512, -(-share // 64) * 64)
-    return cut if longest - cut >= 512 else 0
+    The prompt's kernel runs beside theirs and fills the SMs that they leave, so that the longest request is what counts.  A block takes
+    18 ns a key, 11 where it has an SM to itself (two groups of warps); cut at an SM's share of all keys, the blocks take about 20 ns a
+    key of the cut, and the states 10 us to write and merge.  Cut where that is 2 us less.  Measured at 28 heads over 4 and 40 over 8 of 128, 8 to 64 requests
+    of equal or drawn lengths beside 64 to 1,187 tokens (160 points, both ways each): together 8,895 us uncut, 8,518 by this rule, 8,509 with
+    the better way of each.  (28/4, us a layer, uncut / cut: 8 of up to 4,096 beside 512 tokens 43 / 28; 16 beside 300 43 / 29; 40 beside 64 70 / 53;
+    31 beside 1,187 58 / 72; 64 beside 64 76 / 88; 8 of 2,048 beside 512 26 / 28.  40/8: 16 of up to 4,096 beside 300 43 / 46, 31 beside 1,187 96 / 103.)"""
+    sms = core().tge_device_sm_count()
+    cut = max(512, -(-(-(-keys * kv_heads // sms)) // 64) * 64)
+    alone = 11 if count * kv_heads <= sms and bound >= 1536 else 18
+    return cut if alone * longest - 20 * cut >= 12000 else 0
 
 
 def sample(logits: torch.Tensor, temperature: torch.Tensor, uniform: torch.Tensor,

@@ -866,7 +866,7 @@ def test_side_by_side_attention_sees_what_the_kernels_in_front_have_just_written
     q_lens, begins, n = [1] * len(lead) + portions, lead + starts, len(lead)
     lengths = [a + m for a, m in zip(begins, q_lens)]
     known = dict(lead_keys=sum(lengths[:n]), lead_longest=max(lengths[:n]), rest_ctx_len=max(lengths[n:]))
-    lead_cut = ops.choose_leading_split(known["lead_keys"], known["lead_longest"], kv_heads)
+    lead_cut = ops.choose_leading_split(n, known["lead_keys"], known["lead_longest"], kv_heads, max(lengths))
     rest_cut = ops.choose_attention_split(sum(portions), len(portions), max(portions), known["rest_ctx_len"], heads, kv_heads, bound=known["rest_ctx_len"])
     assert (lead_cut > 0) == lead_is_cut and (rest_cut > 0) == rest_is_cut
     k_pages, v_pages, table, _k, _v = paged_cache(lengths, kv_heads, head_dim, page_size, torch.bfloat16, DEV, seed=5)
