@@ -1759,7 +1759,7 @@ TGE_API int tge_attention_mma(const void* q, int q_stride, const void* k_pages, 
                               window, split_tokens, scratch, status, 0, sink, leave_states, v_pitch, dist_bias, dist_span, keep_first, gate, gate_stride, gate_elements, shared_keys, stream);
   // Side by side where nothing but keys, queries and constants is read (gates may be the kernel in front's work) and where the
   // scratch memory holds the states of one of the two calls only.  (31 single tokens of up to 4,096 beside a prompt of 1,187, 40 heads over 8, us
-  // a layer in a step: 88 and 50 one after the other, 95 and 25 so.)
+  // a layer in a step: 88 and 50 one after the other, 95 and 25 so; eight layers of such a step 6,084 and 6,029.)
   const int rest_ctx = rest_ctx_len > 0 && rest_ctx_len < max_ctx_len ? rest_ctx_len : max_ctx_len;
   const bool rest_cut = split_tokens > 0 && rest_ctx > split_tokens, lead_cut = prefix_split_tokens > 0 && max_ctx_len > prefix_split_tokens;
   LeadingTokens lead;

@@ -142,6 +142,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc2_kernel(
   // Everything above read what the step was given (lengths, positions, the block table) and set up this block's own
   // memory, while the kernel before this one was still running; the queries and the newest keys are its work (or
   // that of the kernel before it, whose ticket says so: p.beside).
+  // (The chain of attention_tc.cuh, a prompt of 2,048 tokens: 157.9 / 157.4 us at 28 heads over 4, 79.0 / 78.5 at 8 over 2.)
   wait_or_take_ticket(p);
   auto s_tmem = [&](int tile, int buffer) { return tmem_base + (uint32_t)((tile * 2 + buffer) * BKV); };
   auto o_tmem = [&](int tile) { return tmem_base + (uint32_t)(2 * QTILES * BKV + tile * HD); };

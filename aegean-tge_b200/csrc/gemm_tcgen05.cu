@@ -51,7 +51,8 @@ constexpr int MAX_STAGES = 8;
 constexpr int EPI_WARPS = 8;              // two per 32-lane quarter of tensor memory, each taking half the columns
 constexpr int NUM_THREADS = (2 + EPI_WARPS) * 32;
 // Pairs of SMs run wide tiles, whose last epilogue nothing hides: four warps to a quarter.  (An SM alone runs a few tokens mostly, one or two
-// groups of sixteen columns to a tile, which eight warps share as well.)
+// groups of sixteen columns to a tile, which eight warps share as well.)  A layer's four products of the 7B shape one after the other, us with
+// eight warps / sixteen: 2,048 tokens 662 / 626, 193 tokens 115 / 115; a whole prompt of 2,048 tokens shows 1 % at most, within its spread.
 constexpr int PAIR_EPI_WARPS = 16;
 constexpr int PAIR_THREADS = (2 + PAIR_EPI_WARPS) * 32;
 constexpr int SMEM_LIMIT = 227 * 1024;
