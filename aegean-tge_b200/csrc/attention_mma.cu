@@ -1663,7 +1663,14 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
         }
         return 1;
       }
-      const size_t smem = tc::smem_bytes(range >> p.page_shift);
+      const int tiles = (tokens - first_token + p.bq - 1) / p.bq + num_seqs;
+      size_t smem = tc::smem_bytes(range >> p.page_shift);
+      // No more blocks than SMs: one to an SM, by more than half of its shared memory.  They start while the kernels in front drain, and were put
+      // two to an SM where those had left first, with other SMs idle.  (Product, store, attention and product in a chain, us two / one to an SM:
+      // 8 heads over 2 of 128, 512 tokens after 3,000 70.6 / 64.9, 192 after 1,000 58.1 / 54.2; 14 over 2 of 64, 768 after 2,000 73.5 / 70.2; 28 over 4,
+      // 256 after 1,000 76.6 / 73.6; 150 points at four sizes of layer: 0.92 to 1.01 of the time.)
+      constexpr size_t ALONE = 116 * 1024;
+      if ((long long)tiles * kv_heads * num_splits <= tge_sm_count() && smem < ALONE) smem = ALONE;
       static size_t configured_tc = 0;
       if (smem > configured_tc) {
         cudaError_t err = cudaFuncSetAttribute(tc::attention_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1673,7 +1680,6 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
         }
         configured_tc = smem;
       }
-      const int tiles = (tokens - first_token + p.bq - 1) / p.bq + num_seqs;
       dim3 grid(tiles * kv_heads, 1, num_splits);
       tge_launch(tc::attention_prefill_tc_kernel, grid, tc::THREADS, smem, stream, *map_k, *map_v, p);
       int rc = tge_check_launch("attention_prefill_tc");

@@ -201,8 +201,7 @@ __global__ void __launch_bounds__(THREADS, 2) attention_prefill_tc_kernel(
   // memory, while the kernel before this one was still running; the queries and the newest keys are its work (or
   // that of the kernel before it, whose ticket says so: p.beside).
   // Product, store, attention and product in a chain, us with the wait ahead of the set-up / so: 28 heads over 4, three prompts of 64 45.5 / 44.9,
-  // one of 193 46.3 / 45.7; 8 over 2 35.9 / 34.5 and 37.3 / 36.0; but 512 tokens after 3,000 at 8 over 2 65 / 70 and at 14 over 2 of 64
-  // 71 / 74, for a reason not found (other cut portions, 32 after 8,000 to 400 after 6,000: no difference).
+  // one of 193 46.3 / 45.7; 8 over 2 35.9 / 34.5 and 37.3 / 36.0.
   wait_or_take_ticket(p);
   const uint32_t s_tmem = tmem_base, o_tmem = tmem_base + 2 * BKV;
 
