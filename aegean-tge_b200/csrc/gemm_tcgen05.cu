@@ -32,8 +32,8 @@
 enum GemmEpilogue : int { GEMM_STORE = 0, GEMM_STORE_F32 = 1, GEMM_ADD_F32 = 2, GEMM_SWIGLU = 3, GEMM_GELU = 4,
                           GEMM_GELU_TANH = 5, GEMM_GLU_CLAMPED = 6 };
 // Added to the epilogue by a caller whose weights and bias no kernel still in flight can have written (a model's, once it is loaded): the
-// products then ask for weights ahead of their wait for the kernel in front.  Without it they let their dependents start only
-// behind that wait, so that the kernel that adds cuts may still ask for the bias ahead of its own.
+// products then ask for weights ahead of their wait for the kernel in front, and the kernel that adds cuts for the bias ahead of its
+// own.  Without it both wait first (see launch()).
 constexpr int GEMM_WEIGHTS_SETTLED = 256;
 // GEMM_GLU_CLAMPED: the gated epilogue with both halves clamped at L = `alpha`: g <- min(g, L), u <- clamp(u, -L, L),
 // out = g sigmoid(1.702 g) (u + 1).
@@ -330,11 +330,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
   const uint32_t tmem_base = *tmem_slot_ptr;
   // Only now may the next kernel be scheduled: this block already holds its tensor memory, so a block of
   // the next kernel that lands on the same SM can at worst wait for it, never starve it.
-  if (!p.settled) pdl_wait();
   pdl_trigger();
   // Set-up above overlapped the previous kernel; from here on its results are read.  The loading warp
   // waits later where weights are nobody's result: it first asks for a ring-full of weight tiles.
-  if (p.settled && warp != 0) pdl_wait();
+  if (warp != 0 || !p.settled) pdl_wait();
 
   const int total_work = p.tiles_w * p.tiles_t * p.splits;
   float* row_factor = nullptr;
@@ -564,11 +563,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
   cluster_sync_all();             // both blocks' barriers exist before either signals the other
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
-  if (!p.settled) pdl_wait();
   pdl_trigger();
   // Settled weights (the caller says so): their loader asks for a ring-full of them while the kernel in front still runs.
   // (193 tokens in three prompts, 12 layers of the 7B shape, with the shorter epilogue: 2,087 -> 1,955 us.)
-  if (p.settled && warp != 0) pdl_wait();
+  if (warp != 0 || !p.settled) pdl_wait();
 
   const int total_work = p.tiles_w * p.tiles_t * p.splits;
   const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
@@ -798,6 +796,22 @@ int make_map(CUtensorMap* map, const void* base, long long rows, long long K, lo
 }
 
 int sm_count() { return tge_sm_count(); }
+
+// A kernel that adds a product's cuts.  It asks for the bias and other numbers of the model ahead of its wait, so only where those are settled
+// may it start while the product still runs: a wait makes visible what came before to the kernel that waits, not to those behind it.
+template <typename... KernelArgs, typename... Args>
+void launch(void (*kernel)(KernelArgs...), bool settled, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  if (settled) {
+    tge_launch(kernel, grid, block, smem, stream, args...);
+    return;
+  }
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = block;
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchKernelEx(&config, kernel, KernelArgs(args)...);
+}
 
 struct Plan {
   int bn, stages, splits;
@@ -1500,14 +1514,14 @@ TGE_API int tge_gemm_tcgen05(const void* x, long long ldx, const void* w, long l
     const long long quad = is_gated ? 4 : is_f32 ? 16 : 8;
     if (N % 4 == 0 && M <= 65535 && (uintptr_t)scratch % 16 == 0 && (uintptr_t)bias % 16 == 0 && (uintptr_t)out % quad == 0 &&
         (ldo * (is_f32 ? 4 : 2)) % quad == 0) {
-      tge_launch(splitk_epilogue_quad_kernel, dim3((N / 4 + QUAD_THREADS - 1) / QUAD_THREADS, M), dim3(QUAD_THREADS), 0, stream, (const float*)scratch,
+      launch(splitk_epilogue_quad_kernel, settled, dim3((N / 4 + QUAD_THREADS - 1) / QUAD_THREADS, M), dim3(QUAD_THREADS), 0, stream, (const float*)scratch,
                  bias, out, ldo, M, N, splits, epilogue, x_ss, x_ss_slices, x_ss_width, x_ss_eps, alpha, act_from);
       return tge_launched("splitk_epilogue", 2);
     }
     const long long count = is_gated ? (long long)M * N / 2 : (long long)M * N;
     long long blocks = (count + 255) / 256;
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
-    tge_launch(splitk_epilogue_kernel, (int)blocks, 256, 0, stream, (const float*)scratch, bias, out, ldo, M, N, splits,
+    launch(splitk_epilogue_kernel, settled, (int)blocks, 256, 0, stream, (const float*)scratch, bias, out, ldo, M, N, splits,
                epilogue, x_ss, x_ss_slices, x_ss_width, x_ss_eps, alpha, act_from);
     return tge_launched("splitk_epilogue", 2);
   }
@@ -1532,7 +1546,7 @@ TGE_API int tge_gemm_tcgen05_add_defer(const void* x, long long ldx, const void*
   int rc = launch_product(x, ldx, w, ldw, nullptr, stream_out, ldo, M, N, K, GEMM_ADD_F32, scratch, scratch_floats, 0, 0,
                           true, status, stream, &splits, settled != 0);
   if (rc != 1) return rc;
-  tge_launch(splitk_add_scale_kernel, dim3((N + SCALE_SLICE - 1) / SCALE_SLICE, M), SCALE_SLICE, 0, stream,
+  launch(splitk_add_scale_kernel, settled != 0, dim3((N + SCALE_SLICE - 1) / SCALE_SLICE, M), SCALE_SLICE, 0, stream,
              (const float*)scratch, bias, stream_out, ldo, norm_weight, (__nv_bfloat16*)scaled_out, ld_scaled, ss_out, M, N,
              splits, alpha);
   return tge_launched("splitk_add_scale", 2);
@@ -1554,7 +1568,7 @@ TGE_API int tge_gemm_tcgen05_add_norm(const void* x, long long ldx, const void* 
   int rc = launch_product(x, ldx, w, ldw, nullptr, stream_out, ldo, M, N, K, GEMM_ADD_F32, scratch, scratch_floats, 0, 0,
                           true, status, stream, &splits, settled != 0);
   if (rc != 1) return rc;
-  tge_launch(splitk_add_norm_kernel, dim3(M), NORM_THREADS, 0, stream,
+  launch(splitk_add_norm_kernel, settled != 0, dim3(M), NORM_THREADS, 0, stream,
              (const float*)scratch, bias, stream_out, ldo, norm_weight, eps, (__nv_bfloat16*)norm_out, ld_norm, M, N,
              splits, alpha);
   return tge_launched("splitk_add_norm", 2);
@@ -1595,7 +1609,7 @@ TGE_API int tge_gemm_tcgen05_qkv_rope(const void* x, long long ldx, const void* 
   int rc = launch_product(x, ldx, w, ldw, nullptr, qkv, ld_qkv, M, N, K, GEMM_STORE, scratch, scratch_floats, 0, 0, true,
                           status, stream, &splits, settled != 0);
   if (rc != 1) return rc;
-  tge_launch(splitk_qkv_rope_store_kernel, dim3(M, heads + 2 * kv_heads), head_dim >= 128 ? 128 : 64,
+  launch(splitk_qkv_rope_store_kernel, settled != 0, dim3(M, heads + 2 * kv_heads), head_dim >= 128 ? 128 : 64,
              (size_t)head_dim * sizeof(float), stream, (const float*)scratch, bias, (__nv_bfloat16*)qkv, ld_qkv, M, N,
              splits, cos_table, sin_table, table_rows, rotary, positions, seq_of_token, block_table, max_pages,
              (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, num_pages, page_size, heads, kv_heads, head_dim, status,
@@ -1634,7 +1648,7 @@ TGE_API int tge_gemm_tcgen05_qkv_norm_act(const void* x, long long ldx, const vo
   if (rc != 1) return rc;
   const size_t smem = 0;
   const int act_blocks = (int)((N - n_qkv + QKV_ACT_SLICE - 1) / QKV_ACT_SLICE);
-  tge_launch(splitk_qkv_norm_act_store_kernel, dim3(M, 1 + act_blocks), QKV_ACT_THREADS, smem, stream,
+  launch(splitk_qkv_norm_act_store_kernel, settled != 0, dim3(M, 1 + act_blocks), QKV_ACT_THREADS, smem, stream,
              (const float*)scratch, M, N, splits, (__nv_bfloat16*)qkv, ld_qkv, (__nv_bfloat16*)act_out, ld_act, activation,
              q_weight, k_weight, eps, (const __nv_bfloat16*)v_other, ld_other, blend, positions, seq_of_token, block_table,
              max_pages, (__nv_bfloat16*)k_pages, (__nv_bfloat16*)v_pages, num_pages, page_size, heads, kv_heads, head_dim,

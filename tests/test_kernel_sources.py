@@ -88,3 +88,12 @@ def test_every_kernel_that_may_start_early_waits():
     names = [name for name in launched if name in defined and name != "attention_simt_kernel"]      # that one is launched with <<< >>>
     assert len(names) > 70
     assert [name for name in names if not waits(name)] == []
+
+
+def test_kernels_that_add_cuts_start_early_beside_settled_weights_only():
+    """They ask for the bias ahead of their wait, which the kernel in front of the product may just have written: the product's own
+    wait makes that visible to the product alone.  So without ``settled`` they are launched to start behind the whole product."""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "gemm_tcgen05.cu").read_text())
+    launches = re.findall(r"(\w+)\(\s*splitk_\w+_kernel\s*,\s*([^,]+),", text)
+    assert len(launches) == 6 and all(how == "launch" and first.startswith("settled") for how, first in launches), launches
+    assert re.search(r"void launch\([^)]*\)\([^)]*\), bool settled.*?if \(settled\) \{\s*tge_launch\(kernel", text, re.S)
