@@ -1669,8 +1669,12 @@ static int attention_dispatch(const void* q, int q_stride, const void* k_pages, 
       // two to an SM where those had left first, with other SMs idle.  (Product, store, attention and product in a chain, us two / one to an SM:
       // 8 heads over 2 of 128, 512 tokens after 3,000 70.6 / 64.9, 192 after 1,000 58.1 / 54.2; 14 over 2 of 64, 768 after 2,000 73.5 / 70.2; 28 over 4,
       // 256 after 1,000 76.6 / 73.6; 150 points at four sizes of layer: 0.92 to 1.01 of the time.)
+      // Beside the single tokens' kernel only where the blocks of both are no more: that kernel's stand on the SMs to its end, and an SM that holds
+      // one has no room for this much.  (28 heads over 4 of 128, 512 tokens beside 31 requests of up to 4,000, us of the chain with the half / without:
+      // 77.4 / 73.8; 8 over 2 beside 16 of up to 1,000 42.6 / 43.9.)
       constexpr size_t ALONE = 116 * 1024;
-      if ((long long)tiles * kv_heads * num_splits <= tge_sm_count() && smem < ALONE) smem = ALONE;
+      const long long others = p.beside ? (long long)first_token * kv_heads : 0;
+      if (others + (long long)tiles * kv_heads * num_splits <= tge_sm_count() && smem < ALONE) smem = ALONE;
       static size_t configured_tc = 0;
       if (smem > configured_tc) {
         cudaError_t err = cudaFuncSetAttribute(tc::attention_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
